@@ -23,7 +23,11 @@ static size_t batched_shmem(int hbins, int threads) {
 
 template <int RULE, int G, int V>
 static BatchedFn pick_g(int canon, int shape, int extra) {
-    if (!canon) return extra ? batched_kernel<RULE, G, false, false, true, V> : batched_kernel<RULE, G, false, false, false, V>;
+    if constexpr ((V & 28) == 28) {   // deals with the path memo are played merged (war_merge.cu); the sample is not
+        if (!canon) return extra ? batched_kernel<RULE, G, false, false, true, V> : nullptr;
+    } else {
+        if (!canon) return extra ? batched_kernel<RULE, G, false, false, true, V> : batched_kernel<RULE, G, false, false, false, V>;
+    }
     if constexpr ((V & 4) != 0 && (V & 16) == 0) return nullptr;   // canonical scans: the path memo only
     if (shape) return extra ? batched_kernel<RULE, G, true, true, true, V> : batched_kernel<RULE, G, true, true, false, V>;
     return extra ? batched_kernel<RULE, G, true, false, true, V> : batched_kernel<RULE, G, true, false, false, V>;

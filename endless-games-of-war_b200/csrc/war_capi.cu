@@ -84,11 +84,22 @@ int ensure_ready() {
     if ((e = cudaStreamCreateWithFlags(&c.own_stream, cudaStreamNonBlocking)) != cudaSuccess) return cuda_fail(e, "stream");
     if ((e = cudaMalloc(&c.d_acc, sizeof(DevAcc))) != cudaSuccess) return cuda_fail(e, "cudaMalloc acc");
     if ((e = cudaMalloc(&c.d_units, sizeof(Unit) * Ctx::UNIT_CAP)) != cudaSuccess) return cuda_fail(e, "cudaMalloc units");
+    if ((e = cudaMalloc(&c.d_blocks, sizeof(MBlock) * MERGE_BLOCK_CAP)) != cudaSuccess) return cuda_fail(e, "cudaMalloc blocks");
+    if ((e = upload_merge_table(&c.d_table)) != cudaSuccess) return cuda_fail(e, "pair lists");
     if ((e = cudaMallocHost(&c.h_acc, sizeof(DevAcc))) != cudaSuccess) return cuda_fail(e, "cudaMallocHost");
     if ((e = cudaEventCreate(&c.ev0)) != cudaSuccess) return cuda_fail(e, "event");
     if ((e = cudaEventCreate(&c.ev1)) != cudaSuccess) return cuda_fail(e, "event");
     c.ready = true;
     return WAR_OK;
+}
+
+cudaError_t upload_merge_table(u32** table) {
+    std::vector<u32> rows(2 * MERGE_ROWS);
+    merge_table(0, rows.data());
+    merge_table(1, rows.data() + MERGE_ROWS);
+    cudaError_t e = cudaMalloc(table, sizeof(u32) * rows.size());
+    if (e == cudaSuccess) e = cudaMemcpy(*table, rows.data(), sizeof(u32) * rows.size(), cudaMemcpyHostToDevice);
+    return e;
 }
 
 cudaStream_t cur_stream() {
@@ -203,9 +214,14 @@ int resolve_tune(const war_job* job, const war_tune* in, Tune& t) {
     if (t.block_m > M) t.block_m = M > 0 ? M : 1;
     int st = ensure_ready();
     if (st) return st;
-    int maxb = batched_max_blocks_per_sm(canon, job->rule, (job->flags & WAR_F_SHAPE) != 0,
-                                         (job->flags & WAR_F_DISTINCT) != 0, (job->flags & WAR_F_SAMPLE) != 0,
-                                         t.threads, t.games, job->hbins, t.variant);
+    // Deals with the path memo are played merged (war_merge.cuh), one game per lane; the sample needs every
+    // deal by itself.  (games = 2 and 4 still ask for blocks of at most 512 and 256 threads.)
+    t.merged = !canon && (t.variant & 28) == 28 && !(job->flags & WAR_F_SAMPLE);
+    int maxb = !t.merged ? batched_max_blocks_per_sm(canon, job->rule, (job->flags & WAR_F_SHAPE) != 0,
+                                                     (job->flags & WAR_F_DISTINCT) != 0,
+                                                     (job->flags & WAR_F_SAMPLE) != 0, t.threads, t.games, job->hbins,
+                                                     t.variant)
+             : t.games * t.threads > 1024 ? 0 : merged_max_blocks_per_sm(job->rule, t.threads, job->hbins);
     if (maxb < 1) return fail(WAR_EINVAL, "launch shape threads=%d games=%d does not fit an SM", t.threads, t.games);
     t.blocks_per_sm = (in && in->blocks_per_sm) ? std::min(in->blocks_per_sm, maxb) : maxb;
     return WAR_OK;
@@ -468,11 +484,18 @@ int war_enumerate_plain(const war_job* job, war_result* out) {
 // states, same packing) or 3 (path entries, (key * C) << bits | value) and shape = 1 when cycle values
 // carry the loop-shape code.  Two layouts never share a table: an entry of one form read as another could
 // name a different state.
-static int prepare_memo(Ctx& c, const war_job* job, int bits, int kind, u64** table) {
+//
+// A job that can only fill part of the table (`want` words or fewer are useful, 0 = no such limit) uses and
+// clears the first 2^*used words of it: clearing 16 GiB takes 2.6 ms, clearing what a slice of 1e8 deals can
+// use takes less than a tenth.  A job that keeps the table uses as much of it as the job before did.
+static int prepare_memo(Ctx& c, const war_job* job, int bits, int kind, u64** table, u64 want = 0, int* used = nullptr) {
     cudaError_t e;
-    const size_t bytes = sizeof(u64) << bits;
     const bool keep = (job->flags & WAR_F_MEMO_KEEP) && c.memo_bits == bits && c.memo_n == job->n &&
                       c.memo_rule == job->rule && c.memo_kind == kind;
+    int ub = bits;
+    while (want && ub > 12 && (1ull << (ub - 1)) >= want) ub--;
+    if (keep) ub = c.memo_used;
+    const size_t bytes = sizeof(u64) << bits;
     if (c.memo_bits != bits) {
         if (c.d_memo) cudaFree(c.d_memo);
         c.d_memo = nullptr;
@@ -483,14 +506,52 @@ static int prepare_memo(Ctx& c, const war_job* job, int bits, int kind, u64** ta
         }
         c.memo_bits = bits;
     }
-    if (!keep && (e = cudaMemsetAsync(c.d_memo, 0, bytes, cur_stream())) != cudaSuccess) {
+    if (!keep && (e = cudaMemsetAsync(c.d_memo, 0, sizeof(u64) << ub, cur_stream())) != cudaSuccess) {
         c.memo_n = -1;
         return cuda_fail(e, "clear cycle memo");
     }
     c.memo_n = job->n;
     c.memo_rule = job->rule;
     c.memo_kind = kind;
+    c.memo_used = ub;
+    if (used) *used = ub;
     *table = c.d_memo;
+    return WAR_OK;
+}
+
+// A deals job with the path memo: each state after the deals' first turns played once (war_merge.cuh).
+static int enumerate_merged(const war_job* job, const Tune& t, war_result* out) {
+    Ctx& c = ctx();
+    MergePlan p;
+    const int blocks = t.blocks_per_sm * c.sm_count;
+    merge_plan(job, (u64)blocks * (u64)(t.threads / 32), p);
+    if (p.units == 0) return WAR_OK;   // (--half: no deal of the range gives card n-1 to player 1)
+    cudaError_t e;
+    if (p.blocks.size() > MERGE_BLOCK_CAP) return fail(WAR_EINVAL, "plan has %zu blocks", p.blocks.size());
+    if ((e = cudaMemcpyAsync(c.d_blocks, p.blocks.data(), sizeof(MBlock) * p.blocks.size(), cudaMemcpyHostToDevice,
+                             cur_stream())) != cudaSuccess)
+        return cuda_fail(e, "copy blocks");
+    MergeArgs a;
+    memset(&a, 0, sizeof a);
+    a.blocks = c.d_blocks;
+    a.nblocks = (u32)p.blocks.size() - 1u;
+    a.table = c.d_table + (job->rule ? MERGE_ROWS : 0);
+    a.lc = p.lc;
+    a.n = job->n; a.hbins = job->hbins; a.W = t.window; a.defer = t.defer;
+    a.tk.k16 = 16u; a.tk.km16 = (u32)-16; a.tk.k2p28 = 1u << 28; a.tk.k4 = 4u; a.tk.one = 1u;
+    a.tk.c0 = 2 * job->n - 4; a.tk.end2 = (u32)(4 * job->n * job->n);
+    int st, used = 0;   // (a game stores at most two states besides the cycles found)
+    if ((st = prepare_memo(c, job, t.memo_bits, 4 * 3, &a.memo, 2 * p.games, &used))) return st;
+    a.memo_bits = (u32)used;
+    for (u64 u = 0; u < p.units; u += MERGE_LAUNCH_UNITS) {
+        a.unit_lo = u;
+        a.unit_hi = std::min(p.units, u + MERGE_LAUNCH_UNITS);
+        st = run_launch([&](cudaStream_t x) { return launch_merged(a, job->rule, t.threads, blocks, c.d_acc, x); },
+                        &out->kernel_ms);
+        if (st) return st;
+        merge_acc(*c.h_acc, out, job->hbins, 0);
+    }
+    out->units += p.units;
     return WAR_OK;
 }
 
@@ -593,6 +654,7 @@ int war_enumerate(const war_job* job, const war_tune* tune, war_result* out) {
     if ((st = resolve_tune(job, tune, t))) return st;
     if ((st = ensure_ready())) return st;
     std::lock_guard<std::mutex> lk(ctx().mu);
+    if (t.merged) return enumerate_merged(job, t, out);
     Ctx& c = ctx();
     Plan p;
     make_plan(job, t.block_m, p);

@@ -15,11 +15,17 @@ typedef unsigned int u32;
 
 #define WAR_FULL_MASK 0xffffffffu
 
-// Variable 64-bit left shift with PTX semantics: shift amounts above 63 give 0 (the amount is
-// clamped, PTX ISA shl).  Used where a retired lane may shift by an out-of-range amount.
+// Variable 64-bit shifts with PTX semantics: shift amounts above 63 give 0 (the amount is
+// clamped, PTX ISA shl, shr).  Used where a retired lane may shift by an out-of-range amount.
 __device__ __forceinline__ u64 shl64(u64 x, u32 s) {
     u64 r;
     asm("shl.b64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s));
+    return r;
+}
+
+__device__ __forceinline__ u64 shr64(u64 x, u32 s) {
+    u64 r;
+    asm("shr.b64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s));
     return r;
 }
 

@@ -20,12 +20,6 @@
 
 namespace war {
 
-__device__ __forceinline__ u64 shr64(u64 x, u32 s) {   // PTX shr: amounts above 63 give 0
-    u64 r;
-    asm("shr.b64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s));
-    return r;
-}
-
 __device__ __forceinline__ u32 h_heap_full(u32 j) {
     u32 f = 0;
     for (u32 i = 1; i < j; i++) f |= i << (4u * i);

@@ -4,6 +4,7 @@
 #include <mutex>
 #include <vector>
 #include "war_kernels.cuh"
+#include "war_merge.cuh"
 
 namespace war {
 
@@ -18,8 +19,11 @@ struct Ctx {
     Unit* d_units = nullptr;        // extra work units of the running job
     ulonglong2* d_sample = nullptr; // Floyd sample buffer
     size_t sample_cap = 0;
+    MBlock* d_blocks = nullptr;     // blocks of the running merged job
+    u32* d_table = nullptr;         // pair lists of both rules (war_merge.cuh)
     u64* d_memo = nullptr;          // cycle memo table of the refill kernel (deals)
-    int memo_bits = 0;
+    int memo_bits = 0;              // log2 of its words,
+    int memo_used = 0;              // and of those that the last job used
     int memo_n = -1, memo_rule = -1;  // job class whose cycles the memo holds
     int memo_kind = 0;                // its entry layout (prepare_memo): engine, memo form, shape values
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -34,11 +38,13 @@ struct Plan {
 
 struct Tune {
     int threads, blocks_per_sm, games, block_m, window, defer, variant, memo_bits, chunk;
+    bool merged;   // deals played merged (war_merge.cuh)
 };
 
 Ctx& ctx();
 int ensure_ready();
 cudaStream_t cur_stream();
+cudaError_t upload_merge_table(u32** table);   // both rules' pair lists, MERGE_ROWS rows each
 int fail(int code, const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);
 u64 fact(int i);

@@ -1,0 +1,168 @@
+// war_merge.cuh — deals played together: the enumeration of the merged kernels (war_merge.cu).
+//
+// The first h = floor(n/2) turns of a deal only use the cards as dealt: turn t takes the cards of deck
+// positions 2t and 2t+1, and the pair goes under the winner's pile.  The state after those h turns is, for
+// each player, the pairs that player won, in the order of the turns (odd n: below the one card of player 1
+// not played yet).  How the two players' wins alternated leaves no trace in it, and every alternation is a
+// deal of its own: which of the two cards of a pair was dealt to which player decides who wins it and
+// nothing else.  So all C(f, a) deals that interleave the same a pairs won by player 1 with the same f - a
+// pairs won by player 2 are in one state after h turns, and the rest of their game is one game: a merged
+// game, played once from turn h and counted C(f, a) times.  No deal is decided before turn h: player 2 has
+// an unplayed card left until then, and a cycle is longer than h turns (a shorter one would bring player
+// 1's first card back on top while a later one of its cards is there).
+//
+// Ranks.  A block of j! consecutive lexicographic ranks (a multiple of j!) fixes the first b = n - j deck
+// positions, and its deals are every order of the other j cards.  Its merged games are: a card for position
+// b if b is odd (dealt against the fixed card before it), a card for position n - 1 if n is odd, an ordered
+// list of f = (the other positions) / 2 unordered pairs, and the number a of them that player 1 wins (the
+// first a of the list).  That is j!/2^f lists of f + 1 games for j!/2^f * 2^f deals: 9.1 deals per game for
+// all 13! deals, 5.3 in a block of 12! of 13 or 15 cards, 3.2 in one of 9!.  A rank range is cut into the
+// fewest aligned blocks.  With no fixed card and even n, a state and its mirror image (the players
+// swapped) are both in the block, and only the one in which player 1 holds card n - 1 is played, twice
+// counted; with --half that one is all there is to play.
+//
+// Work units.  The first f - 4 pairs of a list (with the two single cards) are the unit's outer choice, by
+// mixed-radix index; the last four (fewer in a small block) run through a table of the 2520 ordered lists of
+// four pairs of eight cards, as byte selectors: two byte permutes of the unit's eight cards give a list.
+// A unit is a run of `lc` table rows under one outer choice, with every a.  A warp takes a unit and deals
+// its games to the lanes that need one, so 32 lanes work through it together.
+#pragma once
+#include <vector>
+#include "war_kernels.cuh"
+
+namespace war {
+
+constexpr u32 MERGE_INNER = 4;                       // pairs of a list that the table enumerates
+constexpr u32 MERGE_ROWS = 1 + 1 + 6 + 90 + 2520;    // ordered lists of 0..4 pairs of as many cards
+
+__host__ __device__ __forceinline__ u32 merge_rows(u32 fi) {      // (2 fi)! / 2^fi
+    return fi < 2u ? 1u : (fi == 2u ? 6u : (fi == 3u ? 90u : 2520u));
+}
+__host__ __device__ __forceinline__ u32 merge_row0(u32 fi) {      // first row of the table of fi pairs
+    return fi == 0u ? 0u : (fi == 1u ? 1u : (fi == 2u ? 2u : (fi == 3u ? 8u : 98u)));
+}
+
+typedef unsigned char u8;
+
+// One aligned block of a job.
+struct MBlock {
+    u64 u0;           // its first unit (the last block is followed by a sentinel with the unit total)
+    u32 free_mask;    // cards of the open positions
+    u32 nch;          // units per outer choice: ceil(rows / lc)
+    u8 f;             // pairs of open positions
+    u8 b;             // fixed positions
+    u8 filter;        // play only games in which player 1 holds card n - 1
+    u8 twice;         // and count them twice (their mirror images)
+    u8 prefix[20];    // the fixed cards
+};
+
+struct MergeArgs {
+    const MBlock* blocks;
+    const u32* table;     // MERGE_ROWS byte selectors of the rule (winner's or loser's card first)
+    u64 unit_lo, unit_hi; // units of this launch
+    u32 nblocks, lc;
+    int n, hbins, W, defer;
+    u64* memo;
+    u32 memo_bits;
+    TurnK tk;
+};
+
+// The outer choice of a unit and what its games share.  The piles without the list's pairs (U1, U2, s1 and
+// s2 bits long), the outer pairs (8 bits each), the cards of the inner ones as bytes.
+struct MUnit {
+    u64 U1, U2, O;
+    u32 c0, c1, s1, s2;
+};
+
+// A job's blocks (with the sentinel), units, merged games and rows of a unit.
+struct MergePlan {
+    std::vector<MBlock> blocks;
+    u64 units = 0, games = 0;
+    u32 lc = 0;
+};
+constexpr size_t MERGE_BLOCK_CAP = 512;   // blocks of a range: at most 2 (1 + .. + 16), and the sentinel
+// A launch takes at most this many units: a unit stands for at most 2520 rows x 2^9 deals, and a launch for
+// fewer than 2^38 (a lane's 32-bit turn total is drained with the histograms).
+constexpr u64 MERGE_LAUNCH_UNITS = (1ull << 38) / (2520ull << 9);
+
+void merge_table(int rule, u32* rows);
+void merge_plan(const war_job* job, u64 warps, MergePlan& p);
+cudaError_t launch_merged(const MergeArgs& a, int rule, int threads, int blocks, DevAcc* acc, cudaStream_t st);
+int merged_max_blocks_per_sm(int rule, int threads, int hbins);
+
+// Card of rank d among the set bits of m; m loses it.
+__host__ __device__ __forceinline__ u32 take_card(u32& m, u32 d) {
+    u32 x = m;
+    for (u32 k = 0; k < d; k++) x &= x - 1u;
+    const u32 bit = x & (0u - x);
+    m ^= bit;
+#ifdef __CUDA_ARCH__
+    return (u32)(__ffs((int)bit) - 1);
+#else
+    return (u32)__builtin_ctz(bit);
+#endif
+}
+
+__host__ __device__ __forceinline__ u32 card_count(u32 m) {
+#ifdef __CUDA_ARCH__
+    return (u32)__popc(m);
+#else
+    return (u32)__builtin_popcount(m);
+#endif
+}
+
+// Sets a unit up (every lane of the warp the same): the piles of 4-bit cards after the turns that its fixed and
+// chosen cards decide.
+template <int RULE>
+__host__ __device__ __forceinline__ void merge_unit(const MBlock& B, u64 outer, u32 n, MUnit& m) {
+    u32 free = B.free_mask;
+    const u32 b = B.b, f = B.f, fo = f > MERGE_INNER ? f - MERGE_INNER : 0u;
+    u64 U1 = 0, U2 = 0;
+    u32 s1 = 0, s2 = 0, half = 0;
+    if ((b & 1u) && b < n) {
+        const u32 k = card_count(free);
+        half = take_card(free, (u32)(outer % k));
+        outer /= k;
+    }
+    if (n & 1u) {   // player 1's last card, unplayed after h turns, is on top
+        u32 top;
+        if (b == n) top = B.prefix[n - 1u];
+        else {
+            const u32 k = card_count(free);
+            top = take_card(free, (u32)(outer % k));
+            outer /= k;
+        }
+        U1 = top;
+        s1 = 4u;
+    }
+    for (u32 t = 0; 2u * t < b && 2u * t + 1u < n; t++) {
+        const u32 x = B.prefix[2u * t], y = 2u * t + 1u < b ? B.prefix[2u * t + 1u] : half;
+        const u32 hi = x > y ? x : y, lo = x > y ? y : x;
+        const u64 pair = RULE ? lo | (hi << 4) : hi | (lo << 4);
+        if (x > y) { U1 |= pair << s1; s1 += 8u; }
+        else { U2 |= pair << s2; s2 += 8u; }
+    }
+    u64 O = 0;
+    for (u32 i = 0; i < fo; i++) {
+        const u32 k = card_count(free), np = k * (k - 1u) / 2u;
+        u32 d = (u32)(outer % np), x = 1;
+        outer /= np;
+        while (d >= x) { d -= x; x++; }          // the pair of ranks (x, d), x > d
+        const u32 hi = take_card(free, x), lo = take_card(free, d);
+        O |= (u64)(RULE ? lo | (hi << 4) : hi | (lo << 4)) << (8u * i);
+    }
+    u64 c = 0;
+    for (u32 i = 0; free; i++) c |= (u64)take_card(free, 0u) << (8u * i);
+    m.U1 = U1; m.U2 = U2; m.O = O; m.s1 = s1; m.s2 = s2;
+    m.c0 = (u32)c; m.c1 = (u32)(c >> 32);
+}
+
+// The pairs of a table row as 8-bit pairs of 4-bit cards.
+__device__ __forceinline__ u32 merge_row(u32 c0, u32 c1, u32 sel) {
+    u32 x = __byte_perm(c0, c1, sel), y = __byte_perm(c0, c1, sel >> 16);
+    x |= x >> 4;      // bytes 0 and 2: a card and the next one's nibble
+    y |= y >> 4;
+    return __byte_perm(x, y, 0x6420);
+}
+
+}  // namespace war

@@ -36,12 +36,6 @@ namespace war {
 enum { DET_BRENT = 0, DET_FLOYD = 1, DET_STREAK = 2 };
 enum { K_NONE = 0, K_END = 1, K_CYC = 2, K_UND = 3 };
 
-__device__ __forceinline__ u64 shr64(u64 x, u32 s) {
-    u64 r;
-    asm("shr.b64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(s));
-    return r;
-}
-
 // One turn on 128-bit sentinel piles (a0, a1) and (b0, b1); la = player 1's length, n1 = n - 1.  Returns
 // true if player 1 won.  Rule 0 puts the winning card, then the losing card, under the winner's pile
 // (gpu/war24.py:42-47); rule 1 the losing card first.

@@ -94,8 +94,13 @@ typedef struct war_tune {
                               of each found cycle, games looked up at their current state (n <= 14).  With
                               bits 3 and 4 (the "path memo"): also the states where decided games missed,
                               with their outcome (n <= 16; canonical scans take only this form).
-                              Every form gives the same results; out-of-range forms fall back to none. */
-    int32_t memo_bits;     /* cycle memo: log2 of its 8-byte slots (12..31); 0 = 24 (128 MiB) */
+                              Every form gives the same results; out-of-range forms fall back to none.
+                              Deals with the path memo and no sample are played merged: the states after
+                              the deals' first floor(n/2) turns, each once, in the multiply-add turn form, in
+                              units of the engine's own size (games, block_m and chunk do not apply); `turns`
+                              counts the turns played from there. */
+    int32_t memo_bits;     /* cycle memo: log2 of its 8-byte slots (12..31); 0 = 24 (128 MiB).  A merged job
+                              clears and uses only as much of it as its games can fill */
     int32_t chunk;         /* work units a lane takes from the work counter at a time (1..4096; 0 = 1): each lane
                               walks chunks of chunk x block_m! consecutive ranks (deals) */
 } war_tune;

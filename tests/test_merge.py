@@ -1,0 +1,157 @@
+"""Deals played together (csrc/war_merge.cuh): the first floor(n/2) turns of a deal forget how the two players'
+wins alternated, so C(f, a) deals share the state after them.  On the CPU, a restatement of the enumeration
+(aligned blocks, ordered lists of unordered pairs, the number of them that player 1 wins) against every deal
+of a range played turn by turn; on the GPU, the merged kernels against the oracle and the plain kernel at the
+edges of blocks, units and piles.  Counts are whole numbers: every comparison is equality."""
+import itertools
+import math
+import random
+from collections import Counter
+
+import pytest
+
+
+def unrank(r, n):
+    cards, out = list(range(n)), []
+    for i in range(n):
+        d, r = divmod(r, math.factorial(n - 1 - i))
+        out.append(cards.pop(d))
+    return out
+
+
+def after_first_turns(deck, rule):
+    """Both piles after floor(n/2) turns."""
+    a, b = deck[0::2], deck[1::2]
+    for _ in range(len(deck) // 2):
+        x, y = a.pop(0), b.pop(0)
+        pair = [min(x, y), max(x, y)] if rule else [max(x, y), min(x, y)]
+        (a if x > y else b).extend(pair)
+    return tuple(a), tuple(b)
+
+
+def blocks(lo, hi, n):
+    while lo < hi:
+        j = n
+        while lo % math.factorial(j) or lo + math.factorial(j) > hi:
+            j -= 1
+        yield lo, j
+        lo += math.factorial(j)
+
+
+def pair_lists(cards, f):
+    if f == 0:
+        yield []
+        return
+    for x, y in itertools.combinations(sorted(cards), 2):
+        for rest in pair_lists([c for c in cards if c not in (x, y)], f - 1):
+            yield [(y, x)] + rest
+
+
+def merged(lo, hi, n, rule, half=False):
+    """{state after the first turns: deals of the range in it}, by blocks."""
+    out = Counter()
+    h = n // 2
+    for r, j in blocks(lo, hi, n):
+        b = n - j
+        deck = unrank(r, n)
+        free = deck[b:]
+        f = max(0, (2 * h - (b + b % 2)) // 2)
+        singles = (1 if b % 2 and b < n else 0) + (1 if n % 2 and b < n else 0)
+        for pick in itertools.permutations(free, singles):
+            rest = [c for c in free if c not in pick]
+            pick = list(pick)
+            fixed = deck[:b] + ([pick.pop(0)] if b % 2 and b < n else [])
+            top = [pick.pop(0) if b < n else deck[n - 1]] if n % 2 else []
+            wins = [[], []]
+            for t in range(0, min(len(fixed), 2 * h) - 1, 2):
+                x, y = fixed[t], fixed[t + 1]
+                wins[0 if x > y else 1] += [min(x, y), max(x, y)] if rule else [max(x, y), min(x, y)]
+            for pairs in pair_lists(rest, f):
+                cards = [list(reversed(p)) if rule else list(p) for p in pairs]
+                for a in range(f + 1):
+                    one = tuple(top + wins[0] + sum(cards[:a], []))
+                    two = tuple(wins[1] + sum(cards[a:], []))
+                    if not half or n - 1 in one:
+                        out[one, two] += math.comb(f, a)
+    return out
+
+
+@pytest.mark.parametrize("n,rule", [(2, 0), (3, 1), (4, 0), (5, 0), (6, 1), (7, 0), (8, 1)])
+def test_merged_enumeration_is_every_deal(n, rule):
+    rnd = random.Random(100 * n + rule)
+    total = math.factorial(n)
+    ranges = [(0, total)] if n <= 7 else []
+    for _ in range(5):
+        lo = rnd.randrange(0, total)
+        ranges.append((lo, min(total, lo + rnd.choice([1, 2, 25, 800]))))
+    for lo, hi in ranges:
+        for half in ((False, True) if n % 2 == 0 else (False,)):
+            want = Counter()
+            for r in range(lo, hi):
+                deck = unrank(r, n)
+                if not half or deck.index(n - 1) % 2 == 0:
+                    want[after_first_turns(deck, rule)] += 1
+            assert merged(lo, hi, n, rule, half) == want, (n, rule, lo, hi, half)
+
+
+def memo_tune(wl, **kw):
+    t = dict(variant=31, games=1, threads=256, defer=8, window=32, memo_bits=20)
+    t.update(kw)
+    return wl.make_tune(**t)
+
+
+KEYS = ("cyc", "done", "maxfin", "hist", "endhist")
+
+
+def same(wl, got, want, what):
+    g, w = wl.to_dict(got), wl.to_dict(want)
+    for k in KEYS:
+        assert g[k] == w[k], (what, k)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", range(4, 17))
+def test_merged_ranges(wl, n):
+    """Ranges that begin and end at, before and after block ends, the first and the last deals, one deal, odd
+    lengths; --half; both rules; a table of 2^12 words; several launch shapes."""
+    rnd = random.Random(n)
+    total = math.factorial(n)
+    ranges = [(0, 1), (total - 1, total), (0, min(total, 362880)), (max(0, total - 362881), total)]
+    for j in range(1, min(n, 10)):
+        f = math.factorial(j)
+        k = rnd.randrange(1, total // f) if total // f > 1 else 0
+        ranges.append((k * f, min(total, (k + 1) * f)))
+        ranges.append((max(0, k * f - 1), min(total, k * f + rnd.choice([1, f, 2 * f + 1]))))
+    for _ in range(4):
+        lo = rnd.randrange(0, total)
+        ranges.append((lo, min(total, lo + rnd.choice([3, 1001, 1000003]))))
+    shapes = [dict(), dict(threads=64, defer=4), dict(threads=1024, memo_bits=12), dict(window=1, defer=32),
+              dict(blocks_per_sm=1, threads=128, variant=30)]
+    for i, (lo, hi) in enumerate(ranges):
+        for flags in ([0, wl.F_HALF] if n % 2 == 0 else [0]):
+            job = wl.make_job(n, rule=i % 2, lo=lo, hi=hi, flags=flags, hbins=rnd.choice([0, 64, 256]))
+            same(wl, wl.enumerate_job(job, memo_tune(wl, **shapes[i % len(shapes)])), wl.enumerate_plain(job),
+                 (n, lo, hi, flags, i))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,rule", [(10, 0), (11, 1), (12, 0)])
+def test_merged_whole_spaces(wl, n, rule):
+    """Every deal (even n: mirror images played once, counted twice), and --half."""
+    for flags in ([0, wl.F_HALF] if n % 2 == 0 else [0]):
+        job = wl.make_job(n, rule=rule, flags=flags, hbins=256)
+        want = wl.enumerate_plain(job)
+        for kw in (dict(), dict(memo_bits=12, defer=4)):
+            same(wl, wl.enumerate_job(job, memo_tune(wl, **kw)), want, (n, rule, flags, kw))
+
+
+@pytest.mark.gpu
+def test_merged_table_kept_between_ranges_of_different_sizes(wl):
+    """A job smaller than the one before it with WAR_F_MEMO_KEEP, and one without: the part of the table in use
+    follows the first job, or the job's own size."""
+    t = memo_tune(wl, memo_bits=26)
+    jobs = [(0, 0, 3 * 10 ** 7), (wl.F_MEMO_KEEP, 10 ** 9, 10 ** 9 + 12345), (0, 10 ** 9, 10 ** 9 + 54321),
+            (wl.F_MEMO_KEEP, 5 * 10 ** 8, 5 * 10 ** 8 + 10 ** 7)]
+    for flags, lo, hi in jobs:
+        job = wl.make_job(13, flags=flags, lo=lo, hi=hi, hbins=128)
+        same(wl, wl.enumerate_job(job, t), wl.enumerate_plain(wl.make_job(13, lo=lo, hi=hi, hbins=128)), (lo, hi))
