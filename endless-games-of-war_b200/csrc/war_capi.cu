@@ -526,33 +526,14 @@ static int enumerate_merged(const war_job* job, const Tune& t, war_result* out) 
     const int blocks = t.blocks_per_sm * c.sm_count;
     merge_plan(job, (u64)blocks * (u64)(t.threads / 32), p);
     if (p.units == 0) return WAR_OK;   // (--half: no deal of the range gives card n-1 to player 1)
-    cudaError_t e;
-    if (p.blocks.size() > MERGE_BLOCK_CAP) return fail(WAR_EINVAL, "plan has %zu blocks", p.blocks.size());
-    if ((e = cudaMemcpyAsync(c.d_blocks, p.blocks.data(), sizeof(MBlock) * p.blocks.size(), cudaMemcpyHostToDevice,
-                             cur_stream())) != cudaSuccess)
-        return cuda_fail(e, "copy blocks");
     MergeArgs a;
-    memset(&a, 0, sizeof a);
-    a.blocks = c.d_blocks;
-    a.nblocks = (u32)p.blocks.size() - 1u;
-    a.table = c.d_table + (job->rule ? MERGE_ROWS : 0);
-    a.lc = p.lc;
-    a.n = job->n; a.hbins = job->hbins; a.W = t.window; a.defer = t.defer;
-    a.tk.k16 = 16u; a.tk.km16 = (u32)-16; a.tk.k2p28 = 1u << 28; a.tk.k4 = 4u; a.tk.one = 1u;
-    a.tk.c0 = 2 * job->n - 4; a.tk.end2 = (u32)(4 * job->n * job->n);
-    int st, used = 0;   // (a game stores at most two states besides the cycles found)
+    int st, used = 0;
+    if ((st = merge_args(job, p, job->hbins, t.window, t.defer, a))) return st;
+      // (a game stores at most two states besides the cycles found)
     if ((st = prepare_memo(c, job, t.memo_bits, 4 * 3, &a.memo, 2 * p.games, &used))) return st;
     a.memo_bits = (u32)used;
-    for (u64 u = 0; u < p.units; u += MERGE_LAUNCH_UNITS) {
-        a.unit_lo = u;
-        a.unit_hi = std::min(p.units, u + MERGE_LAUNCH_UNITS);
-        st = run_launch([&](cudaStream_t x) { return launch_merged(a, job->rule, t.threads, blocks, c.d_acc, x); },
-                        &out->kernel_ms);
-        if (st) return st;
-        merge_acc(*c.h_acc, out, job->hbins, 0);
-    }
-    out->units += p.units;
-    return WAR_OK;
+    return run_merged(p, a, job->hbins, out,
+                      [&](cudaStream_t x) { return launch_merged(a, job->rule, t.threads, blocks, c.d_acc, x); });
 }
 
 int war_enumerate_held(const war_job* job, const war_tune* tune, war_result* out) {
@@ -590,12 +571,25 @@ int war_enumerate_held(const war_job* job, const war_tune* tune, war_result* out
     HeldArgs a;
     memset(&a, 0, sizeof a);
     a.W = W; a.defer = defer; a.form = form; a.svc_off = (tune && (tune->variant & 8)) ? 1 : 0;
-    const int maxb = held_max_blocks_per_sm(job->rule, threads, job->hbins, memo, form, held_svc(a));
+    // The default turn plays merged games; that needs the checkpoints after turn 0 to be after the merged turns.
+    const bool merged = !memo && form == 3 && held_svc(a) && W >= job->n / 2;
+    if (!merged && !memo && form == 3) a.svc_off = 1;
+    const int maxb = merged ? held_merged_max_blocks_per_sm(job->rule, threads, job->hbins)
+                            : held_max_blocks_per_sm(job->rule, threads, job->hbins, memo, form, held_svc(a));
     if (maxb < 1) return fail(WAR_EINVAL, "launch shape threads=%d does not fit an SM%s", threads,
                               memo ? " (at most 512 with the memo)" : "");
     const int bps = (tune && tune->blocks_per_sm) ? std::min(tune->blocks_per_sm, maxb) : maxb;
     std::lock_guard<std::mutex> lk(ctx().mu);
     Ctx& c = ctx();
+    if (merged) {
+        MergePlan p;
+        const int blocks = bps * c.sm_count;
+        merge_plan(job, (u64)blocks * (u64)(threads / 32), p);
+        MergeArgs m;
+        if ((st = merge_args(job, p, job->hbins, W, defer, m))) return st;
+        return run_merged(p, m, job->hbins, out,
+                          [&](cudaStream_t x) { return launch_held_merged(m, job->rule, threads, blocks, c.d_acc, x); });
+    }
     Plan p;
     make_plan(job, block_m, p);
     if (p.extra.size() > Ctx::UNIT_CAP) return fail(WAR_EINVAL, "plan has %zu extra units", p.extra.size());

@@ -17,6 +17,7 @@
 // deals as the lexicographic block, so the counts are the same.  With a table (HeldArgs.memo) the engine
 // takes the path memo of war_refill.cuh, with a key of its own state (h_key).
 #include "war_refill.cuh"
+#include "war_merge.cuh"
 
 namespace war {
 
@@ -410,11 +411,224 @@ __global__ void __launch_bounds__(MEMO ? 512 : 1024) held_kernel(const __grid_co
     flush_hist(she, acc->endhist, WAR_EBINS);
 }
 
+// ---- merged games (war_merge.cuh) -----------------------------------------------------------------------
+//
+// held_kernel plays every deal; this kernel plays each state after the deals' first h = floor(n/2) turns once,
+// for the default turn (h_turn_packed_fma) without the memo and with Brent's checkpoint at multiples of the
+// service period (SVC above).  `turns` stays what playing every deal gives: the deals of a game share their
+// path from turn h and so the turn at which Brent's checkpoints W, 3W, ... (all at or after turn h) decide them;
+// only a deal that lies on its own cycle, of length lam <= W, is decided by the checkpoint at turn 0 instead, at
+// turn lam.  At most one deal of a game does (a state on a cycle has one predecessor on it), and held_start
+// finds it.  With the tortoise at the state of turn h until turn W, a game on such a cycle is known at turn
+// h + lam, and counted as decided at W + lam.
+//
+// Services: games start at services, at turn h, so within the service period all games of a warp reach a
+// multiple of it at the same place, (period - h mod period) turns in; the checkpoint is saved there.
+//
+// What bounds it: instruction issue of the turns (about 150 of them per game, as before; ncu of held_kernel
+// issue 82%, ALU pipe 83%), so the gain is the deals per game, and with it the rate: a slice of 1e9 deals
+// of 17 cards (4.9 deals per game on average) 356 -> 58.6 ms on a B200, a period of 32 turns (16: 63.8, 8: 71.3 ms).
+
+// The start of a lane's game, kept for held_start, and its block and holder.
+struct HeldStart {
+    u64 wh, wo;
+    u32 s, tag;    // tag: block, and in bit 31 whether player 1 holds card n-1
+};
+
+// How many deals of the game that is at x at turn h lie on their own cycle of length lam (h < lam): 0, or 1 (2
+// with its mirror image).  Such a deal is the state h turns before x on the cycle; it is a deal if the
+// piles are as dealt, and one of this game's if its first cards are the block's.
+template <int RULE>
+__device__ __noinline__ u32 held_start(const HeldStart x, const MBlock* __restrict__ blocks, u32 n, u32 lam) {
+    const u32 n4m8 = 4u * n - 8u, h = n >> 1;
+    u64 wh = x.wh, wo = x.wo, dh = 0, dv = 0;
+    u32 s = x.s, ds = 0;
+    for (u32 t = 0; t < lam; t++) {
+        if (t == lam - h) { dh = wh; dv = wo; ds = s; }
+        h_turn_packed<RULE>(wh, wo, s, n4m8);
+    }
+    if (wh != x.wh || wo != x.wo || s != x.s) return 0u;      // x is not on the cycle
+    const MBlock& B = blocks[x.tag & 0x7FFFFFFFu];
+    const bool p1 = (x.tag >> 31) != 0u;
+    const u32 lh = (ds & 255u) >> 2, p = ds >> 8;
+    if (lh + 1u != (p1 ? (n + 1u) >> 1 : n >> 1)) return 0u;  // not as dealt
+    for (u32 i = 0; i < B.b; i++) {
+        const u32 k = i >> 1;
+        u32 card;
+        if (((i & 1u) == 0u) == p1) card = k == p ? n - 1u : (u32)(dh >> (4u * (k < p ? k : k - 1u))) & 15u;
+        else card = (u32)(dv >> (4u * k)) & 15u;
+        if (card != B.prefix[i]) return 0u;
+    }
+    return B.twice ? 2u : 1u;
+}
+
+template <int RULE>
+__global__ void __launch_bounds__(1024) held_merge_kernel(const __grid_constant__ MergeArgs a, DevAcc* __restrict__ acc) {
+    extern __shared__ u64 sh64[];
+    __shared__ MUnit units[32];
+    HeldStart* const start = (HeldStart*)sh64 + threadIdx.x;
+    u32* const shh = (u32*)((HeldStart*)sh64 + blockDim.x);
+    u32* const she = shh + a.hbins;
+    const int bins = a.hbins + WAR_EBINS;
+    for (int b = threadIdx.x; b < bins; b += blockDim.x) shh[b] = 0;
+    __syncthreads();
+
+    const u32 n = (u32)a.n, h = n >> 1, W = (u32)a.W, n4m8 = 4u * n - 8u;
+    const TurnK K = a.tk;
+    const u32 hb1 = a.hbins > 0 ? (u32)(a.hbins - 1) : 0u;
+    const u32 period = a.defer > 4 ? (u32)((a.defer + 3) & ~3) : 4u;
+    const u32 after = h % period, before = period - after;   // turns of a period around the checkpoint's place
+    const u32 lane = threadIdx.x & 31u;
+    MUnit& mu = units[threadIdx.x >> 5];
+    u64* const counter = &acc->work_next;
+
+    u64 wh = 0, wo = 0, th = ~0ull, to = 0, turns = 0;
+    u32 s = 0, ts = 0, rounds = 0, next = 0xFFFFFFFFu, wt = 0;
+    bool done = true, kcy = false, active = false;
+    u32 cyc = 0, maxfin = 0, capped = 0;
+    MCursor c;
+
+    auto drain = [&]() {
+        __syncwarp();
+        for (int b = (int)lane; b < bins; b += 32) {
+            const u32 v = atomicExch(&shh[b], 0u);
+            if (v) atomicAdd(b < a.hbins ? &acc->hist[b] : &acc->endhist[b - a.hbins], (u64)v);
+        }
+        const u64 v_cyc = warp_sum((u64)cyc);
+        if (lane == 0u && v_cyc) atomicAdd(&acc->cyc, v_cyc);
+        cyc = 0;
+    };
+    auto setup = [&](const MBlock& B, u64 outer) {
+        MUnit m;
+        merge_unit<RULE>(B, outer, n, m);
+        __syncwarp();
+        if (lane == 0u) mu = m;
+        __syncwarp();
+    };
+    auto over = [&]() -> u32 {
+        return mu.s2 + 8u * (c.f - c.pa) == 0u ? 1u : (mu.s1 + 8u * c.pa == 0u ? 2u : 0u);
+    };
+    auto ended = [&](u32 k) {
+        if (lane == 0u) { atomicAdd(&she[h], k); turns += (u64)k * h; }
+        maxfin = max(maxfin, h);
+    };
+    auto build = [&](u32 sel) -> bool {
+        const u32 a8 = 8u * c.pa;
+        const u64 lw = mu.O | ((u64)merge_row(mu.c0, mu.c1, sel) << (8u * (c.f - c.fi)));
+        const u64 w1 = mu.U1 | shl64(lw & ~shl64(~0ull, a8), mu.s1), w2 = mu.U2 | shl64(shr64(lw, a8), mu.s2);
+        // card n-1: its holder and its depth
+        bool p1;
+        u32 p;
+        if (mu.top >= MTOP_P1) {
+            p1 = mu.top < MTOP_P2;
+            p = mu.top & (p1 ? MTOP_P1 - 1u : MTOP_P2 - 1u);
+        } else {
+            u32 i = mu.top - MTOP_PAIR;
+            if (mu.top == MTOP_INNER) {   // the last of the inner cards: its place in the row
+                const u32 z = sel ^ (0x11111111u * (2u * c.fi - 1u));
+                i = c.f - c.fi + (((u32)__ffs((int)((z - 0x11111111u) & ~z & 0x88888888u)) - 1u) >> 3);
+            }
+            p1 = i < c.pa;
+            p = (p1 ? (mu.s1 >> 2) + 2u * i : (mu.s2 >> 2) + 2u * (i - c.pa)) + (u32)RULE;
+        }
+        if (c.filter && !p1) return false;
+        const u64 w = p1 ? w1 : w2, low = ~shl64(~0ull, 4u * p);
+        wh = (w & low) | (shr64(w, 4u * p + 4u) << (4u * p));
+        wo = p1 ? w2 : w1;
+        const u32 lh = (p1 ? (mu.s1 >> 2) + 2u * c.pa : (mu.s2 >> 2) + 2u * (c.f - c.pa)) - 1u;
+        s = 4u * lh + 256u * p;
+        th = wh; to = wo; ts = s;
+        rounds = h; next = W > h ? W : 3u * W; wt = c.wt;   // (W = h: the tortoise of turn W)
+        done = false; kcy = false; active = true;
+        HeldStart x;
+        x.wh = wh; x.wo = wo; x.s = s; x.tag = c.blk | (p1 ? 0x80000000u : 0u);
+        *start = x;
+        return true;
+    };
+    auto refill = [&](bool want) {
+        if (want) active = false;
+        merge_deal(c, a, counter, want, setup, over, ended, build, drain);
+    };
+    auto turn = [&]() {
+        const bool en = h_turn_packed_fma<RULE>(wh, wo, s, n4m8, K);
+        if (!done) rounds++;
+        const bool cy = (wh == th) & (wo == to) & (s == ts);
+        kcy = done ? kcy : (cy & !en);
+        done = done | cy | en;
+    };
+
+    refill(true);
+    bool running = __any_sync(WAR_FULL_MASK, active);
+    while (running) {
+        for (u32 k = 0; k < before; k++) turn();
+        if (!done && rounds == next) {
+            if (next > WAR_TURN_CAP) { capped++; done = true; }   // abandoned (never expected): the job fails
+            else { th = wh; to = wo; ts = s; next = 2u * next + W; }
+        }
+        for (u32 k = 0; k < after; k++) turn();
+        const bool fin = done & active;
+        if (__any_sync(WAR_FULL_MASK, fin)) {
+            if (fin) {
+                if (kcy) {
+                    // next = W: found with the tortoise at turn h, else at turn (next - W) / 2
+                    const u32 save = next == W ? h : (next - W) >> 1, lam = rounds - save;
+                    cyc += wt;
+                    if (a.hbins) atomicAdd(&shh[lam < hb1 ? lam : hb1], wt);
+                    const u32 t = next == W ? W + lam : rounds;
+                    turns += (u64)wt * t;
+                    if (lam <= W && save <= W) turns -= (u64)held_start<RULE>(*start, a.blocks, n, lam) * (t - lam);
+                } else {
+                    maxfin = max(maxfin, rounds);
+                    turns += (u64)wt * rounds;
+                    atomicAdd(&she[rounds < WAR_EBINS - 1 ? rounds : WAR_EBINS - 1], wt);
+                }
+            }
+            refill(fin);
+            running = __any_sync(WAR_FULL_MASK, active);
+        }
+    }
+
+    const u64 v_cyc = warp_sum((u64)cyc), v_turns = warp_sum(turns), v_max = warp_max((u64)maxfin);
+    const u64 v_cap = warp_sum((u64)capped);
+    if (lane == 0u) {
+        if (c.done) atomicAdd(&acc->done, c.done);
+        if (v_cyc) atomicAdd(&acc->cyc, v_cyc);
+        if (v_turns) atomicAdd(&acc->turns, v_turns);
+        if (v_max) atomicMax(&acc->maxfin, v_max);
+        if (v_cap) atomicAdd(&acc->status, v_cap);
+    }
+    __syncthreads();
+    flush_hist(shh, acc->hist, a.hbins);
+    flush_hist(she, acc->endhist, WAR_EBINS);
+}
+
+static size_t held_merge_shmem(int threads, int hbins) {
+    return sizeof(HeldStart) * (size_t)threads + sizeof(u32) * (size_t)(hbins + WAR_EBINS);
+}
+
+cudaError_t launch_held_merged(const MergeArgs& a, int rule, int threads, int blocks, DevAcc* acc, cudaStream_t st) {
+    (rule ? held_merge_kernel<1> : held_merge_kernel<0>)<<<blocks, threads, held_merge_shmem(threads, a.hbins), st>>>(a, acc);
+    note_launch();
+    return cudaGetLastError();
+}
+
+int held_merged_max_blocks_per_sm(int rule, int threads, int hbins) {
+    int nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rule ? held_merge_kernel<1> : held_merge_kernel<0>, threads,
+                                                      held_merge_shmem(threads, hbins)) != cudaSuccess)
+        return 0;
+    return nb;
+}
+
 typedef void (*HeldFn)(const HeldArgs, DevAcc*);
 
 template <int RULE, bool MEMO>
 static HeldFn held_pick_form(int form, bool svc) {
-    if (form == 3) return svc ? held_kernel<RULE, MEMO, 3, true> : held_kernel<RULE, MEMO, 3, false>;
+    if constexpr (MEMO) {
+        if (form == 3) return svc ? held_kernel<RULE, MEMO, 3, true> : held_kernel<RULE, MEMO, 3, false>;
+    } else {   // with the checkpoint at the services and no memo the default turn plays merged games
+        if (form == 3) return held_kernel<RULE, MEMO, 3, false>;
+    }
     if (form == 2) return svc ? held_kernel<RULE, MEMO, 2, true> : held_kernel<RULE, MEMO, 2, false>;
     if (form == 1) return svc ? held_kernel<RULE, MEMO, 1, true> : held_kernel<RULE, MEMO, 1, false>;
     return svc ? held_kernel<RULE, MEMO, 0, true> : held_kernel<RULE, MEMO, 0, false>;

@@ -53,6 +53,7 @@ int check_job(const war_job* j);
 void make_plan(const war_job* job, int m, Plan& p);
 void merge_acc(const DevAcc& h, war_result* r, int hbins, int dbins);
 void fill_fact(u64* f);
+int merge_args(const war_job* job, const MergePlan& p, int hbins, int window, int defer, MergeArgs& a);
 int resolve_tune(const war_job* job, const war_tune* in, Tune& t);
 int floyd_sample_run(const war_job* job, war_result* out);
 
@@ -74,6 +75,20 @@ inline int run_launch(F launch, double* ms) {
     cudaEventElapsedTime(&f, c.ev0, c.ev1);
     if (ms) *ms += f;
     if (c.h_acc->status) return fail(WAR_ECAP, "%llu game(s) passed the turn cap", (unsigned long long)c.h_acc->status);
+    return WAR_OK;
+}
+
+// Runs a merged job's units in launches of at most MERGE_LAUNCH_UNITS.
+template <typename F>
+inline int run_merged(const MergePlan& p, MergeArgs& a, int hbins, war_result* out, F launch) {
+    for (u64 u = 0; u < p.units; u += MERGE_LAUNCH_UNITS) {
+        a.unit_lo = u;
+        a.unit_hi = p.units - u < MERGE_LAUNCH_UNITS ? p.units : u + MERGE_LAUNCH_UNITS;
+        const int st = run_launch(launch, &out->kernel_ms);
+        if (st) return st;
+        merge_acc(*ctx().h_acc, out, hbins, 0);
+    }
+    out->units += p.units;
     return WAR_OK;
 }
 

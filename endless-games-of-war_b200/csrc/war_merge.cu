@@ -21,11 +21,6 @@
 
 namespace war {
 
-// A warp empties its block's 32-bit histograms into the accumulators before it has dealt out games that count
-// this many deals since it last did.  A bin holds at most what the block's warps dealt out since, so
-// 32 x (2^26 + one unit of at most 2520 x 2^9 deals) stays below 2^32.
-constexpr u32 DRAIN_DEALS = 1u << 26;
-
 // One game slot of the merged kernel.
 struct MGame {
     u64 w1, w2, t1, t2, ka, kb;
@@ -51,14 +46,10 @@ __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restric
     const u32 mbits = a.memo_bits;
     const u32 vmask = (1u << mbits) - 1u;
     const u64 pat = 0x1111111111111111ull * (u64)(n - 1u);
-    const u32 lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    const u32 lane = threadIdx.x & 31u;
     MUnit& mu = units[threadIdx.x >> 5];
 
-    // the warp's place in its unit: row l of [l0, lend) with a of the f pairs won by player 1
-    u32 l = 0, l0 = 0, lend = 0, pa = 0, f = 0, wt = 0, blk = 0, row0 = 0;
-    bool filter = false, dry = false;
-    u32 given = 0;       // deals dealt out since the last drain
-    u64 done = 0;        // deals counted by this warp
+    MCursor c;
     u32 cyc = 0, turns = 0, maxfin = 0, capped = 0, mlook = 0, mhit = 0, mstore = 0;
     MGame g;
     g.active = false; g.done = true; g.kcy = false; g.w1 = g.w2 = 1ull; g.t1 = g.t2 = 0ull; g.q = 0; g.rounds = 0;
@@ -75,80 +66,40 @@ __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restric
             if (v_cyc) atomicAdd(&acc->cyc, v_cyc);
             if (v_turns) atomicAdd(&acc->turns, v_turns);
         }
-        cyc = 0; turns = 0; given = 0;
+        cyc = 0; turns = 0;
     };
-
-    // deals the warp's next games to the lanes that want one
-    auto refill = [&](bool want) {
-        u32 need = __ballot_sync(WAR_FULL_MASK, want);
-        if (want) g.active = false;
-        while (need && !dry) {
-            if (l == lend) {
-                if (pa < f) {
-                    pa++;
-                    wt = wt * (f - pa + 1u) / pa;
-                    l = l0;
-                } else {
-                    u64 u = 0;
-                    if (lane == 0u) u = atomicAdd(counter, 1ull);
-                    u = __shfl_sync(WAR_FULL_MASK, u, 0) + a.unit_lo;
-                    if (u >= a.unit_hi) { dry = true; break; }
-                    while (u >= a.blocks[blk + 1u].u0) blk++;
-                    const MBlock& B = a.blocks[blk];
-                    const u64 v = u - B.u0, outer = v / B.nch;
-                    MUnit m;
-                    merge_unit<RULE>(B, outer, n, m);
-                    __syncwarp();
-                    if (lane == 0u) mu = m;
-                    __syncwarp();
-                    f = B.f;
-                    const u32 fi = min(f, MERGE_INNER);
-                    row0 = merge_row0(fi);
-                    l0 = (u32)(v - outer * B.nch) * a.lc;
-                    lend = min(merge_rows(fi), l0 + a.lc);
-                    l = l0;
-                    pa = 0;
-                    wt = B.twice ? 2u : 1u;
-                    filter = B.filter != 0;
-                    if (given > DRAIN_DEALS) drain();
-                }
-                const u32 q1 = mu.s1 + 8u * pa, q2 = mu.s2 + 8u * (f - pa);
-                if (q1 == 0u || q2 == 0u) {   // one player won every pair: over at turn h
-                    if (q1 != 0u || !filter) {
-                        const u32 c = (lend - l) * wt;
-                        if (lane == 0u) atomicAdd(&she[h], c);
-                        maxfin = max(maxfin, h);
-                        done += c; given += c;
-                    }
-                    l = lend;
-                }
-                continue;
-            }
-            const u32 r = __popc(need & below), take = min((u32)__popc(need), lend - l);
-            bool mine = ((need >> lane) & 1u) && r < take;
-            if (mine) {
-                const u32 fi = min(f, MERGE_INNER), a8 = 8u * pa;
-                const u32 inner = merge_row(mu.c0, mu.c1, __ldg(a.table + row0 + l + r));
-                const u64 lw = mu.O | ((u64)inner << (8u * (f - fi)));
-                g.w1 = mu.U1 | shl64(lw & ~shl64(~0ull, a8), mu.s1) | shl64(1ull, mu.s1 + a8);
-                g.w2 = mu.U2 | shl64(shr64(lw, a8), mu.s2) | shl64(1ull, mu.s2 + 8u * f - a8);
-                g.q = mu.s1 + a8 - n2;
-                if (filter) {   // player 1 must hold card n - 1
-                    const u64 x = g.w1 ^ pat;
-                    mine = ((x - 0x1111111111111111ull) & ~x & 0x8888888888888888ull) != 0ull;
-                }
-            }
-            if (mine) {
-                g.t1 = g.w1; g.t2 = g.w2; g.rounds = h; g.next = 2u * h + W;
-                g.ta = 0; g.tb = 0; g.mv = 0; g.wt = wt;
-                g.done = false; g.kcy = false; g.active = true;
-            }
-            const u32 got = __ballot_sync(WAR_FULL_MASK, mine);
-            need &= ~got;
-            const u32 c = (u32)__popc(got) * wt;
-            done += c; given += c;
-            l += take;
+    auto setup = [&](const MBlock& B, u64 outer) {
+        MUnit m;
+        merge_unit<RULE>(B, outer, n, m);
+        __syncwarp();
+        if (lane == 0u) mu = m;
+        __syncwarp();
+    };
+    auto over = [&]() -> u32 {
+        return mu.s2 + 8u * (c.f - c.pa) == 0u ? 1u : (mu.s1 + 8u * c.pa == 0u ? 2u : 0u);
+    };
+    auto ended = [&](u32 k) {
+        if (lane == 0u) atomicAdd(&she[h], k);
+        maxfin = max(maxfin, h);
+    };
+    auto build = [&](u32 sel) -> bool {
+        const u32 a8 = 8u * c.pa;
+        const u64 lw = mu.O | ((u64)merge_row(mu.c0, mu.c1, sel) << (8u * (c.f - c.fi)));
+        g.w1 = mu.U1 | shl64(lw & ~shl64(~0ull, a8), mu.s1) | shl64(1ull, mu.s1 + a8);
+        g.w2 = mu.U2 | shl64(shr64(lw, a8), mu.s2) | shl64(1ull, mu.s2 + 8u * c.f - a8);
+        if (c.filter) {   // player 1 must hold card n - 1
+            const u64 x = g.w1 ^ pat;
+            if (((x - 0x1111111111111111ull) & ~x & 0x8888888888888888ull) == 0ull) return false;
         }
+        g.q = mu.s1 + a8 - n2;
+        g.t1 = g.w1; g.t2 = g.w2; g.rounds = h; g.next = 2u * h + W;
+        g.ta = 0; g.tb = 0; g.mv = 0; g.wt = c.wt;
+        g.done = false; g.kcy = false; g.active = true;
+        return true;
+    };
+    auto refill = [&](bool want) {
+        if (want) g.active = false;
+        merge_deal(c, a, counter, want, setup, over, ended, build, drain);
     };
 
     refill(true);
@@ -225,7 +176,7 @@ __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restric
     const u64 v_cap = warp_sum((u64)capped), v_l = warp_sum((u64)mlook), v_h = warp_sum((u64)mhit);
     const u64 v_s = warp_sum((u64)mstore);
     if (lane == 0u) {
-        if (done) atomicAdd(&acc->done, done);
+        if (c.done) atomicAdd(&acc->done, c.done);
         if (v_cyc) atomicAdd(&acc->cyc, v_cyc);
         if (v_turns) atomicAdd(&acc->turns, v_turns);
         if (v_max) atomicMax(&acc->maxfin, v_max);
@@ -338,6 +289,24 @@ void merge_plan(const war_job* job, u64 warps, MergePlan& p) {
     memset(&end, 0, sizeof end);
     end.u0 = ~0ull;   // no unit lies past the last block
     p.blocks.push_back(end);
+}
+
+// The arguments of a merged kernel; copies the plan's blocks to the device.
+int merge_args(const war_job* job, const MergePlan& p, int hbins, int window, int defer, MergeArgs& a) {
+    Ctx& c = ctx();
+    cudaError_t e;
+    if (p.blocks.size() > MERGE_BLOCK_CAP) return fail(WAR_EINVAL, "plan has %zu blocks", p.blocks.size());
+    if ((e = cudaMemcpyAsync(c.d_blocks, p.blocks.data(), sizeof(MBlock) * p.blocks.size(), cudaMemcpyHostToDevice,
+                             cur_stream())) != cudaSuccess)
+        return cuda_fail(e, "copy blocks");
+    memset(&a, 0, sizeof a);
+    a.blocks = c.d_blocks;
+    a.table = c.d_table + (job->rule ? MERGE_ROWS : 0);
+    a.lc = p.lc;
+    a.n = job->n; a.hbins = hbins; a.W = window; a.defer = defer;
+    a.tk.k16 = 16u; a.tk.km16 = (u32)-16; a.tk.k2p28 = 1u << 28; a.tk.k4 = 4u; a.tk.one = 1u;
+    a.tk.c0 = 2 * job->n - 4; a.tk.end2 = (u32)(4 * job->n * job->n);
+    return WAR_OK;
 }
 
 static size_t merge_shmem(int hbins) { return sizeof(u32) * (size_t)(hbins + WAR_EBINS); }

@@ -60,7 +60,7 @@ struct MergeArgs {
     const MBlock* blocks;
     const u32* table;     // MERGE_ROWS byte selectors of the rule (winner's or loser's card first)
     u64 unit_lo, unit_hi; // units of this launch
-    u32 nblocks, lc;
+    u32 lc;
     int n, hbins, W, defer;
     u64* memo;
     u32 memo_bits;
@@ -68,11 +68,14 @@ struct MergeArgs {
 };
 
 // The outer choice of a unit and what its games share.  The piles without the list's pairs (U1, U2, s1 and
-// s2 bits long), the outer pairs (8 bits each), the cards of the inner ones as bytes.
+// s2 bits long), the outer pairs (8 bits each), the cards of the inner ones as bytes, and where card n-1 is:
+// MTOP_P1 or MTOP_P2 + its place in that pile, MTOP_PAIR + i in outer pair i, MTOP_INNER among the inner cards
+// (of which it is the last).  Cards are the low 4 bits of their values (card 16 of 17 is told by its place).
 struct MUnit {
     u64 U1, U2, O;
-    u32 c0, c1, s1, s2;
+    u32 c0, c1, s1, s2, top;
 };
+constexpr u32 MTOP_INNER = 0, MTOP_PAIR = 32, MTOP_P1 = 64, MTOP_P2 = 128;
 
 // A job's blocks (with the sentinel), units, merged games and rows of a unit.
 struct MergePlan {
@@ -81,14 +84,16 @@ struct MergePlan {
     u32 lc = 0;
 };
 constexpr size_t MERGE_BLOCK_CAP = 512;   // blocks of a range: at most 2 (1 + .. + 16), and the sentinel
-// A launch takes at most this many units: a unit stands for at most 2520 rows x 2^9 deals, and a launch for
-// fewer than 2^38 (a lane's 32-bit turn total is drained with the histograms).
-constexpr u64 MERGE_LAUNCH_UNITS = (1ull << 38) / (2520ull << 9);
+// A launch takes at most this many units: a unit stands for at most 2520 rows x 2^11 deals, and a launch for
+// fewer than 2^40 (a lane's 32-bit turn total is drained with the histograms).
+constexpr u64 MERGE_LAUNCH_UNITS = (1ull << 40) / (2520ull << 11);
 
 void merge_table(int rule, u32* rows);
 void merge_plan(const war_job* job, u64 warps, MergePlan& p);
 cudaError_t launch_merged(const MergeArgs& a, int rule, int threads, int blocks, DevAcc* acc, cudaStream_t st);
 int merged_max_blocks_per_sm(int rule, int threads, int hbins);
+cudaError_t launch_held_merged(const MergeArgs& a, int rule, int threads, int blocks, DevAcc* acc, cudaStream_t st);
+int held_merged_max_blocks_per_sm(int rule, int threads, int hbins);
 
 // Card of rank d among the set bits of m; m loses it.
 __host__ __device__ __forceinline__ u32 take_card(u32& m, u32 d) {
@@ -111,36 +116,40 @@ __host__ __device__ __forceinline__ u32 card_count(u32 m) {
 #endif
 }
 
+__host__ __device__ __forceinline__ u64 merge_shl(u64 x, u32 s) { return s < 64u ? x << s : 0ull; }
+
 // Sets a unit up (every lane of the warp the same): the piles of 4-bit cards after the turns that its fixed and
 // chosen cards decide.
 template <int RULE>
 __host__ __device__ __forceinline__ void merge_unit(const MBlock& B, u64 outer, u32 n, MUnit& m) {
     u32 free = B.free_mask;
-    const u32 b = B.b, f = B.f, fo = f > MERGE_INNER ? f - MERGE_INNER : 0u;
+    const u32 b = B.b, f = B.f, fo = f > MERGE_INNER ? f - MERGE_INNER : 0u, last = n - 1u;
     u64 U1 = 0, U2 = 0;
-    u32 s1 = 0, s2 = 0, half = 0;
+    u32 s1 = 0, s2 = 0, half = 0, top = MTOP_INNER;
     if ((b & 1u) && b < n) {
         const u32 k = card_count(free);
         half = take_card(free, (u32)(outer % k));
         outer /= k;
     }
     if (n & 1u) {   // player 1's last card, unplayed after h turns, is on top
-        u32 top;
-        if (b == n) top = B.prefix[n - 1u];
+        u32 c;
+        if (b == n) c = B.prefix[n - 1u];
         else {
             const u32 k = card_count(free);
-            top = take_card(free, (u32)(outer % k));
+            c = take_card(free, (u32)(outer % k));
             outer /= k;
         }
-        U1 = top;
+        U1 = c & 15u;
         s1 = 4u;
+        if (c == last) top = MTOP_P1;
     }
     for (u32 t = 0; 2u * t < b && 2u * t + 1u < n; t++) {
         const u32 x = B.prefix[2u * t], y = 2u * t + 1u < b ? B.prefix[2u * t + 1u] : half;
         const u32 hi = x > y ? x : y, lo = x > y ? y : x;
-        const u64 pair = RULE ? lo | (hi << 4) : hi | (lo << 4);
-        if (x > y) { U1 |= pair << s1; s1 += 8u; }
-        else { U2 |= pair << s2; s2 += 8u; }
+        const u64 pair = RULE ? lo | ((hi & 15u) << 4) : (hi & 15u) | (lo << 4);
+        if (hi == last) top = x > y ? MTOP_P1 + s1 / 4u + RULE : MTOP_P2 + s2 / 4u + RULE;
+        if (x > y) { U1 |= merge_shl(pair, s1); s1 += 8u; }
+        else { U2 |= merge_shl(pair, s2); s2 += 8u; }
     }
     u64 O = 0;
     for (u32 i = 0; i < fo; i++) {
@@ -149,11 +158,12 @@ __host__ __device__ __forceinline__ void merge_unit(const MBlock& B, u64 outer, 
         outer /= np;
         while (d >= x) { d -= x; x++; }          // the pair of ranks (x, d), x > d
         const u32 hi = take_card(free, x), lo = take_card(free, d);
-        O |= (u64)(RULE ? lo | (hi << 4) : hi | (lo << 4)) << (8u * i);
+        if (hi == last) top = MTOP_PAIR + i;
+        O |= (u64)(RULE ? lo | ((hi & 15u) << 4) : (hi & 15u) | (lo << 4)) << (8u * i);
     }
     u64 c = 0;
-    for (u32 i = 0; free; i++) c |= (u64)take_card(free, 0u) << (8u * i);
-    m.U1 = U1; m.U2 = U2; m.O = O; m.s1 = s1; m.s2 = s2;
+    for (u32 i = 0; free; i++) c |= (u64)(take_card(free, 0u) & 15u) << (8u * i);
+    m.U1 = U1; m.U2 = U2; m.O = O; m.s1 = s1; m.s2 = s2; m.top = top;
     m.c0 = (u32)c; m.c1 = (u32)(c >> 32);
 }
 
@@ -163,6 +173,80 @@ __device__ __forceinline__ u32 merge_row(u32 c0, u32 c1, u32 sel) {
     x |= x >> 4;      // bytes 0 and 2: a card and the next one's nibble
     y |= y >> 4;
     return __byte_perm(x, y, 0x6420);
+}
+
+// A warp's place in its unit: row l of [l0, lend) with pa of the f pairs won by player 1, games that stand for wt
+// deals each.  Histogram bins of a block are 32 bits: a warp empties them into the accumulators (drain) before
+// it has dealt out games that stand for this many deals since it last did.  A bin holds at most what the block's
+// warps dealt out since, so 32 x (2^26 + one unit of at most 2520 rows x 2^11 deals) stays below 2^32.
+constexpr u32 DRAIN_DEALS = 1u << 26;
+
+struct MCursor {
+    u32 l = 0, l0 = 0, lend = 0, pa = 0, f = 0, fi = 0, wt = 0, blk = 0, row0 = 0;
+    u32 given = 0;       // deals dealt out since the last drain
+    u64 done = 0;        // deals counted by this warp
+    bool filter = false, dry = false;
+};
+
+// Deals the warp's next games to the lanes that want one; called by the whole warp.
+//   setup(B, outer)   sets the unit up for the warp
+//   over()            whether one player won every pair of the unit's games with c.pa (1: player 1, 2: player 2)
+//   ended(count)      counts `count` deals that are over at turn h
+//   build(selectors)  the lane's game from a table row; false if it is not played (filter)
+//   drain()           empties the histograms
+template <class Setup, class Over, class Ended, class Build, class Drain>
+__device__ __forceinline__ u32 merge_deal(MCursor& c, const MergeArgs& a, u64* counter, bool want, Setup setup,
+                                          Over over, Ended ended, Build build, Drain drain) {
+    const u32 lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    u32 need = __ballot_sync(WAR_FULL_MASK, want), served = 0;
+    while (need && !c.dry) {
+        if (c.l == c.lend) {
+            if (c.pa < c.f) {
+                c.pa++;
+                c.wt = c.wt * (c.f - c.pa + 1u) / c.pa;
+                c.l = c.l0;
+            } else {
+                u64 u = 0;
+                if (lane == 0u) u = atomicAdd(counter, 1ull);
+                u = __shfl_sync(WAR_FULL_MASK, u, 0) + a.unit_lo;
+                if (u >= a.unit_hi) { c.dry = true; break; }
+                while (u >= a.blocks[c.blk + 1u].u0) c.blk++;
+                const MBlock& B = a.blocks[c.blk];
+                const u64 v = u - B.u0, outer = v / B.nch;
+                setup(B, outer);
+                c.f = B.f;
+                c.fi = min(c.f, MERGE_INNER);
+                c.row0 = merge_row0(c.fi);
+                c.l0 = (u32)(v - outer * B.nch) * a.lc;
+                c.lend = min(merge_rows(c.fi), c.l0 + a.lc);
+                c.l = c.l0;
+                c.pa = 0;
+                c.wt = B.twice ? 2u : 1u;
+                c.filter = B.filter != 0;
+                if (c.given > DRAIN_DEALS) { drain(); c.given = 0; }
+            }
+            const u32 o = over();
+            if (o) {
+                if (o == 1u || !c.filter) {   // (card n-1 is with the player who won every pair)
+                    const u32 k = (c.lend - c.l) * c.wt;
+                    ended(k);
+                    c.done += k; c.given += k;
+                }
+                c.l = c.lend;
+            }
+            continue;
+        }
+        const u32 r = __popc(need & below), take = min((u32)__popc(need), c.lend - c.l);
+        bool mine = ((need >> lane) & 1u) && r < take;
+        if (mine) mine = build(__ldg(a.table + c.row0 + c.l + r));
+        const u32 got = __ballot_sync(WAR_FULL_MASK, mine);
+        need &= ~got;
+        served |= got;
+        const u32 k = (u32)__popc(got) * c.wt;
+        c.done += k; c.given += k;
+        c.l += take;
+    }
+    return served;
 }
 
 }  // namespace war

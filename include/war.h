@@ -218,7 +218,9 @@ typedef struct war_job_status {
  * fastest), 1 = multiply-adds on separate counts, 2 = packed counts in logic/shift form, 3 = the plain
  * branching turn of gpu/war17.py; bit 2 = the path memo with memo_bits (0 = 28), at most 512 threads then;
  * bit 3 = test Brent's checkpoint after every turn (by default it is saved at the services whenever the
- * window is a multiple of the service period).  NULL = defaults (no memo).  war_enumerate sends n = 17 deal
+ * window is a multiple of the service period).  Variant 0 then plays merged games, each state after the deals'
+ * first floor(n/2) turns once (block_m does not apply), with the same results, `turns` included.  NULL = defaults
+ * (no memo).  war_enumerate sends n = 17 deal
  * jobs here. */
 int war_enumerate_held(const war_job* job, const war_tune* tune, war_result* out);
 

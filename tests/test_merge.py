@@ -155,3 +155,23 @@ def test_merged_table_kept_between_ranges_of_different_sizes(wl):
     for flags, lo, hi in jobs:
         job = wl.make_job(13, flags=flags, lo=lo, hi=hi, hbins=128)
         same(wl, wl.enumerate_job(job, t), wl.enumerate_plain(wl.make_job(13, lo=lo, hi=hi, hbins=128)), (lo, hi))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rule", [0, 1])
+def test_held_merged_games_and_turns(wl, rule):
+    """The held-out-card engine's default turn (merged games) against its turn that plays every deal (variant 8):
+    counts, lengths and the turns that playing every deal takes, with windows around the merged turns and around
+    the cycle lengths of small decks (a deal on its own cycle is decided earlier than the rest of its game)."""
+    keys = KEYS + ("turns",)
+    rnd = random.Random(rule)
+    for n in list(range(2, 12)) + [13, 14, 16, 17, 17]:
+        total = math.factorial(n)
+        lo = 0 if n < 10 else rnd.randrange(0, total - 300000)
+        job = wl.make_job(n, rule=rule, lo=lo, hi=total if n < 10 else lo + 300000, hbins=128)
+        for kw in (dict(), dict(window=16, defer=16, threads=128), dict(window=8, defer=4), dict(window=4, defer=4),
+                   dict(window=64, defer=32, threads=1024)):
+            got = wl.to_dict(wl.enumerate_held(job, wl.make_tune(**kw)))
+            want = wl.to_dict(wl.enumerate_held(job, wl.make_tune(variant=8, **kw)))
+            for k in keys:
+                assert got[k] == want[k], (n, kw, k)
