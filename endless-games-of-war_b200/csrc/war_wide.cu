@@ -30,6 +30,7 @@
 #include <mutex>
 #include "war_kernels.cuh"
 #include "war_host.h"
+#include "war_merge.cuh"
 
 namespace war {
 
@@ -135,10 +136,8 @@ __device__ __forceinline__ bool wide_heap_step(WEnum& E) {
     return true;
 }
 
-// SVC (Brent only): W is a multiple of the service period, so an undecided game (which starts at a service and
-// plays `period` turns between services) reaches each tortoise checkpoint W, 3W, 7W, ... exactly at a service,
-// and the checkpoint is saved there instead of being tested after every turn.
-template <int RULE, int DET, bool SVC>
+// One game per deal: the streak test, and Brent and Floyd where their games cannot be merged (below).
+template <int RULE, int DET>
 __global__ void __launch_bounds__(1024) wide_kernel(const __grid_constant__ WideArgs a, DevAcc* __restrict__ acc) {
     extern __shared__ u32 sh[];
     u32* shh = sh;                    // cycle-length histogram (Brent)
@@ -231,13 +230,10 @@ __global__ void __launch_bounds__(1024) wide_kernel(const __grid_constant__ Wide
                 const u32 kk = en ? (u32)K_END : (cy ? (u32)K_CYC : (r1 > cap ? (u32)K_UND : (u32)K_NONE));
                 rounds = open ? r1 : rounds;
                 kind = open ? kk : kind;
-                if (!SVC && open && kk == K_NONE && r1 == next) {   // Brent: tortoise saved at W, 3W, 7W, ...
+                if (open && kk == K_NONE && r1 == next) {   // Brent: tortoise saved at W, 3W, 7W, ...
                     t0 = a0; t1 = a1; t2 = b0; t3 = b1; next = 2u * next + W;
                 }
             }
-        }
-        if (DET == DET_BRENT && SVC && kind == K_NONE && rounds == next) {   // the checkpoint, at the service
-            t0 = a0; t1 = a1; t2 = b0; t3 = b1; next = 2u * next + W;
         }
         // service: record every decided game, refill its lane
         const bool fin = active & (kind != K_NONE);
@@ -276,27 +272,410 @@ __global__ void __launch_bounds__(1024) wide_kernel(const __grid_constant__ Wide
     flush_hist(she, acc->endhist, WAR_EBINS);
 }
 
-typedef void (*WideFn)(const WideArgs, DevAcc*);
+// ---- merged games (war_merge.cuh) -----------------------------------------------------------------------
+//
+// wide_kernel plays every deal; this kernel plays each state after the deals' first h = floor(n/2) turns once,
+// under any detector, and counts it for all its deals.
+//
+// `turns` stays what playing every deal gives.  Floyd meets at the first multiple of the cycle length that is no
+// earlier than the cycle, the same turn for a deal on its own cycle (a cycle is longer than h turns), so the
+// tortoise waits at turn h until the hare is at turn 2h and both go on from there.  Brent's checkpoints W, 3W, ..
+// (all at or after turn h) decide all deals of a game at the same turn; a deal on its own cycle of length
+// lam <= W is decided at turn lam by the checkpoint at turn 0 instead, and wide_start finds the one that is.
+// With the tortoise at the state of turn h until turn W, a game on such a cycle is known at turn h + lam and
+// counted as decided at W + lam.
+//
+// The streak test (odd n, winner's card first) needs no anchor of its own here.  The piles' sizes change parity
+// every turn, so "the next winner holds an even number of cards" stays true, or stays false, as long as the
+// players alternate, and flips at every turn that the same player wins again (a break).  The test's anchor is
+// therefore the first turn of an alternating run in which it is true, and its period lcm(n+1, W, L-1) is the
+// same all along the run.  While the players alternate a turn can be undone (the winner is known, and its pair
+// is at the bottom of its pile), so a run that reaches its cycle was on it from its first turn, and the test
+// succeeds at the first try: at the run's first turn + the period.  The kernel keeps the turn of the last break,
+// saves the tortoise at the first service after it, finds the cycle one cycle length later and counts that turn.
+// Where there was no break after turn h, the run began before it, for each deal of the game at its own turn:
+// wide_streak_head sums those up.  (A cycle with breaks, or one in which the condition is false, is one that the
+// test never finds: undetermined.)
+//
+// The step cap must not fall before the turns that are not played: at least 2W (Brent), 2h + 2 (Floyd), h + the
+// longest period (streak).
+//
+// What bounds it: instruction issue of the turns, as before; the gain is the deals per game (3.2 in a block of 9!
+// deals of 18 cards, 5.3 in one of 11!) and, in short jobs, units that a whole warp plays instead of one lane.
+// B200: 5e7 deals of 18 cards under Brent 45 -> 2.4 ms, 2e8 of 17 under the streak test 125 -> 16.8 ms (which also
+// plays one cycle length after the last break instead of the period); 256 or 512 threads alike, defer 16 (8: 2.5
+// and 17.8 ms, 32: 2.6 and 17.6 ms).
 
-static WideFn wide_pick(int det, int rule, bool svc) {
-    if (det == DET_FLOYD) return rule ? wide_kernel<1, DET_FLOYD, false> : wide_kernel<0, DET_FLOYD, false>;
-    if (det == DET_STREAK) return wide_kernel<0, DET_STREAK, false>;
-    if (svc) return rule ? wide_kernel<1, DET_BRENT, true> : wide_kernel<0, DET_BRENT, true>;
-    return rule ? wide_kernel<1, DET_BRENT, false> : wide_kernel<0, DET_BRENT, false>;
+// The outer choice of a unit (MUnit with 5-bit cards and 128-bit piles): the outer pairs have 10 bits each.
+struct WUnit {
+    u64 U1l, U1h, U2l, U2h, O;
+    u32 c0, c1, s1, s2;
+    u32 wins;          // bit t: player 1 wins turn t (turns of the fixed cards)
+};
+
+__device__ __forceinline__ void shl128(u64& lo, u64& hi, u32 s) {   // 0 <= s < 128
+    hi = shl64(hi, s) | shl64(lo, s - 64u) | shr64(lo, 64u - s);
+    lo = shl64(lo, s);
+}
+__device__ __forceinline__ void shr128(u64& lo, u64& hi, u32 s) {
+    lo = shr64(lo, s) | shr64(hi, s - 64u) | shl64(hi, 64u - s);
+    hi = shr64(hi, s);
+}
+__device__ __forceinline__ void put128(u64& lo, u64& hi, u64 v, u32 s) {
+    lo |= shl64(v, s);
+    hi |= shl64(v, s - 64u) | (s < 64u ? shr64(v, 64u - s) : 0ull);
 }
 
-// Brent's checkpoints fall on services when W is a multiple of the service period.
-static bool wide_svc(int W, int defer) {
+template <int RULE>
+__device__ __forceinline__ void wide_unit(const MBlock& B, u64 outer, u32 n, WUnit& m) {
+    u32 free = B.free_mask;
+    const u32 b = B.b, f = B.f, fo = f > MERGE_INNER ? f - MERGE_INNER : 0u;
+    m.U1l = m.U1h = m.U2l = m.U2h = m.O = 0ull;
+    u32 s1 = 0, s2 = 0, half = 0, wins = 0;
+    if ((b & 1u) && b < n) {
+        const u32 k = (u32)__popc(free);
+        half = take_card(free, (u32)(outer % k));
+        outer /= k;
+    }
+    if (n & 1u) {   // player 1's last card, unplayed after h turns, is on top
+        if (b == n) m.U1l = B.prefix[n - 1u];
+        else {
+            const u32 k = (u32)__popc(free);
+            m.U1l = take_card(free, (u32)(outer % k));
+            outer /= k;
+        }
+        s1 = 5u;
+    }
+    for (u32 t = 0; 2u * t < b && 2u * t + 1u < n; t++) {
+        const u32 x = B.prefix[2u * t], y = 2u * t + 1u < b ? B.prefix[2u * t + 1u] : half;
+        const u32 hi = max(x, y), lo = min(x, y);
+        const u64 pair = RULE ? lo | (hi << 5) : hi | (lo << 5);
+        if (x > y) { put128(m.U1l, m.U1h, pair, s1); s1 += 10u; wins |= 1u << t; }
+        else { put128(m.U2l, m.U2h, pair, s2); s2 += 10u; }
+    }
+    for (u32 i = 0; i < fo; i++) {
+        const u32 k = (u32)__popc(free), np = k * (k - 1u) / 2u;
+        u32 d = (u32)(outer % np), x = 1;
+        outer /= np;
+        while (d >= x) { d -= x; x++; }
+        const u32 hi = take_card(free, x), lo = take_card(free, d);
+        m.O |= (u64)(RULE ? lo | (hi << 5) : hi | (lo << 5)) << (10u * i);
+    }
+    u64 c = 0;
+    for (u32 i = 0; free; i++) c |= (u64)take_card(free, 0u) << (8u * i);
+    m.s1 = s1; m.s2 = s2; m.wins = wins;
+    m.c0 = (u32)c; m.c1 = (u32)(c >> 32);
+}
+
+// The pairs of a table row as 10-bit pairs of 5-bit cards.
+__device__ __forceinline__ u64 wide_row(u32 c0, u32 c1, u32 sel) {
+    u32 x = __byte_perm(c0, c1, sel), y = __byte_perm(c0, c1, sel >> 16);
+    x = (x & 0x001F001Fu) | ((x >> 3) & 0x03E003E0u);   // bits 0..9 and 16..25: a pair each
+    y = (y & 0x001F001Fu) | ((y >> 3) & 0x03E003E0u);
+    x = (x & 0x3FFu) | ((x >> 6) & 0xFFC00u);
+    y = (y & 0x3FFu) | ((y >> 6) & 0xFFC00u);
+    return (u64)x | ((u64)y << 20);
+}
+
+// The start of a lane's game, kept for wide_start, and its block.
+struct WideStart {
+    u64 a0, a1, b0, b1;
+    u32 la, blk;
+};
+
+// How many deals of the game that is at x at turn h lie on their own cycle of length lam (held_start of
+// war_held.cu): 0, or 1 (2 with its mirror image).
+template <int RULE>
+__device__ __noinline__ u32 wide_start(const WideStart x, const MBlock* __restrict__ blocks, u32 n, u32 lam) {
+    const u32 h = n >> 1;
+    u64 a0 = x.a0, a1 = x.a1, b0 = x.b0, b1 = x.b1, d0 = 0, d1 = 0, e0 = 0, e1 = 0;
+    u32 la = x.la, dla = 0;
+    for (u32 t = 0; t < lam; t++) {
+        if (t == lam - h) { d0 = a0; d1 = a1; e0 = b0; e1 = b1; dla = la; }
+        turn5<RULE>(a0, a1, b0, b1, la, n - 1u);
+    }
+    if (a0 != x.a0 || a1 != x.a1 || b0 != x.b0 || b1 != x.b1) return 0u;   // x is not on the cycle
+    if (dla != (n + 1u) >> 1) return 0u;                                   // not as dealt
+    const MBlock& B = blocks[x.blk];
+    for (u32 i = 0; i < B.b; i++) {
+        u64 lo = i & 1u ? e0 : d0, hi = i & 1u ? e1 : d1;
+        shr128(lo, hi, 5u * (i >> 1));
+        if (((u32)lo & 31u) != B.prefix[i]) return 0u;
+    }
+    return B.twice ? 2u : 1u;
+}
+
+// Turns before turn h that belong to the alternating run at turn h, summed over the deals of a game whose free
+// pairs are won `a` times by player 1: the deals in which every turn from r on (r < h) has the winner who holds
+// an even number of cards, for each r.  wins: the winners of the first p turns.
+__device__ __noinline__ u32 wide_streak_head(u32 n, u32 a, u32 p, u32 wins) {
+    const u32 h = n >> 1, lenA = (n + 1u) / 2u;
+    u32 sum = 0;
+    int r = (int)h - 1;
+    for (; r >= (int)p; r--) {
+        if (((lenA + (u32)r) & 1u) == 0u) {       // player 1's pile is the even one
+            if (a == 0u) return sum;
+            a--;
+        }
+        const u32 rem = (u32)r - p;               // turns of free pairs before r, a of them won by player 1
+        if (a > rem) return sum;
+        u32 c = 1;
+        for (u32 i = 1; i <= a; i++) c = c * (rem - a + i) / i;
+        sum += c;
+    }
+    for (; r >= 0 && a == 0u; r--) {
+        if (((wins >> r) & 1u) == ((lenA + (u32)r) & 1u)) return sum;
+        sum++;
+    }
+    return sum;
+}
+
+// What the kernel needs besides MergeArgs: the step cap, and the streak periods by the next winner's pile.
+struct WideMore {
+    u32 cap;
+    u32 slack;       // streak: turns past the cap after which an undecided game is undetermined for certain
+    u32 lamtab[32];
+};
+
+template <int RULE, int DET>
+__global__ void __launch_bounds__(1024) wide_merge_kernel(const __grid_constant__ MergeArgs a,
+                                                          const __grid_constant__ WideMore more,
+                                                          DevAcc* __restrict__ acc) {
+    extern __shared__ u64 sh64[];
+    __shared__ WUnit units[32];
+    WideStart* const start = (WideStart*)sh64 + threadIdx.x;                     // Brent only
+    u32* const head = (u32*)sh64 + threadIdx.x;                                  // streak only: a, p and wins
+    u32* const shh = DET == DET_BRENT ? (u32*)((WideStart*)sh64 + blockDim.x)
+                                      : (u32*)sh64 + (DET == DET_STREAK ? blockDim.x : 0u);
+    u32* const she = shh + a.hbins;
+    const int bins = a.hbins + WAR_EBINS;
+    for (int b = threadIdx.x; b < bins; b += blockDim.x) shh[b] = 0;
+    __syncthreads();
+
+    const u32 n = (u32)a.n, n1 = n - 1u, h = n >> 1, W = (u32)a.W;
+    const u32 hb1 = a.hbins > 0 ? (u32)(a.hbins - 1) : 0u;
+    const u32 period = a.defer > 4 ? (u32)((a.defer + 3) & ~3) : 4u;
+    const u32 after = DET == DET_BRENT ? h % period : 0u, before = period - after;   // turns around the checkpoint
+    const u32 cap = more.cap + (DET == DET_STREAK ? more.slack : 0u);
+    const u32 lane = threadIdx.x & 31u;
+    WUnit& mu = units[threadIdx.x >> 5];
+    u64* const counter = &acc->work_next;
+
+    u64 a0 = 1, a1 = 0, b0 = 1, b1 = 0, t0 = ~0ull, t1 = 0, t2 = 0, t3 = 0, turns = 0;
+    u32 la = 0, tla = 0, rounds = 0, next = 0xFFFFFFFFu, wt = 0, kind = K_END;
+    u32 run = 0, save = 0, prev = 2u;    // streak: turn of the last break, turn of the tortoise, last winner
+    bool active = false;
+    u32 cyc = 0, maxfin = 0, und = 0;
+    MCursor c;
+
+    auto drain = [&]() {
+        __syncwarp();
+        for (int b = (int)lane; b < bins; b += 32) {
+            const u32 v = atomicExch(&shh[b], 0u);
+            if (v) atomicAdd(b < a.hbins ? &acc->hist[b] : &acc->endhist[b - a.hbins], (u64)v);
+        }
+        const u64 v_cyc = warp_sum((u64)cyc), v_und = warp_sum((u64)und);
+        if (lane == 0u) {
+            if (v_cyc) atomicAdd(&acc->cyc, v_cyc);
+            if (v_und) atomicAdd(&acc->undetermined, v_und);
+        }
+        cyc = 0; und = 0;
+    };
+    auto setup = [&](const MBlock& B, u64 outer) {
+        WUnit m;
+        wide_unit<RULE>(B, outer, n, m);
+        __syncwarp();
+        if (lane == 0u) mu = m;
+        __syncwarp();
+    };
+    auto over = [&]() -> u32 {
+        return mu.s2 + 10u * (c.f - c.pa) == 0u ? 1u : (mu.s1 + 10u * c.pa == 0u ? 2u : 0u);
+    };
+    auto ended = [&](u32 k) {
+        if (lane == 0u) { atomicAdd(&she[h], k); turns += (u64)k * h; }
+        maxfin = max(maxfin, h);
+    };
+    auto build = [&](u32 sel) -> bool {
+        const u32 a10 = 10u * c.pa;
+        const u64 in = wide_row(mu.c0, mu.c1, sel);
+        u64 xl = mu.O, xh = 0;
+        put128(xl, xh, in, 10u * (c.f - c.fi));
+        u64 yl = xl, yh = xh;
+        xl &= ~shl64(~0ull, a10);
+        xh &= a10 > 64u ? ~shl64(~0ull, a10 - 64u) : 0ull;
+        shl128(xl, xh, mu.s1);
+        shr128(yl, yh, a10);
+        shl128(yl, yh, mu.s2);
+        a0 = xl | mu.U1l; a1 = xh | mu.U1h;
+        b0 = yl | mu.U2l; b1 = yh | mu.U2h;
+        la = mu.s1 / 5u + 2u * c.pa;
+        if (c.filter) {   // player 1 must hold card n - 1
+            bool has = false;
+            u64 lo = a0, hi = a1;
+            for (u32 i = 0; i < la; i++) {
+                has |= ((u32)lo & 31u) == n1;
+                shr128(lo, hi, 5u);
+            }
+            if (!has) return false;
+        }
+        put128(a0, a1, 1ull, 5u * la);
+        put128(b0, b1, 1ull, 5u * (n - la));
+        rounds = h; kind = K_NONE; wt = c.wt; active = true;
+        t0 = a0; t1 = a1; t2 = b0; t3 = b1; tla = la;
+        next = W > h ? W : 3u * W;   // (W = h: the tortoise of turn W)
+        if (DET == DET_BRENT) {
+            WideStart x;
+            x.a0 = a0; x.a1 = a1; x.b0 = b0; x.b1 = b1; x.la = la; x.blk = c.blk;
+            *start = x;
+        } else if (DET == DET_STREAK) {
+            run = h; save = h; prev = 2u;
+            *head = c.pa | ((h - c.f) << 8) | (mu.wins << 16);
+        } else if (h & 1u) {         // the hare's turns come in pairs from turn 0
+            turn5<RULE>(a0, a1, b0, b1, la, n1);
+            rounds = h + 1u;
+            if ((la == 0u) | (la == n)) kind = K_END;
+        }
+        return true;
+    };
+    auto refill = [&](bool want) {
+        if (want) { active = false; kind = K_END; }
+        merge_deal(c, a, counter, want, setup, over, ended, build, drain);
+    };
+    auto turn = [&]() {
+        const bool open = kind == K_NONE;
+        if (DET == DET_FLOYD) {
+            turn5<RULE>(a0, a1, b0, b1, la, n1);
+            const bool e1 = (la == 0u) | (la == n);
+            turn5<RULE>(a0, a1, b0, b1, la, n1);
+            const bool e2 = (la == 0u) | (la == n);
+            const u32 r2 = rounds + (e1 ? 1u : 2u);
+            if (r2 > 2u * h) turn5<RULE>(t0, t1, t2, t3, tla, n1);
+            const bool cy = (a0 == t0) & (a1 == t1) & (b0 == t2) & (b1 == t3);
+            const u32 kk = (e1 | e2) ? (u32)K_END : (cy ? (u32)K_CYC : (r2 > cap ? (u32)K_UND : (u32)K_NONE));
+            rounds = open ? r2 : rounds;
+            kind = open ? kk : kind;
+        } else {
+            const u32 w = turn5<RULE>(a0, a1, b0, b1, la, n1) ? 1u : 0u;
+            if (DET == DET_STREAK) {
+                run = open & (w == prev) ? rounds : run;
+                prev = open ? w : prev;
+            }
+            const u32 r1 = rounds + 1u;
+            const bool en = (la == 0u) | (la == n);
+            const bool cy = (a0 == t0) & (a1 == t1) & (b0 == t2) & (b1 == t3);
+            const u32 kk = en ? (u32)K_END : (cy ? (u32)K_CYC : (r1 > cap ? (u32)K_UND : (u32)K_NONE));
+            rounds = open ? r1 : rounds;
+            kind = open ? kk : kind;
+        }
+    };
+
+    refill(true);
+    bool running = __any_sync(WAR_FULL_MASK, active);
+    while (running) {
+        for (u32 k = 0; k < before; k++) turn();
+        if (DET == DET_BRENT) {
+            if (kind == K_NONE && rounds == next) { t0 = a0; t1 = a1; t2 = b0; t3 = b1; next = 2u * next + W; }
+            for (u32 k = 0; k < after; k++) turn();
+        }
+        if (DET == DET_STREAK && kind == K_NONE && run > save) { t0 = a0; t1 = a1; t2 = b0; t3 = b1; tla = la; save = rounds; }
+        const bool fin = active & (kind != K_NONE);
+        if (__any_sync(WAR_FULL_MASK, fin)) {
+            if (fin) {
+                u32 t = rounds;
+                if (DET == DET_STREAK) {   // (what is decided by turn cap + 1 is decided, wide_kernel)
+                    if (kind == K_CYC) {
+                        // the piles are the tortoise's: the next winner's pile and the period are the run's
+                        const u32 ws = ((u32)t0 & 31u) > ((u32)t2 & 31u) ? tla : n - tla;
+                        const u32 lam = more.lamtab[ws & 31u];
+                        if (run > save || lam == 0u || lam % (rounds - save) != 0u || run + lam > more.cap + 1u)
+                            kind = K_UND;
+                        else {
+                            t = run + lam;
+                            if (run == h) turns -= wide_streak_head(n, *head & 255u, (*head >> 8) & 255u, *head >> 16);
+                        }
+                    }
+                    if (kind == K_UND || (kind == K_END && rounds > more.cap + 1u)) { kind = K_UND; t = more.cap + 1u; }
+                }
+                if (kind == K_CYC) {
+                    cyc += wt;
+                    if (DET == DET_BRENT) {
+                        // next = W: found with the tortoise at turn h, else at turn (next - W) / 2
+                        const u32 at = next == W ? h : (next - W) >> 1, lam = rounds - at;
+                        if (a.hbins) atomicAdd(&shh[lam < hb1 ? lam : hb1], wt);
+                        if (next == W) t = W + lam;
+                        if (lam <= W && at <= W) turns -= (u64)wide_start<RULE>(*start, a.blocks, n, lam) * (t - lam);
+                    }
+                } else if (kind == K_END) {
+                    maxfin = max(maxfin, rounds);
+                    atomicAdd(&she[rounds < WAR_EBINS - 1 ? rounds : WAR_EBINS - 1], wt);
+                } else {
+                    und += wt;
+                }
+                turns += (u64)wt * t;
+            }
+            refill(fin);
+            running = __any_sync(WAR_FULL_MASK, active);
+        }
+    }
+
+    const u64 v_cyc = warp_sum((u64)cyc), v_turns = warp_sum(turns), v_max = warp_max((u64)maxfin);
+    const u64 v_und = warp_sum((u64)und);
+    if (lane == 0u) {
+        if (c.done) atomicAdd(&acc->done, c.done);
+        if (v_cyc) atomicAdd(&acc->cyc, v_cyc);
+        if (v_turns) atomicAdd(&acc->turns, v_turns);
+        if (v_max) atomicMax(&acc->maxfin, v_max);
+        if (v_und) atomicAdd(&acc->undetermined, v_und);
+    }
+    __syncthreads();
+    flush_hist(shh, acc->hist, a.hbins);
+    flush_hist(she, acc->endhist, WAR_EBINS);
+}
+
+typedef void (*WideMergeFn)(const MergeArgs, const WideMore, DevAcc*);
+
+static WideMergeFn wide_merge_pick(int det, int rule) {
+    if (det == DET_STREAK) return wide_merge_kernel<0, DET_STREAK>;
+    if (det == DET_FLOYD) return rule ? wide_merge_kernel<1, DET_FLOYD> : wide_merge_kernel<0, DET_FLOYD>;
+    return rule ? wide_merge_kernel<1, DET_BRENT> : wide_merge_kernel<0, DET_BRENT>;
+}
+
+static size_t wide_merge_shmem(int det, int threads, int hbins) {
+    return sizeof(u32) * (size_t)(hbins + WAR_EBINS) +
+           (det == DET_BRENT ? sizeof(WideStart) : det == DET_STREAK ? sizeof(u32) : 0) * (size_t)threads;
+}
+
+// Merged games need every checkpoint after turn 0 at or after turn h and at the service period's multiples (Brent),
+// and the cap at or after the turns that are not played (above).
+static bool wide_merged(int det, int n, int W, int defer, u32 cap, const u32* lamtab) {
     const int period = defer > 4 ? (defer + 3) & ~3 : 4;
-    return W % period == 0;
+    if (det == DET_STREAK) return cap >= (u32)n / 2u + *std::max_element(lamtab, lamtab + 32);
+    if (det == DET_FLOYD) return cap >= (u32)n + 2u;
+    return det == DET_BRENT && W % period == 0 && W >= n / 2 && cap >= 2u * (u32)W;
+}
+
+typedef void (*WideFn)(const WideArgs, DevAcc*);
+
+static WideFn wide_pick(int det, int rule) {
+    if (det == DET_FLOYD) return rule ? wide_kernel<1, DET_FLOYD> : wide_kernel<0, DET_FLOYD>;
+    if (det == DET_STREAK) return wide_kernel<0, DET_STREAK>;
+    return rule ? wide_kernel<1, DET_BRENT> : wide_kernel<0, DET_BRENT>;
 }
 
 static size_t wide_shmem(int hbins) { return sizeof(u32) * (size_t)(hbins + WAR_EBINS + 32); }
 
-static int wide_max_blocks(int det, int rule, bool svc, int threads, int hbins) {
+static int wide_max_blocks(int det, int rule, int threads, int hbins) {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, wide_pick(det, rule, svc), threads, wide_shmem(hbins)) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, wide_pick(det, rule), threads, wide_shmem(hbins)) !=
         cudaSuccess)
+        return 0;
+    return nb;
+}
+
+static int wide_merge_max_blocks(int det, int rule, int threads, int hbins) {
+    int nb = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, wide_merge_pick(det, rule), threads,
+                                                      wide_merge_shmem(det, threads, hbins)) != cudaSuccess)
         return 0;
     return nb;
 }
@@ -341,12 +720,34 @@ extern "C" int war_enumerate_wide(const war_job* job, const war_wide_cfg* cfg, w
     if (job->lo == job->hi) return WAR_OK;
     int st;
     if ((st = ensure_ready())) return st;
-    const bool svc = wide_svc(W, defer);
-    const int maxb = wide_max_blocks(c.det, job->rule, svc, threads, hbins);
+    WideMore more;
+    memset(&more, 0, sizeof more);
+    more.cap = cap;
+    for (int ws = 2; ws + 2 <= job->n; ws += 2) {   // gpu/war24.py:109: lcm(n+1, lcm(W, L-1))
+        auto gcd = [](u64 x, u64 y) { while (y) { u64 t = x % y; x = y; y = t; } return x; };
+        const u64 l1 = (u64)ws / gcd(ws, job->n - ws - 1) * (u64)(job->n - ws - 1);
+        more.lamtab[ws] = (u32)((u64)(job->n + 1) / gcd(job->n + 1, l1) * l1);
+    }
+    more.slack = *std::max_element(more.lamtab, more.lamtab + 32) + 64u;
+    const bool merged = wide_merged(c.det, job->n, W, defer, cap, more.lamtab);
+    const int maxb = merged ? wide_merge_max_blocks(c.det, job->rule, threads, hbins)
+                            : wide_max_blocks(c.det, job->rule, threads, hbins);
     if (maxb < 1) return fail(WAR_EINVAL, "launch shape threads=%d does not fit an SM", threads);
     const int bps = c.blocks_per_sm ? std::min(c.blocks_per_sm, maxb) : maxb;
     std::lock_guard<std::mutex> lk(ctx().mu);
     Ctx& cx = ctx();
+    if (merged) {
+        MergePlan p;
+        const int blocks = bps * cx.sm_count;
+        merge_plan(job, (u64)blocks * (u64)(threads / 32), p);
+        MergeArgs m;
+        if ((st = merge_args(job, p, hbins, W, defer, m))) return st;
+        return run_merged(p, m, hbins, out, [&](cudaStream_t x) {
+            wide_merge_pick(c.det, job->rule)<<<blocks, threads, wide_merge_shmem(c.det, threads, hbins), x>>>(m, more, cx.d_acc);
+            note_launch();
+            return cudaGetLastError();
+        });
+    }
     Plan p;
     make_plan(job, block_m, p);
     if (p.extra.size() > Ctx::UNIT_CAP) return fail(WAR_EINVAL, "plan has %zu extra units", p.extra.size());
@@ -361,15 +762,11 @@ extern "C" int war_enumerate_wide(const war_job* job, const war_wide_cfg* cfg, w
     for (int i = 1; i <= 20; i++) a.fact[i] = a.fact[i - 1] * (u64)i;
     a.n = job->n; a.m = block_m; a.rule = job->rule; a.hbins = hbins; a.W = W; a.defer = defer; a.cap = cap;
     a.units = cx.d_units;
-    for (int ws = 2; ws + 2 <= job->n; ws += 2) {   // gpu/war24.py:109: lcm(n+1, lcm(W, L-1))
-        auto gcd = [](u64 x, u64 y) { while (y) { u64 t = x % y; x = y; y = t; } return x; };
-        const u64 l1 = (u64)ws / gcd(ws, job->n - ws - 1) * (u64)(job->n - ws - 1);
-        a.lamtab[ws] = (u32)((u64)(job->n + 1) / gcd(job->n + 1, l1) * l1);
-    }
+    memcpy(a.lamtab, more.lamtab, sizeof a.lamtab);
     // each launch plays fewer than 2^32 - 2^24 games (32-bit per-lane counters)
     const u64 per_unit = a.fact[block_m];
     const u64 max_units = std::max<u64>(1, ((1ull << 32) - (1ull << 24)) / per_unit);
-    const WideFn fnp = wide_pick(c.det, job->rule, svc);
+    const WideFn fnp = wide_pick(c.det, job->rule);
     const size_t shmem = wide_shmem(hbins);
     u64 done_main = 0;
     bool extras_done = p.extra.empty();

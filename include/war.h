@@ -229,7 +229,9 @@ int war_enumerate_held(const war_job* job, const war_tune* tune, war_result* out
  * one that measures cycle lengths for job.hbins), WAR_DET_FLOYD (gpu/war24.py:85-97) or WAR_DET_STREAK (odd n
  * and rule 0 only: the players alternate for lcm(n+1, W, L-1) turns from an anchor, gpu/war24.py:98-125).  A
  * game still undecided after `cap` turns counts in war_result.undetermined instead of cyc or the ending
- * counts (gpu/war24.py:57).  All zero fields take defaults. */
+ * counts (gpu/war24.py:57).  All zero fields take defaults.  Deals whose first turns lead to one state are played
+ * as one game (`turns` and all counts are those of playing every deal; block_m does not apply) unless the cap is
+ * below the turns that this leaves out, or Brent's window is below n/2 or no multiple of the service period. */
 enum war_det { WAR_DET_BRENT = 0, WAR_DET_FLOYD = 1, WAR_DET_STREAK = 2 };
 typedef struct war_wide_cfg {
     int32_t det;           /* war_det */

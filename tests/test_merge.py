@@ -175,3 +175,50 @@ def test_held_merged_games_and_turns(wl, rule):
             want = wl.to_dict(wl.enumerate_held(job, wl.make_tune(variant=8, **kw)))
             for k in keys:
                 assert got[k] == want[k], (n, kw, k)
+
+
+def ojob(oracle, job):
+    return oracle.make_job(job.n, 0, job.rule, 0, job.lo, job.hi, job.hbins)
+
+
+WIDE_KEYS = KEYS + ("turns", "undetermined")
+
+
+def same_wide(wl, oracle, job, det, window, cap, kw):
+    got = wl.to_dict(wl.enumerate_wide(job, det, cap=cap, **kw))
+    want = oracle.to_dict(oracle.war24(ojob(oracle, job), det, window, cap or 1 << 22))
+    for k in WIDE_KEYS:
+        assert got[k] == want[k], (job.n, job.rule, det, window, cap, kw, k, got[k], want[k])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", range(2, 12))
+def test_wide_merged_small(wl, oracle, n):
+    """The 5-bit engine's merged games, every deal of n <= 11: counts, turns and undetermined games equal the
+    oracle's under every detector, with windows, service periods and step caps at the edges of the rule."""
+    for rule in (0, 1):
+        job = wl.make_job(n, rule=rule, hbins=256)
+        for window, cap, kw in ((32, 0, {}), (16, 0, dict(window=16, defer=4)), (32, 64, {}), (32, 63, {}),
+                                (8, 0, dict(window=8, defer=8, threads=128)), (4, 0, dict(window=4, defer=4)),
+                                (64, 0, dict(window=64, defer=64, threads=1024))):
+            same_wide(wl, oracle, job, wl.DET_BRENT, window, cap, kw)
+        job = wl.make_job(n, rule=rule)
+        for cap, kw in ((0, {}), (0, dict(defer=4)), (2 * n, {}), (n + 2, dict(defer=64)), (n + 1, {})):
+            same_wide(wl, oracle, job, wl.DET_FLOYD, 32, cap, kw)
+        if n % 2 and not rule:
+            for cap, kw in ((0, {}), (0, dict(defer=64, threads=128)), (200, dict(defer=4)), (90, {}), (2 * n, {}),
+                            (n, {})):
+                same_wide(wl, oracle, job, wl.DET_STREAK, 32, cap, kw)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [13, 14, 16, 17, 18, 19, 20])
+def test_wide_merged_ranges(wl, oracle, n):
+    rnd = random.Random(n)
+    total = math.factorial(n)
+    for i in range(3):
+        lo = rnd.randrange(0, total) if i else total - 5041
+        hi = min(total, lo + rnd.choice([1, 5041, 60001]))
+        for det in (0, 1, 2) if n % 2 and i != 1 else (0, 1):
+            job = wl.make_job(n, rule=0 if det == 2 else i % 2, lo=lo, hi=hi, hbins=0 if det else 256)
+            same_wide(wl, oracle, job, det, 32, 0, {})
