@@ -23,14 +23,17 @@ static size_t batched_shmem(int hbins, int threads) {
 
 template <int RULE, int G, int V>
 static BatchedFn pick_g(int canon, int shape, int extra) {
-    if constexpr ((V & 28) == 28) {   // deals with the path memo are played merged (war_merge.cu); the sample is not
-        if (!canon) return extra ? batched_kernel<RULE, G, false, false, true, V> : nullptr;
-    } else {
+    // the path memo: merged deals and canonical scans have kernels of their own (war_merge.cu), which leaves the
+    // sampled deals; the other memo forms are for deals
+    if constexpr ((V & 28) == 28) return canon || !extra ? nullptr : batched_kernel<RULE, G, false, false, true, V>;
+    else {
         if (!canon) return extra ? batched_kernel<RULE, G, false, false, true, V> : batched_kernel<RULE, G, false, false, false, V>;
+        if constexpr ((V & 4) != 0) return nullptr;
+        else {
+            if (shape) return extra ? batched_kernel<RULE, G, true, true, true, V> : batched_kernel<RULE, G, true, true, false, V>;
+            return extra ? batched_kernel<RULE, G, true, false, true, V> : batched_kernel<RULE, G, true, false, false, V>;
+        }
     }
-    if constexpr ((V & 4) != 0 && (V & 16) == 0) return nullptr;   // canonical scans: the path memo only
-    if (shape) return extra ? batched_kernel<RULE, G, true, true, true, V> : batched_kernel<RULE, G, true, true, false, V>;
-    return extra ? batched_kernel<RULE, G, true, false, true, V> : batched_kernel<RULE, G, true, false, false, V>;
 }
 
 template <int V>

@@ -94,9 +94,10 @@ int ensure_ready() {
 }
 
 cudaError_t upload_merge_table(u32** table) {
-    std::vector<u32> rows(2 * MERGE_ROWS);
+    std::vector<u32> rows(2 * MERGE_ROWS + CANON_ROWS);
     merge_table(0, rows.data());
     merge_table(1, rows.data() + MERGE_ROWS);
+    canon_table(rows.data() + 2 * MERGE_ROWS);
     cudaError_t e = cudaMalloc(table, sizeof(u32) * rows.size());
     if (e == cudaSuccess) e = cudaMemcpy(*table, rows.data(), sizeof(u32) * rows.size(), cudaMemcpyHostToDevice);
     return e;
@@ -216,12 +217,16 @@ int resolve_tune(const war_job* job, const war_tune* in, Tune& t) {
     if (st) return st;
     // Deals with the path memo are played merged (war_merge.cuh), one game per lane; the sample needs every
     // deal by itself.  (games = 2 and 4 still ask for blocks of at most 512 and 256 threads.)
-    t.merged = !canon && (t.variant & 28) == 28 && !(job->flags & WAR_F_SAMPLE);
+    // Canonical scans with the path memo have a kernel of the same kind.
+    const bool shape = (job->flags & WAR_F_SHAPE) != 0, extra = (job->flags & (WAR_F_DISTINCT | WAR_F_SAMPLE)) != 0;
+    t.merged = (t.variant & 28) == 28 && (canon || !(job->flags & WAR_F_SAMPLE));
     int maxb = !t.merged ? batched_max_blocks_per_sm(canon, job->rule, (job->flags & WAR_F_SHAPE) != 0,
                                                      (job->flags & WAR_F_DISTINCT) != 0,
                                                      (job->flags & WAR_F_SAMPLE) != 0, t.threads, t.games, job->hbins,
                                                      t.variant)
-             : t.games * t.threads > 1024 ? 0 : merged_max_blocks_per_sm(job->rule, t.threads, job->hbins);
+             : t.games * t.threads > 1024 ? 0
+             : canon ? canon_max_blocks_per_sm(job->rule, shape, extra, t.threads, job->hbins)
+             : merged_max_blocks_per_sm(job->rule, t.threads, job->hbins);
     if (maxb < 1) return fail(WAR_EINVAL, "launch shape threads=%d games=%d does not fit an SM", t.threads, t.games);
     t.blocks_per_sm = (in && in->blocks_per_sm) ? std::min(in->blocks_per_sm, maxb) : maxb;
     return WAR_OK;
@@ -519,21 +524,38 @@ static int prepare_memo(Ctx& c, const war_job* job, int bits, int kind, u64** ta
     return WAR_OK;
 }
 
-// A deals job with the path memo: each state after the deals' first turns played once (war_merge.cuh).
+// A job with the path memo: deals with each state after their first turns played once, or a canonical scan
+// (war_merge.cu).
 static int enumerate_merged(const war_job* job, const Tune& t, war_result* out) {
     Ctx& c = ctx();
     MergePlan p;
+    const bool canon = job->mode == WAR_CANON;
     const int blocks = t.blocks_per_sm * c.sm_count;
-    merge_plan(job, (u64)blocks * (u64)(t.threads / 32), p);
+    const u64 warps = (u64)blocks * (u64)(t.threads / 32);
+    if (canon) canon_plan(job, warps, p);
+    else merge_plan(job, warps, p);
     if (p.units == 0) return WAR_OK;   // (--half: no deal of the range gives card n-1 to player 1)
     MergeArgs a;
     int st, used = 0;
     if ((st = merge_args(job, p, job->hbins, t.window, t.defer, a))) return st;
-      // (a game stores at most two states besides the cycles found)
-    if ((st = prepare_memo(c, job, t.memo_bits, 4 * 3, &a.memo, 2 * p.games, &used))) return st;
+    // the table's layout (prepare_memo); a game stores at most two states besides the cycles found
+    const int kind = 4 * 3 + (canon && (job->flags & WAR_F_SHAPE) ? 2 : 0);
+    if ((st = prepare_memo(c, job, t.memo_bits, kind, &a.memo, 2 * p.games, &used))) return st;
     a.memo_bits = (u32)used;
-    return run_merged(p, a, job->hbins, out,
-                      [&](cudaStream_t x) { return launch_merged(a, job->rule, t.threads, blocks, c.d_acc, x); });
+    if (!canon)
+        return run_merged(p, a, MERGE_LAUNCH_UNITS, job->hbins, 0, out,
+                          [&](cudaStream_t x) { return launch_merged(a, job->rule, t.threads, blocks, c.d_acc, x); });
+    a.dbins = job->dbins;
+    a.blk = out->blk;
+    a.distinct = (job->flags & WAR_F_DISTINCT) ? 1 : 0;
+    a.sample = (job->flags & WAR_F_SAMPLE) ? 1 : 0;
+    a.seed = job->seed;
+    a.thr = ((u64)job->sample_ppm << 32) / 1000000u;
+    const int extra = a.distinct || a.sample;
+    // a launch plays fewer than 2^32 - 2^24 positions (32-bit counters)
+    const u64 per_unit = (u64)p.lc * (u64)(job->n - 1);
+    return run_merged(p, a, ((1ull << 32) - (1ull << 24)) / per_unit, job->hbins, job->dbins, out,
+                      [&](cudaStream_t x) { return launch_canon(a, job->rule, extra, t.threads, blocks, c.d_acc, x); });
 }
 
 int war_enumerate_held(const war_job* job, const war_tune* tune, war_result* out) {
@@ -587,7 +609,7 @@ int war_enumerate_held(const war_job* job, const war_tune* tune, war_result* out
         merge_plan(job, (u64)blocks * (u64)(threads / 32), p);
         MergeArgs m;
         if ((st = merge_args(job, p, job->hbins, W, defer, m))) return st;
-        return run_merged(p, m, job->hbins, out,
+        return run_merged(p, m, MERGE_LAUNCH_UNITS, job->hbins, 0, out,
                           [&](cudaStream_t x) { return launch_held_merged(m, job->rule, threads, blocks, c.d_acc, x); });
     }
     Plan p;
@@ -674,11 +696,8 @@ int war_enumerate(const war_job* job, const war_tune* tune, war_result* out) {
     a.units = c.d_units;
     a.chunk = (u32)t.chunk;
     if (t.variant & 4) {   // the cycle memo
-        // its entry layout: the form the variant selects, and the shape-carrying values of a canonical scan
-        // with the loop-shape test
-        const int form = (t.variant & 24) == 24 ? 3 : ((t.variant & 8) ? 2 : 1);
-        const int kind = 4 * form + ((job->mode == WAR_CANON && (job->flags & WAR_F_SHAPE)) ? 2 : 0);
-        if ((st = prepare_memo(c, job, t.memo_bits, kind, &a.memo))) return st;
+        const int form = (t.variant & 24) == 24 ? 3 : ((t.variant & 8) ? 2 : 1);   // its entry layout
+        if ((st = prepare_memo(c, job, t.memo_bits, 4 * form, &a.memo))) return st;
         a.memo_bits = (u32)t.memo_bits;
     }
     // Each launch plays fewer than 2^32 games, so the 32-bit per-block and per-lane counters cannot wrap.

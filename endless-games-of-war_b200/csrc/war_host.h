@@ -44,7 +44,7 @@ struct Tune {
 Ctx& ctx();
 int ensure_ready();
 cudaStream_t cur_stream();
-cudaError_t upload_merge_table(u32** table);   // both rules' pair lists, MERGE_ROWS rows each
+cudaError_t upload_merge_table(u32** table);   // pair lists of both rules, then orders
 int fail(int code, const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);
 u64 fact(int i);
@@ -78,15 +78,15 @@ inline int run_launch(F launch, double* ms) {
     return WAR_OK;
 }
 
-// Runs a merged job's units in launches of at most MERGE_LAUNCH_UNITS.
+// Runs a merged job's units in launches of at most `most`.
 template <typename F>
-inline int run_merged(const MergePlan& p, MergeArgs& a, int hbins, war_result* out, F launch) {
-    for (u64 u = 0; u < p.units; u += MERGE_LAUNCH_UNITS) {
+inline int run_merged(const MergePlan& p, MergeArgs& a, u64 most, int hbins, int dbins, war_result* out, F launch) {
+    for (u64 u = 0; u < p.units; u += most) {
         a.unit_lo = u;
-        a.unit_hi = p.units - u < MERGE_LAUNCH_UNITS ? p.units : u + MERGE_LAUNCH_UNITS;
+        a.unit_hi = p.units - u < most ? p.units : u + most;
         const int st = run_launch(launch, &out->kernel_ms);
         if (st) return st;
-        merge_acc(*ctx().h_acc, out, hbins, 0);
+        merge_acc(*ctx().h_acc, out, hbins, dbins);
     }
     out->units += p.units;
     return WAR_OK;

@@ -54,6 +54,8 @@ struct MBlock {
     u8 filter;        // play only games in which player 1 holds card n - 1
     u8 twice;         // and count them twice (their mirror images)
     u8 prefix[20];    // the fixed cards
+    u8 inner;         // table cards of a canonical unit
+    u8 k0, k1;        // canonical splits k0 <= k < k1
 };
 
 struct MergeArgs {
@@ -65,6 +67,9 @@ struct MergeArgs {
     u64* memo;
     u32 memo_bits;
     TurnK tk;
+    // canonical scans
+    u64 seed, thr;
+    int dbins, blk, distinct, sample;
 };
 
 // The outer choice of a unit and what its games share.  The piles without the list's pairs (U1, U2, s1 and
@@ -92,6 +97,10 @@ void merge_table(int rule, u32* rows);
 void merge_plan(const war_job* job, u64 warps, MergePlan& p);
 cudaError_t launch_merged(const MergeArgs& a, int rule, int threads, int blocks, DevAcc* acc, cudaStream_t st);
 int merged_max_blocks_per_sm(int rule, int threads, int hbins);
+void canon_table(u32* rows);
+void canon_plan(const war_job* job, u64 warps, MergePlan& p);
+cudaError_t launch_canon(const MergeArgs& a, int rule, int extra, int threads, int blocks, DevAcc* acc, cudaStream_t st);
+int canon_max_blocks_per_sm(int rule, int shape, int extra, int threads, int hbins);
 cudaError_t launch_held_merged(const MergeArgs& a, int rule, int threads, int blocks, DevAcc* acc, cudaStream_t st);
 int held_merged_max_blocks_per_sm(int rule, int threads, int hbins);
 
@@ -175,6 +184,39 @@ __device__ __forceinline__ u32 merge_row(u32 c0, u32 c1, u32 sel) {
     return __byte_perm(x, y, 0x6420);
 }
 
+// Canonical positions are dealt out the same way, one game each: a block is j! consecutive orders of the n - 1
+// other cards with splits k0 <= k < k1, a unit a run of rows of the table of all orders of the last (at most 6)
+// cards under one choice of the others, with every split.
+constexpr u32 CANON_INNER = 6;
+constexpr u32 CANON_ROWS = 1 + 1 + 2 + 6 + 24 + 120 + 720;
+__host__ __device__ __forceinline__ u32 canon_rows(u32 i) {       // i!
+    return i < 2u ? 1u : i == 2u ? 2u : i == 3u ? 6u : i == 4u ? 24u : i == 5u ? 120u : 720u;
+}
+__host__ __device__ __forceinline__ u32 canon_row0(u32 i) {       // first row of the table of i cards
+    return i == 0u ? 0u : i == 1u ? 1u : i == 2u ? 2u : i == 3u ? 4u : i == 4u ? 10u : i == 5u ? 34u : 154u;
+}
+struct CUnit {
+    u64 Q;            // the cards before the inner ones, 4 bits each
+    u32 c0, c1;       // the inner cards as bytes
+};
+__host__ __device__ __forceinline__ void canon_unit(const MBlock& B, u64 outer, u32 m, CUnit& u) {
+    u32 free = B.free_mask;
+    u64 Q = 0, c = 0;
+    for (u32 i = 0; i + B.inner < m; i++) {
+        u32 v;
+        if (i < B.b) v = B.prefix[i];
+        else {
+            const u32 k = card_count(free);
+            v = take_card(free, (u32)(outer % k));
+            outer /= k;
+        }
+        Q |= (u64)v << (4u * i);
+    }
+    for (u32 i = 0; free; i++) c |= (u64)take_card(free, 0u) << (8u * i);
+    u.Q = Q;
+    u.c0 = (u32)c; u.c1 = (u32)(c >> 32);
+}
+
 // A warp's place in its unit: row l of [l0, lend) with pa of the f pairs won by player 1, games that stand for wt
 // deals each.  Histogram bins of a block are 32 bits: a warp empties them into the accumulators (drain) before
 // it has dealt out games that stand for this many deals since it last did.  A bin holds at most what the block's
@@ -188,13 +230,14 @@ struct MCursor {
     bool filter = false, dry = false;
 };
 
-// Deals the warp's next games to the lanes that want one; called by the whole warp.
+// Deals the warp's next games to the lanes that want one; called by the whole warp.  CANON: pa is the split, the
+// rows are orders and every game counts once.
 //   setup(B, outer)   sets the unit up for the warp
 //   over()            whether one player won every pair of the unit's games with c.pa (1: player 1, 2: player 2)
 //   ended(count)      counts `count` deals that are over at turn h
 //   build(selectors)  the lane's game from a table row; false if it is not played (filter)
 //   drain()           empties the histograms
-template <class Setup, class Over, class Ended, class Build, class Drain>
+template <bool CANON = false, class Setup, class Over, class Ended, class Build, class Drain>
 __device__ __forceinline__ u32 merge_deal(MCursor& c, const MergeArgs& a, u64* counter, bool want, Setup setup,
                                           Over over, Ended ended, Build build, Drain drain) {
     const u32 lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
@@ -203,7 +246,7 @@ __device__ __forceinline__ u32 merge_deal(MCursor& c, const MergeArgs& a, u64* c
         if (c.l == c.lend) {
             if (c.pa < c.f) {
                 c.pa++;
-                c.wt = c.wt * (c.f - c.pa + 1u) / c.pa;
+                if (!CANON) c.wt = c.wt * (c.f - c.pa + 1u) / c.pa;
                 c.l = c.l0;
             } else {
                 u64 u = 0;
@@ -214,18 +257,18 @@ __device__ __forceinline__ u32 merge_deal(MCursor& c, const MergeArgs& a, u64* c
                 const MBlock& B = a.blocks[c.blk];
                 const u64 v = u - B.u0, outer = v / B.nch;
                 setup(B, outer);
-                c.f = B.f;
-                c.fi = min(c.f, MERGE_INNER);
-                c.row0 = merge_row0(c.fi);
+                c.f = CANON ? B.k1 - 1u : B.f;
+                c.fi = CANON ? B.inner : min(c.f, MERGE_INNER);
+                c.row0 = CANON ? canon_row0(c.fi) : merge_row0(c.fi);
                 c.l0 = (u32)(v - outer * B.nch) * a.lc;
-                c.lend = min(merge_rows(c.fi), c.l0 + a.lc);
+                c.lend = min(CANON ? canon_rows(c.fi) : merge_rows(c.fi), c.l0 + a.lc);
                 c.l = c.l0;
-                c.pa = 0;
-                c.wt = B.twice ? 2u : 1u;
-                c.filter = B.filter != 0;
+                c.pa = CANON ? B.k0 : 0u;
+                c.wt = !CANON && B.twice ? 2u : 1u;
+                c.filter = !CANON && B.filter != 0;
                 if (c.given > DRAIN_DEALS) { drain(); c.given = 0; }
             }
-            const u32 o = over();
+            const u32 o = CANON ? 0u : over();
             if (o) {
                 if (o == 1u || !c.filter) {   // (card n-1 is with the player who won every pair)
                     const u32 k = (c.lend - c.l) * c.wt;

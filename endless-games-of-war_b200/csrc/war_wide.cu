@@ -742,7 +742,7 @@ extern "C" int war_enumerate_wide(const war_job* job, const war_wide_cfg* cfg, w
         merge_plan(job, (u64)blocks * (u64)(threads / 32), p);
         MergeArgs m;
         if ((st = merge_args(job, p, hbins, W, defer, m))) return st;
-        return run_merged(p, m, hbins, out, [&](cudaStream_t x) {
+        return run_merged(p, m, MERGE_LAUNCH_UNITS, hbins, 0, out, [&](cudaStream_t x) {
             wide_merge_pick(c.det, job->rule)<<<blocks, threads, wide_merge_shmem(c.det, threads, hbins), x>>>(m, more, cx.d_acc);
             note_launch();
             return cudaGetLastError();

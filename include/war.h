@@ -98,7 +98,8 @@ typedef struct war_tune {
                               Deals with the path memo and no sample are played merged: the states after
                               the deals' first floor(n/2) turns, each once, in the multiply-add turn form, in
                               units of the engine's own size (games, block_m and chunk do not apply); `turns`
-                              counts the turns played from there. */
+                              counts the turns played from there.  Canonical scans with the path memo use
+                              the multiply-add turn form and such units too. */
     int32_t memo_bits;     /* cycle memo: log2 of its 8-byte slots (12..31); 0 = 24 (128 MiB).  A merged job
                               clears and uses only as much of it as its games can fill */
     int32_t chunk;         /* work units a lane takes from the work counter at a time (1..4096; 0 = 1): each lane

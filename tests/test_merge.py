@@ -222,3 +222,27 @@ def test_wide_merged_ranges(wl, oracle, n):
         for det in (0, 1, 2) if n % 2 and i != 1 else (0, 1):
             job = wl.make_job(n, rule=0 if det == 2 else i % 2, lo=lo, hi=hi, hbins=0 if det else 256)
             same_wide(wl, oracle, job, det, 32, 0, {})
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [4, 5, 6, 8, 11, 13, 16])
+def test_canonical_units(wl, n):
+    """Canonical scans with the path memo at the edges of orders, blocks and units: one position, part of an order,
+    ranges that begin and end inside orders, the last positions; every output, both rules."""
+    rnd = random.Random(n)
+    total, s = wl.space_size(n, wl.CANON), n - 1
+    ranges = [(0, 1), (total - 1, total), (total - min(total, 720 * s + 3), total), (0, min(total, 721 * s - 1))]
+    for _ in range(4):
+        lo = rnd.randrange(0, total)
+        ranges.append((lo, min(total, lo + rnd.choice([1, s, 2 * s + 1, 100003]))))
+    shapes = [dict(), dict(threads=64, defer=4), dict(threads=1024, memo_bits=12), dict(blocks_per_sm=1, variant=30)]
+    keys = KEYS + ("dhist", "oncycle", "distinct_min", "shape_nonstd", "shape_unchecked", "s_count", "s_cyc",
+                   "s_lamsum", "s_lensum", "s_maxfin")
+    for i, (lo, hi) in enumerate(ranges):
+        for flags in (0, wl.F_SHAPE, wl.F_DISTINCT, wl.F_DISTINCT | wl.F_SHAPE | wl.F_SAMPLE):
+            job = wl.make_job(n, wl.CANON, i % 2, flags, lo, hi, hbins=128, dbins=64 if flags & wl.F_DISTINCT else 0,
+                              sample_ppm=100000, seed=n)
+            got = wl.to_dict(wl.enumerate_job(job, memo_tune(wl, window=128, **shapes[i % len(shapes)])))
+            want = wl.to_dict(wl.enumerate_plain(job))
+            for k in keys:
+                assert got[k] == want[k], (n, lo, hi, flags, k)
