@@ -480,18 +480,12 @@ struct LGame {
     u32 mlam;           // MEMO: the memo's value for this game (0: decided by Brent or by its end)
     u64 ka, kb;         // MEMO_PATH: the keys of the last two states looked up and missed,
     u32 ta, tb;         // at these turns (0: none)
-    u32 pend;           // canonical distinct scan: a memo value held until turn lam of its cycle (0: none)
 };
 
 // With MEMO_LANDMARK, each turn also keeps the state before it when card n-1 is on top (a landmark), and
 // every service looks the kept landmark of each undecided game up in the memo; with MEMO_ALL every
 // service looks up each undecided game's current state.  A game decided by Brent stores its cycle.
-//
-// SHAPE (canonical scans with the loop-shape test, path memo only): the Theorem-3 shape is a property of
-// the cycle, so it travels in the memo with the cycle length — a cycle outcome is 8 lam + 2 code (code 0
-// of the shape, 1 not, 2 loop too long to check) instead of 2 lam — and a cycle found by Brent is checked
-// once with loop_shape_walk from its detection state, which lies on the loop.
-template <int RULE, int G, bool CANON, bool EXTRA, int TV, int MEMO, bool SHAPE = false>
+template <int RULE, int G, bool CANON, bool EXTRA, int TV, int MEMO>
 __device__ __forceinline__ void refill_latched(const BatchArgs& a, DevAcc* __restrict__ acc, u64* __restrict__ counter,
                                                u32* sh) {
     u32* shh = sh;
@@ -516,7 +510,6 @@ __device__ __forceinline__ void refill_latched(const BatchArgs& a, DevAcc* __res
     LGame<EXTRA, MEMO> g[G];
     u32 cyc = 0, done = 0, maxfin = 0, capped = 0, turns = 0;
     u32 sc = 0, scy = 0, slam = 0, slen = 0, smax = 0, oncyc = 0, dmin = 0;
-    u32 nonstd = 0, unchk = 0;             // SHAPE
     u32 mlook = 0, mhit = 0, mstore = 0;   // memo traffic
     const u32 nm1 = n - 1u;
     u64* const memo = MEMO ? a.memo : nullptr;
@@ -532,7 +525,6 @@ __device__ __forceinline__ void refill_latched(const BatchArgs& a, DevAcc* __res
         x.done = !ok; x.kcy = false;
         if (MEMO) { x.m1 = 0ull; x.m2 = 0ull; x.mlam = 0u; }
         if (MEMO == MEMO_PATH) { x.ta = 0u; x.tb = 0u; }
-        if (MEMO) x.pend = 0u;
         if (EXTRA) {
             x.s1 = x.w1; x.s2 = x.w2; x.sq = x.q;
             x.sampled = a.sample && ok && war_pick(a.seed, a.thr, x.w1, x.w2);
@@ -600,7 +592,7 @@ __device__ __forceinline__ void refill_latched(const BatchArgs& a, DevAcc* __res
             for (int i = 0; i < G; i++) {
                 LGame<EXTRA, MEMO>& x = g[i];
                 if (MEMO >= MEMO_ALL) {
-                    look[i] = !x.done & (x.pend == 0u);
+                    look[i] = !x.done;
                     key[i] = memo_key_state(x.w1, x.w2, n);
                 } else {
                     look[i] = !x.done & (x.m1 != 0ull);
@@ -622,18 +614,7 @@ __device__ __forceinline__ void refill_latched(const BatchArgs& a, DevAcc* __res
                     mhit++;
                     const u32 v = MEMO == MEMO_PATH ? (u32)(e[i] & vmask) : (u32)(e[i] >> lsh);
                     const bool vcy = MEMO == MEMO_PATH ? (v & 1u) == 0u : true;
-                    const u32 vlam = MEMO == MEMO_PATH ? v >> (SHAPE ? 3 : 1) : v;
-                    if (CANON && EXTRA && a.distinct && vcy && vlam <= W && x.rounds < vlam) {
-                        // Whether the start lies on its cycle shows at turn vlam: Brent's first window
-                        // compares every state up to W >= vlam with the start.  Play on until then.
-                        x.pend = v;
-                    } else {
-                        x.done = true; x.kcy = vcy; x.mlam = v;
-                    }
-                } else if (CANON && EXTRA && x.pend != 0u && !x.done &&
-                           x.rounds >= (MEMO == MEMO_PATH ? x.pend >> (SHAPE ? 3 : 1) : x.pend)) {
-                    // turn lam passed without the start coming back: on the cycle, not through the start
-                    x.done = true; x.kcy = true; x.mlam = x.pend;
+                    x.done = true; x.kcy = vcy; x.mlam = v;
                 } else if (MEMO == MEMO_PATH && look[i]) {
                     x.kb = x.ka; x.tb = x.ta;
                     x.ka = key[i]; x.ta = x.rounds;
@@ -652,18 +633,10 @@ __device__ __forceinline__ void refill_latched(const BatchArgs& a, DevAcc* __res
                     const bool cy = x.kcy;
                     turns += x.rounds;
                     // the memo's cycle length, or (path memo) the turns left after the memoised state
-                    const u32 mcy = MEMO == MEMO_PATH ? (x.mlam & 1u ? 0u : x.mlam >> (SHAPE ? 3 : 1)) : x.mlam;
+                    const u32 mcy = MEMO == MEMO_PATH ? (x.mlam & 1u ? 0u : x.mlam >> 1) : x.mlam;
                     const u32 len = MEMO == MEMO_PATH && (x.mlam & 1u) ? x.rounds + (x.mlam >> 1) : x.rounds;
                     const u32 lam = (MEMO && mcy) ? mcy : x.rounds - ((x.next - W) >> 1);
-                    // SHAPE: the loop's shape code, from the memo or checked now on the loop
-                    u32 code = 0u;
-                    if (SHAPE && cy) {
-                        code = mcy ? (x.mlam >> 1) & 3u
-                                   : (u32)loop_shape_walk<RULE>(x.w1, x.w2, TV ? x.q + qshift : x.q, k4m4, lam, (u32)a.blk);
-                        if (code == 1u) nonstd++;
-                        if (code == 2u) unchk++;
-                    }
-                    const u64 vcyc = SHAPE ? 8ull * lam + 2ull * code : 2ull * lam;   // the cycle outcome
+                    const u64 vcyc = 2ull * lam;   // the cycle outcome
                     if (MEMO == MEMO_PATH && memo != nullptr) {   // the states it missed, with its outcome
                         if (x.ta) {
                             const u64 v = cy ? vcyc : 2ull * (len - x.ta) + 1ull;
@@ -685,17 +658,13 @@ __device__ __forceinline__ void refill_latched(const BatchArgs& a, DevAcc* __res
                     if (cy) {
                         cyc++;
                         if (MEMO && memo != nullptr && mcy == 0u) {   // found by Brent: store its cycle
-                            memo_store_cycle<RULE, MEMO>(memo, mbits, x.w1, x.w2, TV ? x.q + qshift : x.q, n, lam,
-                                                         SHAPE ? (u32)vcyc : 0u);
+                            memo_store_cycle<RULE, MEMO>(memo, mbits, x.w1, x.w2, TV ? x.q + qshift : x.q, n, lam);
                             mstore += lam;
                         }
                         if (a.hbins) atomicAdd(&shh[lam < hb1 ? lam : hb1], 1u);
                         if (CANON && EXTRA && a.distinct) {
                             const u32 tstep = (x.next - W) >> 1;
-                            // decided by the memo: the start was not seen again within lam <= W turns
-                            // (else Brent's first window would have decided it), or lam > W: walk
-                            bool on = (MEMO && mcy) ? (lam <= W ? false : on_cycle_walk<RULE>(x.s1, x.s2, x.sq, n, lam))
-                                    : (tstep == 0u) ? true
+                            bool on = (tstep == 0u) ? true
                                     : (lam <= W ? false : on_cycle_walk<RULE>(x.s1, x.s2, x.sq, n, lam));
                             if (on) {
                                 CycleWalk cw = cycle_walk<RULE>(x.s1, x.s2, x.sq, n, lam);
@@ -727,13 +696,6 @@ __device__ __forceinline__ void refill_latched(const BatchArgs& a, DevAcc* __res
         }
     }
 
-    if (SHAPE) {
-        u64 v_ns = warp_sum((u64)nonstd), v_un = warp_sum((u64)unchk);
-        if ((threadIdx.x & 31) == 0) {
-            if (v_ns) atomicAdd(&acc->shape_nonstd, v_ns);
-            if (v_un) atomicAdd(&acc->shape_unchecked, v_un);
-        }
-    }
     if (MEMO) {
         u64 v_l = warp_sum((u64)mlook), v_h = warp_sum((u64)mhit), v_s = warp_sum((u64)mstore);
         if ((threadIdx.x & 31) == 0) {
@@ -770,14 +732,13 @@ __device__ __forceinline__ void refill_latched(const BatchArgs& a, DevAcc* __res
 
 // Dispatch: variant V selects the turn form (V & 1: multiply-add), the record scheme (V & 2: latched)
 // and, for deals with the latched scheme, the cycle memo (V & 4: landmarks, V & 12: all states, V & 28:
-// all states and paths); the loop-shape tracker needs the immediate scheme.
+// all states and paths; deals one by one, for the sample: war_merge_body.cuh has the path memo's other
+// jobs); the loop-shape tracker needs the immediate scheme.
 template <int RULE, int G, bool CANON, bool SHAPE, bool EXTRA, int V>
 __device__ __forceinline__ void refill_dispatch(const BatchArgs& a, DevAcc* __restrict__ acc, u64* __restrict__ counter,
                                                 u32* sh) {
-    if constexpr (SHAPE && CANON && (V & 30) == 30)   // the loop-shape test with the path memo
-        refill_latched<RULE, G, CANON, EXTRA, V & 1, MEMO_PATH, true>(a, acc, counter, sh);
-    else if constexpr (SHAPE || (V & 2) == 0) refill_body<RULE, G, CANON, SHAPE, EXTRA, V & 1>(a, acc, counter, sh);
-    else if constexpr ((V & 4) == 0 || (CANON && (V & 8) == 0)) refill_latched<RULE, G, CANON, EXTRA, V & 1, MEMO_NONE>(a, acc, counter, sh);
+    if constexpr (SHAPE || (V & 2) == 0) refill_body<RULE, G, CANON, SHAPE, EXTRA, V & 1>(a, acc, counter, sh);
+    else if constexpr ((V & 4) == 0 || CANON) refill_latched<RULE, G, CANON, EXTRA, V & 1, MEMO_NONE>(a, acc, counter, sh);
     else if constexpr ((V & 24) == 24) refill_latched<RULE, G, CANON, EXTRA, V & 1, MEMO_PATH>(a, acc, counter, sh);
     else if constexpr ((V & 8) != 0) refill_latched<RULE, G, CANON, EXTRA, V & 1, MEMO_ALL>(a, acc, counter, sh);
     else refill_latched<RULE, G, CANON, EXTRA, V & 1, MEMO_LANDMARK>(a, acc, counter, sh);

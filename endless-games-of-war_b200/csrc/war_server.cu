@@ -7,16 +7,22 @@
 // Every "tick" the worker cuts the admitted jobs' remaining ranges into tasks (each a run of work units of
 // one job, about task_ranks ranks), sharing the tick's rank budget round-robin so that a short job is not
 // stuck behind a long one, and runs the whole tick as one launch per kernel variant: each block plays one
-// task with the refill loop of war_refill.cuh and adds its results to that task's job slot.  Jobs of
-// different n and mode therefore run side by side on the device.  Two ticks are in flight at a time (the
-// next one is queued before the previous one is waited for), so the GPU does not wait for the host; a job
-// whose last task was in a finished tick is read back, its slot freed and its result published.
+// task with the loops of war_merge_body.cuh (deals and canonical scans of any n and rule: one variant) or
+// war_refill.cuh and adds its results to that task's job slot.  Jobs of different n and mode therefore run
+// side by side on the device.  Two ticks are in flight at a time (the next one is queued before the previous
+// one is waited for), so the GPU does not wait for the host; the jobs whose last tasks were in a finished tick
+// are read back together, their slots freed and their results published.
+//
+// What bounds a burst of small jobs: the longest task and the jobs whose games find no table to help them.  24 jobs
+// of 1e4 to 3e7 ranks (four mixes, repeated): 38, 32, 45 and 45 ms with one launch per n-and-mode variant of
+// blocks that played units of 720 deals a lane; 33, 5, 12 and 7 ms with this one (B200).
 //
 // Jobs of the same n and rule share one cycle memo (war_refill.cuh): its entries are facts about n and the
 // rule, so every job of that class, now and later, decides its games from what the earlier ones found.
 // The tables come from one arena that war_server_create reserves inside the memory budget (after the
 // accumulator slots); a class takes its table from the arena when its first job is admitted, cleared on
-// the compute stream, and keeps it until the server ends.  The worker thread never calls cudaMalloc, which
+// the compute stream, and keeps it until the server ends; no class takes more than half of what is left, so that
+// a server of several large classes does not leave the last ones without.  The worker thread never calls cudaMalloc, which
 // would synchronise the device in the middle of the tick stream.  A class whose table no longer fits runs
 // without the memo.
 #include <cuda_runtime.h>
@@ -32,29 +38,76 @@
 #include <vector>
 #include "war_host.h"
 #include "war_refill.cuh"
+#include "war_merge_body.cuh"
 
 namespace war {
 
+// A resident job's arguments, kept on the device by accumulator slot while it runs.
+struct ServeJob {
+    union {
+        BatchArgs batch;
+        MergeArgs merge;
+    };
+};
+
+// One block's work: a run of units of a job.
 struct ServeTask {
-    BatchArgs args;   // the job's parameters and this task's units
-    u32 slot;         // accumulator slot of the job
-    u32 pad;
-    u64 counter;      // the task's work-unit counter (zero when uploaded)
+    u64 lo, hi;           // its units [lo, hi) (BatchArgs: main units from main_base = lo, or `hi` extra units)
+    u64 counter;          // the task's work-unit counter (zero when uploaded)
+    const Unit* units;    // extra units, or null
+    u32 slot;             // accumulator slot of the job
+    u32 kind;             // serve_merge_kernel: rule + 2 canon + 2 (canon and distinct or sample)
 };
 
 template <int RULE, int G, bool CANON, bool SHAPE, bool EXTRA, int V>
 __global__ void __launch_bounds__(G == 1 ? 1024 : 512) serve_kernel(ServeTask* __restrict__ tasks,
+                                                                   const ServeJob* __restrict__ jobs,
                                                                    DevAcc* __restrict__ slots) {
     extern __shared__ u32 sh[];
     __shared__ BatchArgs A;
     ServeTask* t = tasks + blockIdx.x;
-    const u32* src = (const u32*)&t->args;
+    const u32* src = (const u32*)&jobs[t->slot].batch;
     for (int i = threadIdx.x; i < (int)(sizeof(BatchArgs) / 4); i += blockDim.x) ((u32*)&A)[i] = src[i];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        A.main_base = t->lo;
+        A.main_count = t->units ? 0ull : t->hi - t->lo;
+        A.n_units = t->units ? t->hi : t->hi - t->lo;
+        A.units = t->units;
+    }
     __syncthreads();
     refill_dispatch<RULE, G, CANON, SHAPE, EXTRA, V>(A, slots + t->slot, &t->counter, sh);
 }
 
-typedef void (*ServeFn)(ServeTask*, DevAcc*);
+// The same for the loops of war_merge_body.cuh, merged deals and canonical scans with or without a table, all in
+// one launch: the tasks of a tick run side by side whatever their kind.
+__global__ void __launch_bounds__(1024) serve_merge_kernel(ServeTask* __restrict__ tasks,
+                                                           const ServeJob* __restrict__ jobs,
+                                                           DevAcc* __restrict__ slots) {
+    extern __shared__ u64 sh64[];
+    __shared__ MergeArgs A;
+    __shared__ UnitStore store;
+    ServeTask* t = tasks + blockIdx.x;
+    const u32* src = (const u32*)&jobs[t->slot].merge;
+    for (int i = threadIdx.x; i < (int)(sizeof(MergeArgs) / 4); i += blockDim.x) ((u32*)&A)[i] = src[i];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        A.unit_lo = t->lo;
+        A.unit_hi = t->hi;
+    }
+    __syncthreads();
+    DevAcc* const acc = slots + t->slot;
+    switch (t->kind) {
+        case 0: merge_body<0>(A, acc, &t->counter, store, (u32*)sh64); break;
+        case 1: merge_body<1>(A, acc, &t->counter, store, (u32*)sh64); break;
+        case 2: canon_body<0, false, false>(A, acc, &t->counter, store, sh64); break;
+        case 3: canon_body<1, false, false>(A, acc, &t->counter, store, sh64); break;
+        case 4: canon_body<0, true, false>(A, acc, &t->counter, store, sh64); break;
+        default: canon_body<1, true, false>(A, acc, &t->counter, store, sh64); break;
+    }
+}
+
+typedef void (*ServeFn)(ServeTask*, const ServeJob*, DevAcc*);
 
 template <int RULE, int G, int V>
 static ServeFn serve_pick(bool canon, bool shape, bool extra) {
@@ -63,27 +116,28 @@ static ServeFn serve_pick(bool canon, bool shape, bool extra) {
     return extra ? serve_kernel<RULE, G, true, false, true, V> : serve_kernel<RULE, G, true, false, false, V>;
 }
 
-// Launch shapes of the serving kernel: one game per thread, 256-thread blocks, the multiply-add turn form;
-// latched records with the path memo where it applies (memo = 1: n <= 14 and a table), with the landmark
-// memo for deals of n = 15 (memo = 2), latched records without a memo otherwise, and the immediate-record
-// loop for the loop-shape test.
+// Launch shapes of the serving kernels: one game per thread, 256-thread blocks, the multiply-add turn form.
+// Merged deals and canonical scans are one kernel (merged = 1, the other fields 0); sampled deals play deal by deal,
+// with the path memo where the class has a table (memo); the loop-shape test has the immediate-record loop, and
+// so have canonical scans and deals of fewer than 4 cards the latched one.
 struct Variant {
-    int canon, rule, shape, extra, memo;
+    int merged, canon, rule, shape, extra, memo;
     bool operator<(const Variant& o) const {
-        return std::tie(canon, rule, shape, extra, memo) < std::tie(o.canon, o.rule, o.shape, o.extra, o.memo);
+        return std::tie(merged, canon, rule, shape, extra, memo) <
+               std::tie(o.merged, o.canon, o.rule, o.shape, o.extra, o.memo);
     }
     bool operator==(const Variant& o) const { return !(*this < o) && !(o < *this); }
-    int games() const { return 1; }
     int threads() const { return 256; }
-    ServeFn fn() const {
-        const bool c = canon != 0;
-        if (rule) return shape ? serve_pick<1, 1, 1>(c, true, extra)
-                         : memo == 1 ? serve_pick<1, 1, 31>(c, false, extra)
-                         : memo == 2 ? serve_pick<1, 1, 7>(c, false, extra) : serve_pick<1, 1, 3>(c, false, extra);
-        return shape ? serve_pick<0, 1, 1>(c, true, extra)
-                     : memo == 1 ? serve_pick<0, 1, 31>(c, false, extra)
-                     : memo == 2 ? serve_pick<0, 1, 7>(c, false, extra) : serve_pick<0, 1, 3>(c, false, extra);
+    size_t shmem(int hbins) const {   // (a merged launch may hold canonical tasks that keep their starts)
+        return sizeof(u32) * (size_t)(hbins + WAR_EBINS) + (merged ? sizeof(ulonglong2) * (size_t)threads() : 0);
     }
+    template <int RULE>
+    ServeFn fn_rule() const {
+        if (shape) return serve_pick<RULE, 1, 1>(true, true, extra);
+        if (memo) return serve_kernel<RULE, 1, false, false, true, 31>;
+        return serve_pick<RULE, 1, 3>(canon != 0, false, extra);
+    }
+    ServeFn fn() const { return merged ? serve_merge_kernel : rule ? fn_rule<1>() : fn_rule<0>(); }
 };
 
 struct SJob {
@@ -96,8 +150,9 @@ struct SJob {
     u64 next_main = 0;
     bool extras_issued = false;
     u64 per_unit = 1;    // ranks per main unit
-    BatchArgs base;
+    MergePlan mplan;     // merged jobs: the plan; next_main counts its units
     Variant var;
+    u32 kind = 0;        // of its tasks (ServeTask)
     war_result* result = nullptr;
 };
 
@@ -108,8 +163,8 @@ struct Tick {
     Unit* d_units = nullptr;
     int ntasks = 0, nunits = 0;
     std::vector<std::pair<Variant, std::pair<int, int>>> groups;   // variant -> [first task, count)
-    std::vector<u64> finishing;     // jobs whose last task is in this tick
-    std::vector<u64> admitted;      // jobs whose slot is cleared before this tick
+    std::vector<std::pair<u64, int>> finishing;      // jobs whose last task is in this tick, and their slots
+    std::vector<std::pair<int, size_t>> admitted;    // slots to be set up before this tick, and their blocks
     cudaEvent_t ev = nullptr;
     bool in_flight = false;
 };
@@ -129,8 +184,13 @@ struct war_server {
     std::map<std::pair<int, int>, std::pair<u64*, int>> memos;   // (n, rule) -> (table, log2 words)
     u64* memo_arena = nullptr;      // reserved at create; tables are carved from it in admission order
     u64 arena_words = 0, arena_used = 0;
+    u32* d_table = nullptr;         // pair lists and orders (war_merge.cuh)
+    war::MBlock* d_blocks = nullptr;     // the resident merged jobs' blocks, SLOT_BLOCKS for each slot
+    war::MBlock* h_blocks = nullptr;     // and their pinned mirror
+    war::ServeJob* d_jobs = nullptr;   // the resident jobs' arguments, by slot
+    war::ServeJob* h_jobs = nullptr;   // and their pinned mirror
     DevAcc* d_slots = nullptr;
-    DevAcc* h_slot = nullptr;   // pinned readback buffer
+    DevAcc* h_slot = nullptr;   // pinned readback buffer, READBACK slots
     cudaStream_t s_comp = nullptr, s_copy = nullptr;
     war::Tick ticks[2];
     uint64_t next_id = 1, nticks = 0, jobs_done = 0, peak_resident = 0, resident = 0;
@@ -145,13 +205,17 @@ struct war_server {
 namespace war {
 namespace {
 
-constexpr u64 TASK_RANKS = 1ull << 16;   // ranks per task (about 15 ms of one block's work at n = 13)
+// Ranks per task: as many as give each SM 16 blocks of the tick's work, so that a small tick spreads over the GPU
+// (2^13: the block's own start and end stay small beside its games).
+constexpr u64 TASK_RANKS_MIN = 1ull << 13, TASK_RANKS_MAX = 1ull << 16;
+constexpr size_t READBACK = 32;          // finished jobs read back at a time
+constexpr size_t SLOT_BLOCKS = 256;      // blocks of a job of at most 16 cards: at most 2 (1 + .. + 15), and the sentinel
 constexpr int UNITS_PER_EXTRA_CAP = 512;   // sizing of the per-tick extra-unit pool
 
 void set_args(war_server* s, SJob& J) {
     const war_job& job = J.job;
     const bool canon = job.mode == WAR_CANON;
-    BatchArgs& a = J.base;
+    BatchArgs a;
     memset(&a, 0, sizeof a);
     fill_fact(a.fact);
     a.n = job.n;
@@ -168,22 +232,32 @@ void set_args(war_server* s, SJob& J) {
     a.distinct = (job.flags & WAR_F_DISTINCT) && canon ? 1 : 0;
     a.seed = job.seed;
     a.thr = ((u64)job.sample_ppm << 32) / 1000000u;
-    J.var.canon = canon ? 1 : 0;
-    J.var.rule = job.rule;
-    J.var.shape = a.blk ? 1 : 0;
-    J.var.extra = (a.distinct || a.sample) ? 1 : 0;
-    J.var.memo = 0;
-    const bool landmarks = !canon && job.n == 15;   // the landmark memo serves n = 15 deals
-    if (!a.blk && job.n >= 4 && (job.n <= 14 || landmarks) && s->cfg.memo_bits >= 0) {
+    const int extra = (a.distinct || a.sample) ? 1 : 0;
+    J.var = Variant();
+    J.var.merged = !a.blk && job.n >= 4 && (canon || !a.sample) ? 1 : 0;
+    if (J.var.merged) {
+        J.kind = (u32)job.rule + (canon ? 2u + 2u * (u32)extra : 0u);
+        const u64 warps = (u64)s->sm_count * 32u;
+        if (canon) canon_plan(&job, warps, J.mplan);
+        else merge_plan(&job, warps, J.mplan);
+        J.per_unit = std::max<u64>(1, (job.hi - job.lo) / std::max<u64>(1, J.mplan.units));
+    } else {
+        J.var.canon = canon ? 1 : 0;
+        J.var.rule = job.rule;
+        J.var.shape = a.blk ? 1 : 0;
+        J.var.extra = extra;
+    }
+    if (!a.blk && job.n >= 4 && s->cfg.memo_bits >= 0) {
         // the class's table: 2^bits words, grown with n (about a thousandth of the class's rank space)
         const std::pair<int, int> cls(job.n, job.rule);
         auto it = s->memos.find(cls);
         if (it == s->memos.end()) {
             const int cap = s->cfg.memo_bits ? s->cfg.memo_bits : 28;
             int bits = std::max(12, std::min(cap, 4 + (int)std::ceil(std::log2((double)fact(job.n)) * 0.75)));
-            // the largest table of at most 2^bits words that the arena still holds (at least 2^12 words)
-            const u64 left = s->arena_words - s->arena_used;
-            while (bits >= 12 && (1ull << bits) > left) bits--;
+            // the largest table of at most 2^bits words in half of what the arena still holds, so that later classes
+            // have one too (in all of it if the arena is below 2^24 words), at least 2^12 words
+            const u64 left = s->arena_words - s->arena_used, most = s->arena_words < (1ull << 24) ? left : left / 2;
+            while (bits >= 12 && (1ull << bits) > most) bits--;
             u64* t = nullptr;
             if (bits >= 12) {
                 t = s->memo_arena + s->arena_used;
@@ -199,32 +273,60 @@ void set_args(war_server* s, SJob& J) {
         if (it->second.first) {
             a.memo = it->second.first;
             a.memo_bits = (u32)it->second.second;
-            J.var.memo = landmarks ? 2 : 1;
+            if (!J.var.merged) J.var.memo = 1;
         }
     }
+    ServeJob& out = s->h_jobs[J.slot];
+    if (!J.var.merged) {
+        out.batch = a;
+        return;
+    }
+    MergeArgs& m = out.merge;
+    memset(&m, 0, sizeof m);
+    MBlock* const h = s->h_blocks + (size_t)J.slot * SLOT_BLOCKS;
+    memcpy(h, J.mplan.blocks.data(), sizeof(MBlock) * J.mplan.blocks.size());
+    m.blocks = s->d_blocks + (size_t)J.slot * SLOT_BLOCKS;
+    m.table = s->d_table + (canon ? 2 * MERGE_ROWS : job.rule ? MERGE_ROWS : 0);
+    m.lc = J.mplan.lc;
+    m.n = a.n; m.hbins = a.hbins; m.W = a.W; m.defer = a.defer;
+    m.memo = a.memo; m.memo_bits = a.memo_bits; m.tk = a.tk;
+    m.seed = a.seed; m.thr = a.thr;
+    m.dbins = a.dbins; m.distinct = a.distinct; m.sample = a.sample;
 }
 
-bool remaining(const SJob& J) { return J.next_main < J.plan.main_count || (!J.extras_issued && !J.plan.extra.empty()); }
+u64 main_units(const SJob& J) { return J.var.merged ? J.mplan.units : J.plan.main_count; }
+bool extras(const SJob& J) { return !J.var.merged && !J.extras_issued && !J.plan.extra.empty(); }
+bool remaining(const SJob& J) { return J.next_main < main_units(J) || extras(J); }
 
-// Finishes a job whose accumulators are complete: reads its slot back and publishes the result.
-void finish_job(war_server* s, u64 id) {
-    SJob& J = s->jobs[id];
-    cudaError_t e = cudaMemcpyAsync(s->h_slot, s->d_slots + J.slot, sizeof(DevAcc), cudaMemcpyDeviceToHost, s->s_copy);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s->s_copy);
-    std::lock_guard<std::mutex> lk(s->mu);
-    if (e != cudaSuccess) {
-        J.state = 3; J.status = WAR_ECUDA;
-    } else if (s->h_slot->status) {
-        J.state = 3; J.status = WAR_ECAP;
-    } else {
-        merge_acc(*s->h_slot, J.result, J.job.hbins, J.job.dbins);
-        J.state = 2;
+// Finishes jobs whose accumulators are complete: reads their slots back, READBACK at a time, and publishes the
+// results.
+void finish_jobs(war_server* s, const std::vector<std::pair<u64, int>>& ids) {
+    for (size_t i0 = 0; i0 < ids.size(); i0 += READBACK) {
+        const size_t k = std::min(READBACK, ids.size() - i0);
+        cudaError_t e = cudaSuccess;
+        for (size_t i = 0; i < k && e == cudaSuccess; i++)
+            e = cudaMemcpyAsync(s->h_slot + i, s->d_slots + ids[i0 + i].second, sizeof(DevAcc),
+                                cudaMemcpyDeviceToHost, s->s_copy);
+        const cudaError_t e2 = cudaStreamSynchronize(s->s_copy);
+        if (e == cudaSuccess) e = e2;
+        std::lock_guard<std::mutex> lk(s->mu);
+        for (size_t i = 0; i < k; i++) {
+            SJob& J = s->jobs[ids[i0 + i].first];
+            if (e != cudaSuccess) {
+                J.state = 3; J.status = WAR_ECUDA;
+            } else if (s->h_slot[i].status) {
+                J.state = 3; J.status = WAR_ECAP;
+            } else {
+                merge_acc(s->h_slot[i], J.result, J.job.hbins, J.job.dbins);
+                J.state = 2;
+            }
+            J.t_finish = s->now_ms();
+            s->free_slots.push_back(J.slot);
+            s->resident--;
+            s->jobs_done++;
+        }
+        s->cv_done.notify_all();
     }
-    J.t_finish = s->now_ms();
-    s->free_slots.push_back(J.slot);
-    s->resident--;
-    s->jobs_done++;
-    s->cv_done.notify_all();
 }
 
 // Admits queued jobs into free slots (caller holds the lock).  Empty jobs finish at once.
@@ -249,13 +351,18 @@ void admit(war_server* s, Tick& T) {
         const int M = canon ? job.n - 1 : job.n;
         make_plan(&job, std::max(1, std::min(canon ? 4 : 6, M)), J.plan);
         J.per_unit = fact(J.plan.m) * J.plan.games_per_order;
-        set_args(s, J);
         J.slot = s->free_slots.back();
+        set_args(s, J);
+        if (J.var.merged && J.mplan.units == 0) {   // --half: no deal of the range gives card n-1 to player 1
+            J.state = 2; J.t_finish = s->now_ms(); s->jobs_done++;
+            s->cv_done.notify_all();
+            continue;
+        }
         s->free_slots.pop_back();
         J.state = 1;
         s->resident++;
         s->peak_resident = std::max<u64>(s->peak_resident, s->resident);
-        T.admitted.push_back(id);
+        T.admitted.push_back({J.slot, J.var.merged ? J.mplan.blocks.size() : 0});
     }
 }
 
@@ -267,69 +374,68 @@ void build_tick(war_server* s, Tick& T) {
         if (kv.second.state == 1 && remaining(kv.second)) run.push_back(kv.first);
     if (run.empty()) return;
     const u64 budget = s->cfg.tick_ranks;
-    const u64 unit_cap = (u64)s->max_units * 8;
-    u64 used = 0, units_used = 0;
-    std::vector<std::pair<Variant, ServeTask>> tasks;
-    std::vector<std::vector<Unit>> task_units;
+    u64 left = 0;
+    for (u64 id : run) {
+        const SJob& J = s->jobs[id];
+        left += (main_units(J) - J.next_main) * J.per_unit;
+    }
+    const u64 task_ranks = std::min(TASK_RANKS_MAX, std::max(TASK_RANKS_MIN, std::min(left, budget) / (16ull * (u64)s->sm_count)));
+    const int unit_cap = s->max_units * 8;
+    u64 used = 0;
+    int ntasks = 0;
+    std::map<Variant, std::vector<ServeTask>> tasks;
     bool progress = true;
-    while (progress && used < budget && (int)tasks.size() < s->max_tasks) {
+    while (progress && used < budget && ntasks < s->max_tasks) {
         progress = false;
         for (u64 id : run) {
-            if (used >= budget || (int)tasks.size() >= s->max_tasks) break;
+            if (used >= budget || ntasks >= s->max_tasks) break;
             SJob& J = s->jobs[id];
             if (!remaining(J)) continue;
             ServeTask t;
             memset(&t, 0, sizeof t);
-            t.args = J.base;
             t.slot = (u32)J.slot;
-            std::vector<Unit> ex;
-            if (J.next_main < J.plan.main_count) {
-                u64 k = std::max<u64>(1, TASK_RANKS / J.per_unit);
-                k = std::min(k, J.plan.main_count - J.next_main);
-                t.args.main_base = J.plan.main_base + J.next_main;
-                t.args.main_count = k;
-                t.args.n_units = k;
+            t.kind = J.kind;
+            if (J.next_main < main_units(J)) {
+                const u64 k = std::min(std::max<u64>(1, task_ranks / J.per_unit), main_units(J) - J.next_main);
+                t.lo = (J.var.merged ? 0 : J.plan.main_base) + J.next_main;
+                t.hi = t.lo + k;
                 J.next_main += k;
                 used += k * J.per_unit;
             } else {
-                if (units_used + J.plan.extra.size() > unit_cap) continue;   // next tick
-                units_used += J.plan.extra.size();
-                ex = J.plan.extra;
-                t.args.main_base = 0;
-                t.args.main_count = 0;
-                t.args.n_units = ex.size();
+                const int k = (int)J.plan.extra.size();
+                if (T.nunits + k > unit_cap) continue;   // next tick
+                memcpy(T.h_units + T.nunits, J.plan.extra.data(), sizeof(Unit) * (size_t)k);
+                t.units = T.d_units + T.nunits;
+                t.hi = (u64)k;
+                T.nunits += k;
                 J.extras_issued = true;
                 used += 1;
             }
-            if (!remaining(J)) T.finishing.push_back(id);
-            tasks.push_back({J.var, t});
-            task_units.push_back(std::move(ex));
+            if (!remaining(J)) T.finishing.push_back({id, J.slot});
+            tasks[J.var].push_back(t);
+            ntasks++;
             progress = true;
         }
     }
-    // group by kernel variant, lay out tasks and extra units
-    std::vector<int> order(tasks.size());
-    for (size_t i = 0; i < order.size(); i++) order[i] = (int)i;
-    std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return tasks[x].first < tasks[y].first; });
-    for (int idx : order) {
-        ServeTask t = tasks[idx].second;
-        const std::vector<Unit>& ex = task_units[idx];
-        if (!ex.empty()) {
-            memcpy(T.h_units + T.nunits, ex.data(), sizeof(Unit) * ex.size());
-            t.args.units = T.d_units + T.nunits;
-            T.nunits += (int)ex.size();
-        }
-        if (T.groups.empty() || !(T.groups.back().first == tasks[idx].first))
-            T.groups.push_back({tasks[idx].first, {T.ntasks, 0}});
-        T.groups.back().second.second++;
-        T.h_tasks[T.ntasks++] = t;
+    for (const auto& kv : tasks) {   // one launch per kernel variant
+        T.groups.push_back({kv.first, {T.ntasks, (int)kv.second.size()}});
+        memcpy(T.h_tasks + T.ntasks, kv.second.data(), sizeof(ServeTask) * kv.second.size());
+        T.ntasks += (int)kv.second.size();
     }
 }
 
 cudaError_t launch_tick(war_server* s, Tick& T) {
     cudaError_t e;
-    for (u64 id : T.admitted) {
-        if ((e = cudaMemsetAsync(s->d_slots + s->jobs[id].slot, 0, sizeof(DevAcc), s->s_comp)) != cudaSuccess) return e;
+    for (const auto& ad : T.admitted) {
+        const int slot = ad.first;
+        if ((e = cudaMemsetAsync(s->d_slots + slot, 0, sizeof(DevAcc), s->s_comp)) != cudaSuccess) return e;
+        if ((e = cudaMemcpyAsync(s->d_jobs + slot, s->h_jobs + slot, sizeof(ServeJob), cudaMemcpyHostToDevice,
+                                 s->s_comp)) != cudaSuccess)
+            return e;
+        const size_t at = (size_t)slot * SLOT_BLOCKS;
+        if (ad.second && (e = cudaMemcpyAsync(s->d_blocks + at, s->h_blocks + at, sizeof(MBlock) * ad.second,
+                                              cudaMemcpyHostToDevice, s->s_comp)) != cudaSuccess)
+            return e;
     }
     T.admitted.clear();
     if (T.ntasks == 0) return cudaSuccess;
@@ -340,10 +446,14 @@ cudaError_t launch_tick(war_server* s, Tick& T) {
         return e;
     for (auto& g : T.groups) {
         int hb = 0;
-        for (int i = g.second.first; i < g.second.first + g.second.second; i++) hb = std::max(hb, T.h_tasks[i].args.hbins);
+        for (int i = g.second.first; i < g.second.first + g.second.second; i++) {
+            const ServeJob& J = s->h_jobs[T.h_tasks[i].slot];
+            hb = std::max(hb, g.first.merged ? J.merge.hbins : J.batch.hbins);
+        }
         // every task of the group zeroes and flushes hbins of its own; the launch provides the largest
-        size_t shmem = sizeof(u32) * (size_t)(hb + WAR_EBINS);
-        g.first.fn()<<<g.second.second, g.first.threads(), shmem, s->s_comp>>>(T.d_tasks + g.second.first, s->d_slots);
+        const size_t shmem = g.first.shmem(hb);
+        g.first.fn()<<<g.second.second, g.first.threads(), shmem, s->s_comp>>>(T.d_tasks + g.second.first, s->d_jobs,
+                                                                              s->d_slots);
         note_launch();
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
@@ -401,7 +511,7 @@ void worker_main(war_server* s) {
                     if (kv.second.state <= 1) { kv.second.state = 3; kv.second.status = WAR_ECUDA; }
                 s->cv_done.notify_all();
             } else {
-                for (u64 id : P.finishing) finish_job(s, id);
+                finish_jobs(s, P.finishing);
             }
             P.finishing.clear();
         }
@@ -457,8 +567,14 @@ int war_server_create(const war_server_cfg* cfg, war_server** out) {
     }
     s->max_tasks = 16384;
     s->max_units = s->max_tasks + 4 * UNITS_PER_EXTRA_CAP;
-    bool ok = cudaMalloc(&s->d_slots, sizeof(DevAcc) * (size_t)s->nslots) == cudaSuccess &&
-              cudaMallocHost(&s->h_slot, sizeof(DevAcc)) == cudaSuccess &&
+    const size_t nblocks = (size_t)s->nslots * SLOT_BLOCKS;
+    bool ok = upload_merge_table(&s->d_table) == cudaSuccess &&
+              cudaMalloc(&s->d_blocks, sizeof(MBlock) * nblocks) == cudaSuccess &&
+              cudaMallocHost(&s->h_blocks, sizeof(MBlock) * nblocks) == cudaSuccess &&
+              cudaMalloc(&s->d_jobs, sizeof(ServeJob) * (size_t)s->nslots) == cudaSuccess &&
+              cudaMallocHost(&s->h_jobs, sizeof(ServeJob) * (size_t)s->nslots) == cudaSuccess &&
+              cudaMalloc(&s->d_slots, sizeof(DevAcc) * (size_t)s->nslots) == cudaSuccess &&
+              cudaMallocHost(&s->h_slot, sizeof(DevAcc) * READBACK) == cudaSuccess &&
               cudaStreamCreateWithFlags(&s->s_comp, cudaStreamNonBlocking) == cudaSuccess &&
               cudaStreamCreateWithFlags(&s->s_copy, cudaStreamNonBlocking) == cudaSuccess;
     for (int i = 0; ok && i < 2; i++) {
@@ -574,6 +690,11 @@ int war_server_destroy(war_server* s) {
         if (T.ev) cudaEventDestroy(T.ev);
     }
     if (s->memo_arena) cudaFree(s->memo_arena);
+    if (s->d_table) cudaFree(s->d_table);
+    if (s->d_jobs) cudaFree(s->d_jobs);
+    if (s->h_jobs) cudaFreeHost(s->h_jobs);
+    if (s->d_blocks) cudaFree(s->d_blocks);
+    if (s->h_blocks) cudaFreeHost(s->h_blocks);
     if (s->d_slots) cudaFree(s->d_slots);
     if (s->h_slot) cudaFreeHost(s->h_slot);
     if (s->s_comp) cudaStreamDestroy(s->s_comp);
