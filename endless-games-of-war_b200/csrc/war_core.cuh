@@ -73,11 +73,12 @@ struct TurnK {
 //   length: qq = 4*len1 - 2n, pos = s*qq + (2n-4) and qq += 4s with s = +1 (player 1 won) or -1;
 //          the game is over when qq*qq == (2n)^2.
 template <int RULE>
-__device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const TurnK& K) {
+__device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const TurnK& K, u32& c1, u32& c2) {
     const u32 l1 = (u32)w1, h1 = (u32)(w1 >> 32), l2 = (u32)w2, h2 = (u32)(w2 >> 32);
     const u32 nl1 = __funnelshift_r(l1, h1, 4), nl2 = __funnelshift_r(l2, h2, 4);
     const u32 nh1 = __umulhi(h1, K.k2p28), nh2 = __umulhi(h2, K.k2p28);
-    const u32 c1 = l1 + nl1 * K.km16, c2 = l2 + nl2 * K.km16;
+    c1 = l1 + nl1 * K.km16;
+    c2 = l2 + nl2 * K.km16;
     const bool p1 = c1 > c2;
     const u32 pa = RULE ? c2 + c1 * K.k16 : c1 + c2 * K.k16;   // player 1 won
     const u32 pb = RULE ? c1 + c2 * K.k16 : c2 + c1 * K.k16;   // player 2 won
@@ -95,6 +96,12 @@ __device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const Tu
     w2 = ((u64)a2h << 32) | (u32)a2;
     qq = qq + (u32)s * K.k4;
     return p1;
+}
+
+template <int RULE>
+__device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const TurnK& K) {
+    u32 c1, c2;   // the cards played
+    return war_turn_fma<RULE>(w1, w2, qq, K, c1, c2);
 }
 
 // The same turn with the rule chosen at run time (serving kernel, checks).

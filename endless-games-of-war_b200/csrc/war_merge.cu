@@ -10,9 +10,9 @@ namespace war {
 
 template <int RULE>
 __global__ void __launch_bounds__(1024) merge_kernel(const __grid_constant__ MergeArgs a, DevAcc* __restrict__ acc) {
-    extern __shared__ u32 sh[];
+    extern __shared__ u64 sh64[];
     __shared__ UnitStore store;
-    merge_body<RULE>(a, acc, &acc->work_next, store, sh);
+    merge_body<RULE>(a, acc, &acc->work_next, store, sh64);
 }
 
 template <int RULE, bool EXTRA, bool SHAPE>
@@ -208,10 +208,12 @@ int merge_args(const war_job* job, const MergePlan& p, int hbins, int window, in
     return WAR_OK;
 }
 
-static size_t merge_shmem(int hbins) { return sizeof(u32) * (size_t)(hbins + WAR_EBINS); }
+static size_t merge_shmem(int threads, int hbins) {
+    return sizeof(Missed) * (size_t)threads + sizeof(u32) * (size_t)(hbins + WAR_EBINS);
+}
 
 cudaError_t launch_merged(const MergeArgs& a, int rule, int threads, int blocks, DevAcc* acc, cudaStream_t st) {
-    (rule ? merge_kernel<1> : merge_kernel<0>)<<<blocks, threads, merge_shmem(a.hbins), st>>>(a, acc);
+    (rule ? merge_kernel<1> : merge_kernel<0>)<<<blocks, threads, merge_shmem(threads, a.hbins), st>>>(a, acc);
     note_launch();
     return cudaGetLastError();
 }
@@ -219,13 +221,13 @@ cudaError_t launch_merged(const MergeArgs& a, int rule, int threads, int blocks,
 int merged_max_blocks_per_sm(int rule, int threads, int hbins) {
     int nb = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rule ? merge_kernel<1> : merge_kernel<0>, threads,
-                                                      merge_shmem(hbins)) != cudaSuccess)
+                                                      merge_shmem(threads, hbins)) != cudaSuccess)
         return 0;
     return nb;
 }
 
 static size_t canon_shmem(int extra, int threads, int hbins) {
-    return sizeof(u32) * (size_t)(hbins + WAR_EBINS) + (extra ? sizeof(ulonglong2) * (size_t)threads : 0);
+    return merge_shmem(threads, hbins) + (extra ? 2 * sizeof(u64) * (size_t)threads : 0);
 }
 
 typedef void (*MergeFn)(const MergeArgs, DevAcc*);

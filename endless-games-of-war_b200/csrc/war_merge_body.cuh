@@ -3,15 +3,20 @@
 //
 // The loop is the latched loop of war_refill.cuh for one game per lane: `defer` turns without a branch or a
 // vote, then a service that saves Brent's checkpoint, looks the game up in the memo, records it if it is
-// decided and gives its lane the next one.  A game starts at turn h, so its tortoise is the state at turn h
-// and its checkpoints follow from there.
+// decided and gives its lane the next one.  A merged game starts at turn h, so its tortoise is the state at turn
+// h and its checkpoints follow from there.
 //
-// What bounds it: random reads and writes of the table in HBM, as in the kernel that played every deal, but
-// nine times fewer (all 13! deals: 5.8e8 lookups and 1.6e8 stores instead of 6.2e9 and 3.8e8) and, for jobs of
-// fewer than about 1e6 games, the longest game.  Measured on a B200 against the one-deal-one-game kernel it
-// replaces: all 13! deals 166 -> 20.1 ms, the end of them from a saved progress 168 -> 33.5 ms, a span of
-// 4.26e9 of 14 cards with --half 124 -> 17.1 ms and of 15 cards 370 -> 168 ms, 1e8 of 13 cards 10.7 -> 2.9 ms,
-// 3e5 of 10 cards 1.71 -> 0.076 ms (there the 720-deal units of one lane each were the time).
+// Landmarks.  What is looked up and stored is not the state at the service but the last landmark before it: a
+// state with card n-1 on top of its holder's pile (every card reaches the top again within a lap of the pile).
+// Games that have met look at the same landmarks whatever turn they have got to, where states at services
+// meet only in games of one phase; and a cycle is stored by its landmarks, about one state in eight.
+//
+// What bounds it: random reads and writes of the table in HBM (13 cards: at the rate of the random-gather ceiling),
+// instruction issue of the turns (canonical scans: ALU pipe 84%), and for jobs of fewer than about 1e6 games the
+// longest game.  Measured on a B200 (states at services -> landmarks -> a found cycle recorded by playing on instead
+// of by a walk): a span of 4.26e9 deals of 15 cards 210 -> 132 -> 85 ms (stores 3.4e9 -> 1.0e9), 1e8 deals of 13 cards
+// 2.5 -> 2.0 -> 1.6 ms, a resumed a(13) 31.2 -> 30.5 -> 29.9 ms, --half span of 14 cards 13.7 -> 13.6 ms, 3e9
+// canonical positions of 14 cards 152 -> 148 ms.  The one-deal-one-game kernel before: 370, 10.7, 168 and 124 ms.
 #pragma once
 #include "war_refill.cuh"
 #include "war_merge.cuh"
@@ -26,17 +31,52 @@ union UnitStore {
 
 // One game slot of the merged kernel.
 struct MGame {
-    u64 w1, w2, t1, t2, ka, kb;
-    u32 q, rounds, next, wt, ta, tb, mv;
+    u64 w1, w2, t1, t2, m1, m2;   // piles, tortoise, the last landmark
+    u32 q, rounds, next, wt, mv, at;
     bool done, kcy, active;
 };
 
+// A game's last two landmarks looked up and missed, and their turns + 1 (0: none), kept in shared memory.
+struct Missed {
+    u64 ka, kb;
+    u32 ta, tb;
+};
+constexpr u32 NO_LANDMARK = 0xFFFFFFFFu;
+// A game whose cycle Brent found plays on around it once more, to the tortoise's state again, and its services store
+// the cycle's landmarks instead of looking them up: the other lanes go on meanwhile, where a walk of the cycle at
+// once holds them up.  (Its checkpoint is this, which is never reached.)
+constexpr u32 RECORDING = 0xFFFFFFFFu;
+
+// Stores the landmarks that a decided game missed, with its outcome: the cycle value vcyc, or (vcyc = 0) the turns
+// from there to its end after len turns.  Returns the entries stored.
+__device__ __forceinline__ u32 store_missed(u64* memo, u32 mbits, const Missed& x, u32 vcyc, u32 len) {
+    const u32 vmask = (1u << mbits) - 1u;
+    u32 k = 0;
+    if (x.ta) {
+        const u32 v = vcyc ? vcyc : 2u * (len + 1u - x.ta) + 1u;
+        if (v <= vmask) {
+            __stcg((unsigned long long*)memo + memo_slot(x.ka, mbits), path_entry(x.ka, mbits, v));
+            k++;
+        }
+    }
+    if (x.tb) {
+        const u32 v = vcyc ? vcyc : 2u * (len + 1u - x.tb) + 1u;
+        if (v <= vmask) {
+            __stcg((unsigned long long*)memo + memo_slot(x.kb, mbits), path_entry(x.kb, mbits, v));
+            k++;
+        }
+    }
+    return k;
+}
+
 template <int RULE>
 __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restrict__ acc, u64* __restrict__ counter,
-                                           UnitStore& store, u32* sh) {
+                                           UnitStore& store, u64* sh64) {
     MUnit* const units = store.m;
-    u32* shh = sh;
-    u32* she = sh + a.hbins;
+    Missed* const miss = (Missed*)sh64 + threadIdx.x;
+    u32* const sh = (u32*)((Missed*)sh64 + blockDim.x);
+    u32* const shh = sh;
+    u32* const she = sh + a.hbins;
     const int bins = a.hbins + WAR_EBINS;
     for (int b = threadIdx.x; b < bins; b += blockDim.x) sh[b] = 0;
     __syncthreads();
@@ -56,7 +96,7 @@ __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restric
     u32 cyc = 0, turns = 0, maxfin = 0, capped = 0, mlook = 0, mhit = 0, mstore = 0;
     MGame g;
     g.active = false; g.done = true; g.kcy = false; g.w1 = g.w2 = 1ull; g.t1 = g.t2 = 0ull; g.q = 0; g.rounds = 0;
-    g.next = 0xFFFFFFFFu; g.ta = g.tb = 0; g.ka = g.kb = 0; g.mv = 0; g.wt = 0;
+    g.next = 0xFFFFFFFFu; g.m1 = g.m2 = 0ull; g.at = NO_LANDMARK; g.mv = 0; g.wt = 0;
 
     auto drain = [&]() {
         __syncwarp();
@@ -96,7 +136,8 @@ __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restric
         }
         g.q = mu.s1 + a8 - n2;
         g.t1 = g.w1; g.t2 = g.w2; g.rounds = h; g.next = 2u * h + W;
-        g.ta = 0; g.tb = 0; g.mv = 0; g.wt = c.wt;
+        g.mv = 0; g.wt = c.wt; g.at = NO_LANDMARK;
+        miss->ta = 0; miss->tb = 0;
         g.done = false; g.kcy = false; g.active = true;
         return true;
     };
@@ -111,7 +152,13 @@ __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restric
         for (int k = 0; k < period; k += 4) {
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                war_turn_fma<RULE>(g.w1, g.w2, g.q, K);
+                const u64 v1 = g.w1, v2 = g.w2;
+                u32 c1, c2;
+                war_turn_fma<RULE>(g.w1, g.w2, g.q, K, c1, c2);
+                const bool top = (c1 == n - 1u) | (c2 == n - 1u);
+                g.m1 = top ? v1 : g.m1;
+                g.m2 = top ? v2 : g.m2;
+                g.at = top ? (u32)(k + u) : g.at;
                 const bool en = g.q * g.q == K.end2;
                 if (!g.done) g.rounds += K.one;
                 const bool cy = (g.w1 == g.t1) & (g.w2 == g.t2);
@@ -124,46 +171,40 @@ __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restric
             if (g.next > WAR_TURN_CAP) { capped++; g.done = true; }   // abandoned (never expected): the job fails
             else { g.t1 = g.w1; g.t2 = g.w2; g.next = 2u * g.rounds + W; }
         }
-        if (memo != nullptr && !g.done) {
-            const u64 key = memo_key_state(g.w1, g.w2, n);
-            const u64 e = __ldcg((const unsigned long long*)memo + memo_slot(key, mbits));
-            mlook++;
-            const u32 v = (u32)e & vmask;
-            if (v != 0u && ((e ^ path_entry(key, mbits, 0ull)) >> mbits) == 0ull) {
-                mhit++;
-                g.done = true; g.kcy = (v & 1u) == 0u; g.mv = v;
+        if (memo != nullptr && g.done && g.kcy && g.mv == 0u) {   // found by Brent: record the cycle
+            const u32 v = 2u * (g.rounds - ((g.next - W) >> 1));
+            if (v <= vmask) { g.mv = v; g.next = RECORDING; g.done = false; }
+        } else if (memo != nullptr && !g.done && g.at != NO_LANDMARK) {
+            const u64 key = memo_key_state(g.m1, g.m2, n);
+            const u32 at = g.rounds - (u32)period + g.at;
+            if (g.next == RECORDING) {
+                __stcg((unsigned long long*)memo + memo_slot(key, mbits), path_entry(key, mbits, g.mv));
+                mstore++;
             } else {
-                g.kb = g.ka; g.tb = g.ta;
-                g.ka = key; g.ta = g.rounds;
+                const u64 e = __ldcg((const unsigned long long*)memo + memo_slot(key, mbits));
+                mlook++;
+                const u32 v = (u32)e & vmask;
+                if (v != 0u && ((e ^ path_entry(key, mbits, 0ull)) >> mbits) == 0ull) {
+                    mhit++;
+                    g.done = true; g.kcy = (v & 1u) == 0u; g.mv = v;
+                    g.next = at + (v >> 1);   // the game's length, if it ends
+                } else {
+                    miss->kb = miss->ka; miss->tb = miss->ta;
+                    miss->ka = key; miss->ta = at + 1u;
+                }
             }
         }
+        g.at = NO_LANDMARK;
         const bool fin = g.done & g.active;
         if (__any_sync(WAR_FULL_MASK, fin)) {
             if (fin) {
                 turns += g.rounds - h;
                 const u32 mcy = (g.mv & 1u) ? 0u : g.mv >> 1;
-                const u32 len = (g.mv & 1u) ? g.rounds + (g.mv >> 1) : g.rounds;
+                const u32 len = (g.mv & 1u) ? g.next : g.rounds;
                 const u32 lam = mcy ? mcy : g.rounds - ((g.next - W) >> 1);
-                if (g.ta) {   // the states it missed, with its outcome (none without a table)
-                    const u32 v = g.kcy ? 2u * lam : 2u * (len - g.ta) + 1u;
-                    if (v <= vmask) {
-                        __stcg((unsigned long long*)memo + memo_slot(g.ka, mbits), path_entry(g.ka, mbits, v));
-                        mstore++;
-                    }
-                }
-                if (g.tb) {
-                    const u32 v = g.kcy ? 2u * lam : 2u * (len - g.tb) + 1u;
-                    if (v <= vmask) {
-                        __stcg((unsigned long long*)memo + memo_slot(g.kb, mbits), path_entry(g.kb, mbits, v));
-                        mstore++;
-                    }
-                }
+                mstore += store_missed(memo, mbits, *miss, g.kcy ? 2u * lam : 0u, len);
                 if (g.kcy) {
                     cyc += g.wt;
-                    if (memo != nullptr && mcy == 0u) {   // found by Brent: store its cycle
-                        memo_store_cycle<RULE, MEMO_PATH>(memo, mbits, g.w1, g.w2, g.q + n2, n, lam);
-                        mstore += lam;
-                    }
                     if (a.hbins) atomicAdd(&shh[lam < hb1 ? lam : hb1], g.wt);
                 } else {
                     maxfin = max(maxfin, len);
@@ -207,17 +248,18 @@ __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restric
 // 152 ms (defer 16; 12: 156, 8: 176 ms; 256 to 1024 threads alike).
 template <bool EXTRA>
 struct CGame {
-    u64 w1, w2, t1, t2, ka, kb;
-    u32 q, rounds, next, ta, tb, mv, pend;
-    bool done, kcy, active, sampled;
+    u64 w1, w2, t1, t2, m1, m2;
+    u32 q, rounds, next, mv, pend, at;
+    bool done, kcy, active, sampled, first;   // first: on the cycle from its start
 };
 
 template <int RULE, bool EXTRA, bool SHAPE>
 __device__ __forceinline__ void canon_body(const MergeArgs& a, DevAcc* __restrict__ acc, u64* __restrict__ counter,
                                            UnitStore& store, u64* sh64) {
     CUnit* const units = store.c;
-    ulonglong2* const start = (ulonglong2*)sh64 + threadIdx.x;      // EXTRA: the starting piles
-    u32* const shh = (u32*)((ulonglong2*)sh64 + (EXTRA ? blockDim.x : 0u));
+    Missed* const miss = (Missed*)sh64 + threadIdx.x;
+    u64* const starts = (u64*)((Missed*)sh64 + blockDim.x);             // EXTRA: the starting piles
+    u32* const shh = (u32*)(starts + (EXTRA ? 2u * blockDim.x : 0u));
     u32* const she = shh + a.hbins;
     const int bins = a.hbins + WAR_EBINS;
     for (int b = threadIdx.x; b < bins; b += blockDim.x) shh[b] = 0;
@@ -237,8 +279,8 @@ __device__ __forceinline__ void canon_body(const MergeArgs& a, DevAcc* __restric
     u32 cyc = 0, turns = 0, maxfin = 0, capped = 0, mlook = 0, mhit = 0, mstore = 0, nonstd = 0, unchk = 0;
     u32 sc = 0, scy = 0, slam = 0, slen = 0, smax = 0, oncyc = 0, dmin = 0;
     CGame<EXTRA> g;
-    g.active = false; g.done = true; g.kcy = false; g.sampled = false; g.w1 = g.w2 = 1ull; g.t1 = g.t2 = 0ull;
-    g.q = 0; g.rounds = 0; g.next = 0xFFFFFFFFu; g.ta = g.tb = 0; g.ka = g.kb = 0; g.mv = 0; g.pend = 0;
+    g.active = false; g.done = true; g.kcy = false; g.sampled = g.first = false; g.w1 = g.w2 = 1ull; g.t1 = g.t2 = 0ull;
+    g.q = 0; g.rounds = 0; g.next = 0xFFFFFFFFu; g.m1 = g.m2 = 0ull; g.at = NO_LANDMARK; g.mv = 0; g.pend = 0;
 
     // (A launch plays fewer than 2^32 positions: no bin and no total of a lane or warp can wrap.)
     auto drain = [&]() {};
@@ -256,10 +298,12 @@ __device__ __forceinline__ void canon_body(const MergeArgs& a, DevAcc* __restric
         canon_position(cu.Q | ((u64)merge_row(cu.c0, cu.c1, sel) << (4u * (m - c.fi))), n, c.pa, g.w1, g.w2, q4);
         g.q = q4 - n2;
         g.t1 = g.w1; g.t2 = g.w2; g.rounds = 0; g.next = W;
-        g.ta = 0; g.tb = 0; g.mv = 0; g.pend = 0;
+        g.mv = 0; g.pend = 0; g.at = NO_LANDMARK; g.first = false;
+        miss->ta = 0; miss->tb = 0;
         g.done = false; g.kcy = false; g.active = true;
         if (EXTRA) {
-            *start = make_ulonglong2(g.w1, g.w2);
+            starts[threadIdx.x] = g.w1;
+            starts[threadIdx.x + blockDim.x] = g.w2;
             g.sampled = a.sample && war_pick(a.seed, a.thr, g.w1, g.w2);
         }
         return true;
@@ -275,7 +319,13 @@ __device__ __forceinline__ void canon_body(const MergeArgs& a, DevAcc* __restric
         for (int k = 0; k < period; k += 4) {
 #pragma unroll
             for (int u = 0; u < 4; u++) {
-                war_turn_fma<RULE>(g.w1, g.w2, g.q, K);
+                const u64 v1 = g.w1, v2 = g.w2;
+                u32 c1, c2;
+                war_turn_fma<RULE>(g.w1, g.w2, g.q, K, c1, c2);
+                const bool top = (c1 == n - 1u) | (c2 == n - 1u);
+                g.m1 = top ? v1 : g.m1;
+                g.m2 = top ? v2 : g.m2;
+                g.at = top ? (u32)(k + u) : g.at;
                 const bool en = g.q * g.q == K.end2;
                 if (!g.done) g.rounds += K.one;
                 const bool cy = (g.w1 == g.t1) & (g.w2 == g.t2);
@@ -288,69 +338,67 @@ __device__ __forceinline__ void canon_body(const MergeArgs& a, DevAcc* __restric
             if (g.next > WAR_TURN_CAP) { capped++; g.done = true; }   // abandoned (never expected): the job fails
             else { g.t1 = g.w1; g.t2 = g.w2; g.next = 2u * g.rounds + W; }
         }
-        if (memo == nullptr) {
-        } else if (!g.done && g.pend == 0u) {
-            const u64 key = memo_key_state(g.w1, g.w2, n);
-            const u64 e = __ldcg((const unsigned long long*)memo + memo_slot(key, mbits));
-            mlook++;
-            const u32 v = (u32)e & vmask;
-            if (v != 0u && ((e ^ path_entry(key, mbits, 0ull)) >> mbits) == 0ull) {
-                mhit++;
-                const bool vcy = (v & 1u) == 0u;
-                if (EXTRA && a.distinct && vcy && (v >> lsh) <= W && g.rounds < (v >> lsh)) g.pend = v;
-                else { g.done = true; g.kcy = vcy; g.mv = v; }
+        if (g.done && g.kcy && g.mv == 0u && g.active) {   // found by Brent: record the cycle
+            const u32 lam = g.rounds - ((g.next - W) >> 1);
+            const u32 code = SHAPE ? (u32)loop_shape_walk<RULE>(g.w1, g.w2, g.q + n2, k4m4, lam, (u32)a.blk) : 0u;
+            const u32 v = SHAPE ? 8u * lam + 2u * code : 2u * lam;
+            g.first = g.next == W;
+            g.mv = v;
+            g.pend = 0u;
+            if (memo != nullptr && v <= vmask) { g.next = RECORDING; g.done = false; }
+        } else if (memo == nullptr) {
+        } else if (!g.done && g.pend == 0u && g.at != NO_LANDMARK) {
+            const u64 key = memo_key_state(g.m1, g.m2, n);
+            const u32 at = g.rounds - (u32)period + g.at;
+            if (g.next == RECORDING) {
+                __stcg((unsigned long long*)memo + memo_slot(key, mbits), path_entry(key, mbits, g.mv));
+                mstore++;
             } else {
-                g.kb = g.ka; g.tb = g.ta;
-                g.ka = key; g.ta = g.rounds;
+                const u64 e = __ldcg((const unsigned long long*)memo + memo_slot(key, mbits));
+                mlook++;
+                const u32 v = (u32)e & vmask;
+                if (v != 0u && ((e ^ path_entry(key, mbits, 0ull)) >> mbits) == 0ull) {
+                    mhit++;
+                    const bool vcy = (v & 1u) == 0u;
+                    if (EXTRA && a.distinct && vcy && (v >> lsh) <= W && g.rounds < (v >> lsh)) g.pend = v;
+                    else {
+                        g.done = true; g.kcy = vcy; g.mv = v;
+                        if (!vcy) g.next = at + (v >> 1);   // the game's length
+                    }
+                } else {
+                    miss->kb = miss->ka; miss->tb = miss->ta;
+                    miss->ka = key; miss->ta = at + 1u;
+                }
             }
-        } else if (EXTRA && !g.done && g.rounds >= (g.pend >> lsh)) {
+        } else if (EXTRA && !g.done && g.pend != 0u && g.rounds >= (g.pend >> lsh)) {
             // turn lam passed without the start coming back: on the cycle, not through the start
             g.done = true; g.kcy = true; g.mv = g.pend;
         }
+        g.at = NO_LANDMARK;
         const bool fin = g.done & g.active;
         if (__any_sync(WAR_FULL_MASK, fin)) {
             if (fin) {
                 turns += g.rounds;
                 const bool cy = g.kcy;
                 const u32 mcy = (g.mv & 1u) ? 0u : g.mv >> lsh;
-                const u32 len = (g.mv & 1u) ? g.rounds + (g.mv >> 1) : g.rounds;
-                const u32 lam = mcy ? mcy : g.rounds - ((g.next - W) >> 1);
-                u32 code = 0;
+                const u32 len = (g.mv & 1u) ? g.next : g.rounds;
+                const u32 lam = mcy;      // (of a cycle: Brent's are values by now, too)
                 if (SHAPE && cy) {
-                    code = mcy ? (g.mv >> 1) & 3u : (u32)loop_shape_walk<RULE>(g.w1, g.w2, g.q + n2, k4m4, lam, (u32)a.blk);
+                    const u32 code = (g.mv >> 1) & 3u;
                     if (code == 1u) nonstd++;
                     if (code == 2u) unchk++;
                 }
-                const u32 vcyc = SHAPE ? 8u * lam + 2u * code : 2u * lam;
-                if (g.ta) {   // the states it missed, with its outcome
-                    const u32 v = cy ? vcyc : 2u * (len - g.ta) + 1u;
-                    if (v <= vmask) {
-                        __stcg((unsigned long long*)memo + memo_slot(g.ka, mbits), path_entry(g.ka, mbits, v));
-                        mstore++;
-                    }
-                }
-                if (g.tb) {
-                    const u32 v = cy ? vcyc : 2u * (len - g.tb) + 1u;
-                    if (v <= vmask) {
-                        __stcg((unsigned long long*)memo + memo_slot(g.kb, mbits), path_entry(g.kb, mbits, v));
-                        mstore++;
-                    }
-                }
+                mstore += store_missed(memo, mbits, *miss, cy ? g.mv : 0u, len);
                 if (cy) {
                     cyc++;
-                    if (memo != nullptr && mcy == 0u) {   // found by Brent: store its cycle
-                        memo_store_cycle<RULE, MEMO_PATH>(memo, mbits, g.w1, g.w2, g.q + n2, n, lam, vcyc);
-                        mstore += lam;
-                    }
                     if (a.hbins) atomicAdd(&shh[lam < hb1 ? lam : hb1], 1u);
                     if (EXTRA && a.distinct) {
                         // decided by the memo: the start was not seen again within lam <= W turns, or lam > W: walk
-                        const ulonglong2 s = *start;
-                        const u32 sq = 4u * pile_len(s.x);
-                        const bool on = mcy == 0u && g.next == W ? true
-                                      : (lam <= W ? false : on_cycle_walk<RULE>(s.x, s.y, sq, n, lam));
+                        const u64 s1 = starts[threadIdx.x], s2 = starts[threadIdx.x + blockDim.x];
+                        const u32 sq = 4u * pile_len(s1);
+                        const bool on = g.first || (lam > W && on_cycle_walk<RULE>(s1, s2, sq, n, lam));
                         if (on) {
-                            const CycleWalk cw = cycle_walk<RULE>(s.x, s.y, sq, n, lam);
+                            const CycleWalk cw = cycle_walk<RULE>(s1, s2, sq, n, lam);
                             oncyc++;
                             if (cw.is_min) dmin++;
                             if (a.dbins) {

@@ -98,8 +98,8 @@ __global__ void __launch_bounds__(1024) serve_merge_kernel(ServeTask* __restrict
     __syncthreads();
     DevAcc* const acc = slots + t->slot;
     switch (t->kind) {
-        case 0: merge_body<0>(A, acc, &t->counter, store, (u32*)sh64); break;
-        case 1: merge_body<1>(A, acc, &t->counter, store, (u32*)sh64); break;
+        case 0: merge_body<0>(A, acc, &t->counter, store, sh64); break;
+        case 1: merge_body<1>(A, acc, &t->counter, store, sh64); break;
         case 2: canon_body<0, false, false>(A, acc, &t->counter, store, sh64); break;
         case 3: canon_body<1, false, false>(A, acc, &t->counter, store, sh64); break;
         case 4: canon_body<0, true, false>(A, acc, &t->counter, store, sh64); break;
@@ -129,7 +129,7 @@ struct Variant {
     bool operator==(const Variant& o) const { return !(*this < o) && !(o < *this); }
     int threads() const { return 256; }
     size_t shmem(int hbins) const {   // (a merged launch may hold canonical tasks that keep their starts)
-        return sizeof(u32) * (size_t)(hbins + WAR_EBINS) + (merged ? sizeof(ulonglong2) * (size_t)threads() : 0);
+        return sizeof(u32) * (size_t)(hbins + WAR_EBINS) + (merged ? (sizeof(Missed) + 2 * sizeof(u64)) * (size_t)threads() : 0);
     }
     template <int RULE>
     ServeFn fn_rule() const {
