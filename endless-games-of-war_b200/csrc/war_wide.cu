@@ -300,69 +300,125 @@ __global__ void __launch_bounds__(1024) wide_kernel(const __grid_constant__ Wide
 // The step cap must not fall before the turns that are not played: at least 2W (Brent), 2h + 2 (Floyd), h + the
 // longest period (streak).
 //
-// What bounds it: instruction issue of the turns, as before; the gain is the deals per game (3.2 in a block of 9!
-// deals of 18 cards, 5.3 in one of 11!) and, in short jobs, units that a whole warp plays instead of one lane.
-// B200: 5e7 deals of 18 cards under Brent 45 -> 2.4 ms, 2e8 of 17 under the streak test 125 -> 16.8 ms (which also
-// plays one cycle length after the last break instead of the period); 256 or 512 threads alike, defer 16 (8: 2.5
-// and 17.8 ms, 32: 2.6 and 17.6 ms).
+// What bounds it: instruction issue of the turns; the gain over wide_kernel is the deals per game (3.2 in a block of
+// 9! deals of 18 cards, 5.3 in one of 11!), in short jobs units that a whole warp plays instead of one lane, and a
+// turn of half the operations (turn5_pred).  B200: 5e7 deals of 18 cards under Brent 45 -> 2.4 (turn5) -> 1.6 ms, 2e8
+// of 17 under the streak test 125 -> 16.8 -> 10.3 ms (which also plays one cycle length after the last break instead
+// of the period), 2e8 of 17 under Floyd 24.4 -> 15.3 ms; 256 or 512 threads alike, defer 16 (8: 1.8 and 11.7 ms, 32:
+// 1.6 and 10.2 ms).
+//
+// Piles here are 96 bits (a u64 and a u32) of cards 1..n in 5 bits each, without a sentinel: no card is 0, so the
+// words still tell the length, and 19 cards, the most a player can hold while the game goes on, fit.
 
-// The outer choice of a unit (MUnit with 5-bit cards and 128-bit piles): the outer pairs have 10 bits each.
+// Constants of turn5_pred as operands (war_core.cuh, TurnK).
+struct Turn5K {
+    u32 one, m1, m32, k32, k2p27, c1, c2;   // 1, -1, -32, 32, 2^27, -5, 5n - 5
+};
+
+// One turn.  qa = 5 * player 1's length.  Both tops are popped (two funnel shifts and a multiply-high each, the
+// card as lo - 32 lo'), the pair is built, placed and added to the winner's pile by multiply-adds, those of player 1's
+// win under a predicate: 9 operations are left to the ALU pipe (turn5: about 35), 17 go to the FMA pipe, which
+// balances the two with the loop's tests, which only the ALU pipe has.  Returns 1 if player 1 won.
+template <int RULE>
+__device__ __forceinline__ u32 turn5_pred(u64& a0, u32& a1, u64& b0, u32& b1, u32& qa, const Turn5K& K) {
+    const u32 l1 = (u32)a0, h1 = (u32)(a0 >> 32), l2 = (u32)b0, h2 = (u32)(b0 >> 32);
+    const u32 nl1 = __funnelshift_r(l1, h1, 5), nh1 = __funnelshift_r(h1, a1, 5);
+    const u32 nl2 = __funnelshift_r(l2, h2, 5), nh2 = __funnelshift_r(h2, b1, 5);
+    a1 = __umulhi(a1, K.k2p27);
+    b1 = __umulhi(b1, K.k2p27);
+    const u32 c1 = l1 + nl1 * K.m32, c2 = l2 + nl2 * K.m32;
+    const u32 f = RULE ? c1 : c2, g = RULE ? c2 : c1;   // player 2 won: f first in the pair; player 1: g
+    u64 x1 = ((u64)nh1 << 32) | nl1, x2 = ((u64)nh2 << 32) | nl2;
+    u32 w;
+    asm("{\n\t"
+        ".reg .pred p;\n\t"
+        ".reg .u32 t, ps, pt, xl, xh, yl, yh, al, ah, q;\n\t"
+        ".reg .u64 x, y;\n\t"
+        "setp.gt.u32 p, %6, %7;\n\t"
+        "mad.lo.u32 t, %9, %10, %8;\n\t"         // f + 32 g
+        "@p mad.lo.u32 t, %8, %10, %9;\n\t"      // g + 32 f
+        "mad.lo.u32 ps, %4, %12, %14;\n\t"       // the place under the winner's pile after the pop
+        "@p mad.lo.u32 ps, %4, %11, %13;\n\t"
+        "mad.lo.u32 q, %4, %11, -5;\n\t"
+        "@p mad.lo.u32 q, %4, %11, 5;\n\t"
+        "mov.u32 %4, q;\n\t"
+        "mad.lo.u32 pt, ps, %11, -32;\n\t"
+        "cvt.u64.u32 x, t;\n\t"
+        "shl.b64 y, x, pt;\n\t"
+        "shl.b64 x, x, ps;\n\t"
+        "mov.b64 {xl, xh}, x;\n\t"
+        "mov.b64 {yl, yh}, y;\n\t"
+        "@p mad.wide.u32 %0, xl, %11, %0;\n\t"
+        "@!p mad.wide.u32 %2, xl, %11, %2;\n\t"
+        "mov.b64 {al, ah}, %0;\n\t"
+        "@p mad.lo.u32 ah, xh, %11, ah;\n\t"
+        "mov.b64 %0, {al, ah};\n\t"
+        "mov.b64 {al, ah}, %2;\n\t"
+        "@!p mad.lo.u32 ah, xh, %11, ah;\n\t"
+        "mov.b64 %2, {al, ah};\n\t"
+        "@p mad.lo.u32 %1, yh, %11, %1;\n\t"
+        "@!p mad.lo.u32 %3, yh, %11, %3;\n\t"
+        "selp.u32 %5, 1, 0, p;\n\t"
+        "}"
+        : "+l"(x1), "+r"(a1), "+l"(x2), "+r"(b1), "+r"(qa), "=r"(w)
+        : "r"(c1), "r"(c2), "r"(f), "r"(g), "r"(K.k32), "r"(K.one), "r"(K.m1), "r"(K.c1), "r"(K.c2));
+    a0 = x1;
+    b0 = x2;
+    return w;
+}
+
+// The outer choice of a unit (MUnit with such cards and piles): the outer pairs have 10 bits each.
 struct WUnit {
-    u64 U1l, U1h, U2l, U2h, O;
+    u64 U1l, U2l, O;
+    u32 U1h, U2h;
     u32 c0, c1, s1, s2;
     u32 wins;          // bit t: player 1 wins turn t (turns of the fixed cards)
 };
 
-__device__ __forceinline__ void shl128(u64& lo, u64& hi, u32 s) {   // 0 <= s < 128
-    hi = shl64(hi, s) | shl64(lo, s - 64u) | shr64(lo, 64u - s);
-    lo = shl64(lo, s);
-}
-__device__ __forceinline__ void shr128(u64& lo, u64& hi, u32 s) {
-    lo = shr64(lo, s) | shr64(hi, s - 64u) | shl64(hi, 64u - s);
-    hi = shr64(hi, s);
-}
-__device__ __forceinline__ void put128(u64& lo, u64& hi, u64 v, u32 s) {
+// Adds v << s to a 96-bit pile; v << s may reach past bit 63 (s < 128).
+__device__ __forceinline__ void put96(u64& lo, u32& hi, u64 v, u32 s) {
     lo |= shl64(v, s);
-    hi |= shl64(v, s - 64u) | (s < 64u ? shr64(v, 64u - s) : 0ull);
+    hi |= (u32)(s < 64u ? shr64(v, 64u - s) : shl64(v, s - 64u));
 }
 
 template <int RULE>
 __device__ __forceinline__ void wide_unit(const MBlock& B, u64 outer, u32 n, WUnit& m) {
     u32 free = B.free_mask;
     const u32 b = B.b, f = B.f, fo = f > MERGE_INNER ? f - MERGE_INNER : 0u;
-    m.U1l = m.U1h = m.U2l = m.U2h = m.O = 0ull;
+    m.U1l = m.U2l = m.O = 0ull;
+    m.U1h = m.U2h = 0u;
     u32 s1 = 0, s2 = 0, half = 0, wins = 0;
     if ((b & 1u) && b < n) {
         const u32 k = (u32)__popc(free);
-        half = take_card(free, (u32)(outer % k));
+        half = take_card(free, (u32)(outer % k)) + 1u;
         outer /= k;
     }
     if (n & 1u) {   // player 1's last card, unplayed after h turns, is on top
-        if (b == n) m.U1l = B.prefix[n - 1u];
+        if (b == n) m.U1l = B.prefix[n - 1u] + 1u;
         else {
             const u32 k = (u32)__popc(free);
-            m.U1l = take_card(free, (u32)(outer % k));
+            m.U1l = take_card(free, (u32)(outer % k)) + 1u;
             outer /= k;
         }
         s1 = 5u;
     }
     for (u32 t = 0; 2u * t < b && 2u * t + 1u < n; t++) {
-        const u32 x = B.prefix[2u * t], y = 2u * t + 1u < b ? B.prefix[2u * t + 1u] : half;
+        const u32 x = B.prefix[2u * t] + 1u, y = 2u * t + 1u < b ? B.prefix[2u * t + 1u] + 1u : half;
         const u32 hi = max(x, y), lo = min(x, y);
         const u64 pair = RULE ? lo | (hi << 5) : hi | (lo << 5);
-        if (x > y) { put128(m.U1l, m.U1h, pair, s1); s1 += 10u; wins |= 1u << t; }
-        else { put128(m.U2l, m.U2h, pair, s2); s2 += 10u; }
+        if (x > y) { put96(m.U1l, m.U1h, pair, s1); s1 += 10u; wins |= 1u << t; }
+        else { put96(m.U2l, m.U2h, pair, s2); s2 += 10u; }
     }
     for (u32 i = 0; i < fo; i++) {
         const u32 k = (u32)__popc(free), np = k * (k - 1u) / 2u;
         u32 d = (u32)(outer % np), x = 1;
         outer /= np;
         while (d >= x) { d -= x; x++; }
-        const u32 hi = take_card(free, x), lo = take_card(free, d);
+        const u32 hi = take_card(free, x) + 1u, lo = take_card(free, d) + 1u;
         m.O |= (u64)(RULE ? lo | (hi << 5) : hi | (lo << 5)) << (10u * i);
     }
     u64 c = 0;
-    for (u32 i = 0; free; i++) c |= (u64)take_card(free, 0u) << (8u * i);
+    for (u32 i = 0; free; i++) c |= (u64)(take_card(free, 0u) + 1u) << (8u * i);
     m.s1 = s1; m.s2 = s2; m.wins = wins;
     m.c0 = (u32)c; m.c1 = (u32)(c >> 32);
 }
@@ -379,28 +435,27 @@ __device__ __forceinline__ u64 wide_row(u32 c0, u32 c1, u32 sel) {
 
 // The start of a lane's game, kept for wide_start, and its block.
 struct WideStart {
-    u64 a0, a1, b0, b1;
-    u32 la, blk;
+    u64 a0, b0;
+    u32 a1, b1, qa, blk;
 };
 
 // How many deals of the game that is at x at turn h lie on their own cycle of length lam (held_start of
 // war_held.cu): 0, or 1 (2 with its mirror image).
 template <int RULE>
-__device__ __noinline__ u32 wide_start(const WideStart x, const MBlock* __restrict__ blocks, u32 n, u32 lam) {
+__device__ __noinline__ u32 wide_start(const WideStart x, const MBlock* __restrict__ blocks, u32 n, u32 lam, const Turn5K K) {
     const u32 h = n >> 1;
-    u64 a0 = x.a0, a1 = x.a1, b0 = x.b0, b1 = x.b1, d0 = 0, d1 = 0, e0 = 0, e1 = 0;
-    u32 la = x.la, dla = 0;
+    u64 a0 = x.a0, b0 = x.b0, d0 = 0, e0 = 0;
+    u32 a1 = x.a1, b1 = x.b1, qa = x.qa, d1 = 0, e1 = 0, dq = 0;
     for (u32 t = 0; t < lam; t++) {
-        if (t == lam - h) { d0 = a0; d1 = a1; e0 = b0; e1 = b1; dla = la; }
-        turn5<RULE>(a0, a1, b0, b1, la, n - 1u);
+        if (t == lam - h) { d0 = a0; d1 = a1; e0 = b0; e1 = b1; dq = qa; }
+        turn5_pred<RULE>(a0, a1, b0, b1, qa, K);
     }
     if (a0 != x.a0 || a1 != x.a1 || b0 != x.b0 || b1 != x.b1) return 0u;   // x is not on the cycle
-    if (dla != (n + 1u) >> 1) return 0u;                                   // not as dealt
+    if (dq != 5u * ((n + 1u) >> 1)) return 0u;                             // not as dealt
     const MBlock& B = blocks[x.blk];
-    for (u32 i = 0; i < B.b; i++) {
-        u64 lo = i & 1u ? e0 : d0, hi = i & 1u ? e1 : d1;
-        shr128(lo, hi, 5u * (i >> 1));
-        if (((u32)lo & 31u) != B.prefix[i]) return 0u;
+    for (u32 i = 0; i < B.b; i++) {   // (10 cards a player: the low 60 bits)
+        const u64 lo = i & 1u ? e0 : d0;
+        if (((u32)(lo >> (5u * (i >> 1))) & 31u) != B.prefix[i] + 1u) return 0u;
     }
     return B.twice ? 2u : 1u;
 }
@@ -434,6 +489,7 @@ __device__ __noinline__ u32 wide_streak_head(u32 n, u32 a, u32 p, u32 wins) {
 struct WideMore {
     u32 cap;
     u32 slack;       // streak: turns past the cap after which an undecided game is undetermined for certain
+    Turn5K tk;
     u32 lamtab[32];
 };
 
@@ -461,8 +517,12 @@ __global__ void __launch_bounds__(1024) wide_merge_kernel(const __grid_constant_
     WUnit& mu = units[threadIdx.x >> 5];
     u64* const counter = &acc->work_next;
 
-    u64 a0 = 1, a1 = 0, b0 = 1, b1 = 0, t0 = ~0ull, t1 = 0, t2 = 0, t3 = 0, turns = 0;
-    u32 la = 0, tla = 0, rounds = 0, next = 0xFFFFFFFFu, wt = 0, kind = K_END;
+    const Turn5K K = more.tk;
+    const u32 n5 = 5u * n;
+    u64 a0 = 1, b0 = 1, t0 = ~0ull, t2 = 0, turns = 0;          // the piles' low words, the tortoise's,
+    u32 a1 = 0, b1 = 0, t1 = 0, t3 = 0, qa = 0, tqa = 0;        // their high words, 5 * player 1's cards
+    u32 rounds = 0, next = 0xFFFFFFFFu, wt = 0, kind = K_END;
+    bool done = true, kcy = false;                              // (Brent, streak: decided, by a cycle)
     u32 run = 0, save = 0, prev = 2u;    // streak: turn of the last break, turn of the tortoise, last winner
     bool active = false;
     u32 cyc = 0, maxfin = 0, und = 0;
@@ -496,76 +556,73 @@ __global__ void __launch_bounds__(1024) wide_merge_kernel(const __grid_constant_
         maxfin = max(maxfin, h);
     };
     auto build = [&](u32 sel) -> bool {
-        const u32 a10 = 10u * c.pa;
+        const u32 a10 = 10u * c.pa, in_at = 10u * (c.f - c.fi);
         const u64 in = wide_row(mu.c0, mu.c1, sel);
-        u64 xl = mu.O, xh = 0;
-        put128(xl, xh, in, 10u * (c.f - c.fi));
-        u64 yl = xl, yh = xh;
-        xl &= ~shl64(~0ull, a10);
-        xh &= a10 > 64u ? ~shl64(~0ull, a10 - 64u) : 0ull;
-        shl128(xl, xh, mu.s1);
-        shr128(yl, yh, a10);
-        shl128(yl, yh, mu.s2);
-        a0 = xl | mu.U1l; a1 = xh | mu.U1h;
-        b0 = yl | mu.U2l; b1 = yh | mu.U2h;
-        la = mu.s1 / 5u + 2u * c.pa;
+        // the list: outer pairs, then inner ones; player 1's first c.pa pairs and player 2's others
+        const u64 xl = mu.O | shl64(in, in_at), xh = in_at ? shr64(in, 64u - in_at) : 0ull;
+        u64 yl = xl & ~shl64(~0ull, a10), yh = a10 > 64u ? xh & ~shl64(~0ull, a10 - 64u) : 0ull;
+        a0 = mu.U1l; a1 = mu.U1h;
+        put96(a0, a1, yl, mu.s1);
+        if (yh) a1 |= (u32)shl64(yh, mu.s1);
+        yl = shr64(xl, a10) | shl64(xh, 64u - a10) | shr64(xh, a10 - 64u);
+        yh = shr64(xh, a10);
+        b0 = mu.U2l; b1 = mu.U2h;
+        put96(b0, b1, yl, mu.s2);
+        if (yh) b1 |= (u32)shl64(yh, mu.s2);
+        qa = mu.s1 + a10;
         if (c.filter) {   // player 1 must hold card n - 1
             bool has = false;
-            u64 lo = a0, hi = a1;
-            for (u32 i = 0; i < la; i++) {
-                has |= ((u32)lo & 31u) == n1;
-                shr128(lo, hi, 5u);
-            }
+            for (u32 i = 0; i < qa; i += 5u) has |= ((u32)(i < 60u ? a0 >> i : ((u64)a1 << 32 | a0 >> 32) >> (i - 32u)) & 31u) == n;
             if (!has) return false;
         }
-        put128(a0, a1, 1ull, 5u * la);
-        put128(b0, b1, 1ull, 5u * (n - la));
-        rounds = h; kind = K_NONE; wt = c.wt; active = true;
-        t0 = a0; t1 = a1; t2 = b0; t3 = b1; tla = la;
+        rounds = h; kind = K_NONE; wt = c.wt; active = true; done = false; kcy = false;
+        t0 = a0; t1 = DET == DET_FLOYD ? a1 : a1 + b1; t2 = b0; t3 = b1; tqa = qa;   // (t1: both high words)
         next = W > h ? W : 3u * W;   // (W = h: the tortoise of turn W)
         if (DET == DET_BRENT) {
             WideStart x;
-            x.a0 = a0; x.a1 = a1; x.b0 = b0; x.b1 = b1; x.la = la; x.blk = c.blk;
+            x.a0 = a0; x.a1 = a1; x.b0 = b0; x.b1 = b1; x.qa = qa; x.blk = c.blk;
             *start = x;
         } else if (DET == DET_STREAK) {
             run = h; save = h; prev = 2u;
             *head = c.pa | ((h - c.f) << 8) | (mu.wins << 16);
         } else if (h & 1u) {         // the hare's turns come in pairs from turn 0
-            turn5<RULE>(a0, a1, b0, b1, la, n1);
+            turn5_pred<RULE>(a0, a1, b0, b1, qa, K);
             rounds = h + 1u;
-            if ((la == 0u) | (la == n)) kind = K_END;
+            if ((qa == 0u) | (qa == n5)) kind = K_END;
         }
         return true;
     };
     auto refill = [&](bool want) {
-        if (want) { active = false; kind = K_END; }
+        if (want) { active = false; kind = K_END; done = true; }
         merge_deal(c, a, counter, want, setup, over, ended, build, drain);
     };
+    // Brent and the streak test latch `done` (and by what) and look at the cap at the services; what is decided by
+    // turn cap + 1 is decided (wide_kernel).
     auto turn = [&]() {
-        const bool open = kind == K_NONE;
         if (DET == DET_FLOYD) {
-            turn5<RULE>(a0, a1, b0, b1, la, n1);
-            const bool e1 = (la == 0u) | (la == n);
-            turn5<RULE>(a0, a1, b0, b1, la, n1);
-            const bool e2 = (la == 0u) | (la == n);
+            const bool open = kind == K_NONE;
+            turn5_pred<RULE>(a0, a1, b0, b1, qa, K);
+            const bool e1 = (qa == 0u) | (qa == n5);
+            turn5_pred<RULE>(a0, a1, b0, b1, qa, K);
+            const bool e2 = (qa == 0u) | (qa == n5);
             const u32 r2 = rounds + (e1 ? 1u : 2u);
-            if (r2 > 2u * h) turn5<RULE>(t0, t1, t2, t3, tla, n1);
-            const bool cy = (a0 == t0) & (a1 == t1) & (b0 == t2) & (b1 == t3);
+            if (r2 > 2u * h) turn5_pred<RULE>(t0, t1, t2, t3, tqa, K);
+            const bool cy = (a0 == t0) & (b0 == t2) & (a1 * K.one + b1 == t1 * K.one + t3);
             const u32 kk = (e1 | e2) ? (u32)K_END : (cy ? (u32)K_CYC : (r2 > cap ? (u32)K_UND : (u32)K_NONE));
             rounds = open ? r2 : rounds;
             kind = open ? kk : kind;
         } else {
-            const u32 w = turn5<RULE>(a0, a1, b0, b1, la, n1) ? 1u : 0u;
+            const u32 w = turn5_pred<RULE>(a0, a1, b0, b1, qa, K);
             if (DET == DET_STREAK) {
-                run = open & (w == prev) ? rounds : run;
-                prev = open ? w : prev;
+                if (!done & (w == prev)) run = rounds * K.one;
+                prev = w;
             }
-            const u32 r1 = rounds + 1u;
-            const bool en = (la == 0u) | (la == n);
-            const bool cy = (a0 == t0) & (a1 == t1) & (b0 == t2) & (b1 == t3);
-            const u32 kk = en ? (u32)K_END : (cy ? (u32)K_CYC : (r1 > cap ? (u32)K_UND : (u32)K_NONE));
-            rounds = open ? r1 : rounds;
-            kind = open ? kk : kind;
+            if (!done) rounds = rounds * K.one + K.one;
+            const bool en = qa * K.one - 5u >= n5 - 5u;          // 0 or 5n
+            // (at most one of the piles reaches its high word, and equal low words say which)
+            const bool cy = (a0 == t0) & (b0 == t2) & (a1 * K.one + b1 == t1);
+            kcy = done ? kcy : (cy & !en);
+            done = done | cy | en;
         }
     };
 
@@ -574,18 +631,20 @@ __global__ void __launch_bounds__(1024) wide_merge_kernel(const __grid_constant_
     while (running) {
         for (u32 k = 0; k < before; k++) turn();
         if (DET == DET_BRENT) {
-            if (kind == K_NONE && rounds == next) { t0 = a0; t1 = a1; t2 = b0; t3 = b1; next = 2u * next + W; }
+            if (!done && rounds == next) { t0 = a0; t1 = a1 + b1; t2 = b0; next = 2u * next + W; }
             for (u32 k = 0; k < after; k++) turn();
         }
-        if (DET == DET_STREAK && kind == K_NONE && run > save) { t0 = a0; t1 = a1; t2 = b0; t3 = b1; tla = la; save = rounds; }
+        if (DET == DET_STREAK && !done && run > save) { t0 = a0; t1 = a1 + b1; t2 = b0; tqa = qa; save = rounds; }
+        if (DET != DET_FLOYD && active)
+            kind = done ? (rounds > cap + 1u ? (u32)K_UND : (kcy ? (u32)K_CYC : (u32)K_END)) : (rounds > cap ? (u32)K_UND : (u32)K_NONE);
         const bool fin = active & (kind != K_NONE);
         if (__any_sync(WAR_FULL_MASK, fin)) {
             if (fin) {
                 u32 t = rounds;
-                if (DET == DET_STREAK) {   // (what is decided by turn cap + 1 is decided, wide_kernel)
+                if (DET == DET_STREAK) {
                     if (kind == K_CYC) {
                         // the piles are the tortoise's: the next winner's pile and the period are the run's
-                        const u32 ws = ((u32)t0 & 31u) > ((u32)t2 & 31u) ? tla : n - tla;
+                        const u32 ws = ((u32)t0 & 31u) > ((u32)t2 & 31u) ? tqa / 5u : n - tqa / 5u;
                         const u32 lam = more.lamtab[ws & 31u];
                         if (run > save || lam == 0u || lam % (rounds - save) != 0u || run + lam > more.cap + 1u)
                             kind = K_UND;
@@ -594,7 +653,7 @@ __global__ void __launch_bounds__(1024) wide_merge_kernel(const __grid_constant_
                             if (run == h) turns -= wide_streak_head(n, *head & 255u, (*head >> 8) & 255u, *head >> 16);
                         }
                     }
-                    if (kind == K_UND || (kind == K_END && rounds > more.cap + 1u)) { kind = K_UND; t = more.cap + 1u; }
+                    if (kind == K_END && rounds > more.cap + 1u) kind = K_UND;
                 }
                 if (kind == K_CYC) {
                     cyc += wt;
@@ -603,13 +662,14 @@ __global__ void __launch_bounds__(1024) wide_merge_kernel(const __grid_constant_
                         const u32 at = next == W ? h : (next - W) >> 1, lam = rounds - at;
                         if (a.hbins) atomicAdd(&shh[lam < hb1 ? lam : hb1], wt);
                         if (next == W) t = W + lam;
-                        if (lam <= W && at <= W) turns -= (u64)wide_start<RULE>(*start, a.blocks, n, lam) * (t - lam);
+                        if (lam <= W && at <= W) turns -= (u64)wide_start<RULE>(*start, a.blocks, n, lam, K) * (t - lam);
                     }
                 } else if (kind == K_END) {
                     maxfin = max(maxfin, rounds);
                     atomicAdd(&she[rounds < WAR_EBINS - 1 ? rounds : WAR_EBINS - 1], wt);
                 } else {
                     und += wt;
+                    if (DET != DET_FLOYD) t = more.cap + 1u;
                 }
                 turns += (u64)wt * t;
             }
@@ -723,6 +783,8 @@ extern "C" int war_enumerate_wide(const war_job* job, const war_wide_cfg* cfg, w
     WideMore more;
     memset(&more, 0, sizeof more);
     more.cap = cap;
+    more.tk.one = 1u; more.tk.m1 = (u32)-1; more.tk.m32 = (u32)-32; more.tk.k32 = 32u; more.tk.k2p27 = 1u << 27;
+    more.tk.c1 = (u32)-5; more.tk.c2 = 5u * (u32)job->n - 5u;
     for (int ws = 2; ws + 2 <= job->n; ws += 2) {   // gpu/war24.py:109: lcm(n+1, lcm(W, L-1))
         auto gcd = [](u64 x, u64 y) { while (y) { u64 t = x % y; x = y; y = t; } return x; };
         const u64 l1 = (u64)ws / gcd(ws, job->n - ws - 1) * (u64)(job->n - ws - 1);
