@@ -73,12 +73,11 @@ struct TurnK {
 //   length: qq = 4*len1 - 2n, pos = s*qq + (2n-4) and qq += 4s with s = +1 (player 1 won) or -1;
 //          the game is over when qq*qq == (2n)^2.
 template <int RULE>
-__device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const TurnK& K, u32& c1, u32& c2) {
+__device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const TurnK& K) {
     const u32 l1 = (u32)w1, h1 = (u32)(w1 >> 32), l2 = (u32)w2, h2 = (u32)(w2 >> 32);
     const u32 nl1 = __funnelshift_r(l1, h1, 4), nl2 = __funnelshift_r(l2, h2, 4);
     const u32 nh1 = __umulhi(h1, K.k2p28), nh2 = __umulhi(h2, K.k2p28);
-    c1 = l1 + nl1 * K.km16;
-    c2 = l2 + nl2 * K.km16;
+    const u32 c1 = l1 + nl1 * K.km16, c2 = l2 + nl2 * K.km16;
     const bool p1 = c1 > c2;
     const u32 pa = RULE ? c2 + c1 * K.k16 : c1 + c2 * K.k16;   // player 1 won
     const u32 pb = RULE ? c1 + c2 * K.k16 : c2 + c1 * K.k16;   // player 2 won
@@ -98,10 +97,80 @@ __device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const Tu
     return p1;
 }
 
-template <int RULE>
-__device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const TurnK& K) {
-    u32 c1, c2;   // the cards played
-    return war_turn_fma<RULE>(w1, w2, qq, K, c1, c2);
+// A turn of the latched loops with its tests, in one block so that the predicates stay predicates.  Both pipes that
+// can do its work are half rate (ALU: logic, shifts, compares, selects; FMA: multiply-adds), so it is split between
+// them: what follows from "player 1 won" is written by a multiply-add for player 2's win and overwritten by one
+// under the predicate, moves under a predicate are multiplications by one, and the ALU is left the shifts, the
+// cards' masks and the compares: about 18 operations on each.
+//
+//   pair        first card f + 16 (second card g) of the winner's two, + 0xFF: see war_turn_fma
+//   landmark    if one of the cards played is `top` (card n-1): the piles before the turn, and the turn
+//   end, cycle  a pile is empty; both piles are the tortoise's (t1, t2): ev = 2 (turn in the period) + (1 if an end),
+//               and the game is frozen: its length word gets an odd value far out of range, so it never signals
+//               again (an odd length word is no end; the pushed pairs shift out, and with fewer than n cards the piles
+//               are no tortoise)
+// k2: twice the number of the unrolled turn 0 in the period; U the unrolled turn.
+constexpr u32 NO_EVENT = 0xFFFFFFFFu;
+constexpr u32 FROZEN = 0x80000001u;
+
+template <int RULE, int U>
+__device__ __forceinline__ void war_turn_tests(u64& w1, u64& w2, u32& qq, u64 t1, u64 t2, u64& m1, u64& m2, u32& at,
+                                               u32& ev, u32 k2, u32 top, const TurnK& K) {
+    const u32 l1 = (u32)w1, h1 = (u32)(w1 >> 32), l2 = (u32)w2, h2 = (u32)(w2 >> 32);
+    const u32 nl1 = __funnelshift_r(l1, h1, 4), nl2 = __funnelshift_r(l2, h2, 4);
+    const u32 nh1 = __umulhi(h1, K.k2p28), nh2 = __umulhi(h2, K.k2p28);
+    const u32 c1 = l1 & 15u, c2 = l2 & 15u;
+    const u32 f = RULE ? c1 : c2, g = RULE ? c2 : c1;   // player 2 won: f first in the pair; player 1: g
+    u64 a1 = ((u64)nh1 << 32) | nl1, a2 = ((u64)nh2 << 32) | nl2;
+    u32 ma = (u32)m1, mb = (u32)(m1 >> 32), mc = (u32)m2, md = (u32)(m2 >> 32);
+    asm("{\n\t"
+        ".reg .pred p, q, e, y;\n\t"
+        ".reg .u32 t, s, ps, xl, xh, al, ah, bl, bh, sq;\n\t"
+        ".reg .u64 x;\n\t"
+        "setp.eq.u32 q, %9, %13;\n\t"
+        "setp.eq.or.u32 q, %10, %13, q;\n\t"
+        "setp.gt.u32 p, %9, %10;\n\t"
+        "@q mov.b32 %3, %14;\n\t"
+        "@q mad.lo.u32 %4, %15, %19, 0;\n\t"
+        "@q mad.lo.u32 %5, %16, %19, 0;\n\t"
+        "@q mad.lo.u32 %6, %17, %19, 0;\n\t"
+        "@q mad.lo.u32 %7, %22, %19, %23;\n\t"
+        "mad.lo.u32 t, %12, %18, %11;\n\t"       // f + 16 g
+        "@p mad.lo.u32 t, %11, %18, %12;\n\t"    // g + 16 f
+        "selp.b32 s, 1, -1, p;\n\t"
+        "mad.lo.u32 t, t, %19, 255;\n\t"
+        "mad.lo.u32 ps, s, %2, %20;\n\t"         // the winner's sentinel after the pop
+        "mad.lo.u32 %2, s, %21, %2;\n\t"
+        "cvt.u64.u32 x, t;\n\t"
+        "shl.b64 x, x, ps;\n\t"
+        "mov.b64 {xl, xh}, x;\n\t"
+        "@p mad.wide.u32 %0, xl, %19, %0;\n\t"
+        "@!p mad.wide.u32 %1, xl, %19, %1;\n\t"
+        "mov.b64 {al, ah}, %0;\n\t"
+        "@p mad.lo.u32 ah, xh, %19, ah;\n\t"
+        "mov.b64 %0, {al, ah};\n\t"
+        "mov.b64 {bl, bh}, %1;\n\t"
+        "@!p mad.lo.u32 bh, xh, %19, bh;\n\t"
+        "mov.b64 %1, {bl, bh};\n\t"
+        "mul.lo.u32 sq, %2, %2;\n\t"
+        "setp.eq.u32 e, sq, %24;\n\t"
+        "setp.eq.u32 y, al, %25;\n\t"
+        "setp.eq.and.u32 y, ah, %26, y;\n\t"
+        "setp.eq.and.u32 y, bl, %27, y;\n\t"
+        "setp.eq.and.u32 y, bh, %28, y;\n\t"
+        "@e mad.lo.u32 %8, %22, %19, %29;\n\t"
+        "@y mad.lo.u32 %8, %22, %19, %23;\n\t"
+        "@e mad.lo.u32 %2, %30, %19, 0;\n\t"
+        "@y mad.lo.u32 %2, %30, %19, 0;\n\t"
+        "}"
+        : "+l"(a1), "+l"(a2), "+r"(qq), "+r"(ma), "+r"(mb), "+r"(mc), "+r"(md), "+r"(at), "+r"(ev)
+        : "r"(c1), "r"(c2), "r"(f), "r"(g), "r"(top), "r"(l1), "r"(h1), "r"(l2), "r"(h2), "r"(K.k16), "r"(K.one),
+          "r"(K.c0), "r"(K.k4), "r"(k2), "n"(2 * U), "r"(K.end2), "r"((u32)t1), "r"((u32)(t1 >> 32)), "r"((u32)t2),
+          "r"((u32)(t2 >> 32)), "n"(2 * U + 1), "r"(FROZEN));
+    m1 = ((u64)mb << 32) | ma;
+    m2 = ((u64)md << 32) | mc;
+    w1 = a1;
+    w2 = a2;
 }
 
 // The same turn with the rule chosen at run time (serving kernel, checks).

@@ -547,7 +547,7 @@ __global__ void __launch_bounds__(1024) held_merge_kernel(const __grid_constant_
     };
     auto refill = [&](bool want) {
         if (want) active = false;
-        merge_deal(c, a, counter, want, setup, over, ended, build, drain);
+        merge_deal(c, a, counter, __ballot_sync(WAR_FULL_MASK, want), setup, []() {}, over, ended, build, drain);
     };
     auto turn = [&]() {
         const bool en = h_turn_packed_fma<RULE>(wh, wo, s, n4m8, K);

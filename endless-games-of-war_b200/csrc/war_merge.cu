@@ -102,9 +102,10 @@ void canon_plan(const war_job* job, u64 warps, MergePlan& p) {
         }
         if (job->hi % m) add(y, 0, 0, (u32)(job->hi % m));
     }
-    // about 24 units for each warp, of at least a warp's worth of games
+    // about 24 units for each warp, so that the last ones end together, of at least 300 games: setting a unit up costs
+    // about what ten games do (2e6 positions of 11 cards: units of 40 games 469 us, 200: 370, 300: 351, 400: 344, 800: 363)
     u64 lc = rows / std::max<u64>(1, warps * 24);
-    lc = std::min<u64>(std::max<u64>(lc, (32 + m - 1) / m), 720);
+    lc = std::min<u64>(std::max<u64>(lc, (300 + m - 1) / m), 720);
     const u64 parts = (720 + lc - 1) / lc;
     p.lc = (u32)((720 + parts - 1) / parts);
     u64 u = 0;
@@ -171,9 +172,11 @@ void merge_plan(const war_job* job, u64 warps, MergePlan& p) {
         p.games += lists * (B.f + 1u);
         rows4 += lists;
     }
-    // About 24 units for each warp, so that the last ones end together, of at least a warp's worth of games.
+    // About 24 units for each warp, so that the last ones end together, of at least 40 rows (200 games in a block of
+    // ten cards): 5e6 deals of 11 cards take 235 us with units of 7 rows, 169 with 40, 177 with 80, 236 with 160,
+    // 3e5 of 10 cards 84, 83, 90 and 117.  (6 units for each warp: a span of 14 cards 14.4 ms instead of 14.1.)
     u64 lc = rows4 / std::max<u64>(1, warps * 24);
-    lc = std::min<u64>(std::max<u64>(lc, 7), 2520);
+    lc = std::min<u64>(std::max<u64>(lc, 40), 2520);
     const u64 parts = (2520 + lc - 1) / lc;
     p.lc = (u32)((2520 + parts - 1) / parts);
     u64 u = 0;
@@ -227,7 +230,7 @@ int merged_max_blocks_per_sm(int rule, int threads, int hbins) {
 }
 
 static size_t canon_shmem(int extra, int threads, int hbins) {
-    return merge_shmem(threads, hbins) + (extra ? 2 * sizeof(u64) * (size_t)threads : 0);
+    return merge_shmem(threads, hbins) + (extra ? 2 * sizeof(u64) * (size_t)threads + sizeof(StartQueue) * (size_t)(threads / 32) : 0);
 }
 
 typedef void (*MergeFn)(const MergeArgs, DevAcc*);
@@ -239,7 +242,7 @@ static MergeFn canon_pick(int shape, int extra) {
 }
 
 cudaError_t launch_canon(const MergeArgs& a, int rule, int extra, int threads, int blocks, DevAcc* acc, cudaStream_t st) {
-    const MergeFn fn = rule ? canon_pick<1>(a.blk, extra) : canon_pick<0>(a.blk, extra);
+    const MergeFn fn = rule ? canon_pick<1>(a.blk, extra) : canon_pick<0>(a.blk, extra);   // (shared memory: set below)
     fn<<<blocks, threads, canon_shmem(extra, threads, a.hbins), st>>>(a, acc);
     note_launch();
     return cudaGetLastError();
@@ -249,6 +252,11 @@ int canon_max_blocks_per_sm(int rule, int shape, int extra, int threads, int hbi
     const MergeFn fn = rule ? canon_pick<1>(shape, extra) : canon_pick<0>(shape, extra);
     const size_t shmem = canon_shmem(extra, threads, hbins);
     int nb = 0;
+    if (shmem > 48 * 1024 &&
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, threads, shmem) != cudaSuccess) return 0;
     return nb;
 }

@@ -79,6 +79,11 @@ struct MergeArgs {
 struct MUnit {
     u64 U1, U2, O;
     u32 c0, c1, s1, s2, top;
+    // of the number of pairs in hand that player 1 wins: the piles with their sentinels and without the list, the
+    // list's pairs that are player 1's
+    u64 A1, A2, mask;
+    u32 at;           // where the inner pairs go, in bits
+    u32 a8;           // 8 * pairs won by player 1
 };
 constexpr u32 MTOP_INNER = 0, MTOP_PAIR = 32, MTOP_P1 = 64, MTOP_P2 = 128;
 
@@ -198,6 +203,10 @@ __host__ __device__ __forceinline__ u32 canon_row0(u32 i) {       // first row o
 struct CUnit {
     u64 Q;            // the cards before the inner ones, 4 bits each
     u32 c0, c1;       // the inner cards as bytes
+    // of the split in hand: the piles without the other cards (player 1's card n-1, sentinels), player 1's cards
+    u64 A1, A2, mask;
+    u32 at;           // where the inner cards go, in bits
+    u32 k4;           // 4 * split
 };
 __host__ __device__ __forceinline__ void canon_unit(const MBlock& B, u64 outer, u32 m, CUnit& u) {
     u32 free = B.free_mask;
@@ -230,18 +239,18 @@ struct MCursor {
     bool filter = false, dry = false;
 };
 
-// Deals the warp's next games to the lanes that want one; called by the whole warp.  CANON: pa is the split, the
+// Deals the warp's next games to the lanes of `need`; called by the whole warp.  CANON: pa is the split, the
 // rows are orders and every game counts once.
 //   setup(B, outer)   sets the unit up for the warp
+//   split()           sets up what depends on c.pa
 //   over()            whether one player won every pair of the unit's games with c.pa (1: player 1, 2: player 2)
 //   ended(count)      counts `count` deals that are over at turn h
 //   build(selectors)  the lane's game from a table row; false if it is not played (filter)
 //   drain()           empties the histograms
-template <bool CANON = false, class Setup, class Over, class Ended, class Build, class Drain>
-__device__ __forceinline__ u32 merge_deal(MCursor& c, const MergeArgs& a, u64* counter, bool want, Setup setup,
-                                          Over over, Ended ended, Build build, Drain drain) {
+template <bool CANON = false, class Setup, class Split, class Over, class Ended, class Build, class Drain>
+__device__ __forceinline__ void merge_deal(MCursor& c, const MergeArgs& a, u64* counter, u32 need, Setup setup,
+                                           Split split, Over over, Ended ended, Build build, Drain drain) {
     const u32 lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-    u32 need = __ballot_sync(WAR_FULL_MASK, want), served = 0;
     while (need && !c.dry) {
         if (c.l == c.lend) {
             if (c.pa < c.f) {
@@ -268,6 +277,7 @@ __device__ __forceinline__ u32 merge_deal(MCursor& c, const MergeArgs& a, u64* c
                 c.filter = !CANON && B.filter != 0;
                 if (c.given > DRAIN_DEALS) { drain(); c.given = 0; }
             }
+            split();
             const u32 o = CANON ? 0u : over();
             if (o) {
                 if (o == 1u || !c.filter) {   // (card n-1 is with the player who won every pair)
@@ -284,12 +294,10 @@ __device__ __forceinline__ u32 merge_deal(MCursor& c, const MergeArgs& a, u64* c
         if (mine) mine = build(__ldg(a.table + c.row0 + c.l + r));
         const u32 got = __ballot_sync(WAR_FULL_MASK, mine);
         need &= ~got;
-        served |= got;
         const u32 k = (u32)__popc(got) * c.wt;
         c.done += k; c.given += k;
         c.l += take;
     }
-    return served;
 }
 
 }  // namespace war

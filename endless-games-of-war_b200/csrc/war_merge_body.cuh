@@ -11,12 +11,18 @@
 // Games that have met look at the same landmarks whatever turn they have got to, where states at services
 // meet only in games of one phase; and a cycle is stored by its landmarks, about one state in eight.
 //
-// What bounds it: random reads and writes of the table in HBM (13 cards: at the rate of the random-gather ceiling),
-// instruction issue of the turns (canonical scans: ALU pipe 84%), and for jobs of fewer than about 1e6 games the
-// longest game.  Measured on a B200 (states at services -> landmarks -> a found cycle recorded by playing on instead
-// of by a walk): a span of 4.26e9 deals of 15 cards 210 -> 132 -> 85 ms (stores 3.4e9 -> 1.0e9), 1e8 deals of 13 cards
-// 2.5 -> 2.0 -> 1.6 ms, a resumed a(13) 31.2 -> 30.5 -> 29.9 ms, --half span of 14 cards 13.7 -> 13.6 ms, 3e9
-// canonical positions of 14 cards 152 -> 148 ms.  The one-deal-one-game kernel before: 370, 10.7, 168 and 124 ms.
+// The service is as long as the turns of its period, so it is written for few operations and branches: a decided
+// game is frozen in the turn (war_turn_tests), its outcome is one word from any source, what is rare (Brent's own
+// finds, their recording, checkpoints) is behind one branch, a miss goes to one of two slots in shared memory, both
+// histograms are one array, and what a unit's games share is prepared once per (unit, split).
+//
+// What bounds it: instruction issue (12! deals of 13 cards: ALU pipe 82%, issue 75%, beside random accesses at 0.9 of
+// the random-gather ceiling), and for jobs of fewer than about 1e6 games the longest game.  Measured on a B200 (states
+// at services -> landmarks -> a found cycle recorded by playing on instead of by a walk -> this service and turn): a
+// span of 4.26e9 deals of 15 cards 210 -> 132 -> 85 -> 81 ms (stores 3.4e9 -> 1.0e9), 1e8 deals of 13 cards 2.5 -> 2.0
+// -> 1.6 -> 1.5 ms, a resumed a(13) 31.2 -> 30.5 -> 29.9 -> 28.8 ms, --half span of 14 cards 13.7 -> 12.9 ms, 3e9
+// canonical positions of 14 cards 152 -> 148 -> 148 -> 143 ms and 125 with the queue of starts.  The one-deal-one-game
+// kernel before: 370, 10.7, 168, 124 and 164 ms.
 #pragma once
 #include "war_refill.cuh"
 #include "war_merge.cuh"
@@ -29,74 +35,85 @@ union UnitStore {
     CUnit c[32];
 };
 
-// One game slot of the merged kernel.
+// One game slot of the merged kernel.  next: Brent's next checkpoint, or RECORDING, or IDLE for a lane without a game.
 struct MGame {
     u64 w1, w2, t1, t2, m1, m2;   // piles, tortoise, the last landmark
-    u32 q, rounds, next, wt, mv, at;
-    bool done, kcy, active;
+    u32 q, rounds, next, wt, mv, at, missed;
 };
 
-// A game's last two landmarks looked up and missed, and their turns + 1 (0: none), kept in shared memory.
+// The hashes of a game's last two landmarks looked up and missed, and their turns, kept in shared memory: the k-th
+// miss in slot k mod 2.
 struct Missed {
-    u64 ka, kb;
-    u32 ta, tb;
+    u64 h[2];
+    u32 t[2];
 };
 constexpr u32 NO_LANDMARK = 0xFFFFFFFFu;
 // A game whose cycle Brent found plays on around it once more, to the tortoise's state again, and its services store
 // the cycle's landmarks instead of looking them up: the other lanes go on meanwhile, where a walk of the cycle at
-// once holds them up.  (Its checkpoint is this, which is never reached.)
-constexpr u32 RECORDING = 0xFFFFFFFFu;
+// once holds them up.  (As checkpoints, these are never reached.)
+constexpr u32 RECORDING = 0xFFFFFFFFu, IDLE = 0xFFFFFFFEu;
 
-// Stores the landmarks that a decided game missed, with its outcome: the cycle value vcyc, or (vcyc = 0) the turns
-// from there to its end after len turns.  Returns the entries stored.
-__device__ __forceinline__ u32 store_missed(u64* memo, u32 mbits, const Missed& x, u32 vcyc, u32 len) {
-    const u32 vmask = (1u << mbits) - 1u;
-    u32 k = 0;
-    if (x.ta) {
-        const u32 v = vcyc ? vcyc : 2u * (len + 1u - x.ta) + 1u;
-        if (v <= vmask) {
-            __stcg((unsigned long long*)memo + memo_slot(x.ka, mbits), path_entry(x.ka, mbits, v));
-            k++;
-        }
+// The table: its words, log2 of their number, the largest value, and the key's constants (memo_key_state): the cards
+// that a key holds, and 4(n-1) as a factor.
+struct MemoTable {
+    u64* T;
+    u32 bits, vmask, lenlo, lenhi;
+    u64 cards;
+    __device__ __forceinline__ MemoTable(u64* t, u32 b, u32 n) : T(t), bits(b), vmask((1u << b) - 1u) {
+        const u32 kb = 4u * (n - 1u);
+        cards = (1ull << kb) - 1ull;
+        lenlo = (u32)(1ull << kb);
+        lenhi = (u32)((1ull << kb) >> 32);
     }
-    if (x.tb) {
-        const u32 v = vcyc ? vcyc : 2u * (len + 1u - x.tb) + 1u;
-        if (v <= vmask) {
-            __stcg((unsigned long long*)memo + memo_slot(x.kb, mbits), path_entry(x.kb, mbits, v));
-            k++;
-        }
+    // The hash of a state: memo_key_state(w1, w2) * MEMO_MUL, with the length field added by multiply-adds.
+    __device__ __forceinline__ u64 hash(u64 w1, u64 w2) const {
+        const bool sw = w2 < w1;
+        const u64 h = sw ? w2 : w1, o = sw ? w1 : w2;
+        const u32 len = pile_len(h);
+        const u64 k = (h ^ ((o ^ 1ull) << (4u * len))) & cards;      // (the sentinel of h goes with o's lowest bit)
+        return (((u64)(len * lenhi + (u32)(k >> 32)) << 32) | (len * lenlo + (u32)k)) * MEMO_MUL;
     }
-    return k;
-}
+    __device__ __forceinline__ u64* word(u64 h) const { return T + ((u32)(h >> 32) >> (32u - bits)); }
+    __device__ __forceinline__ void store(u64 h, u32 v) const {
+        __stcg((unsigned long long*)word(h), (unsigned long long)((h << bits) | v));
+    }
+    // The missed landmarks of a decided game, with its outcome: 2 lam (and the like) for a cycle, else 2 len + 1, from
+    // a landmark 2 (turns left) + 1.  Returns the entries stored.
+    __device__ __forceinline__ u32 store_missed(const Missed& x, u32 missed, u32 out) const {
+        u32 k = 0;
+#pragma unroll
+        for (u32 i = 0; i < 2u; i++) {
+            const u32 v = out - ((out & 1u) ? 2u * x.t[i] : 0u);
+            if (missed > i && v <= vmask) { store(x.h[i], v); k++; }
+        }
+        return k;
+    }
+};
 
 template <int RULE>
 __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restrict__ acc, u64* __restrict__ counter,
                                            UnitStore& store, u64* sh64) {
-    MUnit* const units = store.m;
     Missed* const miss = (Missed*)sh64 + threadIdx.x;
-    u32* const sh = (u32*)((Missed*)sh64 + blockDim.x);
-    u32* const shh = sh;
-    u32* const she = sh + a.hbins;
+    u32* const sh = (u32*)((Missed*)sh64 + blockDim.x);      // cycle lengths, then ending lengths
+    const u32 hbins = (u32)a.hbins;
     const int bins = a.hbins + WAR_EBINS;
     for (int b = threadIdx.x; b < bins; b += blockDim.x) sh[b] = 0;
     __syncthreads();
 
     const u32 n = (u32)a.n, h = n >> 1, W = (u32)a.W, n2 = 2u * n;
     const TurnK K = a.tk;
-    const u32 hb1 = a.hbins > 0 ? (u32)(a.hbins - 1) : 0u;
-    const int period = a.defer > 4 ? (a.defer + 3) & ~3 : 4;
-    u64* const memo = a.memo;
-    const u32 mbits = a.memo_bits;
-    const u32 vmask = (1u << mbits) - 1u;
+    const u32 hb1 = hbins ? hbins - 1u : 0u;
+    const u32 period = a.defer > 4 ? (u32)((a.defer + 3) & ~3) : 4u;
+    const MemoTable memo(a.memo, a.memo_bits, n);
+    const bool table = a.memo != nullptr;
     const u64 pat = 0x1111111111111111ull * (u64)(n - 1u);
     const u32 lane = threadIdx.x & 31u;
-    MUnit& mu = units[threadIdx.x >> 5];
+    MUnit& mu = store.m[threadIdx.x >> 5];
 
     MCursor c;
     u32 cyc = 0, turns = 0, maxfin = 0, capped = 0, mlook = 0, mhit = 0, mstore = 0;
     MGame g;
-    g.active = false; g.done = true; g.kcy = false; g.w1 = g.w2 = 1ull; g.t1 = g.t2 = 0ull; g.q = 0; g.rounds = 0;
-    g.next = 0xFFFFFFFFu; g.m1 = g.m2 = 0ull; g.at = NO_LANDMARK; g.mv = 0; g.wt = 0;
+    g.w1 = g.w2 = 1ull; g.m1 = g.m2 = 0ull; g.rounds = g.mv = g.wt = g.missed = 0; g.at = NO_LANDMARK;
 
     auto drain = [&]() {
         __syncwarp();
@@ -118,101 +135,110 @@ __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restric
         if (lane == 0u) mu = m;
         __syncwarp();
     };
+    auto split = [&]() {
+        const u32 a8 = 8u * c.pa, q1 = mu.s1 + a8, q2 = mu.s2 + 8u * c.f - a8;
+        const u64 A1 = mu.U1 | shl64(1ull, q1), A2 = mu.U2 | shl64(1ull, q2);
+        __syncwarp();
+        if (lane == 0u) {
+            mu.A1 = A1; mu.A2 = A2;
+            mu.mask = ~shl64(~0ull, a8);
+            mu.at = 8u * (c.f - c.fi);
+            mu.a8 = a8;
+        }
+        __syncwarp();
+    };
     auto over = [&]() -> u32 {
         return mu.s2 + 8u * (c.f - c.pa) == 0u ? 1u : (mu.s1 + 8u * c.pa == 0u ? 2u : 0u);
     };
     auto ended = [&](u32 k) {
-        if (lane == 0u) atomicAdd(&she[h], k);
+        if (lane == 0u) atomicAdd(&sh[hbins + h], k);
         maxfin = max(maxfin, h);
     };
     auto build = [&](u32 sel) -> bool {
-        const u32 a8 = 8u * c.pa;
-        const u64 lw = mu.O | ((u64)merge_row(mu.c0, mu.c1, sel) << (8u * (c.f - c.fi)));
-        g.w1 = mu.U1 | shl64(lw & ~shl64(~0ull, a8), mu.s1) | shl64(1ull, mu.s1 + a8);
-        g.w2 = mu.U2 | shl64(shr64(lw, a8), mu.s2) | shl64(1ull, mu.s2 + 8u * c.f - a8);
+        const u32 a8 = mu.a8, s1 = mu.s1;
+        const u64 lw = mu.O | shl64((u64)merge_row(mu.c0, mu.c1, sel), mu.at);
+        const u64 w1 = mu.A1 | shl64(lw & mu.mask, s1), w2 = mu.A2 | shl64(shr64(lw, a8), mu.s2);
         if (c.filter) {   // player 1 must hold card n - 1
-            const u64 x = g.w1 ^ pat;
+            const u64 x = w1 ^ pat;
             if (((x - 0x1111111111111111ull) & ~x & 0x8888888888888888ull) == 0ull) return false;
         }
-        g.q = mu.s1 + a8 - n2;
-        g.t1 = g.w1; g.t2 = g.w2; g.rounds = h; g.next = 2u * h + W;
-        g.mv = 0; g.wt = c.wt; g.at = NO_LANDMARK;
-        miss->ta = 0; miss->tb = 0;
-        g.done = false; g.kcy = false; g.active = true;
+        g.w1 = g.t1 = w1; g.w2 = g.t2 = w2;
+        g.q = s1 + a8 - n2;
+        g.rounds = h; g.next = 2u * h + W;
+        g.mv = 0; g.wt = c.wt; g.missed = 0;
         return true;
     };
-    auto refill = [&](bool want) {
-        if (want) g.active = false;
-        merge_deal(c, a, counter, want, setup, over, ended, build, drain);
+    auto refill = [&](u32 need) {
+        if ((need >> lane) & 1u) { g.next = IDLE; g.q = FROZEN; g.t1 = g.t2 = ~0ull; }
+        merge_deal(c, a, counter, need, setup, split, over, ended, build, drain);
     };
 
-    refill(true);
-    bool running = __any_sync(WAR_FULL_MASK, g.active);
+    refill(WAR_FULL_MASK);
+    bool running = __any_sync(WAR_FULL_MASK, g.next != IDLE);
     while (running) {
-        for (int k = 0; k < period; k += 4) {
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const u64 v1 = g.w1, v2 = g.w2;
-                u32 c1, c2;
-                war_turn_fma<RULE>(g.w1, g.w2, g.q, K, c1, c2);
-                const bool top = (c1 == n - 1u) | (c2 == n - 1u);
-                g.m1 = top ? v1 : g.m1;
-                g.m2 = top ? v2 : g.m2;
-                g.at = top ? (u32)(k + u) : g.at;
-                const bool en = g.q * g.q == K.end2;
-                if (!g.done) g.rounds += K.one;
-                const bool cy = (g.w1 == g.t1) & (g.w2 == g.t2);
-                const bool fin = (cy | en) & !g.done;
-                g.kcy = fin ? cy : g.kcy;
-                g.done = g.done | fin;
-            }
-        }
-        if (!g.done && g.rounds >= g.next) {   // Brent's checkpoint (war_refill.cuh)
-            if (g.next > WAR_TURN_CAP) { capped++; g.done = true; }   // abandoned (never expected): the job fails
-            else { g.t1 = g.w1; g.t2 = g.w2; g.next = 2u * g.rounds + W; }
-        }
-        if (memo != nullptr && g.done && g.kcy && g.mv == 0u) {   // found by Brent: record the cycle
-            const u32 v = 2u * (g.rounds - ((g.next - W) >> 1));
-            if (v <= vmask) { g.mv = v; g.next = RECORDING; g.done = false; }
-        } else if (memo != nullptr && !g.done && g.at != NO_LANDMARK) {
-            const u64 key = memo_key_state(g.m1, g.m2, n);
-            const u32 at = g.rounds - (u32)period + g.at;
-            if (g.next == RECORDING) {
-                __stcg((unsigned long long*)memo + memo_slot(key, mbits), path_entry(key, mbits, g.mv));
-                mstore++;
-            } else {
-                const u64 e = __ldcg((const unsigned long long*)memo + memo_slot(key, mbits));
-                mlook++;
-                const u32 v = (u32)e & vmask;
-                if (v != 0u && ((e ^ path_entry(key, mbits, 0ull)) >> mbits) == 0ull) {
-                    mhit++;
-                    g.done = true; g.kcy = (v & 1u) == 0u; g.mv = v;
-                    g.next = at + (v >> 1);   // the game's length, if it ends
-                } else {
-                    miss->kb = miss->ka; miss->tb = miss->ta;
-                    miss->ka = key; miss->ta = at + 1u;
-                }
-            }
-        }
+        u32 ev = NO_EVENT;
         g.at = NO_LANDMARK;
-        const bool fin = g.done & g.active;
-        if (__any_sync(WAR_FULL_MASK, fin)) {
-            if (fin) {
-                turns += g.rounds - h;
-                const u32 mcy = (g.mv & 1u) ? 0u : g.mv >> 1;
-                const u32 len = (g.mv & 1u) ? g.next : g.rounds;
-                const u32 lam = mcy ? mcy : g.rounds - ((g.next - W) >> 1);
-                mstore += store_missed(memo, mbits, *miss, g.kcy ? 2u * lam : 0u, len);
-                if (g.kcy) {
-                    cyc += g.wt;
-                    if (a.hbins) atomicAdd(&shh[lam < hb1 ? lam : hb1], g.wt);
-                } else {
-                    maxfin = max(maxfin, len);
-                    atomicAdd(&she[len < WAR_EBINS - 1 ? len : WAR_EBINS - 1], g.wt);
+        for (u32 k2 = 0; k2 < 2u * period; k2 += 8u) {
+            war_turn_tests<RULE, 0>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, n - 1u, K);
+            war_turn_tests<RULE, 1>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, n - 1u, K);
+            war_turn_tests<RULE, 2>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, n - 1u, K);
+            war_turn_tests<RULE, 3>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, n - 1u, K);
+        }
+        // out: a decided game's outcome, 2 lam for a cycle, 2 len + 1 for an end
+        const u32 base = g.rounds;
+        const bool open = ev == NO_EVENT;
+        g.rounds = base + (open ? period : (ev >> 1) + 1u);
+        bool fin = !open;
+        u32 out = (ev & 1u) ? 2u * g.rounds + 1u : g.mv;
+        const bool mark = open & (g.at != NO_LANDMARK);
+        const u32 at = base + (g.at >> 1);
+        u64 hash = 0;
+        if (table) hash = memo.hash(g.m1, g.m2);
+        if (open ? (g.rounds >= g.next || (g.next == RECORDING && mark)) : out == 0u) {
+            if (!open) {                         // Brent found the cycle: record it
+                out = 2u * (g.rounds - ((g.next - W) >> 1));
+                if (table && out <= memo.vmask) {
+                    fin = false;
+                    g.mv = out; g.next = RECORDING;
+                    g.w1 = g.t1; g.w2 = g.t2; g.q = 4u * pile_len(g.t1) - n2;   // (the game stands frozen)
                 }
+            } else if (g.next == RECORDING) {
+                memo.store(hash, g.mv);
+                mstore++;
+            } else if (g.next > WAR_TURN_CAP) {  // abandoned (never expected): the job fails
+                capped++; fin = true; out = 1u;
+            } else {                             // Brent's checkpoint (war_refill.cuh)
+                g.t1 = g.w1; g.t2 = g.w2; g.next = 2u * g.rounds + W;
             }
-            refill(fin);
-            running = __any_sync(WAR_FULL_MASK, g.active);
+        }
+        const bool look = table & mark & (g.next < IDLE);
+        u64 e = 0;
+        if (look) e = __ldcg((const unsigned long long*)memo.word(hash));
+        e ^= hash << memo.bits;                  // the value, if the entry is the landmark's
+        const u32 v = (u32)e;
+        const bool hit = look & ((u32)(e >> 32) == 0u) & (v - 1u < memo.vmask);
+        mlook += look ? 1u : 0u;
+        mhit += hit ? 1u : 0u;
+        if (hit) out = v + ((v & 1u) ? 2u * at : 0u);
+        if (look & !hit) {
+            miss->h[g.missed & 1u] = hash;
+            miss->t[g.missed & 1u] = at;
+            g.missed++;
+        }
+        fin = fin | hit;
+        const u32 need = __ballot_sync(WAR_FULL_MASK, fin);
+        if (need) {
+            if (fin) {
+                const bool cy = (out & 1u) == 0u;
+                turns += g.rounds - h;
+                if (g.missed) mstore += memo.store_missed(*miss, g.missed, out);
+                const u32 len = out >> 1, bin = cy ? min(len, hb1) : hbins + min(len, (u32)WAR_EBINS - 1u);
+                if (!cy | (hbins != 0u)) atomicAdd(&sh[bin], g.wt);
+                cyc += cy ? g.wt : 0u;
+                maxfin = max(maxfin, cy ? 0u : len);
+            }
+            refill(need);
+            running = __any_sync(WAR_FULL_MASK, g.next != IDLE);
         }
     }
 
@@ -230,57 +256,65 @@ __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restric
         if (v_s) atomicAdd(&acc->memo_stores, v_s);
     }
     __syncthreads();
-    flush_hist(shh, acc->hist, a.hbins);
-    flush_hist(she, acc->endhist, WAR_EBINS);
+    flush_hist(sh, acc->hist, a.hbins);
+    flush_hist(sh + hbins, acc->endhist, WAR_EBINS);
 }
 
 // ---- canonical scans ----------------------------------------------------------------------------------
 //
 // The same loop for canonical positions with the path memo, one game each.  EXTRA: the distinct-cycle outputs and
 // the sample (gpu/war_gpu.py:217-235); SHAPE: the loop-shape test, whose code travels in the memo with the cycle
-// length (war_refill.cuh).  Whether the start of a game lies on its cycle (distinct) shows within Brent's first
-// window, which compares every state up to turn W with the start: a memo hit "cycle of length lam" before turn
-// lam <= W is held (pend) until then.
+// length (war_refill.cuh).  Whether the start of a game lies on its cycle (distinct): Brent's first window compares
+// every state up to turn W with the start; the starts of games that the memo decides are queued and walked around
+// 32 at a time, without the tests of the loop (playing such games on to turn lam cost a fifth of the n = 14 scan, where
+// 3% of the positions cycle).
 //
 // What bounds it: instruction issue and the random reads of the table, about equally; in a small scan the number
 // of warps at work, which is why a warp, not a lane, takes a unit (a lane of the kernel it replaces played 120
 // orders with all their splits alone).  B200: 2e6 positions of 11 cards 8.9 -> 0.40 ms, 3e9 of 14 cards 164 ->
 // 152 ms (defer 16; 12: 156, 8: 176 ms; 256 to 1024 threads alike).
-template <bool EXTRA>
 struct CGame {
     u64 w1, w2, t1, t2, m1, m2;
-    u32 q, rounds, next, mv, pend, at;
-    bool done, kcy, active, sampled, first;   // first: on the cycle from its start
+    u32 q, rounds, next, mv, at, missed;
+    bool sampled, first;          // first: on its cycle from the start
+};
+
+// Starts of a warp's games that the memo found to cycle, with their cycle lengths, until 32 of them are walked
+// around together to see which lie on their cycle.
+struct StartQueue {
+    u64 s1[64], s2[64];
+    u32 lam[64];
 };
 
 template <int RULE, bool EXTRA, bool SHAPE>
 __device__ __forceinline__ void canon_body(const MergeArgs& a, DevAcc* __restrict__ acc, u64* __restrict__ counter,
                                            UnitStore& store, u64* sh64) {
-    CUnit* const units = store.c;
     Missed* const miss = (Missed*)sh64 + threadIdx.x;
-    u64* const starts = (u64*)((Missed*)sh64 + blockDim.x);             // EXTRA: the starting piles
-    u32* const shh = (u32*)(starts + (EXTRA ? 2u * blockDim.x : 0u));
-    u32* const she = shh + a.hbins;
+    u64* const starts = (u64*)((Missed*)sh64 + blockDim.x);             // EXTRA: the starting piles,
+    StartQueue* const queues = (StartQueue*)(starts + (EXTRA ? 2u * blockDim.x : 0u));   // and the warps' queues
+    StartQueue& queue = queues[threadIdx.x >> 5];
+    u32* const sh = (u32*)(queues + (EXTRA ? blockDim.x >> 5 : 0u));     // cycle lengths, then ending lengths
+    const u32 hbins = (u32)a.hbins;
     const int bins = a.hbins + WAR_EBINS;
-    for (int b = threadIdx.x; b < bins; b += blockDim.x) shh[b] = 0;
+    for (int b = threadIdx.x; b < bins; b += blockDim.x) sh[b] = 0;
     __syncthreads();
 
     const u32 n = (u32)a.n, m = n - 1u, k4m4 = 4u * m, W = (u32)a.W, n2 = 2u * n;
     const TurnK K = a.tk;
-    const u32 hb1 = a.hbins > 0 ? (u32)(a.hbins - 1) : 0u;
-    const int period = a.defer > 4 ? (a.defer + 3) & ~3 : 4;
-    u64* const memo = a.memo;
-    const u32 mbits = a.memo_bits, lsh = SHAPE ? 3u : 1u;          // a memo value: 8 lam + 2 code, or 2 lam
-    const u32 vmask = (1u << mbits) - 1u;
+    const u32 hb1 = hbins ? hbins - 1u : 0u;
+    const u32 period = a.defer > 4 ? (u32)((a.defer + 3) & ~3) : 4u;
+    const MemoTable memo(a.memo, a.memo_bits, n);
+    const bool table = a.memo != nullptr;
+    constexpr u32 lsh = SHAPE ? 3u : 1u;                               // a memo value: 8 lam + 2 code, or 2 lam
     const u32 lane = threadIdx.x & 31u;
-    CUnit& cu = units[threadIdx.x >> 5];
+    CUnit& cu = store.c[threadIdx.x >> 5];
 
     MCursor c;
     u32 cyc = 0, turns = 0, maxfin = 0, capped = 0, mlook = 0, mhit = 0, mstore = 0, nonstd = 0, unchk = 0;
     u32 sc = 0, scy = 0, slam = 0, slen = 0, smax = 0, oncyc = 0, dmin = 0;
-    CGame<EXTRA> g;
-    g.active = false; g.done = true; g.kcy = false; g.sampled = g.first = false; g.w1 = g.w2 = 1ull; g.t1 = g.t2 = 0ull;
-    g.q = 0; g.rounds = 0; g.next = 0xFFFFFFFFu; g.m1 = g.m2 = 0ull; g.at = NO_LANDMARK; g.mv = 0; g.pend = 0;
+    CGame g;
+    g.w1 = g.w2 = 1ull; g.m1 = g.m2 = 0ull; g.rounds = g.mv = g.missed = 0; g.at = NO_LANDMARK;
+    g.sampled = g.first = false;
 
     // (A launch plays fewer than 2^32 positions: no bin and no total of a lane or warp can wrap.)
     auto drain = [&]() {};
@@ -291,16 +325,53 @@ __device__ __forceinline__ void canon_body(const MergeArgs& a, DevAcc* __restric
         if (lane == 0u) cu = u;
         __syncwarp();
     };
+    auto split = [&]() {   // canon_position (war_core.cuh) of split c.pa without the other cards
+        __syncwarp();
+        if (lane == 0u) {
+            cu.A1 = (u64)m | (1ull << (4u * (c.pa + 1u)));
+            cu.A2 = 1ull << (4u * (m - c.pa));
+            cu.mask = ~shl64(~0ull, 4u * c.pa);
+            cu.at = 4u * (m - c.fi);
+            cu.k4 = 4u * c.pa;
+        }
+        __syncwarp();
+    };
+    // a start on its cycle of length lam: the distinct-cycle counts (gpu/war_gpu.py:217-235)
+    auto on_cycle = [&](u64 s1, u64 s2, u32 lam) {
+        const CycleWalk cw = cycle_walk<RULE>(s1, s2, 4u * pile_len(s1), n, lam);
+        oncyc++;
+        if (cw.is_min) dmin++;
+        if (a.dbins) {
+            const u32 d = cw.sym ? cw.c1 : cw.c1 + cw.c2, db1 = (u32)(a.dbins - 1);
+            atomicAdd(&acc->dhist[d < db1 ? d : db1], 1ull);
+        }
+    };
+    // walks up to 32 queued starts around, one per lane
+    u32 queued = 0;
+    auto walk_queue = [&]() {
+        __syncwarp();
+        const u32 k = min(queued, 32u);
+        queued -= k;
+        if (lane < k) {
+            const u64 s1 = queue.s1[queued + lane], s2 = queue.s2[queued + lane];
+            const u32 lam = queue.lam[queued + lane];
+            u64 v1 = s1, v2 = s2;
+            u32 q = 4u * pile_len(s1) - n2;
+            for (u32 t = 0; t < lam; t++) war_turn_fma<RULE>(v1, v2, q, K);
+            if (v1 == s1 && v2 == s2) on_cycle(s1, s2, lam);
+        }
+        __syncwarp();
+    };
     auto over = []() -> u32 { return 0u; };
     auto ended = [](u32) {};
     auto build = [&](u32 sel) -> bool {
-        u32 q4;
-        canon_position(cu.Q | ((u64)merge_row(cu.c0, cu.c1, sel) << (4u * (m - c.fi))), n, c.pa, g.w1, g.w2, q4);
-        g.q = q4 - n2;
-        g.t1 = g.w1; g.t2 = g.w2; g.rounds = 0; g.next = W;
-        g.mv = 0; g.pend = 0; g.at = NO_LANDMARK; g.first = false;
-        miss->ta = 0; miss->tb = 0;
-        g.done = false; g.kcy = false; g.active = true;
+        const u64 q = cu.Q | shl64((u64)merge_row(cu.c0, cu.c1, sel), cu.at);
+        const u32 k4 = cu.k4;
+        g.w1 = g.t1 = cu.A1 | ((q & cu.mask) << 4);
+        g.w2 = g.t2 = cu.A2 | shr64(q, k4);
+        g.q = k4 + 4u - n2;
+        g.rounds = 0; g.next = W;
+        g.mv = 0; g.missed = 0; g.first = false;
         if (EXTRA) {
             starts[threadIdx.x] = g.w1;
             starts[threadIdx.x + blockDim.x] = g.w2;
@@ -308,119 +379,113 @@ __device__ __forceinline__ void canon_body(const MergeArgs& a, DevAcc* __restric
         }
         return true;
     };
-    auto refill = [&](bool want) {
-        if (want) g.active = false;
-        merge_deal<true>(c, a, counter, want, setup, over, ended, build, drain);
+    auto refill = [&](u32 need) {
+        if ((need >> lane) & 1u) { g.next = IDLE; g.q = FROZEN; g.t1 = g.t2 = ~0ull; }
+        merge_deal<true>(c, a, counter, need, setup, split, over, ended, build, drain);
     };
 
-    refill(true);
-    bool running = __any_sync(WAR_FULL_MASK, g.active);
+    refill(WAR_FULL_MASK);
+    bool running = __any_sync(WAR_FULL_MASK, g.next != IDLE);
     while (running) {
-        for (int k = 0; k < period; k += 4) {
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const u64 v1 = g.w1, v2 = g.w2;
-                u32 c1, c2;
-                war_turn_fma<RULE>(g.w1, g.w2, g.q, K, c1, c2);
-                const bool top = (c1 == n - 1u) | (c2 == n - 1u);
-                g.m1 = top ? v1 : g.m1;
-                g.m2 = top ? v2 : g.m2;
-                g.at = top ? (u32)(k + u) : g.at;
-                const bool en = g.q * g.q == K.end2;
-                if (!g.done) g.rounds += K.one;
-                const bool cy = (g.w1 == g.t1) & (g.w2 == g.t2);
-                const bool fin = (cy | en) & !g.done;
-                g.kcy = fin ? cy : g.kcy;
-                g.done = g.done | fin;
-            }
-        }
-        if (!g.done && g.rounds >= g.next) {   // Brent's checkpoint (war_refill.cuh)
-            if (g.next > WAR_TURN_CAP) { capped++; g.done = true; }   // abandoned (never expected): the job fails
-            else { g.t1 = g.w1; g.t2 = g.w2; g.next = 2u * g.rounds + W; }
-        }
-        if (g.done && g.kcy && g.mv == 0u && g.active) {   // found by Brent: record the cycle
-            const u32 lam = g.rounds - ((g.next - W) >> 1);
-            const u32 code = SHAPE ? (u32)loop_shape_walk<RULE>(g.w1, g.w2, g.q + n2, k4m4, lam, (u32)a.blk) : 0u;
-            const u32 v = SHAPE ? 8u * lam + 2u * code : 2u * lam;
-            g.first = g.next == W;
-            g.mv = v;
-            g.pend = 0u;
-            if (memo != nullptr && v <= vmask) { g.next = RECORDING; g.done = false; }
-        } else if (memo == nullptr) {
-        } else if (!g.done && g.pend == 0u && g.at != NO_LANDMARK) {
-            const u64 key = memo_key_state(g.m1, g.m2, n);
-            const u32 at = g.rounds - (u32)period + g.at;
-            if (g.next == RECORDING) {
-                __stcg((unsigned long long*)memo + memo_slot(key, mbits), path_entry(key, mbits, g.mv));
-                mstore++;
-            } else {
-                const u64 e = __ldcg((const unsigned long long*)memo + memo_slot(key, mbits));
-                mlook++;
-                const u32 v = (u32)e & vmask;
-                if (v != 0u && ((e ^ path_entry(key, mbits, 0ull)) >> mbits) == 0ull) {
-                    mhit++;
-                    const bool vcy = (v & 1u) == 0u;
-                    if (EXTRA && a.distinct && vcy && (v >> lsh) <= W && g.rounds < (v >> lsh)) g.pend = v;
-                    else {
-                        g.done = true; g.kcy = vcy; g.mv = v;
-                        if (!vcy) g.next = at + (v >> 1);   // the game's length
-                    }
-                } else {
-                    miss->kb = miss->ka; miss->tb = miss->ta;
-                    miss->ka = key; miss->ta = at + 1u;
-                }
-            }
-        } else if (EXTRA && !g.done && g.pend != 0u && g.rounds >= (g.pend >> lsh)) {
-            // turn lam passed without the start coming back: on the cycle, not through the start
-            g.done = true; g.kcy = true; g.mv = g.pend;
-        }
+        u32 ev = NO_EVENT;
         g.at = NO_LANDMARK;
-        const bool fin = g.done & g.active;
-        if (__any_sync(WAR_FULL_MASK, fin)) {
+        for (u32 k2 = 0; k2 < 2u * period; k2 += 8u) {
+            war_turn_tests<RULE, 0>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, m, K);
+            war_turn_tests<RULE, 1>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, m, K);
+            war_turn_tests<RULE, 2>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, m, K);
+            war_turn_tests<RULE, 3>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, m, K);
+        }
+        // out: a decided game's outcome, the memo value of a cycle, 2 len + 1 for an end
+        const u32 base = g.rounds;
+        const bool open = ev == NO_EVENT;
+        g.rounds = base + (open ? period : (ev >> 1) + 1u);
+        bool fin = !open;
+        u32 out = (ev & 1u) ? 2u * g.rounds + 1u : g.mv;
+        const bool mark = open & (g.at != NO_LANDMARK);
+        const u32 at = base + (g.at >> 1);
+        u64 hash = 0;
+        if (table) hash = memo.hash(g.m1, g.m2);
+        if (open ? (g.rounds >= g.next || (g.next == RECORDING && mark)) : out == 0u) {
+            if (!open) {                         // Brent found the cycle: record it
+                const u32 lam = g.rounds - ((g.next - W) >> 1);
+                out = 2u * lam;
+                if (SHAPE)
+                    out = 8u * lam + 2u * (u32)loop_shape_walk<RULE>(g.t1, g.t2, 4u * pile_len(g.t1), k4m4, lam, (u32)a.blk);
+                g.first = g.next == W;
+                if (table && out <= memo.vmask) {
+                    fin = false;
+                    g.mv = out; g.next = RECORDING;
+                    g.w1 = g.t1; g.w2 = g.t2; g.q = 4u * pile_len(g.t1) - n2;   // (the game stands frozen)
+                }
+            } else if (g.next == RECORDING) {
+                memo.store(hash, g.mv);
+                mstore++;
+            } else if (g.next > WAR_TURN_CAP) {  // abandoned (never expected): the job fails
+                capped++; fin = true; out = 1u;
+            } else {                             // Brent's checkpoint (war_refill.cuh)
+                g.t1 = g.w1; g.t2 = g.w2; g.next = 2u * g.rounds + W;
+            }
+        }
+        const bool look = table & mark & (g.next < IDLE);
+        u64 e = 0;
+        if (look) e = __ldcg((const unsigned long long*)memo.word(hash));
+        e ^= hash << memo.bits;                  // the value, if the entry is the landmark's
+        const u32 v = (u32)e;
+        const bool hit = look & ((u32)(e >> 32) == 0u) & (v - 1u < memo.vmask);
+        mlook += look ? 1u : 0u;
+        mhit += hit ? 1u : 0u;
+        if (look & !hit) {
+            miss->h[g.missed & 1u] = hash;
+            miss->t[g.missed & 1u] = at;
+            g.missed++;
+        }
+        if (hit) out = v + ((v & 1u) ? 2u * at : 0u);
+        fin = fin | hit;
+        const u32 need = __ballot_sync(WAR_FULL_MASK, fin);
+        if (need) {
+            bool push = false;
             if (fin) {
+                const bool cy = (out & 1u) == 0u;
+                const u32 len = cy ? out >> lsh : out >> 1;
                 turns += g.rounds;
-                const bool cy = g.kcy;
-                const u32 mcy = (g.mv & 1u) ? 0u : g.mv >> lsh;
-                const u32 len = (g.mv & 1u) ? g.next : g.rounds;
-                const u32 lam = mcy;      // (of a cycle: Brent's are values by now, too)
                 if (SHAPE && cy) {
-                    const u32 code = (g.mv >> 1) & 3u;
+                    const u32 code = (out >> 1) & 3u;
                     if (code == 1u) nonstd++;
                     if (code == 2u) unchk++;
                 }
-                mstore += store_missed(memo, mbits, *miss, cy ? g.mv : 0u, len);
-                if (cy) {
-                    cyc++;
-                    if (a.hbins) atomicAdd(&shh[lam < hb1 ? lam : hb1], 1u);
-                    if (EXTRA && a.distinct) {
-                        // decided by the memo: the start was not seen again within lam <= W turns, or lam > W: walk
-                        const u64 s1 = starts[threadIdx.x], s2 = starts[threadIdx.x + blockDim.x];
-                        const u32 sq = 4u * pile_len(s1);
-                        const bool on = g.first || (lam > W && on_cycle_walk<RULE>(s1, s2, sq, n, lam));
-                        if (on) {
-                            const CycleWalk cw = cycle_walk<RULE>(s1, s2, sq, n, lam);
-                            oncyc++;
-                            if (cw.is_min) dmin++;
-                            if (a.dbins) {
-                                const u32 d = cw.sym ? cw.c1 : cw.c1 + cw.c2, db1 = (u32)(a.dbins - 1);
-                                atomicAdd(&acc->dhist[d < db1 ? d : db1], 1ull);
-                            }
-                        }
-                    }
-                } else {
-                    maxfin = max(maxfin, len);
-                    atomicAdd(&she[len < WAR_EBINS - 1 ? len : WAR_EBINS - 1], 1u);
+                if (g.missed) mstore += memo.store_missed(*miss, g.missed, out);
+                const u32 bin = cy ? min(len, hb1) : hbins + min(len, (u32)WAR_EBINS - 1u);
+                if (!cy | (hbins != 0u)) atomicAdd(&sh[bin], 1u);
+                cyc += cy ? 1u : 0u;
+                maxfin = max(maxfin, cy ? 0u : len);
+                if (EXTRA && cy && a.distinct) {
+                    if (g.first) on_cycle(starts[threadIdx.x], starts[threadIdx.x + blockDim.x], len);
+                    // if Brent's first window saw lam turns pass, it would have seen the start again
+                    push = !g.first && (len > W || g.rounds < len);
                 }
                 if (EXTRA && g.sampled) {
                     sc++;
-                    if (cy) { scy++; slam += lam; }
+                    if (cy) { scy++; slam += len; }
                     else { slen += len; smax = max(smax, len); }
                 }
             }
-            refill(fin);
-            running = __any_sync(WAR_FULL_MASK, g.active);
+            if (EXTRA && a.distinct) {
+                const u32 pb = __ballot_sync(WAR_FULL_MASK, push);
+                if (push) {
+                    const u32 i = queued + (u32)__popc(pb & ((1u << lane) - 1u));
+                    queue.s1[i] = starts[threadIdx.x];
+                    queue.s2[i] = starts[threadIdx.x + blockDim.x];
+                    queue.lam[i] = out >> lsh;
+                }
+                queued += (u32)__popc(pb);
+                if (queued >= 32u) walk_queue();
+            }
+            refill(need);
+            running = __any_sync(WAR_FULL_MASK, g.next != IDLE);
         }
     }
+
+    if (EXTRA) while (queued) walk_queue();
 
     const u64 v_cyc = warp_sum((u64)cyc), v_turns = warp_sum((u64)turns), v_max = warp_max((u64)maxfin);
     const u64 v_cap = warp_sum((u64)capped), v_l = warp_sum((u64)mlook), v_h = warp_sum((u64)mhit);
@@ -456,8 +521,8 @@ __device__ __forceinline__ void canon_body(const MergeArgs& a, DevAcc* __restric
         }
     }
     __syncthreads();
-    flush_hist(shh, acc->hist, a.hbins);
-    flush_hist(she, acc->endhist, WAR_EBINS);
+    flush_hist(sh, acc->hist, a.hbins);
+    flush_hist(sh + hbins, acc->endhist, WAR_EBINS);
 }
 
 }  // namespace war

@@ -443,18 +443,16 @@ template <int MODE>
 __device__ __forceinline__ u32 memo_lam_shift(u32 n) { return MODE >= MEMO_ALL ? 4u * n : 4u * (n - 1u); }
 
 // Walks the cycle of length lam through the state (w1, w2, q4 = 4*len1) once and stores its landmarks
-// (MEMO_LANDMARK; MEMO_PATH with TOPS, as path entries) or all its states (MEMO_ALL, MEMO_PATH).
-template <int RULE, int MODE, bool TOPS = false>
-__device__ __noinline__ void memo_store_cycle(u64* T, u32 bits, u64 w1, u64 w2, u32 q4, u32 n, u32 lam,
-                                              u32 pv = 0u) {
+// (MEMO_LANDMARK) or all its states (MEMO_ALL, MEMO_PATH).
+template <int RULE, int MODE>
+__device__ __noinline__ void memo_store_cycle(u64* T, u32 bits, u64 w1, u64 w2, u32 q4, u32 n, u32 lam) {
     const u32 lsh = memo_lam_shift<MODE>(n);
-    const u32 v = MODE == MEMO_PATH ? (pv ? pv : 2u * lam) : lam;   // pv: the path value, if not 2 lam
+    const u32 v = MODE == MEMO_PATH ? 2u * lam : lam;
     if (lam == 0u || (u64)v >> (MODE == MEMO_PATH ? bits : 64u - lsh) != 0ull) return;
     const u32 k4m4 = 4u * (n - 1u);
     const u64 top = (u64)(n - 1u);
     for (u32 t = 0; t < lam; t++) {
         if (MODE == MEMO_PATH) {
-            if (TOPS && (w1 & 15ull) != top && (w2 & 15ull) != top) { war_turn<RULE>(w1, w2, q4, k4m4); continue; }
             const u64 k = memo_key_state(w1, w2, n);
             __stcg((unsigned long long*)T + memo_slot(k, bits), (unsigned long long)path_entry(k, bits, v));
         } else if (MODE == MEMO_ALL) memo_put(T, bits, memo_key_state(w1, w2, n), lsh, lam);

@@ -129,7 +129,7 @@ struct Variant {
     bool operator==(const Variant& o) const { return !(*this < o) && !(o < *this); }
     int threads() const { return 256; }
     size_t shmem(int hbins) const {   // (a merged launch may hold canonical tasks that keep their starts)
-        return sizeof(u32) * (size_t)(hbins + WAR_EBINS) + (merged ? (sizeof(Missed) + 2 * sizeof(u64)) * (size_t)threads() : 0);
+        return sizeof(u32) * (size_t)(hbins + WAR_EBINS) + (merged ? (sizeof(Missed) + 2 * sizeof(u64) + sizeof(StartQueue) / 32) * (size_t)threads() : 0);
     }
     template <int RULE>
     ServeFn fn_rule() const {

@@ -594,7 +594,7 @@ __global__ void __launch_bounds__(1024) wide_merge_kernel(const __grid_constant_
     };
     auto refill = [&](bool want) {
         if (want) { active = false; kind = K_END; done = true; }
-        merge_deal(c, a, counter, want, setup, over, ended, build, drain);
+        merge_deal(c, a, counter, __ballot_sync(WAR_FULL_MASK, want), setup, []() {}, over, ended, build, drain);
     };
     // Brent and the streak test latch `done` (and by what) and look at the cap at the services; what is decided by
     // turn cap + 1 is decided (wide_kernel).
