@@ -76,18 +76,19 @@ def load_cache():
 
 
 def default_tune(n, mode, rule, flags):
-    """The tune for a job class with no stored entry: the path memo with a table that grows with n (the
-    n = 13 deal and n = 14 canonical measurements: 6! (deals) or 5! x splits (canonical) work units,
-    services every 8 (deals) or 16 (canonical) turns, one game per lane); none below 4 cards."""
+    """The tune for a job class with no stored entry: the path memo with a table that grows with n and services
+    every 8 to 16 turns; none below 4 cards.  Services: a resumed a(13) takes 28.8 ms with one every 8 turns
+    and 33.8 with 12; a span of 14 cards 12.9 and 12.4 (16: 12.8), of 15 cards 81.4 and 75.7 (16: 74.8); 3e9
+    canonical positions of 14 cards 125 with 12 and 134 with 16, 2e6 of 11 cards 0.49 with 12 and 0.42 with 16."""
     if n < 4:
         return None
     # from 13 cards a 2^31-word table (16 GiB): all 13! deals 166.0 ms against 170.7 ms at 2^30
     bits = {4: 12, 5: 12, 6: 14, 7: 16, 8: 18, 9: 20, 10: 22, 11: 24, 12: 27}.get(n, 31)
     variant = 31 if n <= 16 else 3   # the path memo up to 16 cards (it loses on 17-card slices)
     if mode == warlib.CANON:
-        return {"block_m": min(5, n - 1), "blocks_per_sm": 0, "defer": 16, "games": 1, "threads": 512,
+        return {"block_m": min(5, n - 1), "blocks_per_sm": 0, "defer": 16 if n < 13 else 12, "games": 1, "threads": 512,
                 "window": 128, "variant": variant, "memo_bits": bits}
-    return {"block_m": min(6, n), "blocks_per_sm": 0, "defer": 8, "games": 1, "threads": 256, "window": 32,
+    return {"block_m": min(6, n), "blocks_per_sm": 0, "defer": {14: 12, 15: 16, 16: 16}.get(n, 8), "games": 1, "threads": 256, "window": 32,
             "variant": variant, "memo_bits": bits}
 
 

@@ -102,10 +102,12 @@ void canon_plan(const war_job* job, u64 warps, MergePlan& p) {
         }
         if (job->hi % m) add(y, 0, 0, (u32)(job->hi % m));
     }
-    // about 24 units for each warp, so that the last ones end together, of at least 300 games: setting a unit up costs
-    // about what ten games do (2e6 positions of 11 cards: units of 40 games 469 us, 200: 370, 300: 351, 400: 344, 800: 363)
+    // about 24 units for each warp, so that the last ones end together, of at least 64 to 400 games, as many as give
+    // every warp one: setting a unit up costs about what ten games do (2e6 positions of 11 cards: units of 40 games
+    // 469 us, 200: 370, 300: 351, 400: 344, 800: 363)
     u64 lc = rows / std::max<u64>(1, warps * 24);
-    lc = std::min<u64>(std::max<u64>(lc, (300 + m - 1) / m), 720);
+    const u64 least = std::min<u64>(std::max<u64>(rows / std::max<u64>(1, warps), (64 + m - 1) / m), (400 + m - 1) / m);
+    lc = std::min<u64>(std::max(lc, least), 720);
     const u64 parts = (720 + lc - 1) / lc;
     p.lc = (u32)((720 + parts - 1) / parts);
     u64 u = 0;
@@ -172,11 +174,13 @@ void merge_plan(const war_job* job, u64 warps, MergePlan& p) {
         p.games += lists * (B.f + 1u);
         rows4 += lists;
     }
-    // About 24 units for each warp, so that the last ones end together, of at least 40 rows (200 games in a block of
-    // ten cards): 5e6 deals of 11 cards take 235 us with units of 7 rows, 169 with 40, 177 with 80, 236 with 160,
-    // 3e5 of 10 cards 84, 83, 90 and 117.  (6 units for each warp: a span of 14 cards 14.4 ms instead of 14.1.)
+    // About 24 units for each warp, so that the last ones end together, of at least 14 to 60 rows (five games each in a
+    // block of ten cards), as many as give every warp one: kernel times with units of 7, 14, 20, 30, 40 and 60 rows
+    // 43.0, 41.0, 41.9, 46.2, 47.1 and 54.0 us for 3e5 deals of 10 cards, 193, 154, 141, 129, 123 and 119 us for 5e6 of
+    // 11.  (6 units for each warp: a span of 14 cards 14.4 ms instead of 14.1.)
     u64 lc = rows4 / std::max<u64>(1, warps * 24);
-    lc = std::min<u64>(std::max<u64>(lc, 40), 2520);
+    const u64 least = std::min<u64>(std::max<u64>(rows4 / std::max<u64>(1, warps), 14), 60);
+    lc = std::min<u64>(std::max(lc, least), 2520);
     const u64 parts = (2520 + lc - 1) / lc;
     p.lc = (u32)((2520 + parts - 1) / parts);
     u64 u = 0;
@@ -204,6 +208,7 @@ int merge_args(const war_job* job, const MergePlan& p, int hbins, int window, in
     memset(&a, 0, sizeof a);
     a.blocks = c.d_blocks;
     a.table = c.d_table + (job->mode == WAR_CANON ? 2 * MERGE_ROWS : job->rule ? MERGE_ROWS : 0);
+    a.nblocks = (u32)p.blocks.size() - 1u;
     a.lc = p.lc;
     a.n = job->n; a.hbins = hbins; a.W = window; a.defer = defer;
     a.tk.k16 = 16u; a.tk.km16 = (u32)-16; a.tk.k2p28 = 1u << 28; a.tk.k4 = 4u; a.tk.one = 1u;
@@ -252,7 +257,7 @@ int canon_max_blocks_per_sm(int rule, int shape, int extra, int threads, int hbi
     const MergeFn fn = rule ? canon_pick<1>(shape, extra) : canon_pick<0>(shape, extra);
     const size_t shmem = canon_shmem(extra, threads, hbins);
     int nb = 0;
-    if (shmem > 48 * 1024 &&
+    if (shmem > 32 * 1024 &&   // (with the static part it may pass the 48 KB that need no asking)
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem) != cudaSuccess) {
         cudaGetLastError();
         return 0;

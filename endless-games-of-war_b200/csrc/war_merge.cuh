@@ -62,7 +62,7 @@ struct MergeArgs {
     const MBlock* blocks;
     const u32* table;     // MERGE_ROWS byte selectors of the rule (winner's or loser's card first)
     u64 unit_lo, unit_hi; // units of this launch
-    u32 lc;
+    u32 nblocks, lc;      // blocks[nblocks]: the sentinel
     int n, hbins, W, defer;
     u64* memo;
     u32 memo_bits;
@@ -130,6 +130,19 @@ __host__ __device__ __forceinline__ u32 card_count(u32 m) {
 #endif
 }
 
+// x mod k, and x /= k: in 32 bits where x allows (a 64-bit division is some 100 operations).
+__host__ __device__ __forceinline__ u32 take_digit(u64& x, u32 k) {
+    if ((x >> 32) == 0ull) {
+        const u32 y = (u32)x, q = y / k;
+        x = q;
+        return y - q * k;
+    }
+    const u64 q = x / k;
+    const u32 r = (u32)(x - q * k);
+    x = q;
+    return r;
+}
+
 __host__ __device__ __forceinline__ u64 merge_shl(u64 x, u32 s) { return s < 64u ? x << s : 0ull; }
 
 // Sets a unit up (every lane of the warp the same): the piles of 4-bit cards after the turns that its fixed and
@@ -142,16 +155,14 @@ __host__ __device__ __forceinline__ void merge_unit(const MBlock& B, u64 outer, 
     u32 s1 = 0, s2 = 0, half = 0, top = MTOP_INNER;
     if ((b & 1u) && b < n) {
         const u32 k = card_count(free);
-        half = take_card(free, (u32)(outer % k));
-        outer /= k;
+        half = take_card(free, take_digit(outer, k));
     }
     if (n & 1u) {   // player 1's last card, unplayed after h turns, is on top
         u32 c;
         if (b == n) c = B.prefix[n - 1u];
         else {
             const u32 k = card_count(free);
-            c = take_card(free, (u32)(outer % k));
-            outer /= k;
+            c = take_card(free, take_digit(outer, k));
         }
         U1 = c & 15u;
         s1 = 4u;
@@ -168,8 +179,7 @@ __host__ __device__ __forceinline__ void merge_unit(const MBlock& B, u64 outer, 
     u64 O = 0;
     for (u32 i = 0; i < fo; i++) {
         const u32 k = card_count(free), np = k * (k - 1u) / 2u;
-        u32 d = (u32)(outer % np), x = 1;
-        outer /= np;
+        u32 d = take_digit(outer, np), x = 1;
         while (d >= x) { d -= x; x++; }          // the pair of ranks (x, d), x > d
         const u32 hi = take_card(free, x), lo = take_card(free, d);
         if (hi == last) top = MTOP_PAIR + i;
@@ -215,9 +225,7 @@ __host__ __device__ __forceinline__ void canon_unit(const MBlock& B, u64 outer, 
         u32 v;
         if (i < B.b) v = B.prefix[i];
         else {
-            const u32 k = card_count(free);
-            v = take_card(free, (u32)(outer % k));
-            outer /= k;
+            v = take_card(free, take_digit(outer, card_count(free)));
         }
         Q |= (u64)v << (4u * i);
     }
@@ -262,14 +270,22 @@ __device__ __forceinline__ void merge_deal(MCursor& c, const MergeArgs& a, u64* 
                 if (lane == 0u) u = atomicAdd(counter, 1ull);
                 u = __shfl_sync(WAR_FULL_MASK, u, 0) + a.unit_lo;
                 if (u >= a.unit_hi) { c.dry = true; break; }
-                while (u >= a.blocks[c.blk + 1u].u0) c.blk++;
+                // its block: the last one that begins at or before it, 32 at a time from the warp's last block on (a
+                // job has up to 380 blocks; the last is followed by a sentinel that begins after every unit)
+                for (;;) {
+                    const u32 i = min(c.blk + 1u + lane, a.nblocks);
+                    const u32 adv = (u32)__popc(__ballot_sync(WAR_FULL_MASK, u >= a.blocks[i].u0));
+                    c.blk += adv;
+                    if (adv < 32u) break;
+                }
                 const MBlock& B = a.blocks[c.blk];
-                const u64 v = u - B.u0, outer = v / B.nch;
+                u64 outer = u - B.u0;
+                const u32 part = take_digit(outer, B.nch);
                 setup(B, outer);
                 c.f = CANON ? B.k1 - 1u : B.f;
                 c.fi = CANON ? B.inner : min(c.f, MERGE_INNER);
                 c.row0 = CANON ? canon_row0(c.fi) : merge_row0(c.fi);
-                c.l0 = (u32)(v - outer * B.nch) * a.lc;
+                c.l0 = part * a.lc;
                 c.lend = min(CANON ? canon_rows(c.fi) : merge_rows(c.fi), c.l0 + a.lc);
                 c.l = c.l0;
                 c.pa = CANON ? B.k0 : 0u;

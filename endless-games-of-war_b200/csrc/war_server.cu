@@ -224,7 +224,7 @@ void set_args(war_server* s, SJob& J) {
     a.dbins = job.dbins;
     a.blk = (job.flags & WAR_F_SHAPE) && canon ? (job.blk ? job.blk : (job.n & -job.n)) : 0;
     a.W = canon ? 128 : 32;
-    a.defer = canon ? 16 : 8;
+    a.defer = canon ? (job.n < 13 ? 16 : 12) : job.n < 14 ? 8 : job.n == 14 ? 12 : 16;   // (autotune.py's defaults)
     a.tk.k16 = 16u; a.tk.km16 = (u32)-16; a.tk.k2p28 = 1u << 28; a.tk.k4 = 4u; a.tk.one = 1u;
     a.tk.c0 = 2 * job.n - 4; a.tk.end2 = (u32)(4 * job.n * job.n);
     a.half = (job.flags & WAR_F_HALF) ? 1 : 0;
@@ -287,6 +287,7 @@ void set_args(war_server* s, SJob& J) {
     memcpy(h, J.mplan.blocks.data(), sizeof(MBlock) * J.mplan.blocks.size());
     m.blocks = s->d_blocks + (size_t)J.slot * SLOT_BLOCKS;
     m.table = s->d_table + (canon ? 2 * MERGE_ROWS : job.rule ? MERGE_ROWS : 0);
+    m.nblocks = (u32)J.mplan.blocks.size() - 1u;
     m.lc = J.mplan.lc;
     m.n = a.n; m.hbins = a.hbins; m.W = a.W; m.defer = a.defer;
     m.memo = a.memo; m.memo_bits = a.memo_bits; m.tk = a.tk;

@@ -390,15 +390,13 @@ __device__ __forceinline__ void wide_unit(const MBlock& B, u64 outer, u32 n, WUn
     u32 s1 = 0, s2 = 0, half = 0, wins = 0;
     if ((b & 1u) && b < n) {
         const u32 k = (u32)__popc(free);
-        half = take_card(free, (u32)(outer % k)) + 1u;
-        outer /= k;
+        half = take_card(free, take_digit(outer, k)) + 1u;
     }
     if (n & 1u) {   // player 1's last card, unplayed after h turns, is on top
         if (b == n) m.U1l = B.prefix[n - 1u] + 1u;
         else {
             const u32 k = (u32)__popc(free);
-            m.U1l = take_card(free, (u32)(outer % k)) + 1u;
-            outer /= k;
+            m.U1l = take_card(free, take_digit(outer, k)) + 1u;
         }
         s1 = 5u;
     }
@@ -411,8 +409,7 @@ __device__ __forceinline__ void wide_unit(const MBlock& B, u64 outer, u32 n, WUn
     }
     for (u32 i = 0; i < fo; i++) {
         const u32 k = (u32)__popc(free), np = k * (k - 1u) / 2u;
-        u32 d = (u32)(outer % np), x = 1;
-        outer /= np;
+        u32 d = take_digit(outer, np), x = 1;
         while (d >= x) { d -= x; x++; }
         const u32 hi = take_card(free, x) + 1u, lo = take_card(free, d) + 1u;
         m.O |= (u64)(RULE ? lo | (hi << 5) : hi | (lo << 5)) << (10u * i);

@@ -27,10 +27,13 @@ import time
 sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
 import warlib  # noqa: E402
 
-# Ranks enumerated per call of the engine: a few seconds of work, so progress is written about as
-# often as the reference writes it (every 10 s) and an interrupted run loses little.  Just under 2^32,
-# so that a span of deals is one launch of the engine (a launch plays fewer than 2^32 - 2^24 games).
-SPAN_RANKS = (1 << 32) - (1 << 25)
+# Deals enumerated per call of the engine, 14!: a second or two of work, so progress is written about as often
+# as the reference writes it (every 10 s) and an interrupted run loses little.  A factorial, because deals are
+# played together in blocks of as many orders, the larger the fewer games (csrc/war_merge.cuh): all 13! deals in
+# one call 20 ms, in two calls split at 2^32 - 2^25 30 ms.
+SPAN_RANKS = 87178291200
+# The same for canonical positions and for the plain kernel (--plain): just under 2^32, one launch.
+CALL_RANKS = (1 << 32) - (1 << 25)
 
 
 def _tune_for(n, canon, rule, flags):
@@ -96,7 +99,7 @@ def run(n, half=False, per=256, threads=256, batch_threads=1 << 18, out=None, re
     mult_pos = (n - 1) if canon else 1                    # engine ranks per order
     if tune is None and not plain:
         tune = _tune_for(n, canon, rule, flags)
-    span = max(batch_threads * per, SPAN_RANKS // mult_pos if mult_pos else SPAN_RANKS)
+    span = max(batch_threads * per, min(SPAN_RANKS, CALL_RANKS) // mult_pos if canon or plain else SPAN_RANKS)
     t0 = time.time()
     last_write = 0.0
     slowest = 0.0
