@@ -99,7 +99,7 @@ def run(n, half=False, per=256, threads=256, batch_threads=1 << 18, out=None, re
     mult_pos = (n - 1) if canon else 1                    # engine ranks per order
     if tune is None and not plain:
         tune = _tune_for(n, canon, rule, flags)
-    span = max(batch_threads * per, min(SPAN_RANKS, CALL_RANKS) // mult_pos if canon or plain else SPAN_RANKS)
+    span = max(batch_threads * per, min(SPAN_RANKS, CALL_RANKS) // max(1, mult_pos) if canon or plain else SPAN_RANKS)
     t0 = time.time()
     last_write = 0.0
     slowest = 0.0
