@@ -36,12 +36,13 @@ sys.path.insert(0, PKG)
 
 # Algorithmic integer operations per turn: the turn step (pop both tops, compare, build the pair, place it
 # under the winner: 22), Brent's test and bookkeeping (6), the end test (2).  Fixed from the source of
-# war_turn / batched_kernel, not from compiled code.
+# war_turn / batched_kernel, not from compiled code.  (`turns` counts the turns that were played: deals that
+# reach one state are played together from there.)
 K_OPS_PER_TURN = 30
-# DRAM bytes (read + write) per deal of the path-memo refill kernel at this line's configuration (all 13!
-# deals, 16 GiB table): one-pass ncu capture of both launches of a timed step, 699.5 GB read and 11.4 GB
-# written for 6,227,020,800 deals (112.3 + 1.8 B per deal); each random 8-byte lookup costs a DRAM line.
-MEMO_DRAM_BYTES_PER_DEAL = 114.2
+# DRAM bytes (read + write) per deal of the merged path-memo kernel at this line's configuration (all 13! deals in
+# one launch, 16 GiB table): one-pass ncu capture, 58.74 GB read and 1.82 GB written for 6,227,020,800 deals (9.43 +
+# 0.29 B per deal: 681 million games stand for them, and each random 8-byte lookup costs a DRAM line).
+MEMO_DRAM_BYTES_PER_DEAL = 9.73
 # Turns of the reference's own schedule (Brent with the tortoise saved at powers of two from the first turn)
 # over all 13! deals, as counted by an instrumented copy of cpu/war.cpp; the plain kernel reproduces it
 # exactly (its `turns`).
@@ -292,6 +293,27 @@ def deal_extra_units(lo, hi, m):
     return blocks(lo, a2) + blocks(b2, hi) if a2 < b2 else blocks(lo, hi)
 
 
+def range_blocks(lo, hi, n, mode):
+    """How many blocks the path-memo engine copies to the device for ranks [lo, hi): the fewest aligned blocks of
+    j! orders, for canonical positions one more for each order cut by the range, and the sentinel."""
+    f = math.factorial
+    k, m, x, y = 1, n, lo, hi
+    if mode:
+        m = n - 1
+        x, y = lo // m, hi // m
+        if x == y:
+            return 2
+        k += (1 if lo % m else 0) + (1 if hi % m else 0)
+        x += 1 if lo % m else 0
+    while x < y:
+        j = m
+        while j > 0 and (x % f(j) or x + f(j) > y):
+            j -= 1
+        x += f(j)
+        k += 1
+    return k
+
+
 def peaks(warlib, table_bits, clk_mhz=None):
     """The measured ceilings on this GPU: integer issue (LOP3+IMAD), the ALU pipe alone, random 8-byte and
     32-byte gathers from a table of 2^table_bits words, and the nominal issue rate (SMs x 4 schedulers x 32
@@ -502,18 +524,21 @@ def main():
         torch.cuda.synchronize()
         barrier(ws)
         e2e_s = max_over_ranks((time.perf_counter() - t0) / reps, ws)
-        # per step: the extra work units copied in for each engine call, and the accumulator block read back
+        # per step: the blocks (48 bytes) or extra work units (24) copied in for each engine call, and the accumulator
+        # block read back
         spans = []
         if ws == 1 and "lo" not in w:
             mult = (n - 1) if mode else 1
             orders = hi0 // mult
-            span = max(war_gpu.SPAN_RANKS // mult, 1)
+            span = max((war_gpu.CALL_RANKS if mode else war_gpu.SPAN_RANKS) // mult, 1)
             spans = [(a * mult, min(orders, a + span) * mult) for a in range(0, orders, span)]
         else:
             spans = [(lo, hi)]
         h2d = 0
         for a, b in spans:
-            if mode == 0:
+            if tune is not None and tune.variant & 28 == 28 and (mode or not w["flags"] & warlib.F_SAMPLE):
+                h2d += 48 * range_blocks(a, b, n, mode)
+            elif mode == 0:
                 h2d += 24 * deal_extra_units(a, b, min(n, tune.block_m if tune else 6))
             else:
                 h2d += 24 * len(warlib.plan(warlib.make_job(n, mode, 0, w["flags"], a, b), tune.block_m)[2])
