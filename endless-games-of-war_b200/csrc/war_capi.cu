@@ -538,9 +538,13 @@ static int enumerate_merged(const war_job* job, const Tune& t, war_result* out) 
     MergeArgs a;
     int st, used = 0;
     if ((st = merge_args(job, p, job->hbins, t.window, t.defer, a))) return st;
-    // the table's layout (prepare_memo); a game stores at most two states besides the cycles found
+    // the table's layout (prepare_memo)
     const int kind = 4 * 3 + (canon && (job->flags & WAR_F_SHAPE) ? 2 : 0);
-    if ((st = prepare_memo(c, job, t.memo_bits, kind, &a.memo, 2 * p.games, &used))) return st;
+    // Words worth clearing: a game stores at most two landmarks besides the cycles found, most store none.  All 13!
+    // deals (6.8e8 games) take 18.0 ms with 2^29 words, 18.3 with 2^30, 19.3 with 2^31, its end from a saved progress
+    // (1.2e9 games) 30.2 with 2^29 or 2^30 and 31.0 with 2^31; from 15 cards the many cycles fill what there is.
+    const u64 want = canon ? 2 * p.games : job->n >= 15 ? 4 * p.games : p.games / 4 * 3 + 1;
+    if ((st = prepare_memo(c, job, t.memo_bits, kind, &a.memo, want, &used))) return st;
     a.memo_bits = (u32)used;
     if (!canon)
         return run_merged(p, a, MERGE_LAUNCH_UNITS, job->hbins, 0, out,
@@ -596,7 +600,7 @@ int war_enumerate_held(const war_job* job, const war_tune* tune, war_result* out
     // The default turn plays merged games; that needs the checkpoints after turn 0 to be after the merged turns.
     const bool merged = !memo && form == 3 && held_svc(a) && W >= job->n / 2;
     if (!merged && !memo && form == 3) a.svc_off = 1;
-    const int maxb = merged ? held_merged_max_blocks_per_sm(job->rule, threads, job->hbins)
+    const int maxb = merged ? held_merged_max_blocks_per_sm(job->n, job->rule, true, threads, job->hbins)
                             : held_max_blocks_per_sm(job->rule, threads, job->hbins, memo, form, held_svc(a));
     if (maxb < 1) return fail(WAR_EINVAL, "launch shape threads=%d does not fit an SM%s", threads,
                               memo ? " (at most 512 with the memo)" : "");
@@ -609,8 +613,15 @@ int war_enumerate_held(const war_job* job, const war_tune* tune, war_result* out
         merge_plan(job, (u64)blocks * (u64)(threads / 32), p);
         MergeArgs m;
         if ((st = merge_args(job, p, job->hbins, W, defer, m))) return st;
-        return run_merged(p, m, MERGE_LAUNCH_UNITS, job->hbins, 0, out,
-                          [&](cudaStream_t x) { return launch_held_merged(m, job->rule, threads, blocks, c.d_acc, x); });
+        for (bool run : {true, false}) {   // (again without the run test if it left a game open; see the kernel)
+            memset(out, 0, sizeof *out);
+            out->hbins = job->hbins;
+            st = run_merged(p, m, MERGE_LAUNCH_UNITS, job->hbins, 0, out, [&](cudaStream_t x) {
+                return launch_held_merged(m, job->rule, run, threads, blocks, c.d_acc, x);
+            });
+            if (st || !out->undetermined) return st;
+        }
+        return WAR_OK;
     }
     Plan p;
     make_plan(job, block_m, p);

@@ -226,6 +226,137 @@ __device__ __forceinline__ bool h_turn_packed_fma(u64& wh, u64& wo, u32& s, u32 
     return hw & (q == n4m8);
 }
 
+// The packed-count turn with the tests of the merged loop, in the manner of war_turn_tests (war_core.cuh): what goes
+// under the winner's pile, its place, the holder's pop and the new count word are each written by a multiply-add for
+// the usual case and overwritten under "the holder won" and "card n-1 was on top"; a decided game notes 2 (turn in
+// the period) + (1 if it ended) in ev and is frozen by an odd count word far out of range (its low byte never is an
+// opponent's last card, the word no tortoise's, and card n-1 never on top).  HeldK: -1, -260, -252, 65 and 4n - 8 as
+// operands.
+template <int RULE>
+__device__ __forceinline__ void h_turn_tests(u64& wh, u64& wo, u32& s, u64 th, u64 to, u32 ts, u32& ev, u32 k2,
+                                   u32& prev, u32& brk, u32& brk_cy, const TurnK& K, const HeldK& H) {
+    const u32 ol = (u32)wo, oh = (u32)(wo >> 32), hl = (u32)wh, hh = (u32)(wh >> 32);
+    const u32 nol = __funnelshift_r(ol, oh, 4), noh = __umulhi(oh, K.k2p28);
+    const u32 nhl = __funnelshift_r(hl, hh, 4), nhh = __umulhi(hh, K.k2p28);
+    const u32 c = ol & 15u, h = hl & 15u;                     // the two top cards
+    const u32 f = RULE ? h : c, g = RULE ? c : h;             // the opponent won: f first in the pair; the holder: g
+    const u32 q = s & 255u;
+    u64 ao = ((u64)noh << 32) | nol;
+    u32 al = hl, ah = hh;
+    asm("{\n\t"
+        ".reg .pred z, w, e, y, b;\n\t"
+        ".reg .u32 t, ps, xl, xh, bl, bh, s1;\n\t"
+        ".reg .u64 x, a;\n\t"
+        "setp.lt.u32 z, %3, 256;\n\t"                 // the holder plays card n-1
+        "setp.gt.or.u32 w, %9, %8, z;\n\t"            // the holder wins
+        "mad.lo.u32 t, %11, %12, %10;\n\t"               // f + 16 g
+        "@w mad.lo.u32 t, %10, %12, %11;\n\t"            // g + 16 f
+        "@z mad.lo.u32 t, %8, %13, 0;\n\t"            // only the captured card
+        "mad.lo.u32 ps, %14, %15, %16;\n\t"           // 4 (n - 2 - lh)
+        "@w mad.lo.u32 ps, %14, %13, -4;\n\t"
+        "@z mad.lo.u32 ps, %14, %13, 0;\n\t"
+        "@!z mov.b32 %0, %17;\n\t"                    // the holder's pop, unless card n-1 was on top
+        "@!z mov.b32 %1, %18;\n\t"
+        "mad.lo.u32 s1, %3, %13, %19;\n\t"            // one card popped from each pile, card n-1 one place up
+        "@w mad.lo.u32 s1, %3, %13, %20;\n\t"         // and the pair under the holder's
+        "@z mad.lo.u32 s1, %14, %21, %22;\n\t"        // lh + 1 cards, card n-1 at depth lh (rule 0) or lh + 1
+        "setp.eq.and.u32 e, %14, %16, w;\n\t"         // the holder won the opponent's last card
+        "cvt.u64.u32 x, t;\n\t"
+        "shl.b64 x, x, ps;\n\t"
+        "mov.b64 {xl, xh}, x;\n\t"
+        "mov.b64 a, {%0, %1};\n\t"
+        "@w mad.wide.u32 a, xl, %13, a;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t"
+        "@w mad.lo.u32 %1, xh, %13, %1;\n\t"
+        "@!w mad.wide.u32 %2, xl, %13, %2;\n\t"
+        "mov.b64 {bl, bh}, %2;\n\t"
+        "@!w mad.lo.u32 bh, xh, %13, bh;\n\t"
+        "mov.b64 %2, {bl, bh};\n\t"
+        "setp.eq.u32 y, %0, %23;\n\t"
+        "setp.eq.and.u32 y, %1, %24, y;\n\t"
+        "setp.eq.and.u32 y, bl, %25, y;\n\t"
+        "setp.eq.and.u32 y, bh, %26, y;\n\t"
+        "setp.eq.and.u32 y, s1, %27, y;\n\t"
+        "@y mad.lo.u32 %4, %28, %13, 0;\n\t"
+        "@e mad.lo.u32 %4, %28, %13, 1;\n\t"
+        "@y mad.lo.u32 s1, %29, %13, 0;\n\t"
+        "@e mad.lo.u32 s1, %29, %13, 0;\n\t"
+        "mov.u32 %3, s1;\n\t"
+        "}"
+        : "+r"(al), "+r"(ah), "+l"(ao), "+r"(s), "+r"(ev), "+r"(prev), "+r"(brk), "+r"(brk_cy)
+        : "r"(c), "r"(h), "r"(f), "r"(g), "r"(K.k16), "r"(K.one), "r"(q), "r"(H.m1), "r"(H.n4m8), "r"(nhl), "r"(nhh),
+          "r"(H.m260), "r"(H.m252), "r"(H.k65), "n"(4 + 256 * RULE), "r"((u32)th), "r"((u32)(th >> 32)), "r"((u32)to),
+          "r"((u32)(to >> 32)), "r"(ts), "r"(k2), "r"(FROZEN));
+    wh = ((u64)ah << 32) | al;
+    wo = ao;
+}
+
+// The same, noting the last turn at which the player who won the turn before won again (brk, as ev; brk_cy at a
+// cycle), for the run test of the merged loop.
+template <int RULE>
+__device__ __forceinline__ void h_turn_tests_run(u64& wh, u64& wo, u32& s, u64 th, u64 to, u32 ts, u32& ev, u32 k2,
+                                   u32& prev, u32& brk, u32& brk_cy, const TurnK& K, const HeldK& H) {
+    const u32 ol = (u32)wo, oh = (u32)(wo >> 32), hl = (u32)wh, hh = (u32)(wh >> 32);
+    const u32 nol = __funnelshift_r(ol, oh, 4), noh = __umulhi(oh, K.k2p28);
+    const u32 nhl = __funnelshift_r(hl, hh, 4), nhh = __umulhi(hh, K.k2p28);
+    const u32 c = ol & 15u, h = hl & 15u;                     // the two top cards
+    const u32 f = RULE ? h : c, g = RULE ? c : h;             // the opponent won: f first in the pair; the holder: g
+    const u32 q = s & 255u;
+    u64 ao = ((u64)noh << 32) | nol;
+    u32 al = hl, ah = hh;
+    asm("{\n\t"
+        ".reg .pred z, w, e, y, b;\n\t"
+        ".reg .u32 t, ps, xl, xh, bl, bh, s1;\n\t"
+        ".reg .u64 x, a;\n\t"
+        "setp.lt.u32 z, %3, 256;\n\t"                 // the holder plays card n-1
+        "setp.gt.or.u32 w, %9, %8, z;\n\t"            // the holder wins
+        "setp.ne.u32 b, %5, 0;\n\t"                   // the holder won the turn before
+        "xor.pred b, b, w;\n\t"
+        "@!b mad.lo.u32 %6, %28, %13, 0;\n\t"         // the same player again: a break
+        "selp.u32 %5, 1, 0, w;\n\t"
+        "mad.lo.u32 t, %11, %12, %10;\n\t"               // f + 16 g
+        "@w mad.lo.u32 t, %10, %12, %11;\n\t"            // g + 16 f
+        "@z mad.lo.u32 t, %8, %13, 0;\n\t"            // only the captured card
+        "mad.lo.u32 ps, %14, %15, %16;\n\t"           // 4 (n - 2 - lh)
+        "@w mad.lo.u32 ps, %14, %13, -4;\n\t"
+        "@z mad.lo.u32 ps, %14, %13, 0;\n\t"
+        "@!z mov.b32 %0, %17;\n\t"                    // the holder's pop, unless card n-1 was on top
+        "@!z mov.b32 %1, %18;\n\t"
+        "mad.lo.u32 s1, %3, %13, %19;\n\t"            // one card popped from each pile, card n-1 one place up
+        "@w mad.lo.u32 s1, %3, %13, %20;\n\t"         // and the pair under the holder's
+        "@z mad.lo.u32 s1, %14, %21, %22;\n\t"        // lh + 1 cards, card n-1 at depth lh (rule 0) or lh + 1
+        "setp.eq.and.u32 e, %14, %16, w;\n\t"         // the holder won the opponent's last card
+        "cvt.u64.u32 x, t;\n\t"
+        "shl.b64 x, x, ps;\n\t"
+        "mov.b64 {xl, xh}, x;\n\t"
+        "mov.b64 a, {%0, %1};\n\t"
+        "@w mad.wide.u32 a, xl, %13, a;\n\t"
+        "mov.b64 {%0, %1}, a;\n\t"
+        "@w mad.lo.u32 %1, xh, %13, %1;\n\t"
+        "@!w mad.wide.u32 %2, xl, %13, %2;\n\t"
+        "mov.b64 {bl, bh}, %2;\n\t"
+        "@!w mad.lo.u32 bh, xh, %13, bh;\n\t"
+        "mov.b64 %2, {bl, bh};\n\t"
+        "setp.eq.u32 y, %0, %23;\n\t"
+        "setp.eq.and.u32 y, %1, %24, y;\n\t"
+        "setp.eq.and.u32 y, bl, %25, y;\n\t"
+        "setp.eq.and.u32 y, bh, %26, y;\n\t"
+        "setp.eq.and.u32 y, s1, %27, y;\n\t"
+        "@y mad.lo.u32 %4, %28, %13, 0;\n\t"
+        "@e mad.lo.u32 %4, %28, %13, 1;\n\t"
+        "@y mad.lo.u32 s1, %29, %13, 0;\n\t"
+        "@e mad.lo.u32 s1, %29, %13, 0;\n\t"
+        "@y mad.lo.u32 %7, %6, %13, 0;\n\t"
+        "mov.u32 %3, s1;\n\t"
+        "}"
+        : "+r"(al), "+r"(ah), "+l"(ao), "+r"(s), "+r"(ev), "+r"(prev), "+r"(brk), "+r"(brk_cy)
+        : "r"(c), "r"(h), "r"(f), "r"(g), "r"(K.k16), "r"(K.one), "r"(q), "r"(H.m1), "r"(H.n4m8), "r"(nhl), "r"(nhh),
+          "r"(H.m260), "r"(H.m252), "r"(H.k65), "n"(4 + 256 * RULE), "r"((u32)th), "r"((u32)(th >> 32)), "r"((u32)to),
+          "r"((u32)(to >> 32)), "r"(ts), "r"(k2), "r"(FROZEN));
+    wh = ((u64)ah << 32) | al;
+    wo = ao;
+}
+
 // Path-memo key of a held-out state (the entry format of war_refill.cuh: the key itself is not stored, the
 // slot and entry give it back).  The n-1 other cards in the order holder's then opponent's, the holder's
 // count lh and the depth p; the last card is the one missing.  At 17 cards that is 15 nibbles + 8 bits =
@@ -414,7 +545,7 @@ __global__ void __launch_bounds__(MEMO ? 512 : 1024) held_kernel(const __grid_co
 // ---- merged games (war_merge.cuh) -----------------------------------------------------------------------
 //
 // held_kernel plays every deal; this kernel plays each state after the deals' first h = floor(n/2) turns once,
-// for the default turn (h_turn_packed_fma) without the memo and with Brent's checkpoint at multiples of the
+// for the default turn (the packed counts with multiply-adds) without the memo and with Brent's checkpoint at multiples of the
 // service period (SVC above).  `turns` stays what playing every deal gives: the deals of a game share their
 // path from turn h and so the turn at which Brent's checkpoints W, 3W, ... (all at or after turn h) decide them;
 // only a deal that lies on its own cycle, of length lam <= W, is decided by the checkpoint at turn 0 instead, at
@@ -422,12 +553,22 @@ __global__ void __launch_bounds__(MEMO ? 512 : 1024) held_kernel(const __grid_co
 // finds it.  With the tortoise at the state of turn h until turn W, a game on such a cycle is known at turn
 // h + lam, and counted as decided at W + lam.
 //
+// RUN (odd n, winner's card first): where the players alternate, a turn can be undone (war_wide.cu), so a game's cycle
+// begins where its last break is, a turn at which the player who won the turn before won again.  The tortoise
+// follows the last break at the next place where checkpoints are saved, the cycle is found one cycle length later, and
+// `turns` counts the turn at which Brent's checkpoints would have found it.  A game that this does not decide (a cycle
+// with a break in it, which no odd n has, or none by turn RUN_CAP) is counted in DevAcc.undetermined, and the host
+// plays the job again without RUN.
+//
 // Services: games start at services, at turn h, so within the service period all games of a warp reach a
 // multiple of it at the same place, (period - h mod period) turns in; the checkpoint is saved there.
 //
-// What bounds it: instruction issue of the turns (about 150 of them per game, as before; ncu of held_kernel
-// issue 82%, ALU pipe 83%), so the gain is the deals per game, and with it the rate: a slice of 1e9 deals
-// of 17 cards (4.9 deals per game on average) 356 -> 58.6 ms on a B200, a period of 32 turns (16: 63.8, 8: 71.3 ms).
+// What bounds it: instruction issue of the turns; the gain over held_kernel is the deals per game and the turn with
+// its tests in one block (h_turn_tests).  A slice of 1e9 deals of 17 cards (4.9 deals per game on average) on a B200:
+// 356 ms -> 58.6 (merged, h_turn_packed_fma) -> 50.5 (h_turn_tests) -> 46.1 (RUN), with a period of 32 turns (16:
+// 49.4, 8: 57.8 ms).
+
+constexpr u32 RUN_CAP = 1u << 16, RUN_LOST = 0xFFFFFFFDu;   // (RUN_LOST: an odd event, recorded as an end)
 
 // The start of a lane's game, kept for held_start, and its block and holder.
 struct HeldStart {
@@ -462,7 +603,7 @@ __device__ __noinline__ u32 held_start(const HeldStart x, const MBlock* __restri
     return B.twice ? 2u : 1u;
 }
 
-template <int RULE>
+template <int RULE, bool RUN>
 __global__ void __launch_bounds__(1024) held_merge_kernel(const __grid_constant__ MergeArgs a, DevAcc* __restrict__ acc) {
     extern __shared__ u64 sh64[];
     __shared__ MUnit units[32];
@@ -473,8 +614,9 @@ __global__ void __launch_bounds__(1024) held_merge_kernel(const __grid_constant_
     for (int b = threadIdx.x; b < bins; b += blockDim.x) shh[b] = 0;
     __syncthreads();
 
-    const u32 n = (u32)a.n, h = n >> 1, W = (u32)a.W, n4m8 = 4u * n - 8u;
+    const u32 n = (u32)a.n, h = n >> 1, W = (u32)a.W;
     const TurnK K = a.tk;
+    const HeldK H = a.held;
     const u32 hb1 = a.hbins > 0 ? (u32)(a.hbins - 1) : 0u;
     const u32 period = a.defer > 4 ? (u32)((a.defer + 3) & ~3) : 4u;
     const u32 after = h % period, before = period - after;   // turns of a period around the checkpoint's place
@@ -483,9 +625,10 @@ __global__ void __launch_bounds__(1024) held_merge_kernel(const __grid_constant_
     u64* const counter = &acc->work_next;
 
     u64 wh = 0, wo = 0, th = ~0ull, to = 0, turns = 0;
-    u32 s = 0, ts = 0, rounds = 0, next = 0xFFFFFFFFu, wt = 0;
-    bool done = true, kcy = false, active = false;
-    u32 cyc = 0, maxfin = 0, capped = 0;
+    u32 s = FROZEN, ts = 0, rounds = 0, next = 0xFFFFFFFFu, wt = 0;
+    u32 prev = 0, run = 0, save = 0;     // RUN: the last winner, the turn of the last break, of the tortoise
+    bool active = false;
+    u32 cyc = 0, maxfin = 0;
     MCursor c;
 
     auto drain = [&]() {
@@ -539,49 +682,76 @@ __global__ void __launch_bounds__(1024) held_merge_kernel(const __grid_constant_
         s = 4u * lh + 256u * p;
         th = wh; to = wo; ts = s;
         rounds = h; next = W > h ? W : 3u * W; wt = c.wt;   // (W = h: the tortoise of turn W)
-        done = false; kcy = false; active = true;
+        run = save = h;
+        active = true;
         HeldStart x;
         x.wh = wh; x.wo = wo; x.s = s; x.tag = c.blk | (p1 ? 0x80000000u : 0u);
         *start = x;
         return true;
     };
     auto refill = [&](bool want) {
-        if (want) active = false;
+        if (want) { active = false; s = FROZEN; }
         merge_deal(c, a, counter, __ballot_sync(WAR_FULL_MASK, want), setup, []() {}, over, ended, build, drain);
     };
-    auto turn = [&]() {
-        const bool en = h_turn_packed_fma<RULE>(wh, wo, s, n4m8, K);
-        if (!done) rounds++;
-        const bool cy = (wh == th) & (wo == to) & (s == ts);
-        kcy = done ? kcy : (cy & !en);
-        done = done | cy | en;
-    };
-
     refill(true);
     bool running = __any_sync(WAR_FULL_MASK, active);
     while (running) {
-        for (u32 k = 0; k < before; k++) turn();
-        if (!done && rounds == next) {
-            if (next > WAR_TURN_CAP) { capped++; done = true; }   // abandoned (never expected): the job fails
-            else { th = wh; to = wo; ts = s; next = 2u * next + W; }
+        u32 ev = NO_EVENT, brk = NO_EVENT, brk_cy = NO_EVENT;
+        const u32 base = rounds;
+        auto turn = [&](u32 k) {
+            if (RUN) h_turn_tests_run<RULE>(wh, wo, s, th, to, ts, ev, 2u * k, prev, brk, brk_cy, K, H);
+            else h_turn_tests<RULE>(wh, wo, s, th, to, ts, ev, 2u * k, prev, brk, brk_cy, K, H);
+        };
+        auto keep = [&](u32 at) {   // RUN: the tortoise follows the last break
+            if (ev == NO_EVENT) {
+                if (brk != NO_EVENT) run = base + (brk >> 1);
+                if (run > save) { th = wh; to = wo; ts = s; save = at; }
+            }
+            brk = NO_EVENT;
+        };
+#pragma unroll 4
+        for (u32 k = 0; k < before; k++) turn(k);
+        if (RUN) keep(base + before);
+        else if (ev == NO_EVENT && base + before == next) {
+            if (next > WAR_TURN_CAP) {       // abandoned (never expected): the job fails
+                atomicAdd(&acc->status, 1ull);
+                ev = 2u * before - 1u; s = FROZEN;
+            } else { th = wh; to = wo; ts = s; next = 2u * next + W; }
         }
-        for (u32 k = 0; k < after; k++) turn();
-        const bool fin = done & active;
+#pragma unroll 4
+        for (u32 k = before; k < period; k++) turn(k);
+        if (RUN) keep(base + period);
+        rounds = base + (ev == NO_EVENT ? period : (ev >> 1) + 1u);
+        if (RUN && active && ev == NO_EVENT && rounds > RUN_CAP) ev = RUN_LOST;
+        const bool fin = ev != NO_EVENT, kcy = (ev & 1u) == 0u;
         if (__any_sync(WAR_FULL_MASK, fin)) {
             if (fin) {
-                if (kcy) {
+                if (RUN && kcy) {
+                    if (brk_cy != NO_EVENT) run = max(run, base + (brk_cy >> 1));
+                    const u32 lam = rounds - save;
+                    if (run > save) ev = RUN_LOST;     // a cycle with a break
+                    cyc += wt;
+                    if (a.hbins) atomicAdd(&shh[lam < hb1 ? lam : hb1], wt);
+                    // Brent's checkpoint that finds it: the first one at or after the run's first turn (turn 0 aside) with
+                    // lam turns to the next
+                    u32 c0 = W;
+                    while ((c0 < run && run > h) || lam > c0 + W) c0 = 2u * c0 + W;
+                    turns += (u64)wt * (c0 + lam);
+                    if (run == h && lam <= W) turns -= (u64)held_start<RULE>(*start, a.blocks, n, lam) * c0;
+                } else if (kcy) {
                     // next = W: found with the tortoise at turn h, else at turn (next - W) / 2
-                    const u32 save = next == W ? h : (next - W) >> 1, lam = rounds - save;
+                    const u32 at = next == W ? h : (next - W) >> 1, lam = rounds - at;
                     cyc += wt;
                     if (a.hbins) atomicAdd(&shh[lam < hb1 ? lam : hb1], wt);
                     const u32 t = next == W ? W + lam : rounds;
                     turns += (u64)wt * t;
-                    if (lam <= W && save <= W) turns -= (u64)held_start<RULE>(*start, a.blocks, n, lam) * (t - lam);
+                    if (lam <= W && at <= W) turns -= (u64)held_start<RULE>(*start, a.blocks, n, lam) * (t - lam);
                 } else {
                     maxfin = max(maxfin, rounds);
                     turns += (u64)wt * rounds;
                     atomicAdd(&she[rounds < WAR_EBINS - 1 ? rounds : WAR_EBINS - 1], wt);
                 }
+                if (RUN && ev == RUN_LOST) atomicAdd(&acc->undetermined, 1ull);
             }
             refill(fin);
             running = __any_sync(WAR_FULL_MASK, active);
@@ -589,13 +759,11 @@ __global__ void __launch_bounds__(1024) held_merge_kernel(const __grid_constant_
     }
 
     const u64 v_cyc = warp_sum((u64)cyc), v_turns = warp_sum(turns), v_max = warp_max((u64)maxfin);
-    const u64 v_cap = warp_sum((u64)capped);
     if (lane == 0u) {
         if (c.done) atomicAdd(&acc->done, c.done);
         if (v_cyc) atomicAdd(&acc->cyc, v_cyc);
         if (v_turns) atomicAdd(&acc->turns, v_turns);
         if (v_max) atomicMax(&acc->maxfin, v_max);
-        if (v_cap) atomicAdd(&acc->status, v_cap);
     }
     __syncthreads();
     flush_hist(shh, acc->hist, a.hbins);
@@ -606,15 +774,23 @@ static size_t held_merge_shmem(int threads, int hbins) {
     return sizeof(HeldStart) * (size_t)threads + sizeof(u32) * (size_t)(hbins + WAR_EBINS);
 }
 
-cudaError_t launch_held_merged(const MergeArgs& a, int rule, int threads, int blocks, DevAcc* acc, cudaStream_t st) {
-    (rule ? held_merge_kernel<1> : held_merge_kernel<0>)<<<blocks, threads, held_merge_shmem(threads, a.hbins), st>>>(a, acc);
+typedef void (*HeldMergeFn)(const MergeArgs, DevAcc*);
+
+// The run test holds for odd n and the winner's card first.
+static HeldMergeFn held_merge_pick(int n, int rule, bool run) {
+    if (rule) return held_merge_kernel<1, false>;
+    return run && (n & 1) ? held_merge_kernel<0, true> : held_merge_kernel<0, false>;
+}
+
+cudaError_t launch_held_merged(const MergeArgs& a, int rule, bool run, int threads, int blocks, DevAcc* acc, cudaStream_t st) {
+    held_merge_pick(a.n, rule, run)<<<blocks, threads, held_merge_shmem(threads, a.hbins), st>>>(a, acc);
     note_launch();
     return cudaGetLastError();
 }
 
-int held_merged_max_blocks_per_sm(int rule, int threads, int hbins) {
+int held_merged_max_blocks_per_sm(int n, int rule, bool run, int threads, int hbins) {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, rule ? held_merge_kernel<1> : held_merge_kernel<0>, threads,
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, held_merge_pick(n, rule, run), threads,
                                                       held_merge_shmem(threads, hbins)) != cudaSuccess)
         return 0;
     return nb;

@@ -58,6 +58,8 @@ struct MBlock {
     u8 k0, k1;        // canonical splits k0 <= k < k1
 };
 
+struct HeldK { u32 m1, m260, m252, k65, n4m8; };   // constants of the held-out engine's turn (war_held.cu)
+
 struct MergeArgs {
     const MBlock* blocks;
     const u32* table;     // MERGE_ROWS byte selectors of the rule (winner's or loser's card first)
@@ -67,6 +69,7 @@ struct MergeArgs {
     u64* memo;
     u32 memo_bits;
     TurnK tk;
+    HeldK held;
     // canonical scans
     u64 seed, thr;
     int dbins, blk, distinct, sample;
@@ -106,8 +109,8 @@ void canon_table(u32* rows);
 void canon_plan(const war_job* job, u64 warps, MergePlan& p);
 cudaError_t launch_canon(const MergeArgs& a, int rule, int extra, int threads, int blocks, DevAcc* acc, cudaStream_t st);
 int canon_max_blocks_per_sm(int rule, int shape, int extra, int threads, int hbins);
-cudaError_t launch_held_merged(const MergeArgs& a, int rule, int threads, int blocks, DevAcc* acc, cudaStream_t st);
-int held_merged_max_blocks_per_sm(int rule, int threads, int hbins);
+cudaError_t launch_held_merged(const MergeArgs& a, int rule, bool run, int threads, int blocks, DevAcc* acc, cudaStream_t st);
+int held_merged_max_blocks_per_sm(int n, int rule, bool run, int threads, int hbins);
 
 // Card of rank d among the set bits of m; m loses it.
 __host__ __device__ __forceinline__ u32 take_card(u32& m, u32 d) {
