@@ -100,8 +100,10 @@ __device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const Tu
 // A turn of the latched loops with its tests, in one block so that the predicates stay predicates.  Both pipes that
 // can do its work are half rate (ALU: logic, shifts, compares, selects; FMA: multiply-adds), so it is split between
 // them: what follows from "player 1 won" is written by a multiply-add for player 2's win and overwritten by one
-// under the predicate, moves under a predicate are multiplications by one, and the ALU is left the shifts, the
-// cards' masks and the compares: about 18 operations on each.
+// under the predicate, moves under a predicate are multiplications by one, a card is the word less 16 times the popped
+// word, and the ALU is left the shifts and the compares.  B200: with the cards masked and one move left as a move
+// 1.47, 12.4, 74.4 and 125.1 ms (2^28 deals of 13, 7!! 14!/2 of 14, 14! of 15 cards, 2e8 canonical of 14), so 1.45, 12.1,
+// 72.2 and 124.2.
 //
 //   pair        first card f + 16 (second card g) of the winner's two, + 0xFF: see war_turn_fma
 //   landmark    if one of the cards played is `top` (card n-1): the piles before the turn, and the turn
@@ -119,7 +121,7 @@ __device__ __forceinline__ void war_turn_tests(u64& w1, u64& w2, u32& qq, u64 t1
     const u32 l1 = (u32)w1, h1 = (u32)(w1 >> 32), l2 = (u32)w2, h2 = (u32)(w2 >> 32);
     const u32 nl1 = __funnelshift_r(l1, h1, 4), nl2 = __funnelshift_r(l2, h2, 4);
     const u32 nh1 = __umulhi(h1, K.k2p28), nh2 = __umulhi(h2, K.k2p28);
-    const u32 c1 = l1 & 15u, c2 = l2 & 15u;
+    const u32 c1 = l1 + nl1 * K.km16, c2 = l2 + nl2 * K.km16;
     const u32 f = RULE ? c1 : c2, g = RULE ? c2 : c1;   // player 2 won: f first in the pair; player 1: g
     u64 a1 = ((u64)nh1 << 32) | nl1, a2 = ((u64)nh2 << 32) | nl2;
     u32 ma = (u32)m1, mb = (u32)(m1 >> 32), mc = (u32)m2, md = (u32)(m2 >> 32);
@@ -130,7 +132,7 @@ __device__ __forceinline__ void war_turn_tests(u64& w1, u64& w2, u32& qq, u64 t1
         "setp.eq.u32 q, %9, %13;\n\t"
         "setp.eq.or.u32 q, %10, %13, q;\n\t"
         "setp.gt.u32 p, %9, %10;\n\t"
-        "@q mov.b32 %3, %14;\n\t"
+        "@q mad.lo.u32 %3, %14, %19, 0;\n\t"
         "@q mad.lo.u32 %4, %15, %19, 0;\n\t"
         "@q mad.lo.u32 %5, %16, %19, 0;\n\t"
         "@q mad.lo.u32 %6, %17, %19, 0;\n\t"

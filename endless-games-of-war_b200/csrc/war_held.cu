@@ -230,7 +230,10 @@ __device__ __forceinline__ bool h_turn_packed_fma(u64& wh, u64& wo, u32& s, u32 
 // under the winner's pile, its place, the holder's pop and the new count word are each written by a multiply-add for
 // the usual case and overwritten under "the holder won" and "card n-1 was on top"; a decided game notes 2 (turn in
 // the period) + (1 if it ended) in ev and is frozen by an odd count word far out of range (its low byte never is an
-// opponent's last card, the word no tortoise's, and card n-1 never on top).  HeldK: -1, -260, -252, 65 and 4n - 8 as
+// opponent's last card, the word no tortoise's, and card n-1 never on top).  The
+// cards are ol - 16 ol' (the popped word), and half of the holder's pop is a multiplication: the ALU pipe was 82%
+// busy, the FMA pipe 62% (masks and moves 50.7 ms for 2e8 deals of 17 cards, so 49.2, both halves of the pop 50.2).
+// HeldK: -1, -260, -252, 65 and 4n - 8 as
 // operands.
 template <int RULE>
 __device__ __forceinline__ void h_turn_tests(u64& wh, u64& wo, u32& s, u64 th, u64 to, u32 ts, u32& ev, u32 k2,
@@ -238,7 +241,7 @@ __device__ __forceinline__ void h_turn_tests(u64& wh, u64& wo, u32& s, u64 th, u
     const u32 ol = (u32)wo, oh = (u32)(wo >> 32), hl = (u32)wh, hh = (u32)(wh >> 32);
     const u32 nol = __funnelshift_r(ol, oh, 4), noh = __umulhi(oh, K.k2p28);
     const u32 nhl = __funnelshift_r(hl, hh, 4), nhh = __umulhi(hh, K.k2p28);
-    const u32 c = ol & 15u, h = hl & 15u;                     // the two top cards
+    const u32 c = ol + nol * K.km16, h = hl + nhl * K.km16;   // the two top cards
     const u32 f = RULE ? h : c, g = RULE ? c : h;             // the opponent won: f first in the pair; the holder: g
     const u32 q = s & 255u;
     u64 ao = ((u64)noh << 32) | nol;
@@ -255,7 +258,7 @@ __device__ __forceinline__ void h_turn_tests(u64& wh, u64& wo, u32& s, u64 th, u
         "mad.lo.u32 ps, %14, %15, %16;\n\t"           // 4 (n - 2 - lh)
         "@w mad.lo.u32 ps, %14, %13, -4;\n\t"
         "@z mad.lo.u32 ps, %14, %13, 0;\n\t"
-        "@!z mov.b32 %0, %17;\n\t"                    // the holder's pop, unless card n-1 was on top
+        "@!z mad.lo.u32 %0, %17, %13, 0;\n\t"         // the holder's pop, unless card n-1 was on top
         "@!z mov.b32 %1, %18;\n\t"
         "mad.lo.u32 s1, %3, %13, %19;\n\t"            // one card popped from each pile, card n-1 one place up
         "@w mad.lo.u32 s1, %3, %13, %20;\n\t"         // and the pair under the holder's
@@ -299,7 +302,7 @@ __device__ __forceinline__ void h_turn_tests_run(u64& wh, u64& wo, u32& s, u64 t
     const u32 ol = (u32)wo, oh = (u32)(wo >> 32), hl = (u32)wh, hh = (u32)(wh >> 32);
     const u32 nol = __funnelshift_r(ol, oh, 4), noh = __umulhi(oh, K.k2p28);
     const u32 nhl = __funnelshift_r(hl, hh, 4), nhh = __umulhi(hh, K.k2p28);
-    const u32 c = ol & 15u, h = hl & 15u;                     // the two top cards
+    const u32 c = ol + nol * K.km16, h = hl + nhl * K.km16;   // the two top cards
     const u32 f = RULE ? h : c, g = RULE ? c : h;             // the opponent won: f first in the pair; the holder: g
     const u32 q = s & 255u;
     u64 ao = ((u64)noh << 32) | nol;
@@ -320,7 +323,7 @@ __device__ __forceinline__ void h_turn_tests_run(u64& wh, u64& wo, u32& s, u64 t
         "mad.lo.u32 ps, %14, %15, %16;\n\t"           // 4 (n - 2 - lh)
         "@w mad.lo.u32 ps, %14, %13, -4;\n\t"
         "@z mad.lo.u32 ps, %14, %13, 0;\n\t"
-        "@!z mov.b32 %0, %17;\n\t"                    // the holder's pop, unless card n-1 was on top
+        "@!z mad.lo.u32 %0, %17, %13, 0;\n\t"         // the holder's pop, unless card n-1 was on top
         "@!z mov.b32 %1, %18;\n\t"
         "mad.lo.u32 s1, %3, %13, %19;\n\t"            // one card popped from each pile, card n-1 one place up
         "@w mad.lo.u32 s1, %3, %13, %20;\n\t"         // and the pair under the holder's
