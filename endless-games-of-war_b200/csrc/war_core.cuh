@@ -59,6 +59,7 @@ struct TurnK {
     u32 k2p28;  // 2^28
     u32 k4;     // 4
     u32 one;    // 1
+    u32 m1;     // -1; with it the struct is 32 bytes and the last three words stand where they measured best
     int c0;     // 2n - 4
     u32 end2;   // (2n)^2
 };
@@ -103,10 +104,12 @@ __device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const Tu
 // under the predicate, moves under a predicate are multiplications by one, a card is the word less 16 times the popped
 // word, and the ALU is left the shifts and the compares.  B200: with the cards masked and one move left as a move
 // 1.47, 12.4, 74.4 and 125.1 ms (2^28 deals of 13, 7!! 14!/2 of 14, 14! of 15 cards, 2e8 canonical of 14), so 1.45, 12.1,
-// 72.2 and 124.2.
+// 72.2 and 124.2; with MERGED 1.42, 11.9, 70.3, and 124.0 for the
+// canonical kernel's 123.6, which keeps the two compares.
 //
 //   pair        first card f + 16 (second card g) of the winner's two, + 0xFF: see war_turn_fma
-//   landmark    if one of the cards played is `top` (card n-1): the piles before the turn, and the turn
+//   landmark    if one of the cards played is `top` (card n-1): the piles before the turn, and the turn.  MERGED: told
+//               by the winner's card in the pair, which `top` always is: a multiply-add and a compare for two compares
 //   end, cycle  a pile is empty; both piles are the tortoise's (t1, t2): ev = 2 (turn in the period) + (1 if an end),
 //               and the game is frozen: its length word gets an odd value far out of range, so it never signals
 //               again (an odd length word is no end; the pushed pairs shift out, and with fewer than n cards the piles
@@ -115,7 +118,56 @@ __device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const Tu
 constexpr u32 NO_EVENT = 0xFFFFFFFFu;
 constexpr u32 FROZEN = 0x80000001u;
 
-template <int RULE, int U>
+// The piles before the turn and its number; the turn (MARK: q from the cards, MARK_PAIR: from the pair, TOP: `top` in
+// the form that q is compared with).
+#define WAR_LANDMARK \
+        "@q mad.lo.u32 %3, %14, %19, 0;\n\t" \
+        "@q mad.lo.u32 %4, %15, %19, 0;\n\t" \
+        "@q mad.lo.u32 %5, %16, %19, 0;\n\t" \
+        "@q mad.lo.u32 %6, %17, %19, 0;\n\t" \
+        "@q mad.lo.u32 %7, %22, %19, %23;\n\t"
+#define WAR_TURN_TESTS(MARK, MARK_PAIR, TOP) \
+    asm("{\n\t" \
+        ".reg .pred p, q, e, y;\n\t" \
+        ".reg .u32 t, s, ps, xl, xh, al, ah, bl, bh, sq;\n\t" \
+        ".reg .u64 x;\n\t" \
+        "setp.gt.u32 p, %9, %10;\n\t" \
+        MARK \
+        "mad.lo.u32 t, %12, %18, %11;\n\t"       /* f + 16 g */ \
+        "@p mad.lo.u32 t, %11, %18, %12;\n\t"    /* g + 16 f */ \
+        MARK_PAIR \
+        "selp.b32 s, 1, -1, p;\n\t" \
+        "mad.lo.u32 t, t, %19, 255;\n\t" \
+        "mad.lo.u32 ps, s, %2, %20;\n\t"         /* the winner's sentinel after the pop */ \
+        "mad.lo.u32 %2, s, %21, %2;\n\t" \
+        "cvt.u64.u32 x, t;\n\t" \
+        "shl.b64 x, x, ps;\n\t" \
+        "mov.b64 {xl, xh}, x;\n\t" \
+        "@p mad.wide.u32 %0, xl, %19, %0;\n\t" \
+        "@!p mad.wide.u32 %1, xl, %19, %1;\n\t" \
+        "mov.b64 {al, ah}, %0;\n\t" \
+        "@p mad.lo.u32 ah, xh, %19, ah;\n\t" \
+        "mov.b64 %0, {al, ah};\n\t" \
+        "mov.b64 {bl, bh}, %1;\n\t" \
+        "@!p mad.lo.u32 bh, xh, %19, bh;\n\t" \
+        "mov.b64 %1, {bl, bh};\n\t" \
+        "mul.lo.u32 sq, %2, %2;\n\t" \
+        "setp.eq.u32 e, sq, %24;\n\t" \
+        "setp.eq.u32 y, al, %25;\n\t" \
+        "setp.eq.and.u32 y, ah, %26, y;\n\t" \
+        "setp.eq.and.u32 y, bl, %27, y;\n\t" \
+        "setp.eq.and.u32 y, bh, %28, y;\n\t" \
+        "@e mad.lo.u32 %8, %22, %19, %29;\n\t" \
+        "@y mad.lo.u32 %8, %22, %19, %23;\n\t" \
+        "@e mad.lo.u32 %2, %30, %19, 0;\n\t" \
+        "@y mad.lo.u32 %2, %30, %19, 0;\n\t" \
+        "}" \
+        : "+l"(a1), "+l"(a2), "+r"(qq), "+r"(ma), "+r"(mb), "+r"(mc), "+r"(md), "+r"(at), "+r"(ev) \
+        : "r"(c1), "r"(c2), "r"(f), "r"(g), "r"(TOP), "r"(l1), "r"(h1), "r"(l2), "r"(h2), "r"(K.k16), "r"(K.one), \
+          "r"(K.c0), "r"(K.k4), "r"(k2), "n"(2 * U), "r"(K.end2), "r"((u32)t1), "r"((u32)(t1 >> 32)), "r"((u32)t2), \
+          "r"((u32)(t2 >> 32)), "n"(2 * U + 1), "r"(FROZEN), "r"(K.k2p28))
+
+template <int RULE, int U, bool MERGED>
 __device__ __forceinline__ void war_turn_tests(u64& w1, u64& w2, u32& qq, u64 t1, u64 t2, u64& m1, u64& m2, u32& at,
                                                u32& ev, u32 k2, u32 top, const TurnK& K) {
     const u32 l1 = (u32)w1, h1 = (u32)(w1 >> 32), l2 = (u32)w2, h2 = (u32)(w2 >> 32);
@@ -125,55 +177,19 @@ __device__ __forceinline__ void war_turn_tests(u64& w1, u64& w2, u32& qq, u64 t1
     const u32 f = RULE ? c1 : c2, g = RULE ? c2 : c1;   // player 2 won: f first in the pair; player 1: g
     u64 a1 = ((u64)nh1 << 32) | nl1, a2 = ((u64)nh2 << 32) | nl2;
     u32 ma = (u32)m1, mb = (u32)(m1 >> 32), mc = (u32)m2, md = (u32)(m2 >> 32);
-    asm("{\n\t"
-        ".reg .pred p, q, e, y;\n\t"
-        ".reg .u32 t, s, ps, xl, xh, al, ah, bl, bh, sq;\n\t"
-        ".reg .u64 x;\n\t"
-        "setp.eq.u32 q, %9, %13;\n\t"
-        "setp.eq.or.u32 q, %10, %13, q;\n\t"
-        "setp.gt.u32 p, %9, %10;\n\t"
-        "@q mad.lo.u32 %3, %14, %19, 0;\n\t"
-        "@q mad.lo.u32 %4, %15, %19, 0;\n\t"
-        "@q mad.lo.u32 %5, %16, %19, 0;\n\t"
-        "@q mad.lo.u32 %6, %17, %19, 0;\n\t"
-        "@q mad.lo.u32 %7, %22, %19, %23;\n\t"
-        "mad.lo.u32 t, %12, %18, %11;\n\t"       // f + 16 g
-        "@p mad.lo.u32 t, %11, %18, %12;\n\t"    // g + 16 f
-        "selp.b32 s, 1, -1, p;\n\t"
-        "mad.lo.u32 t, t, %19, 255;\n\t"
-        "mad.lo.u32 ps, s, %2, %20;\n\t"         // the winner's sentinel after the pop
-        "mad.lo.u32 %2, s, %21, %2;\n\t"
-        "cvt.u64.u32 x, t;\n\t"
-        "shl.b64 x, x, ps;\n\t"
-        "mov.b64 {xl, xh}, x;\n\t"
-        "@p mad.wide.u32 %0, xl, %19, %0;\n\t"
-        "@!p mad.wide.u32 %1, xl, %19, %1;\n\t"
-        "mov.b64 {al, ah}, %0;\n\t"
-        "@p mad.lo.u32 ah, xh, %19, ah;\n\t"
-        "mov.b64 %0, {al, ah};\n\t"
-        "mov.b64 {bl, bh}, %1;\n\t"
-        "@!p mad.lo.u32 bh, xh, %19, bh;\n\t"
-        "mov.b64 %1, {bl, bh};\n\t"
-        "mul.lo.u32 sq, %2, %2;\n\t"
-        "setp.eq.u32 e, sq, %24;\n\t"
-        "setp.eq.u32 y, al, %25;\n\t"
-        "setp.eq.and.u32 y, ah, %26, y;\n\t"
-        "setp.eq.and.u32 y, bl, %27, y;\n\t"
-        "setp.eq.and.u32 y, bh, %28, y;\n\t"
-        "@e mad.lo.u32 %8, %22, %19, %29;\n\t"
-        "@y mad.lo.u32 %8, %22, %19, %23;\n\t"
-        "@e mad.lo.u32 %2, %30, %19, 0;\n\t"
-        "@y mad.lo.u32 %2, %30, %19, 0;\n\t"
-        "}"
-        : "+l"(a1), "+l"(a2), "+r"(qq), "+r"(ma), "+r"(mb), "+r"(mc), "+r"(md), "+r"(at), "+r"(ev)
-        : "r"(c1), "r"(c2), "r"(f), "r"(g), "r"(top), "r"(l1), "r"(h1), "r"(l2), "r"(h2), "r"(K.k16), "r"(K.one),
-          "r"(K.c0), "r"(K.k4), "r"(k2), "n"(2 * U), "r"(K.end2), "r"((u32)t1), "r"((u32)(t1 >> 32)), "r"((u32)t2),
-          "r"((u32)(t2 >> 32)), "n"(2 * U + 1), "r"(FROZEN));
+    if (MERGED && RULE)        // the winner's card is the pair's high nibble
+        WAR_TURN_TESTS("", "setp.ge.u32 q, t, %13;\n\t" WAR_LANDMARK, top << 4);
+    else if (MERGED)           // its low nibble
+        WAR_TURN_TESTS("", "mul.lo.u32 s, t, %31;\n\t setp.ge.u32 q, s, %13;\n\t" WAR_LANDMARK, top << 28);
+    else
+        WAR_TURN_TESTS("setp.eq.u32 q, %9, %13;\n\t setp.eq.or.u32 q, %10, %13, q;\n\t" WAR_LANDMARK, "", top);
     m1 = ((u64)mb << 32) | ma;
     m2 = ((u64)md << 32) | mc;
     w1 = a1;
     w2 = a2;
 }
+#undef WAR_TURN_TESTS
+#undef WAR_LANDMARK
 
 // The same turn with the rule chosen at run time (serving kernel, checks).
 __device__ __forceinline__ bool war_turn_rt(u64& w1, u64& w2, u32& q, u32 k4m4, int rule) {

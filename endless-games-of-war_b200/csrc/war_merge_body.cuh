@@ -21,8 +21,9 @@
 // at services -> landmarks -> a found cycle recorded by playing on instead of by a walk -> this service and turn): a
 // span of 4.26e9 deals of 15 cards 210 -> 132 -> 85 -> 81 ms (stores 3.4e9 -> 1.0e9), 1e8 deals of 13 cards 2.5 -> 2.0
 // -> 1.6 -> 1.5 ms, a resumed a(13) 31.2 -> 30.5 -> 29.9 -> 28.8 ms, --half span of 14 cards 13.7 -> 12.9 ms, 3e9
-// canonical positions of 14 cards 152 -> 148 -> 148 -> 143 ms and 125 with the queue of starts.  The one-deal-one-game
-// kernel before: 370, 10.7, 168, 124 and 164 ms.
+// canonical positions of 14 cards 152 -> 148 -> 148 -> 143 ms and 125 with the queue of starts; with services every 16
+// turns from 15 cards and the later steps of the turn (war_turn_tests) 70.3, 1.42, 27.9, 11.9 and 123.6 ms.  The
+// one-deal-one-game kernel before: 370, 10.7, 168, 124 and 164 ms.
 #pragma once
 #include "war_refill.cuh"
 #include "war_merge.cuh"
@@ -179,10 +180,10 @@ __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restric
         u32 ev = NO_EVENT;
         g.at = NO_LANDMARK;
         for (u32 k2 = 0; k2 < 2u * period; k2 += 8u) {
-            war_turn_tests<RULE, 0>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, n - 1u, K);
-            war_turn_tests<RULE, 1>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, n - 1u, K);
-            war_turn_tests<RULE, 2>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, n - 1u, K);
-            war_turn_tests<RULE, 3>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, n - 1u, K);
+            war_turn_tests<RULE, 0, true>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, n - 1u, K);
+            war_turn_tests<RULE, 1, true>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, n - 1u, K);
+            war_turn_tests<RULE, 2, true>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, n - 1u, K);
+            war_turn_tests<RULE, 3, true>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, n - 1u, K);
         }
         // out: a decided game's outcome, 2 lam for a cycle, 2 len + 1 for an end
         const u32 base = g.rounds;
@@ -390,10 +391,10 @@ __device__ __forceinline__ void canon_body(const MergeArgs& a, DevAcc* __restric
         u32 ev = NO_EVENT;
         g.at = NO_LANDMARK;
         for (u32 k2 = 0; k2 < 2u * period; k2 += 8u) {
-            war_turn_tests<RULE, 0>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, m, K);
-            war_turn_tests<RULE, 1>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, m, K);
-            war_turn_tests<RULE, 2>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, m, K);
-            war_turn_tests<RULE, 3>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, m, K);
+            war_turn_tests<RULE, 0, false>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, m, K);
+            war_turn_tests<RULE, 1, false>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, m, K);
+            war_turn_tests<RULE, 2, false>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, m, K);
+            war_turn_tests<RULE, 3, false>(g.w1, g.w2, g.q, g.t1, g.t2, g.m1, g.m2, g.at, ev, k2, m, K);
         }
         // out: a decided game's outcome, the memo value of a cycle, 2 len + 1 for an end
         const u32 base = g.rounds;
