@@ -30,6 +30,7 @@
 #include <cmath>
 #include <chrono>
 #include <condition_variable>
+#include <cstdlib>
 #include <cstring>
 #include <deque>
 #include <map>
@@ -186,9 +187,11 @@ struct war_server {
     u64 arena_words = 0, arena_used = 0;
     u32* d_table = nullptr;         // pair lists and orders (war_merge.cuh)
     war::MBlock* d_blocks = nullptr;     // the resident merged jobs' blocks, SLOT_BLOCKS for each slot
-    war::MBlock* h_blocks = nullptr;     // and their pinned mirror
+    war::MBlock* h_blocks = nullptr;     // and their mirror: pageable, a slot's few KB are staged by the copy, where
+                                         // pinning the 4 MB of 256 slots takes longer than all the copies
     war::ServeJob* d_jobs = nullptr;   // the resident jobs' arguments, by slot
-    war::ServeJob* h_jobs = nullptr;   // and their pinned mirror
+    war::ServeJob* h_jobs = nullptr;   // and their mirror: pageable, a slot's few KB are staged by the copy, where
+                                         // pinning the 4 MB of 256 slots takes longer than all the copies
     DevAcc* d_slots = nullptr;
     DevAcc* h_slot = nullptr;   // pinned readback buffer, READBACK slots
     cudaStream_t s_comp = nullptr, s_copy = nullptr;
@@ -571,7 +574,7 @@ int war_server_create(const war_server_cfg* cfg, war_server** out) {
     const size_t nblocks = (size_t)s->nslots * SLOT_BLOCKS;
     bool ok = upload_merge_table(&s->d_table) == cudaSuccess &&
               cudaMalloc(&s->d_blocks, sizeof(MBlock) * nblocks) == cudaSuccess &&
-              cudaMallocHost(&s->h_blocks, sizeof(MBlock) * nblocks) == cudaSuccess &&
+              (s->h_blocks = (MBlock*)calloc(nblocks, sizeof(MBlock))) != nullptr &&
               cudaMalloc(&s->d_jobs, sizeof(ServeJob) * (size_t)s->nslots) == cudaSuccess &&
               cudaMallocHost(&s->h_jobs, sizeof(ServeJob) * (size_t)s->nslots) == cudaSuccess &&
               cudaMalloc(&s->d_slots, sizeof(DevAcc) * (size_t)s->nslots) == cudaSuccess &&
@@ -695,7 +698,7 @@ int war_server_destroy(war_server* s) {
     if (s->d_jobs) cudaFree(s->d_jobs);
     if (s->h_jobs) cudaFreeHost(s->h_jobs);
     if (s->d_blocks) cudaFree(s->d_blocks);
-    if (s->h_blocks) cudaFreeHost(s->h_blocks);
+    free(s->h_blocks);
     if (s->d_slots) cudaFree(s->d_slots);
     if (s->h_slot) cudaFreeHost(s->h_slot);
     if (s->s_comp) cudaStreamDestroy(s->s_comp);
