@@ -568,7 +568,8 @@ __global__ void __launch_bounds__(MEMO ? 512 : 1024) held_kernel(const __grid_co
 //
 // What bounds it: instruction issue of the turns; the gain over held_kernel is the deals per game and the turn with
 // its tests in one block (h_turn_tests).  A slice of 1e9 deals of 17 cards (4.9 deals per game on average) on a B200:
-// 356 ms -> 58.6 (merged, h_turn_packed_fma) -> 50.5 (h_turn_tests) -> 46.1 (RUN), with a period of 32 turns (16:
+// 356 ms -> 58.6 (merged, h_turn_packed_fma) -> 50.5 (h_turn_tests) -> 46.1 (RUN) -> 44.4 (cards and half a pop as
+// multiply-adds), with a period of 32 turns (16:
 // 49.4, 8: 57.8 ms).
 
 constexpr u32 RUN_CAP = 1u << 16, RUN_LOST = 0xFFFFFFFDu;   // (RUN_LOST: an odd event, recorded as an end)
