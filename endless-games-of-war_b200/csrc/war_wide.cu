@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(1024) wide_merge_kernel(const __grid_constant_
     for (int b = threadIdx.x; b < bins; b += blockDim.x) shh[b] = 0;
     __syncthreads();
 
-    const u32 n = (u32)a.n, n1 = n - 1u, h = n >> 1, W = (u32)a.W;
+    const u32 n = (u32)a.n, h = n >> 1, W = (u32)a.W;
     const u32 hb1 = a.hbins > 0 ? (u32)(a.hbins - 1) : 0u;
     const u32 period = a.defer > 4 ? (u32)((a.defer + 3) & ~3) : 4u;
     const u32 after = DET == DET_BRENT ? h % period : 0u, before = period - after;   // turns around the checkpoint
