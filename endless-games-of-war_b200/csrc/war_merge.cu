@@ -259,8 +259,10 @@ int canon_max_blocks_per_sm(int rule, int shape, int extra, int threads, int hbi
     const MergeFn fn = rule ? canon_pick<1>(shape, extra) : canon_pick<0>(shape, extra);
     const size_t shmem = canon_shmem(extra, threads, hbins);
     int nb = 0;
-    if (shmem > 32 * 1024 &&   // (with the static part it may pass the 48 KB that need no asking)
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem) != cudaSuccess) {
+    // large blocks with starts and queues pass the 48 KB that need no asking; the limit asked for is the same from every
+    // call, so that a thread cannot lower it under another one's launch
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)canon_shmem(extra, 1024, WAR_HBINS_MAX)) != cudaSuccess) {
         cudaGetLastError();
         return 0;
     }

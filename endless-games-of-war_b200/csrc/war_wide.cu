@@ -731,6 +731,14 @@ static int wide_max_blocks(int det, int rule, int threads, int hbins) {
 
 static int wide_merge_max_blocks(int det, int rule, int threads, int hbins) {
     int nb = 0;
+    // 1024 threads with more than about 2,500 bins pass the 48 KB that need no asking.  The limit asked for is the
+    // same from every call, so that a thread cannot lower it under another one's launch.
+    const size_t most = wide_merge_shmem(det, 1024, WAR_HBINS_MAX);
+    if (cudaFuncSetAttribute(wide_merge_pick(det, rule), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) !=
+        cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, wide_merge_pick(det, rule), threads,
                                                       wide_merge_shmem(det, threads, hbins)) != cudaSuccess)
         return 0;

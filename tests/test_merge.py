@@ -225,6 +225,18 @@ def test_wide_merged_ranges(wl, oracle, n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("det", [0, 1, 2])
+def test_wide_merged_largest_launch_shape(wl, det):
+    """Blocks of 1024 threads with the most histogram bins: more shared memory than a launch has unasked."""
+    lo = 10 ** 13
+    job = wl.make_job(17, lo=lo, hi=lo + 5041, hbins=wl.WAR_HBINS_MAX)
+    got = wl.to_dict(wl.enumerate_wide(job, det, threads=1024))
+    want = wl.to_dict(wl.enumerate_wide(job, det))
+    for k in WIDE_KEYS:
+        assert got[k] == want[k], (det, k)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("n", [4, 5, 6, 8, 11, 13, 16])
 def test_canonical_units(wl, n):
     """Canonical scans with the path memo at the edges of orders, blocks and units: one position, part of an order,
