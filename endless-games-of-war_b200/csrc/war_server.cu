@@ -190,8 +190,7 @@ struct war_server {
     war::MBlock* h_blocks = nullptr;     // and their mirror: pageable, a slot's few KB are staged by the copy, where
                                          // pinning the 4 MB of 256 slots takes longer than all the copies
     war::ServeJob* d_jobs = nullptr;   // the resident jobs' arguments, by slot
-    war::ServeJob* h_jobs = nullptr;   // and their mirror: pageable, a slot's few KB are staged by the copy, where
-                                         // pinning the 4 MB of 256 slots takes longer than all the copies
+    war::ServeJob* h_jobs = nullptr;   // and their mirror, pinned
     DevAcc* d_slots = nullptr;
     DevAcc* h_slot = nullptr;   // pinned readback buffer, READBACK slots
     cudaStream_t s_comp = nullptr, s_copy = nullptr;
