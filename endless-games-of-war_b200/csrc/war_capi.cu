@@ -492,13 +492,15 @@ int war_enumerate_plain(const war_job* job, war_result* out) {
 //
 // A job that can only fill part of the table (`want` words or fewer are useful, 0 = no such limit) uses and
 // clears the first 2^*used words of it: clearing 16 GiB takes 2.6 ms, clearing what a slice of 1e8 deals can
-// use takes less than a tenth.  A job that keeps the table uses as much of it as the job before did.
+// use takes less than a tenth.  A job that keeps the table uses as much of it as the job before did, unless that
+// is less than half of what it can use itself: what so small a table holds is worth less than the room, and it starts
+// from a clear one.
 static int prepare_memo(Ctx& c, const war_job* job, int bits, int kind, u64** table, u64 want = 0, int* used = nullptr) {
     cudaError_t e;
-    const bool keep = (job->flags & WAR_F_MEMO_KEEP) && c.memo_bits == bits && c.memo_n == job->n &&
-                      c.memo_rule == job->rule && c.memo_kind == kind;
     int ub = bits;
     while (want && ub > 12 && (1ull << (ub - 1)) >= want) ub--;
+    const bool keep = (job->flags & WAR_F_MEMO_KEEP) && c.memo_bits == bits && c.memo_n == job->n &&
+                      c.memo_rule == job->rule && c.memo_kind == kind && ub <= c.memo_used + 1;
     if (keep) ub = c.memo_used;
     const size_t bytes = sizeof(u64) << bits;
     if (c.memo_bits != bits) {

@@ -225,6 +225,20 @@ def test_wide_merged_ranges(wl, oracle, n):
 
 
 @pytest.mark.gpu
+def test_merged_table_kept_after_a_much_smaller_job(wl):
+    """WAR_F_MEMO_KEEP after a job of a few deals: the job takes the table that it would take by itself, so that it
+    looks its games up as often and finds as many (to a few in a thousand: lanes race for what to store)."""
+    t = memo_tune(wl, memo_bits=26)
+    lo, hi = 10 ** 9, 10 ** 9 + 3 * 10 ** 7
+    alone = wl.to_dict(wl.enumerate_job(wl.make_job(13, lo=lo, hi=hi, hbins=128), t))
+    wl.enumerate_job(wl.make_job(13, lo=0, hi=1000, hbins=128), t)
+    kept = wl.to_dict(wl.enumerate_job(wl.make_job(13, flags=wl.F_MEMO_KEEP, lo=lo, hi=hi, hbins=128), t))
+    for k in KEYS:
+        assert kept[k] == alone[k], k
+    assert kept["turns"] < 1.05 * alone["turns"]
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("det", [0, 1, 2])
 def test_wide_merged_largest_launch_shape(wl, det):
     """Blocks of 1024 threads with the most histogram bins: more shared memory than a launch has unasked."""
