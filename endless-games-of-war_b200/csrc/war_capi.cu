@@ -492,10 +492,11 @@ int war_enumerate_plain(const war_job* job, war_result* out) {
 //
 // A job that can only fill part of the table (`want` words or fewer are useful, 0 = no such limit) uses and
 // clears the first 2^*used words of it: clearing 16 GiB takes 2.6 ms, clearing what a slice of 1e8 deals can
-// use takes less than a tenth.  A job that keeps the table uses as much of it as the job before did, unless that
-// is less than half of what it can use itself: what so small a table holds is worth less than the room, and it starts
-// from a clear one.
-static int prepare_memo(Ctx& c, const war_job* job, int bits, int kind, u64** table, u64 want = 0, int* used = nullptr) {
+// use takes less than a tenth.  The kernel must read the table with *used, whatever the job asked for: entries are
+// packed for that many words, and the words past them were not cleared.  A job that keeps the table uses as much of
+// it as the job before did, unless that is less than half of what it can use itself: what so small a table holds is
+// worth less than the room, and it starts from a clear one.
+static int prepare_memo(Ctx& c, const war_job* job, int bits, int kind, u64 want, u64** table, u32* used) {
     cudaError_t e;
     int ub = bits;
     while (want && ub > 12 && (1ull << (ub - 1)) >= want) ub--;
@@ -521,7 +522,7 @@ static int prepare_memo(Ctx& c, const war_job* job, int bits, int kind, u64** ta
     c.memo_rule = job->rule;
     c.memo_kind = kind;
     c.memo_used = ub;
-    if (used) *used = ub;
+    *used = (u32)ub;
     *table = c.d_memo;
     return WAR_OK;
 }
@@ -538,7 +539,7 @@ static int enumerate_merged(const war_job* job, const Tune& t, war_result* out) 
     else merge_plan(job, warps, p);
     if (p.units == 0) return WAR_OK;   // (--half: no deal of the range gives card n-1 to player 1)
     MergeArgs a;
-    int st, used = 0;
+    int st;
     if ((st = merge_args(job, p, job->hbins, t.window, t.defer, a))) return st;
     // the table's layout (prepare_memo)
     const int kind = 4 * 3 + (canon && (job->flags & WAR_F_SHAPE) ? 2 : 0);
@@ -546,8 +547,7 @@ static int enumerate_merged(const war_job* job, const Tune& t, war_result* out) 
     // deals (6.8e8 games) take 18.0 ms with 2^29 words, 18.3 with 2^30, 19.3 with 2^31, its end from a saved progress
     // (1.2e9 games) 30.2 with 2^29 or 2^30 and 31.0 with 2^31; from 15 cards the many cycles fill what there is.
     const u64 want = canon ? 2 * p.games : job->n >= 15 ? 4 * p.games : p.games / 4 * 3 + 1;
-    if ((st = prepare_memo(c, job, t.memo_bits, kind, &a.memo, want, &used))) return st;
-    a.memo_bits = (u32)used;
+    if ((st = prepare_memo(c, job, t.memo_bits, kind, want, &a.memo, &a.memo_bits))) return st;
     if (!canon)
         return run_merged(p, a, MERGE_LAUNCH_UNITS, job->hbins, 0, out,
                           [&](cudaStream_t x) { return launch_merged(a, job->rule, t.threads, blocks, c.d_acc, x); });
@@ -638,8 +638,7 @@ int war_enumerate_held(const war_job* job, const war_tune* tune, war_result* out
     a.units = c.d_units;
     a.tk.k16 = 16u; a.tk.km16 = (u32)-16; a.tk.k2p28 = 1u << 28; a.tk.k4 = 4u; a.tk.one = 1u; a.tk.m1 = (u32)-1;
     if (memo) {
-        if ((st = prepare_memo(c, job, memo_bits, 1, &a.memo))) return st;
-        a.memo_bits = (u32)memo_bits;
+        if ((st = prepare_memo(c, job, memo_bits, 1, 0, &a.memo, &a.memo_bits))) return st;
     }
     // each launch plays fewer than 2^32 - 2^24 games (32-bit per-lane counters)
     const u64 per_unit = fact(block_m);
@@ -710,8 +709,7 @@ int war_enumerate(const war_job* job, const war_tune* tune, war_result* out) {
     a.chunk = (u32)t.chunk;
     if (t.variant & 4) {   // the cycle memo
         const int form = (t.variant & 24) == 24 ? 3 : ((t.variant & 8) ? 2 : 1);   // its entry layout
-        if ((st = prepare_memo(c, job, t.memo_bits, 4 * form, &a.memo))) return st;
-        a.memo_bits = (u32)t.memo_bits;
+        if ((st = prepare_memo(c, job, t.memo_bits, 4 * form, 0, &a.memo, &a.memo_bits))) return st;
     }
     // Each launch plays fewer than 2^32 games, so the 32-bit per-block and per-lane counters cannot wrap.
     const u64 per_unit = fact(t.block_m) * p.games_per_order;
