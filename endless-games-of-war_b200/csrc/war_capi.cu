@@ -487,7 +487,7 @@ int war_enumerate_plain(const war_job* job, war_result* out) {
 // previous job of the same n, rule and entry layout left.  kind names the layout: 1 the held-out engine;
 // for the main engine 4 * form + 2 * shape, with form 1 (landmarks, key | lam << shift), 2 (all cycle
 // states, same packing) or 3 (path entries, (key * C) << bits | value) and shape = 1 when cycle values
-// carry the loop-shape code.  Two layouts never share a table: an entry of one form read as another could
+// carry the loop-shape code, plus 16 * the block length that the code was found with.  Two layouts never share a table: an entry of one form read as another could
 // name a different state.
 //
 // A job that can only fill part of the table (`want` words or fewer are useful, 0 = no such limit) uses and
@@ -542,7 +542,7 @@ static int enumerate_merged(const war_job* job, const Tune& t, war_result* out) 
     int st;
     if ((st = merge_args(job, p, job->hbins, t.window, t.defer, a))) return st;
     // the table's layout (prepare_memo)
-    const int kind = 4 * 3 + (canon && (job->flags & WAR_F_SHAPE) ? 2 : 0);
+    const int kind = 4 * 3 + (canon && (job->flags & WAR_F_SHAPE) ? 2 + 16 * out->blk : 0);
     // Words worth clearing: a game stores at most two landmarks besides the cycles found, most store none.  All 13!
     // deals (6.8e8 games) take 18.0 ms with 2^29 words, 18.3 with 2^30, 19.3 with 2^31, its end from a saved progress
     // (1.2e9 games) 30.2 with 2^29 or 2^30 and 31.0 with 2^31; from 15 cards the many cycles fill what there is.

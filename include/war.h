@@ -53,9 +53,9 @@ enum war_flags {
     WAR_F_SAMPLE = 8,   /* accumulate the seeded sample aggregates used by the Floyd cross-check */
     WAR_F_MEMO_KEEP = 16 /* jobs with the cycle memo (war_tune.variant bit 2): start from the memo left by the
                             previous war_enumerate of the same n and rule instead of an empty one (its entries
-                            are facts about n and the rule, not about the range; one of less than half
-                            the words that a merged job can use is started anew); no other effect (no
-                            reference counterpart) */
+                            are facts about n and the rule, with WAR_F_SHAPE also about blk, not about the
+                            range; one of less than half the words that a job can use is started anew); no
+                            other effect (no reference counterpart) */
 };
 
 /* One enumeration job: the ranks [lo, hi) of one space.

@@ -45,3 +45,12 @@ def test_sampled_deals_after_a_job_that_used_half_of_the_table(wl, n, canon):
     check(wl, bits, n, flags=wl.F_SAMPLE | wl.F_MEMO_KEEP)
     check(wl, bits, n, flags=wl.F_MEMO_KEEP)
     check(wl, bits, n, mode=1, flags=wl.F_MEMO_KEEP)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [9, 11])
+def test_shape_scans_of_different_block_lengths(wl, n):
+    """The loop-shape codes in a table are those of one block length: a job with another one does not read them."""
+    bits = words(2 * math.factorial(n - 1) * (n - 1))
+    for i, blk in enumerate((2, 1, 1, 4, 0)):
+        check(wl, bits, n, mode=1, flags=wl.F_SHAPE | (wl.F_MEMO_KEEP if i else 0), blk=blk)
