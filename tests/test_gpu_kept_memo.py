@@ -10,7 +10,7 @@ KEYS = ("cyc", "done", "maxfin", "hist", "endhist", "s_count", "s_cyc", "s_lamsu
 
 
 def tune(wl, canon, memo_bits):
-    return wl.make_tune(variant=31, games=1, threads=256, defer=8, window=128 if canon else 32, memo_bits=memo_bits)
+    return wl.make_tune(variant=31, games=1, threads=256, defer=4, window=128 if canon else 32, memo_bits=memo_bits)
 
 
 def check(wl, memo_bits, n, mode=0, rule=0, flags=0, **kw):
@@ -31,9 +31,10 @@ def words(useful):
 @pytest.mark.parametrize("n", [9, 11])
 @pytest.mark.parametrize("canon", [False, True])
 def test_sampled_deals_after_a_job_that_used_half_of_the_table(wl, n, canon):
-    """A sampled job of the other rule fills the whole table; a merged (or canonical) job clears and uses half of
-    it; a sampled job keeps that; a merged job keeps what the sampled one left.  (Sampled deals are played one by
-    one, by another kernel than the merged ones, in the same table.)"""
+    """Jobs of the other rule fill the whole table, canonical positions among them: their starts are states that
+    games of both rules can reach (after a turn the pair under the winner's pile tells the rules apart).  A merged
+    (or canonical) job clears and uses half of the table, a sampled job keeps that, a merged and a canonical one
+    what the sampled one left.  (Sampled deals are played by another kernel than the others, in the same table.)"""
     if canon:
         games = 2 * math.factorial(n - 1) * (n - 1)
     else:
@@ -41,6 +42,7 @@ def test_sampled_deals_after_a_job_that_used_half_of_the_table(wl, n, canon):
         games = math.factorial(n) // 2 ** f * (f + 1) // 4 * 3 + 1
     bits = words(games) + 1
     check(wl, bits, n, rule=1, flags=wl.F_SAMPLE)
+    check(wl, bits, n, mode=1, rule=1, flags=wl.F_MEMO_KEEP)
     check(wl, bits, n, mode=1 if canon else 0)
     check(wl, bits, n, flags=wl.F_SAMPLE | wl.F_MEMO_KEEP)
     check(wl, bits, n, flags=wl.F_MEMO_KEEP)
