@@ -636,7 +636,7 @@ int war_enumerate_held(const war_job* job, const war_tune* tune, war_result* out
     for (int i = 0; i <= 17; i++) a.fact[i] = fact(i);
     a.n = job->n; a.m = block_m; a.rule = job->rule; a.hbins = job->hbins;
     a.units = c.d_units;
-    a.tk.k16 = 16u; a.tk.km16 = (u32)-16; a.tk.k2p28 = 1u << 28; a.tk.k4 = 4u; a.tk.one = 1u; a.tk.m1 = (u32)-1;
+    set_turn(a.tk, job->n);
     if (memo) {
         if ((st = prepare_memo(c, job, memo_bits, 1, 0, &a.memo, &a.memo_bits))) return st;
     }
@@ -698,8 +698,7 @@ int war_enumerate(const war_job* job, const war_tune* tune, war_result* out) {
     fill_fact(a.fact);
     a.n = job->n; a.m = t.block_m; a.hbins = job->hbins; a.dbins = job->dbins;
     a.blk = out->blk; a.W = t.window; a.defer = t.defer;
-    a.tk.k16 = 16u; a.tk.km16 = (u32)-16; a.tk.k2p28 = 1u << 28; a.tk.k4 = 4u; a.tk.one = 1u; a.tk.m1 = (u32)-1;
-    a.tk.c0 = 2 * job->n - 4; a.tk.end2 = (u32)(4 * job->n * job->n);
+    set_turn(a.tk, job->n);
     a.half = (job->flags & WAR_F_HALF) ? 1 : 0;
     a.sample = (job->flags & WAR_F_SAMPLE) ? 1 : 0;
     a.distinct = (job->flags & WAR_F_DISTINCT) && job->mode == WAR_CANON ? 1 : 0;

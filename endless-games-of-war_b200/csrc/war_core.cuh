@@ -59,10 +59,24 @@ struct TurnK {
     u32 k2p28;  // 2^28
     u32 k4;     // 4
     u32 one;    // 1
-    u32 m1;     // -1; with it the struct is 32 bytes and the last three words stand where they measured best
     int c0;     // 2n - 4
     u32 end2;   // (2n)^2
 };
+
+// The same for the turns with tests (war_turn_tests, h_turn_tests).  Another layout, with the last two words from a
+// 16-byte boundary on: the merged kernels measured best with it (71.2 ms for 14! ranks), and the one-game-per-deal
+// kernels with the one above (3e4 deals of 13 cards without a memo 7.5 ms, with this one 8.5).
+struct TestK {
+    u32 k16, km16, k2p28, k4, one, pad;
+    int c0;
+    u32 end2;
+};
+
+template <class Constants>
+inline void set_turn(Constants& k, int n) {
+    k.k16 = 16u; k.km16 = (u32)-16; k.k2p28 = 1u << 28; k.k4 = 4u; k.one = 1u;
+    k.c0 = 2 * n - 4; k.end2 = (u32)(4 * n * n);
+}
 
 // The same turn as war_turn, written so that about half of its integer operations are multiply-adds
 // (the FMA pipe) rather than logic / shift operations (the ALU pipe, half rate on sm_100):
@@ -73,8 +87,8 @@ struct TurnK {
 //          by mad.wide, so no select or mask is needed
 //   length: qq = 4*len1 - 2n, pos = s*qq + (2n-4) and qq += 4s with s = +1 (player 1 won) or -1;
 //          the game is over when qq*qq == (2n)^2.
-template <int RULE>
-__device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const TurnK& K) {
+template <int RULE, class Constants>
+__device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const Constants& K) {
     const u32 l1 = (u32)w1, h1 = (u32)(w1 >> 32), l2 = (u32)w2, h2 = (u32)(w2 >> 32);
     const u32 nl1 = __funnelshift_r(l1, h1, 4), nl2 = __funnelshift_r(l2, h2, 4);
     const u32 nh1 = __umulhi(h1, K.k2p28), nh2 = __umulhi(h2, K.k2p28);
@@ -169,7 +183,7 @@ constexpr u32 FROZEN = 0x80000001u;
 
 template <int RULE, int U, bool MERGED>
 __device__ __forceinline__ void war_turn_tests(u64& w1, u64& w2, u32& qq, u64 t1, u64 t2, u64& m1, u64& m2, u32& at,
-                                               u32& ev, u32 k2, u32 top, const TurnK& K) {
+                                               u32& ev, u32 k2, u32 top, const TestK& K) {
     const u32 l1 = (u32)w1, h1 = (u32)(w1 >> 32), l2 = (u32)w2, h2 = (u32)(w2 >> 32);
     const u32 nl1 = __funnelshift_r(l1, h1, 4), nl2 = __funnelshift_r(l2, h2, 4);
     const u32 nh1 = __umulhi(h1, K.k2p28), nh2 = __umulhi(h2, K.k2p28);

@@ -237,7 +237,7 @@ __device__ __forceinline__ bool h_turn_packed_fma(u64& wh, u64& wo, u32& s, u32 
 // operands.
 template <int RULE>
 __device__ __forceinline__ void h_turn_tests(u64& wh, u64& wo, u32& s, u64 th, u64 to, u32 ts, u32& ev, u32 k2,
-                                   u32& prev, u32& brk, u32& brk_cy, const TurnK& K, const HeldK& H) {
+                                   u32& prev, u32& brk, u32& brk_cy, const TestK& K, const HeldK& H) {
     const u32 ol = (u32)wo, oh = (u32)(wo >> 32), hl = (u32)wh, hh = (u32)(wh >> 32);
     const u32 nol = __funnelshift_r(ol, oh, 4), noh = __umulhi(oh, K.k2p28);
     const u32 nhl = __funnelshift_r(hl, hh, 4), nhh = __umulhi(hh, K.k2p28);
@@ -298,7 +298,7 @@ __device__ __forceinline__ void h_turn_tests(u64& wh, u64& wo, u32& s, u64 th, u
 // cycle), for the run test of the merged loop.
 template <int RULE>
 __device__ __forceinline__ void h_turn_tests_run(u64& wh, u64& wo, u32& s, u64 th, u64 to, u32 ts, u32& ev, u32 k2,
-                                   u32& prev, u32& brk, u32& brk_cy, const TurnK& K, const HeldK& H) {
+                                   u32& prev, u32& brk, u32& brk_cy, const TestK& K, const HeldK& H) {
     const u32 ol = (u32)wo, oh = (u32)(wo >> 32), hl = (u32)wh, hh = (u32)(wh >> 32);
     const u32 nol = __funnelshift_r(ol, oh, 4), noh = __umulhi(oh, K.k2p28);
     const u32 nhl = __funnelshift_r(hl, hh, 4), nhh = __umulhi(hh, K.k2p28);
@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(1024) held_merge_kernel(const __grid_constant_
     __syncthreads();
 
     const u32 n = (u32)a.n, h = n >> 1, W = (u32)a.W;
-    const TurnK K = a.tk;
+    const TestK K = a.tk;
     const HeldK H = a.held;
     const u32 hb1 = a.hbins > 0 ? (u32)(a.hbins - 1) : 0u;
     const u32 period = a.defer > 4 ? (u32)((a.defer + 3) & ~3) : 4u;

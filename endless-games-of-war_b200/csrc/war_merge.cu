@@ -211,8 +211,7 @@ int merge_args(const war_job* job, const MergePlan& p, int hbins, int window, in
     a.nblocks = (u32)p.blocks.size() - 1u;
     a.lc = p.lc;
     a.n = job->n; a.hbins = hbins; a.W = window; a.defer = defer;
-    a.tk.k16 = 16u; a.tk.km16 = (u32)-16; a.tk.k2p28 = 1u << 28; a.tk.k4 = 4u; a.tk.one = 1u; a.tk.m1 = (u32)-1;
-    a.tk.c0 = 2 * job->n - 4; a.tk.end2 = (u32)(4 * job->n * job->n);
+    set_turn(a.tk, job->n);
     a.held.m1 = (u32)-1; a.held.m260 = (u32)-260; a.held.m252 = (u32)-252; a.held.k65 = 65u;
     a.held.n4m8 = 4u * (u32)job->n - 8u;
     return WAR_OK;

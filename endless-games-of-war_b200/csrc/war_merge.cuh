@@ -68,7 +68,7 @@ struct MergeArgs {
     int n, hbins, W, defer;
     u64* memo;
     u32 memo_bits;
-    TurnK tk;
+    TestK tk;
     HeldK held;
     // canonical scans
     u64 seed, thr;

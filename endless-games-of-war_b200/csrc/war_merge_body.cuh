@@ -102,7 +102,7 @@ __device__ __forceinline__ void merge_body(const MergeArgs& a, DevAcc* __restric
     __syncthreads();
 
     const u32 n = (u32)a.n, h = n >> 1, W = (u32)a.W, n2 = 2u * n;
-    const TurnK K = a.tk;
+    const TestK K = a.tk;
     const u32 hb1 = hbins ? hbins - 1u : 0u;
     const u32 period = a.defer > 4 ? (u32)((a.defer + 3) & ~3) : 4u;
     const MemoTable memo(a.memo, a.memo_bits, n);
@@ -301,7 +301,7 @@ __device__ __forceinline__ void canon_body(const MergeArgs& a, DevAcc* __restric
     __syncthreads();
 
     const u32 n = (u32)a.n, m = n - 1u, k4m4 = 4u * m, W = (u32)a.W, n2 = 2u * n;
-    const TurnK K = a.tk;
+    const TestK K = a.tk;
     const u32 hb1 = hbins ? hbins - 1u : 0u;
     const u32 period = a.defer > 4 ? (u32)((a.defer + 3) & ~3) : 4u;
     const MemoTable memo(a.memo, a.memo_bits, n);

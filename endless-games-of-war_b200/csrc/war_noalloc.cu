@@ -183,8 +183,7 @@ extern "C" int war_enumerate_noalloc(const war_job* job, const war_tune* tune, w
     fill_fact(a.fact);
     a.n = job->n; a.m = block_m; a.hbins = job->hbins; a.dbins = job->dbins;
     a.blk = out->blk; a.W = window; a.defer = defer;
-    a.tk.k16 = 16u; a.tk.km16 = (u32)-16; a.tk.k2p28 = 1u << 28; a.tk.k4 = 4u; a.tk.one = 1u; a.tk.m1 = (u32)-1;
-    a.tk.c0 = 2 * job->n - 4; a.tk.end2 = (u32)(4 * job->n * job->n);
+    set_turn(a.tk, job->n);
     a.half = (job->flags & WAR_F_HALF) ? 1 : 0;
     a.sample = (job->flags & WAR_F_SAMPLE) ? 1 : 0;
     a.distinct = (job->flags & WAR_F_DISTINCT) && canon ? 1 : 0;

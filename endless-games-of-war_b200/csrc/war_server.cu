@@ -227,8 +227,7 @@ void set_args(war_server* s, SJob& J) {
     a.blk = (job.flags & WAR_F_SHAPE) && canon ? (job.blk ? job.blk : (job.n & -job.n)) : 0;
     a.W = canon ? 128 : 32;
     a.defer = canon ? (job.n < 13 ? 16 : 12) : job.n < 14 ? 8 : job.n == 14 ? 12 : 16;   // (autotune.py's defaults)
-    a.tk.k16 = 16u; a.tk.km16 = (u32)-16; a.tk.k2p28 = 1u << 28; a.tk.k4 = 4u; a.tk.one = 1u; a.tk.m1 = (u32)-1;
-    a.tk.c0 = 2 * job.n - 4; a.tk.end2 = (u32)(4 * job.n * job.n);
+    set_turn(a.tk, job.n);
     a.half = (job.flags & WAR_F_HALF) ? 1 : 0;
     a.sample = (job.flags & WAR_F_SAMPLE) ? 1 : 0;
     a.distinct = (job.flags & WAR_F_DISTINCT) && canon ? 1 : 0;
@@ -292,7 +291,7 @@ void set_args(war_server* s, SJob& J) {
     m.nblocks = (u32)J.mplan.blocks.size() - 1u;
     m.lc = J.mplan.lc;
     m.n = a.n; m.hbins = a.hbins; m.W = a.W; m.defer = a.defer;
-    m.memo = a.memo; m.memo_bits = a.memo_bits; m.tk = a.tk;
+    m.memo = a.memo; m.memo_bits = a.memo_bits; set_turn(m.tk, job.n);
     m.seed = a.seed; m.thr = a.thr;
     m.dbins = a.dbins; m.distinct = a.distinct; m.sample = a.sample;
 }
