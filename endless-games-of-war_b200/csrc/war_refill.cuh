@@ -591,8 +591,10 @@ __device__ __forceinline__ void refill_latched(const BatchArgs& a, DevAcc* __res
             for (int i = 0; i < G; i++) {
                 LGame<EXTRA, MEMO>& x = g[i];
                 if (MEMO >= MEMO_ALL) {
+                    // (the key under the test: the sampled kernel spills 32 bytes with it, 40 without, and 1e8 sampled
+                    // deals of 13 cards take 10.8 ms instead of 13.8)
                     look[i] = !x.done;
-                    key[i] = memo_key_state(x.w1, x.w2, n);
+                    key[i] = look[i] ? memo_key_state(x.w1, x.w2, n) : 0ull;
                 } else {
                     look[i] = !x.done & (x.m1 != 0ull);
                     const bool h1 = ((u32)x.m1 & 15u) == nm1;
