@@ -207,8 +207,10 @@ struct war_server {
 namespace war {
 namespace {
 
-// Ranks per task: as many as give each SM 16 blocks of the tick's work, so that a small tick spreads over the GPU
-// (2^13: the block's own start and end stay small beside its games).
+// Ranks per task of a merged job: as many as give each SM 16 blocks of the tick's work, so that a small tick spreads
+// over the GPU (2^13: the block's own start and end stay small beside its games).  Tasks of the other jobs have the
+// most: there a lane, not a warp, plays a unit (720 deals), and a smaller task leaves more of a block's lanes without
+// one (1e8 sampled deals of 13 cards 6.8 ms, with tasks by the tick's work 11.2).
 constexpr u64 TASK_RANKS_MIN = 1ull << 13, TASK_RANKS_MAX = 1ull << 16;
 constexpr size_t READBACK = 32;          // finished jobs read back at a time
 constexpr size_t SLOT_BLOCKS = 256;      // blocks of a job of at most 16 cards: at most 2 (1 + .. + 15), and the sentinel
@@ -398,7 +400,8 @@ void build_tick(war_server* s, Tick& T) {
             t.slot = (u32)J.slot;
             t.kind = J.kind;
             if (J.next_main < main_units(J)) {
-                const u64 k = std::min(std::max<u64>(1, task_ranks / J.per_unit), main_units(J) - J.next_main);
+                const u64 ranks = J.var.merged ? task_ranks : TASK_RANKS_MAX;
+                const u64 k = std::min(std::max<u64>(1, ranks / J.per_unit), main_units(J) - J.next_main);
                 t.lo = (J.var.merged ? 0 : J.plan.main_base) + J.next_main;
                 t.hi = t.lo + k;
                 J.next_main += k;
