@@ -601,7 +601,6 @@ int war_enumerate_held(const war_job* job, const war_tune* tune, war_result* out
     a.W = W; a.defer = defer; a.form = form; a.svc_off = (tune && (tune->variant & 8)) ? 1 : 0;
     // The default turn plays merged games; that needs the checkpoints after turn 0 to be after the merged turns.
     const bool merged = !memo && form == 3 && held_svc(a) && W >= job->n / 2;
-    if (!merged && !memo && form == 3) a.svc_off = 1;
     const int maxb = merged ? held_merged_max_blocks_per_sm(job->n, job->rule, true, threads, job->hbins)
                             : held_max_blocks_per_sm(job->rule, threads, job->hbins, memo, form, held_svc(a));
     if (maxb < 1) return fail(WAR_EINVAL, "launch shape threads=%d does not fit an SM%s", threads,

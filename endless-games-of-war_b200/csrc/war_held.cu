@@ -804,11 +804,7 @@ typedef void (*HeldFn)(const HeldArgs, DevAcc*);
 
 template <int RULE, bool MEMO>
 static HeldFn held_pick_form(int form, bool svc) {
-    if constexpr (MEMO) {
-        if (form == 3) return svc ? held_kernel<RULE, MEMO, 3, true> : held_kernel<RULE, MEMO, 3, false>;
-    } else {   // with the checkpoint at the services and no memo the default turn plays merged games
-        if (form == 3) return held_kernel<RULE, MEMO, 3, false>;
-    }
+    if (form == 3) return svc ? held_kernel<RULE, MEMO, 3, true> : held_kernel<RULE, MEMO, 3, false>;
     if (form == 2) return svc ? held_kernel<RULE, MEMO, 2, true> : held_kernel<RULE, MEMO, 2, false>;
     if (form == 1) return svc ? held_kernel<RULE, MEMO, 1, true> : held_kernel<RULE, MEMO, 1, false>;
     return svc ? held_kernel<RULE, MEMO, 0, true> : held_kernel<RULE, MEMO, 0, false>;
