@@ -32,7 +32,8 @@ import warlib  # noqa: E402
 # played together in blocks of as many orders, the larger the fewer games (csrc/war_merge.cuh): all 13! deals in
 # one call 20 ms, in two calls split at 2^32 - 2^25 30 ms.
 SPAN_RANKS = 87178291200
-# The same for canonical positions and for the plain kernel (--plain): just under 2^32, one launch.
+# The same where the engine plays every game: canonical positions, the plain kernel (--plain), tunes without the path
+# memo.  Just under 2^32, one launch, a second or so at 14 and 15 cards, where 14! deals one by one take 10 to 20 s.
 CALL_RANKS = (1 << 32) - (1 << 25)
 
 
@@ -99,7 +100,8 @@ def run(n, half=False, per=256, threads=256, batch_threads=1 << 18, out=None, re
     mult_pos = (n - 1) if canon else 1                    # engine ranks per order
     if tune is None and not plain:
         tune = _tune_for(n, canon, rule, flags)
-    span = max(batch_threads * per, min(SPAN_RANKS, CALL_RANKS) // max(1, mult_pos) if canon or plain else SPAN_RANKS)
+    merged = not canon and not plain and tune is not None and tune.variant & 30 == 30 and n <= 16
+    span = max(batch_threads * per, SPAN_RANKS if merged else min(SPAN_RANKS, CALL_RANKS) // max(1, mult_pos))
     t0 = time.time()
     last_write = 0.0
     slowest = 0.0
