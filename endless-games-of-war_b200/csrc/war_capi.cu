@@ -85,7 +85,7 @@ int ensure_ready() {
     if ((e = cudaMalloc(&c.d_acc, sizeof(DevAcc))) != cudaSuccess) return cuda_fail(e, "cudaMalloc acc");
     if ((e = cudaMalloc(&c.d_units, sizeof(Unit) * Ctx::UNIT_CAP)) != cudaSuccess) return cuda_fail(e, "cudaMalloc units");
     if ((e = cudaMalloc(&c.d_blocks, sizeof(MBlock) * MERGE_BLOCK_CAP)) != cudaSuccess) return cuda_fail(e, "cudaMalloc blocks");
-    if ((e = upload_merge_table(&c.d_table)) != cudaSuccess) return cuda_fail(e, "pair lists");
+    if ((e = upload_merge_table(&c.d_table, c.own_stream)) != cudaSuccess) return cuda_fail(e, "pair lists");
     if ((e = cudaMallocHost(&c.h_acc, sizeof(DevAcc))) != cudaSuccess) return cuda_fail(e, "cudaMallocHost");
     if ((e = cudaEventCreate(&c.ev0)) != cudaSuccess) return cuda_fail(e, "event");
     if ((e = cudaEventCreate(&c.ev1)) != cudaSuccess) return cuda_fail(e, "event");
@@ -93,13 +93,22 @@ int ensure_ready() {
     return WAR_OK;
 }
 
-cudaError_t upload_merge_table(u32** table) {
+cudaError_t upload_merge_table(u32** table, cudaStream_t st) {
     std::vector<u32> rows(2 * MERGE_ROWS + CANON_ROWS);
     merge_table(0, rows.data());
     merge_table(1, rows.data() + MERGE_ROWS);
     canon_table(rows.data() + 2 * MERGE_ROWS);
     cudaError_t e = cudaMalloc(table, sizeof(u32) * rows.size());
-    if (e == cudaSuccess) e = cudaMemcpy(*table, rows.data(), sizeof(u32) * rows.size(), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) {
+        *table = nullptr;
+        return e;
+    }
+    e = cudaMemcpyAsync(*table, rows.data(), sizeof(u32) * rows.size(), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {
+        cudaFree(*table);
+        *table = nullptr;
+    }
     return e;
 }
 

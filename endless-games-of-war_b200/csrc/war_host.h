@@ -44,7 +44,9 @@ struct Tune {
 Ctx& ctx();
 int ensure_ready();
 cudaStream_t cur_stream();
-cudaError_t upload_merge_table(u32** table);   // pair lists of both rules, then orders
+// Allocates and fills the pair lists of both rules, then orders; they are there for every stream when it returns (the
+// streams here are non-blocking and wait for no other one).  On an error there is no table.
+cudaError_t upload_merge_table(u32** table, cudaStream_t st);
 int fail(int code, const char* fmt, ...);
 int cuda_fail(cudaError_t e, const char* what);
 u64 fact(int i);

@@ -573,14 +573,14 @@ int war_server_create(const war_server_cfg* cfg, war_server** out) {
     s->max_tasks = 16384;
     s->max_units = s->max_tasks + 4 * UNITS_PER_EXTRA_CAP;
     const size_t nblocks = (size_t)s->nslots * SLOT_BLOCKS;
-    bool ok = upload_merge_table(&s->d_table) == cudaSuccess &&
+    bool ok = cudaStreamCreateWithFlags(&s->s_comp, cudaStreamNonBlocking) == cudaSuccess &&
+              upload_merge_table(&s->d_table, s->s_comp) == cudaSuccess &&
               cudaMalloc(&s->d_blocks, sizeof(MBlock) * nblocks) == cudaSuccess &&
               (s->h_blocks = (MBlock*)calloc(nblocks, sizeof(MBlock))) != nullptr &&
               cudaMalloc(&s->d_jobs, sizeof(ServeJob) * (size_t)s->nslots) == cudaSuccess &&
               cudaMallocHost(&s->h_jobs, sizeof(ServeJob) * (size_t)s->nslots) == cudaSuccess &&
               cudaMalloc(&s->d_slots, sizeof(DevAcc) * (size_t)s->nslots) == cudaSuccess &&
               cudaMallocHost(&s->h_slot, sizeof(DevAcc) * READBACK) == cudaSuccess &&
-              cudaStreamCreateWithFlags(&s->s_comp, cudaStreamNonBlocking) == cudaSuccess &&
               cudaStreamCreateWithFlags(&s->s_copy, cudaStreamNonBlocking) == cudaSuccess;
     for (int i = 0; ok && i < 2; i++) {
         Tick& T = s->ticks[i];
