@@ -71,8 +71,11 @@ Ctx& ctx() {
     return c;
 }
 
+// What the context holds on the device; several threads may come here first, the context is made by one of them.
 int ensure_ready() {
     Ctx& c = ctx();
+    static std::mutex first;
+    std::lock_guard<std::mutex> lk(first);
     if (c.ready) return WAR_OK;
     int ndev = 0;
     cudaError_t e = cudaGetDeviceCount(&ndev);

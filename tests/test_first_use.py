@@ -38,3 +38,12 @@ def test_server_tables_are_on_the_device_before_the_first_launch(play):
     assert play("h = ctypes.c_void_p()\n"
                 "print(war.war_server_create(None, ctypes.byref(h)), fake.fake_unsynced())\n"
                 "war.war_server_destroy(h)\n") == [0, 0]
+
+
+def test_first_use_by_several_threads(play):
+    """The context is made once: a thread that came second would replace its buffers under the first one's job."""
+    one = play("print(war.war_set_stream(None), fake.fake_streams_made(), fake.fake_live())")
+    two = play("t = [threading.Thread(target=war.war_set_stream, args=(None,)) for _ in range(4)]\n"
+               "[x.start() for x in t]\n[x.join() for x in t]\n"
+               "print(war.war_set_stream(None), fake.fake_streams_made(), fake.fake_live())")
+    assert one[:2] == [0, 1] and two == one
