@@ -71,12 +71,8 @@ Ctx& ctx() {
     return c;
 }
 
-// What the context holds on the device; several threads may come here first, the context is made by one of them.
-int ensure_ready() {
-    Ctx& c = ctx();
-    static std::mutex first;
-    std::lock_guard<std::mutex> lk(first);
-    if (c.ready) return WAR_OK;
+// Makes what the context holds on the device.
+static int make_context(Ctx& c) {
     int ndev = 0;
     cudaError_t e = cudaGetDeviceCount(&ndev);
     if (e != cudaSuccess || ndev == 0) return fail(WAR_ENODEV, "no CUDA device (%s)", cudaGetErrorString(e));
@@ -92,8 +88,32 @@ int ensure_ready() {
     if ((e = cudaMallocHost(&c.h_acc, sizeof(DevAcc))) != cudaSuccess) return cuda_fail(e, "cudaMallocHost");
     if ((e = cudaEventCreate(&c.ev0)) != cudaSuccess) return cuda_fail(e, "event");
     if ((e = cudaEventCreate(&c.ev1)) != cudaSuccess) return cuda_fail(e, "event");
-    c.ready = true;
     return WAR_OK;
+}
+
+// Several threads may come here first: one makes the context.  One that could not be made gives back what it had, so
+// that a later call can try again.
+int ensure_ready() {
+    Ctx& c = ctx();
+    static std::mutex first;
+    std::lock_guard<std::mutex> lk(first);
+    if (c.ready) return WAR_OK;
+    const int st = make_context(c);
+    if (st == WAR_OK) {
+        c.ready = true;
+        return st;
+    }
+    cudaGetLastError();   // (the next launch does not report it)
+    if (c.ev0) cudaEventDestroy(c.ev0);
+    if (c.h_acc) cudaFreeHost(c.h_acc);
+    if (c.d_table) cudaFree(c.d_table);
+    if (c.d_blocks) cudaFree(c.d_blocks);
+    if (c.d_units) cudaFree(c.d_units);
+    if (c.d_acc) cudaFree(c.d_acc);
+    if (c.own_stream) cudaStreamDestroy(c.own_stream);
+    c.ev0 = c.ev1 = nullptr; c.h_acc = nullptr; c.d_table = nullptr; c.d_blocks = nullptr; c.d_units = nullptr;
+    c.d_acc = nullptr; c.own_stream = nullptr;
+    return st;
 }
 
 cudaError_t upload_merge_table(u32** table, cudaStream_t st) {

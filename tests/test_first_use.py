@@ -47,3 +47,12 @@ def test_first_use_by_several_threads(play):
                "[x.start() for x in t]\n[x.join() for x in t]\n"
                "print(war.war_set_stream(None), fake.fake_streams_made(), fake.fake_live())")
     assert one[:2] == [0, 1] and two == one
+
+
+def test_first_use_that_fails_gives_back_what_it_had(play):
+    """The upload of the pair lists fails twice: nothing is left, and the third call makes one whole context."""
+    one = play("print(war.war_set_stream(None), fake.fake_live())")
+    got = play("fake.fake_fail_copies(2)\n"
+               "for i in range(3): print(war.war_set_stream(None), fake.fake_live())")
+    ecuda = -2
+    assert got == [ecuda, 0, ecuda, 0] + one
