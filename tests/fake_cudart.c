@@ -1,4 +1,4 @@
-/* A CUDA runtime for tests of host code without a GPU: one device, memory from the heap, no kernels.  Loaded before
+/* A CUDA runtime for tests of host code without a GPU: one device, memory from the heap, kernels that do nothing.  Loaded before
  * the real one (LD_PRELOAD), it counts what is alive and notes the order of copies, synchronisations and launches. */
 #include <cuda_runtime_api.h>
 #include <stdatomic.h>
@@ -32,6 +32,30 @@ static cudaError_t copy(void* d, const void* s, size_t n) {
 static cudaError_t handle(void** p) {
     usleep(20000);      /* long enough for a second thread to come in */
     return take(p, 16);
+}
+
+/* Launches: no kernel runs; launch i finds the given words in its accumulators. */
+enum { LAUNCHES = 4, WORDS = 32 };
+static unsigned long long words[LAUNCHES][WORDS];
+static const void* fns[LAUNCHES];
+static atomic_int launches;
+void fake_set_word(int launch, int word, unsigned long long v) { words[launch][word] = v; }
+int fake_launches(void) { return launches; }
+int fake_same_kernel(int i, int j) { return fns[i] == fns[j]; }
+cudaError_t cudaLaunchKernel(const void* f, dim3 grid, dim3 block, void** args, size_t sh, cudaStream_t st) {
+    const int i = launches++;
+    if (i >= LAUNCHES) return cudaErrorUnknown;
+    memcpy(*(void**)args[1], words[i], sizeof words[i]);      /* (arguments, accumulators) */
+    fns[i] = f;
+    return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* f, int threads, size_t sh, unsigned fl) {
+    *n = 2;
+    return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void* f, int threads, size_t sh) {
+    *n = 2;
+    return cudaSuccess;
 }
 
 cudaError_t cudaMalloc(void** p, size_t n) { return take(p, n); }
