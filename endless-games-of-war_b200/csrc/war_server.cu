@@ -43,39 +43,33 @@
 
 namespace war {
 
-// A resident job's arguments, kept on the device by accumulator slot while it runs.
-struct ServeJob {
-    union {
-        BatchArgs batch;
-        MergeArgs merge;
-    };
+// One block's work: a run of units of a merged job, whose arguments are kept on the device by accumulator slot
+// while it runs.
+struct ServeTask {
+    u64 lo, hi;           // its units [lo, hi)
+    u64 counter;          // the task's work-unit counter (zero when uploaded)
+    u32 slot;             // accumulator slot of the job
+    u32 kind;             // rule + 2 canon + 2 (canon and distinct or sample)
 };
 
-// One block's work: a run of units of a job.
-struct ServeTask {
-    u64 lo, hi;           // its units [lo, hi) (BatchArgs: main units from main_base = lo, or `hi` extra units)
-    u64 counter;          // the task's work-unit counter (zero when uploaded)
-    const Unit* units;    // extra units, or null
-    u32 slot;             // accumulator slot of the job
-    u32 kind;             // serve_merge_kernel: rule + 2 canon + 2 (canon and distinct or sample)
+// The same for the other jobs, whose tasks are few (2^16 ranks each).  The arguments come with the task, units and
+// all: put together in the kernel from a job's and a task's, the sampled deals' loop without a table is compiled for 56
+// registers instead of 64 (3e7 deals of 13 cards 21.5 ms, so 23.7).
+struct RefillTask {
+    BatchArgs args;   // the job's parameters and this task's units
+    u32 slot;         // accumulator slot of the job
+    u32 pad;
+    u64 counter;      // the task's work-unit counter (zero when uploaded)
 };
 
 template <int RULE, int G, bool CANON, bool SHAPE, bool EXTRA, int V>
-__global__ void __launch_bounds__(G == 1 ? 1024 : 512) serve_kernel(ServeTask* __restrict__ tasks,
-                                                                   const ServeJob* __restrict__ jobs,
+__global__ void __launch_bounds__(G == 1 ? 1024 : 512) serve_kernel(RefillTask* __restrict__ tasks,
                                                                    DevAcc* __restrict__ slots) {
     extern __shared__ u32 sh[];
     __shared__ BatchArgs A;
-    ServeTask* t = tasks + blockIdx.x;
-    const u32* src = (const u32*)&jobs[t->slot].batch;
+    RefillTask* t = tasks + blockIdx.x;
+    const u32* src = (const u32*)&t->args;
     for (int i = threadIdx.x; i < (int)(sizeof(BatchArgs) / 4); i += blockDim.x) ((u32*)&A)[i] = src[i];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        A.main_base = t->lo;
-        A.main_count = t->units ? 0ull : t->hi - t->lo;
-        A.n_units = t->units ? t->hi : t->hi - t->lo;
-        A.units = t->units;
-    }
     __syncthreads();
     refill_dispatch<RULE, G, CANON, SHAPE, EXTRA, V>(A, slots + t->slot, &t->counter, sh);
 }
@@ -83,13 +77,13 @@ __global__ void __launch_bounds__(G == 1 ? 1024 : 512) serve_kernel(ServeTask* _
 // The same for the loops of war_merge_body.cuh, merged deals and canonical scans with or without a table, all in
 // one launch: the tasks of a tick run side by side whatever their kind.
 __global__ void __launch_bounds__(1024) serve_merge_kernel(ServeTask* __restrict__ tasks,
-                                                           const ServeJob* __restrict__ jobs,
+                                                           const MergeArgs* __restrict__ jobs,
                                                            DevAcc* __restrict__ slots) {
     extern __shared__ u64 sh64[];
     __shared__ MergeArgs A;
     __shared__ UnitStore store;
     ServeTask* t = tasks + blockIdx.x;
-    const u32* src = (const u32*)&jobs[t->slot].merge;
+    const u32* src = (const u32*)&jobs[t->slot];
     for (int i = threadIdx.x; i < (int)(sizeof(MergeArgs) / 4); i += blockDim.x) ((u32*)&A)[i] = src[i];
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -108,7 +102,7 @@ __global__ void __launch_bounds__(1024) serve_merge_kernel(ServeTask* __restrict
     }
 }
 
-typedef void (*ServeFn)(ServeTask*, const ServeJob*, DevAcc*);
+typedef void (*ServeFn)(RefillTask*, DevAcc*);
 
 template <int RULE, int G, int V>
 static ServeFn serve_pick(bool canon, bool shape, bool extra) {
@@ -118,7 +112,7 @@ static ServeFn serve_pick(bool canon, bool shape, bool extra) {
 }
 
 // Launch shapes of the serving kernels: one game per thread, 256-thread blocks, the multiply-add turn form.
-// Merged deals and canonical scans are one kernel (merged = 1, the other fields 0); sampled deals play deal by deal,
+// Merged deals and canonical scans are one kernel, serve_merge_kernel (merged = 1, the other fields 0); sampled deals play deal by deal,
 // with the path memo where the class has a table (memo); the loop-shape test has the immediate-record loop, and
 // so have canonical scans and deals of fewer than 4 cards the latched one.
 struct Variant {
@@ -127,19 +121,21 @@ struct Variant {
         return std::tie(merged, canon, rule, shape, extra, memo) <
                std::tie(o.merged, o.canon, o.rule, o.shape, o.extra, o.memo);
     }
-    bool operator==(const Variant& o) const { return !(*this < o) && !(o < *this); }
-    int threads() const { return 256; }
-    size_t shmem(int hbins) const {   // (a merged launch may hold canonical tasks that keep their starts)
-        return sizeof(u32) * (size_t)(hbins + WAR_EBINS) + (merged ? (sizeof(Missed) + 2 * sizeof(u64) + sizeof(StartQueue) / 32) * (size_t)threads() : 0);
-    }
     template <int RULE>
     ServeFn fn_rule() const {
         if (shape) return serve_pick<RULE, 1, 1>(true, true, extra);
         if (memo) return serve_kernel<RULE, 1, false, false, true, 31>;
         return serve_pick<RULE, 1, 3>(canon != 0, false, extra);
     }
-    ServeFn fn() const { return merged ? serve_merge_kernel : rule ? fn_rule<1>() : fn_rule<0>(); }
+    ServeFn fn() const { return rule ? fn_rule<1>() : fn_rule<0>(); }
 };
+
+constexpr int SERVE_THREADS = 256;
+
+size_t serve_shmem(int hbins, bool merged) {   // (a merged launch may hold canonical tasks that keep their starts)
+    return sizeof(u32) * (size_t)(hbins + WAR_EBINS) +
+           (merged ? (sizeof(Missed) + 2 * sizeof(u64) + sizeof(StartQueue) / 32) * (size_t)SERVE_THREADS : 0);
+}
 
 struct SJob {
     war_job job;
@@ -152,6 +148,7 @@ struct SJob {
     bool extras_issued = false;
     u64 per_unit = 1;    // ranks per main unit
     MergePlan mplan;     // merged jobs: the plan; next_main counts its units
+    BatchArgs base;      // the other jobs: the arguments of their tasks, without units
     Variant var;
     u32 kind = 0;        // of its tasks (ServeTask)
     war_result* result = nullptr;
@@ -159,11 +156,13 @@ struct SJob {
 
 struct Tick {
     ServeTask* h_tasks = nullptr;   // pinned
+    RefillTask* h_refill = nullptr; // pinned
     Unit* h_units = nullptr;        // pinned
     ServeTask* d_tasks = nullptr;
+    RefillTask* d_refill = nullptr;
     Unit* d_units = nullptr;
-    int ntasks = 0, nunits = 0;
-    std::vector<std::pair<Variant, std::pair<int, int>>> groups;   // variant -> [first task, count)
+    int ntasks = 0, nrefill = 0, nunits = 0;
+    std::vector<std::pair<Variant, std::pair<int, int>>> groups;   // kernels of the other jobs -> [first task, count)
     std::vector<std::pair<u64, int>> finishing;      // jobs whose last task is in this tick, and their slots
     std::vector<std::pair<int, size_t>> admitted;    // slots to be set up before this tick, and their blocks
     cudaEvent_t ev = nullptr;
@@ -189,8 +188,8 @@ struct war_server {
     war::MBlock* d_blocks = nullptr;     // the resident merged jobs' blocks, SLOT_BLOCKS for each slot
     war::MBlock* h_blocks = nullptr;     // and their mirror: pageable, a slot's few KB are staged by the copy, where
                                          // pinning the 4 MB of 256 slots takes longer than all the copies
-    war::ServeJob* d_jobs = nullptr;   // the resident jobs' arguments, by slot
-    war::ServeJob* h_jobs = nullptr;   // and their mirror, pinned
+    war::MergeArgs* d_jobs = nullptr;   // the resident merged jobs' arguments, by slot
+    war::MergeArgs* h_jobs = nullptr;   // and their mirror, pinned
     DevAcc* d_slots = nullptr;
     DevAcc* h_slot = nullptr;   // pinned readback buffer, READBACK slots
     cudaStream_t s_comp = nullptr, s_copy = nullptr;
@@ -212,6 +211,9 @@ namespace {
 // most: there a lane, not a warp, plays a unit (720 deals), and a smaller task leaves more of a block's lanes without
 // one (1e8 sampled deals of 13 cards 6.8 ms, with tasks by the tick's work 11.2).
 constexpr u64 TASK_RANKS_MIN = 1ull << 13, TASK_RANKS_MAX = 1ull << 16;
+// Refill tasks of a tick: what a tick's ranks make by default, and two more for the ends of each of 256 jobs (room for
+// 16384 took 7 ms to pin when the server is made, a third of all).
+constexpr int MAX_REFILL = 2560;
 constexpr size_t READBACK = 32;          // finished jobs read back at a time
 constexpr size_t SLOT_BLOCKS = 256;      // blocks of a job of at most 16 cards: at most 2 (1 + .. + 15), and the sentinel
 constexpr int UNITS_PER_EXTRA_CAP = 512;   // sizing of the per-tick extra-unit pool
@@ -279,12 +281,9 @@ void set_args(war_server* s, SJob& J) {
             if (!J.var.merged) J.var.memo = 1;
         }
     }
-    ServeJob& out = s->h_jobs[J.slot];
-    if (!J.var.merged) {
-        out.batch = a;
-        return;
-    }
-    MergeArgs& m = out.merge;
+    J.base = a;
+    if (!J.var.merged) return;
+    MergeArgs& m = s->h_jobs[J.slot];
     memset(&m, 0, sizeof m);
     MBlock* const h = s->h_blocks + (size_t)J.slot * SLOT_BLOCKS;
     memcpy(h, J.mplan.blocks.data(), sizeof(MBlock) * J.mplan.blocks.size());
@@ -372,7 +371,7 @@ void admit(war_server* s, Tick& T) {
 
 // Cuts the running jobs' remaining work into this tick's tasks (caller holds the lock).
 void build_tick(war_server* s, Tick& T) {
-    T.ntasks = 0; T.nunits = 0; T.groups.clear(); T.finishing.clear();
+    T.ntasks = 0; T.nrefill = 0; T.nunits = 0; T.groups.clear(); T.finishing.clear();
     std::vector<u64> run;
     for (auto& kv : s->jobs)
         if (kv.second.state == 1 && remaining(kv.second)) run.push_back(kv.first);
@@ -386,46 +385,52 @@ void build_tick(war_server* s, Tick& T) {
     const u64 task_ranks = std::min(TASK_RANKS_MAX, std::max(TASK_RANKS_MIN, std::min(left, budget) / (16ull * (u64)s->sm_count)));
     const int unit_cap = s->max_units * 8;
     u64 used = 0;
-    int ntasks = 0;
-    std::map<Variant, std::vector<ServeTask>> tasks;
+    std::map<Variant, std::vector<RefillTask>> refill;
     bool progress = true;
-    while (progress && used < budget && ntasks < s->max_tasks) {
+    while (progress && used < budget && T.ntasks + T.nrefill < s->max_tasks) {
         progress = false;
         for (u64 id : run) {
-            if (used >= budget || ntasks >= s->max_tasks) break;
+            if (used >= budget || T.ntasks + T.nrefill >= s->max_tasks) break;
             SJob& J = s->jobs[id];
-            if (!remaining(J)) continue;
-            ServeTask t;
-            memset(&t, 0, sizeof t);
-            t.slot = (u32)J.slot;
-            t.kind = J.kind;
-            if (J.next_main < main_units(J)) {
-                const u64 ranks = J.var.merged ? task_ranks : TASK_RANKS_MAX;
-                const u64 k = std::min(std::max<u64>(1, ranks / J.per_unit), main_units(J) - J.next_main);
-                t.lo = (J.var.merged ? 0 : J.plan.main_base) + J.next_main;
-                t.hi = t.lo + k;
-                J.next_main += k;
-                used += k * J.per_unit;
+            if (!remaining(J) || (!J.var.merged && T.nrefill >= MAX_REFILL)) continue;
+            const u64 lo = J.next_main, ranks = J.var.merged ? task_ranks : TASK_RANKS_MAX;
+            const u64 k = std::min(std::max<u64>(1, ranks / J.per_unit), main_units(J) - lo);
+            J.next_main += k;
+            used += k * J.per_unit;
+            if (J.var.merged) {
+                ServeTask& t = T.h_tasks[T.ntasks++];
+                t.lo = lo; t.hi = lo + k; t.counter = 0;
+                t.slot = (u32)J.slot; t.kind = J.kind;
             } else {
-                const int k = (int)J.plan.extra.size();
-                if (T.nunits + k > unit_cap) continue;   // next tick
-                memcpy(T.h_units + T.nunits, J.plan.extra.data(), sizeof(Unit) * (size_t)k);
-                t.units = T.d_units + T.nunits;
-                t.hi = (u64)k;
-                T.nunits += k;
-                J.extras_issued = true;
-                used += 1;
+                RefillTask t;
+                memset(&t, 0, sizeof t);
+                t.args = J.base;
+                t.slot = (u32)J.slot;
+                if (k) {
+                    t.args.main_base = J.plan.main_base + lo;
+                    t.args.main_count = t.args.n_units = k;
+                } else {
+                    const int x = (int)J.plan.extra.size();
+                    if (T.nunits + x > unit_cap) continue;   // next tick
+                    memcpy(T.h_units + T.nunits, J.plan.extra.data(), sizeof(Unit) * (size_t)x);
+                    t.args.units = T.d_units + T.nunits;
+                    t.args.n_units = (u64)x;
+                    T.nunits += x;
+                    J.extras_issued = true;
+                    used += 1;
+                }
+                refill[J.var].push_back(t);
+                T.nrefill++;
             }
             if (!remaining(J)) T.finishing.push_back({id, J.slot});
-            tasks[J.var].push_back(t);
-            ntasks++;
             progress = true;
         }
     }
-    for (const auto& kv : tasks) {   // one launch per kernel variant
-        T.groups.push_back({kv.first, {T.ntasks, (int)kv.second.size()}});
-        memcpy(T.h_tasks + T.ntasks, kv.second.data(), sizeof(ServeTask) * kv.second.size());
-        T.ntasks += (int)kv.second.size();
+    int at = 0;
+    for (const auto& kv : refill) {   // one launch per kernel variant
+        T.groups.push_back({kv.first, {at, (int)kv.second.size()}});
+        memcpy(T.h_refill + at, kv.second.data(), sizeof(RefillTask) * kv.second.size());
+        at += (int)kv.second.size();
     }
 }
 
@@ -434,31 +439,39 @@ cudaError_t launch_tick(war_server* s, Tick& T) {
     for (const auto& ad : T.admitted) {
         const int slot = ad.first;
         if ((e = cudaMemsetAsync(s->d_slots + slot, 0, sizeof(DevAcc), s->s_comp)) != cudaSuccess) return e;
-        if ((e = cudaMemcpyAsync(s->d_jobs + slot, s->h_jobs + slot, sizeof(ServeJob), cudaMemcpyHostToDevice,
+        if (!ad.second) continue;   // not merged
+        if ((e = cudaMemcpyAsync(s->d_jobs + slot, s->h_jobs + slot, sizeof(MergeArgs), cudaMemcpyHostToDevice,
                                  s->s_comp)) != cudaSuccess)
             return e;
         const size_t at = (size_t)slot * SLOT_BLOCKS;
-        if (ad.second && (e = cudaMemcpyAsync(s->d_blocks + at, s->h_blocks + at, sizeof(MBlock) * ad.second,
-                                              cudaMemcpyHostToDevice, s->s_comp)) != cudaSuccess)
+        if ((e = cudaMemcpyAsync(s->d_blocks + at, s->h_blocks + at, sizeof(MBlock) * ad.second, cudaMemcpyHostToDevice,
+                                 s->s_comp)) != cudaSuccess)
             return e;
     }
     T.admitted.clear();
-    if (T.ntasks == 0) return cudaSuccess;
-    if ((e = cudaMemcpyAsync(T.d_tasks, T.h_tasks, sizeof(ServeTask) * T.ntasks, cudaMemcpyHostToDevice, s->s_comp)))
+    if (T.ntasks + T.nrefill == 0) return cudaSuccess;
+    if (T.ntasks &&
+        (e = cudaMemcpyAsync(T.d_tasks, T.h_tasks, sizeof(ServeTask) * T.ntasks, cudaMemcpyHostToDevice, s->s_comp)))
+        return e;
+    if (T.nrefill &&
+        (e = cudaMemcpyAsync(T.d_refill, T.h_refill, sizeof(RefillTask) * T.nrefill, cudaMemcpyHostToDevice, s->s_comp)))
         return e;
     if (T.nunits &&
         (e = cudaMemcpyAsync(T.d_units, T.h_units, sizeof(Unit) * T.nunits, cudaMemcpyHostToDevice, s->s_comp)))
         return e;
+    // every task of a launch zeroes and flushes hbins of its own; the launch provides the largest
     for (auto& g : T.groups) {
         int hb = 0;
-        for (int i = g.second.first; i < g.second.first + g.second.second; i++) {
-            const ServeJob& J = s->h_jobs[T.h_tasks[i].slot];
-            hb = std::max(hb, g.first.merged ? J.merge.hbins : J.batch.hbins);
-        }
-        // every task of the group zeroes and flushes hbins of its own; the launch provides the largest
-        const size_t shmem = g.first.shmem(hb);
-        g.first.fn()<<<g.second.second, g.first.threads(), shmem, s->s_comp>>>(T.d_tasks + g.second.first, s->d_jobs,
-                                                                              s->d_slots);
+        for (int i = g.second.first; i < g.second.first + g.second.second; i++) hb = std::max(hb, T.h_refill[i].args.hbins);
+        g.first.fn()<<<g.second.second, SERVE_THREADS, serve_shmem(hb, false), s->s_comp>>>(T.d_refill + g.second.first,
+                                                                                         s->d_slots);
+        note_launch();
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    if (T.ntasks) {
+        int hb = 0;
+        for (int i = 0; i < T.ntasks; i++) hb = std::max(hb, s->h_jobs[T.h_tasks[i].slot].hbins);
+        serve_merge_kernel<<<T.ntasks, SERVE_THREADS, serve_shmem(hb, true), s->s_comp>>>(T.d_tasks, s->d_jobs, s->d_slots);
         note_launch();
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
@@ -489,7 +502,7 @@ void worker_main(war_server* s) {
             if (!s->fatal) {
                 admit(s, T);
                 build_tick(s, T);
-                built = T.ntasks > 0 || !T.admitted.empty();
+                built = T.ntasks + T.nrefill > 0 || !T.admitted.empty();
             }
         }
         if (built) {
@@ -500,7 +513,7 @@ void worker_main(war_server* s) {
                 for (auto& kv : s->jobs)
                     if (kv.second.state <= 1) { kv.second.state = 3; kv.second.status = WAR_ECUDA; }
                 s->cv_done.notify_all();
-            } else if (T.ntasks > 0) {
+            } else if (T.ntasks + T.nrefill > 0) {
                 T.in_flight = true;
                 s->nticks++;
             }
@@ -577,16 +590,18 @@ int war_server_create(const war_server_cfg* cfg, war_server** out) {
               upload_merge_table(&s->d_table, s->s_comp) == cudaSuccess &&
               cudaMalloc(&s->d_blocks, sizeof(MBlock) * nblocks) == cudaSuccess &&
               (s->h_blocks = (MBlock*)calloc(nblocks, sizeof(MBlock))) != nullptr &&
-              cudaMalloc(&s->d_jobs, sizeof(ServeJob) * (size_t)s->nslots) == cudaSuccess &&
-              cudaMallocHost(&s->h_jobs, sizeof(ServeJob) * (size_t)s->nslots) == cudaSuccess &&
+              cudaMalloc(&s->d_jobs, sizeof(MergeArgs) * (size_t)s->nslots) == cudaSuccess &&
+              cudaMallocHost(&s->h_jobs, sizeof(MergeArgs) * (size_t)s->nslots) == cudaSuccess &&
               cudaMalloc(&s->d_slots, sizeof(DevAcc) * (size_t)s->nslots) == cudaSuccess &&
               cudaMallocHost(&s->h_slot, sizeof(DevAcc) * READBACK) == cudaSuccess &&
               cudaStreamCreateWithFlags(&s->s_copy, cudaStreamNonBlocking) == cudaSuccess;
     for (int i = 0; ok && i < 2; i++) {
         Tick& T = s->ticks[i];
         ok = cudaMallocHost(&T.h_tasks, sizeof(ServeTask) * s->max_tasks) == cudaSuccess &&
+             cudaMallocHost(&T.h_refill, sizeof(RefillTask) * MAX_REFILL) == cudaSuccess &&
              cudaMallocHost(&T.h_units, sizeof(Unit) * (size_t)s->max_units * 8) == cudaSuccess &&
              cudaMalloc(&T.d_tasks, sizeof(ServeTask) * s->max_tasks) == cudaSuccess &&
+             cudaMalloc(&T.d_refill, sizeof(RefillTask) * MAX_REFILL) == cudaSuccess &&
              cudaMalloc(&T.d_units, sizeof(Unit) * (size_t)s->max_units * 8) == cudaSuccess &&
              cudaEventCreateWithFlags(&T.ev, cudaEventDisableTiming) == cudaSuccess;
     }
@@ -689,8 +704,10 @@ int war_server_destroy(war_server* s) {
     for (int i = 0; i < 2; i++) {
         Tick& T = s->ticks[i];
         if (T.h_tasks) cudaFreeHost(T.h_tasks);
+        if (T.h_refill) cudaFreeHost(T.h_refill);
         if (T.h_units) cudaFreeHost(T.h_units);
         if (T.d_tasks) cudaFree(T.d_tasks);
+        if (T.d_refill) cudaFree(T.d_refill);
         if (T.d_units) cudaFree(T.d_units);
         if (T.ev) cudaEventDestroy(T.ev);
     }
