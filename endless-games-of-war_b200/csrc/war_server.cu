@@ -21,8 +21,8 @@
 // rule, so every job of that class, now and later, decides its games from what the earlier ones found.
 // The tables come from one arena that war_server_create reserves inside the memory budget (after the
 // accumulator slots); a class takes its table from the arena when its first job is admitted, cleared on
-// the compute stream, and keeps it until the server ends; no class takes more than half of what is left, so that
-// a server of several large classes does not leave the last ones without.  The worker thread never calls cudaMalloc, which
+// the compute stream, and keeps it until the server ends; a class of merged jobs takes at most half of what is left, so
+// that a server of several large classes does not leave the last ones without.  The worker thread never calls cudaMalloc, which
 // would synchronise the device in the middle of the tick stream.  A class whose table no longer fits runs
 // without the memo.
 #include <cuda_runtime.h>
@@ -260,8 +260,10 @@ void set_args(war_server* s, SJob& J) {
             const int cap = s->cfg.memo_bits ? s->cfg.memo_bits : 28;
             int bits = std::max(12, std::min(cap, 4 + (int)std::ceil(std::log2((double)fact(job.n)) * 0.75)));
             // the largest table of at most 2^bits words in half of what the arena still holds, so that later classes
-            // have one too (in all of it if the arena is below 2^24 words), at least 2^12 words
-            const u64 left = s->arena_words - s->arena_used, most = s->arena_words < (1ull << 24) ? left : left / 2;
+            // have one too (in all of it if the arena is below 2^24 words, or for sampled deals, which look every deal
+            // up: 5e7 of 13 cards in an arena of 2^25 words 12.1 ms, with half of it 13.6), at least 2^12 words
+            const u64 left = s->arena_words - s->arena_used;
+            const u64 most = s->arena_words < (1ull << 24) || !J.var.merged ? left : left / 2;
             while (bits >= 12 && (1ull << bits) > most) bits--;
             u64* t = nullptr;
             if (bits >= 12) {

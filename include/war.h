@@ -200,7 +200,8 @@ typedef struct war_server_cfg {
     int32_t memo_bits;       /* cycle memo shared by all jobs of one n and rule, log2 of its 8-byte words
                                 (grown with n up to this, shrunk to what the arena has left; 0 = 28, i.e.
                                 2 GiB per class; < 0 = no memo).  A class takes at most half of what is left
-                                of an arena of 128 MiB or more.  A class whose table does not fit runs
+                                of an arena of 128 MiB or more, all of it if its first job is deals with
+                                WAR_F_SAMPLE.  A class whose table does not fit runs
                                 without the memo, with the same results */
     int32_t reserved[3];
 } war_server_cfg;
