@@ -78,8 +78,10 @@ def load_cache():
 def default_tune(n, mode, rule, flags):
     """The tune for a job class with no stored entry: the path memo with a table that grows with n and services
     every 8 to 16 turns; none below 4 cards.  Services: a resumed a(13) takes 28.8 ms with one every 8 turns
-    and 33.8 with 12; a span of 14 cards 12.9 and 12.4 (16: 12.8), of 15 cards 81.4 and 75.7 (16: 74.8); 3e9
-    canonical positions of 14 cards 125 with 12 and 134 with 16, 2e6 of 11 cards 0.49 with 12 and 0.42 with 16."""
+    and 33.8 with 12; a span of 4.26e9 ranks of 14 cards 12.9 and 12.4 (16: 12.8), of 15 cards 81.4 and 75.7 (16:
+    74.8), one of 14! of 15 cards 480 and 450 (16: 472), of 16 cards 532 and 455 (16: 453, 20: 466), --half 390
+    and 338 (16: 333, 20: 327); all canonical positions of 14 cards 3001 with 12 and 3263 with 16 (8: 3434), 2e6 of
+    11 cards 0.49 with 12 and 0.42 with 16."""
     if n < 4:
         return None
     # the largest table a job may take (it uses what its games can fill): from 13 cards 2^31 words, 16 GiB
