@@ -64,7 +64,7 @@ struct TurnK {
 };
 
 // The same for the turns with tests (war_turn_tests, h_turn_tests).  Another layout, with the last two words from a
-// 16-byte boundary on: the merged kernels measured best with it (71.2 ms for 14! ranks), and the one-game-per-deal
+// 16-byte boundary on: the merged kernels measured best with it (71.2 ms for 4.26e9 deals of 15 cards), and the one-game-per-deal
 // kernels with the one above (3e4 deals of 13 cards without a memo 7.5 ms, with this one 8.5).
 struct TestK {
     u32 k16, km16, k2p28, k4, one, pad;
@@ -116,9 +116,9 @@ __device__ __forceinline__ bool war_turn_fma(u64& w1, u64& w2, u32& qq, const Co
 // can do its work are half rate (ALU: logic, shifts, compares, selects; FMA: multiply-adds), so it is split between
 // them: what follows from "player 1 won" is written by a multiply-add for player 2's win and overwritten by one
 // under the predicate, moves under a predicate are multiplications by one, a card is the word less 16 times the popped
-// word, and the ALU is left the shifts and the compares.  B200: with the cards masked and one move left as a move
-// 1.47, 12.4, 74.4 and 125.1 ms (2^28 deals of 13, 7!! 14!/2 of 14, 14! of 15 cards, 2e8 canonical of 14), so 1.45, 12.1,
-// 72.2 and 124.2; with MERGED 1.42, 11.9, 70.3, and 124.0 for the
+// word, and the ALU is left the shifts and the compares.  B200, kernel times of 1e8 deals of 13 cards, 4.26e9 ranks of 14
+// with --half, 4.26e9 deals of 15 and 3e9 canonical positions of 14: with the cards masked and one move left as a move
+// 1.47, 12.4, 74.4 and 125.1 ms, so 1.45, 12.1, 72.2 and 124.2; with MERGED 1.42, 11.9 and 70.3, and 124.0 for the
 // canonical kernel's 123.6, which keeps the two compares.
 //
 //   pair        first card f + 16 (second card g) of the winner's two, + 0xFF: see war_turn_fma

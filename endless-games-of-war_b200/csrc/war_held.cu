@@ -232,9 +232,8 @@ __device__ __forceinline__ bool h_turn_packed_fma(u64& wh, u64& wo, u32& s, u32 
 // the period) + (1 if it ended) in ev and is frozen by an odd count word far out of range (its low byte never is an
 // opponent's last card, the word no tortoise's, and card n-1 never on top).  The
 // cards are ol - 16 ol' (the popped word), and half of the holder's pop is a multiplication: the ALU pipe was 82%
-// busy, the FMA pipe 62% (masks and moves 50.7 ms for 2e8 deals of 17 cards, so 49.2, both halves of the pop 50.2).
-// HeldK: -1, -260, -252, 65 and 4n - 8 as
-// operands.
+// busy, the FMA pipe 62% (masks and moves 50.7 ms for 1e9 deals of 17 cards, so 49.2, both halves of the pop 50.2).
+// HeldK: -1, -260, -252, 65 and 4n - 8 as operands.
 template <int RULE>
 __device__ __forceinline__ void h_turn_tests(u64& wh, u64& wo, u32& s, u64 th, u64 to, u32 ts, u32& ev, u32 k2,
                                    u32& prev, u32& brk, u32& brk_cy, const TestK& K, const HeldK& H) {
