@@ -3,9 +3,9 @@
     python bench.py [--gpus N] [--steps K] [--warmup W] [--workload deals13|canon14|deals11|deals13slice]
                     [--impl ours|reference] [--peaks]
 
-One step = one complete enumeration of the workload's rank space by the persistent refill kernel
-(war_enumerate), every step checked bit-exactly against the reference's recorded values.  Workloads (the
-rank spaces are the inputs; nothing is random):
+One step = one complete enumeration of the workload's rank space by the engine (war_enumerate), every step
+checked bit-exactly against the reference's recorded values.  Workloads (the rank spaces are the inputs;
+nothing is random):
   deals13  all 13! = 6,227,020,800 deals, cycle-length and ending-length histograms   (default)
   canon14  all 13!*13 = 80,951,270,400 canonical positions of n = 14, distinct cycles, cycle-length
            histogram and the seeded 1% Floyd cross-check
@@ -40,9 +40,9 @@ sys.path.insert(0, PKG)
 # reach one state are played together from there.)
 K_OPS_PER_TURN = 30
 # DRAM bytes (read + write) per deal of the merged path-memo kernel at this line's configuration (all 13! deals in
-# one launch, 16 GiB table): one-pass ncu capture, 58.74 GB read and 1.82 GB written for 6,227,020,800 deals (9.43 +
-# 0.29 B per deal: 681 million games stand for them, and each random 8-byte lookup costs a DRAM line).
-MEMO_DRAM_BYTES_PER_DEAL = 9.73
+# one launch, 2^29 words of the table in use, 4 GiB): ncu capture, 58.59 GB read and 2.06 GB written for 6,227,020,800
+# deals (9.41 + 0.33 B per deal: 681 million games stand for them, and each random 8-byte lookup costs a DRAM line).
+MEMO_DRAM_BYTES_PER_DEAL = 9.74
 # Turns of the reference's own schedule (Brent with the tortoise saved at powers of two from the first turn)
 # over all 13! deals, as counted by an instrumented copy of cpu/war.cpp; the plain kernel reproduces it
 # exactly (its `turns`).
@@ -293,25 +293,45 @@ def deal_extra_units(lo, hi, m):
     return blocks(lo, a2) + blocks(b2, hi) if a2 < b2 else blocks(lo, hi)
 
 
-def range_blocks(lo, hi, n, mode):
-    """How many blocks the path-memo engine copies to the device for ranks [lo, hi): the fewest aligned blocks of
-    j! orders, for canonical positions one more for each order cut by the range, and the sentinel."""
+def aligned_blocks(x, y, m):
+    """The fewest aligned blocks of j! orders of m cards that make up [x, y): their j."""
     f = math.factorial
-    k, m, x, y = 1, n, lo, hi
-    if mode:
-        m = n - 1
-        x, y = lo // m, hi // m
-        if x == y:
-            return 2
-        k += (1 if lo % m else 0) + (1 if hi % m else 0)
-        x += 1 if lo % m else 0
+    out = []
     while x < y:
         j = m
         while j > 0 and (x % f(j) or x + f(j) > y):
             j -= 1
         x += f(j)
-        k += 1
-    return k
+        out.append(j)
+    return out
+
+
+def range_blocks(lo, hi, n, mode):
+    """How many blocks the path-memo engine copies to the device for ranks [lo, hi): the fewest aligned blocks of
+    j! orders, for canonical positions one more for each order cut by the range, and the sentinel."""
+    if not mode:
+        return 1 + len(aligned_blocks(lo, hi, n))
+    m = n - 1
+    x, y = lo // m, hi // m
+    if x == y:
+        return 2
+    return (1 + (1 if lo % m else 0) + (1 if hi % m else 0) +
+            len(aligned_blocks(x + (1 if lo % m else 0), y, m)))
+
+
+def memo_table_bits(lo, hi, n, mode, bits):
+    """log2 of the words that the path-memo engine clears and uses of a table of 2^bits for ranks [lo, hi)
+    (csrc/war_capi.cu, enumerate_merged): deals have (f + 1) j!/2^f games in a block of j! with f open pairs."""
+    want = 2 * (hi - lo)
+    if not mode:
+        games = 0
+        for j in aligned_blocks(lo, hi, n):
+            f = max(0, (n - (n & 1) - (n - j) - ((n - j) & 1)) // 2)
+            games += (math.factorial(j) >> f) * (f + 1)
+        want = 4 * games if n >= 15 else games // 4 * 3 + 1
+    while bits > 12 and 1 << (bits - 1) >= want:
+        bits -= 1
+    return bits
 
 
 def peaks(warlib, table_bits, clk_mhz=None):
@@ -567,8 +587,12 @@ def main():
 
     if rank == 0:
         cs = clk.summary()
-        pk = peaks(warlib, (tune.memo_bits or 24) if tune is not None and (tune.variant & 4) else 30,
-                   clk_mhz=cs["sm_mhz"])
+        table_bits = 30
+        if tune is not None and (tune.variant & 4):
+            table_bits = tune.memo_bits or 24
+            if tune.variant & 28 == 28 and (mode or not w["flags"] & warlib.F_SAMPLE):
+                table_bits = memo_table_bits(lo, hi, n, mode, table_bits)
+        pk = peaks(warlib, max(20, table_bits), clk_mhz=cs["sm_mhz"])
         issue_peak, alu_peak, nominal = pk["int_issue_ops_per_s"], pk["alu_ops_per_s"], pk["nominal_issue_ops_per_s"]
         kops = K_OPS_PER_TURN_ENGINE[engine]
         achieved = turns * kops / (kernel_ms * 1e-3)    # algorithmic int ops/s of the enumeration kernel
@@ -578,7 +602,7 @@ def main():
             hbm_peak, hbm_src = measured_hbm_peak()
             mbytes = 8.0 * (res.memo_lookups + res.memo_stores)
             lps = res.memo_lookups / (kernel_ms * 1e-3)
-            memo = {"variant": tune.variant, "table_bytes": 8 << (tune.memo_bits or 24),
+            memo = {"variant": tune.variant, "table_bytes": 8 << table_bits,
                     "lookups_per_game": res.memo_lookups / res.done, "hit_rate": res.memo_hits / res.memo_lookups,
                     "stores_per_game": res.memo_stores / res.done, "turns_per_game": res.turns / res.done,
                     "lookups_per_s": lps, "gather_peak_lookups_per_s": pk["gather8_lookups_per_s"],
@@ -596,6 +620,11 @@ def main():
                      "turns_per_launch": turns / max(1, launches // args.steps),
                      "peak_source": "war_measure_int_peak on this GPU (LOP3+IMAD issue ceiling, measured); "
                                     "nominal = SMs x 4 x 32 x median SM clock"}
+        if engine != "refill":
+            # `turns` of these engines are those of playing every deal; merged games play fewer, and do not count them
+            int_issue.update(dict.fromkeys(("achieved", "frac", "frac_of_nominal", "frac_of_alu_pipe",
+                                            "turns_per_launch")),
+                             note="not measured: the engine's turns are those of every deal, merged games play fewer")
         per_launch = total / max(1, launches // args.steps)
         if memo:
             roofline = {"bound": "hbm_random_access", "achieved": memo["lookups_per_s"] / 1e9,
