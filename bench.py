@@ -350,7 +350,7 @@ def peaks(warlib, table_bits, clk_mhz=None):
 
 def canon14_leg(warlib, war_gpu, golden, stream):
     """The reference's long run `war_gpu.py 14 --canon --distinct --shape --hist 256` (data/long_runs.txt:20-23)
-    with the seeded 1% sample of the north-star's canonical configuration: every canonical position of n = 14
+    with a seeded 1% Floyd sample: every canonical position of n = 14
     once per rep through war_enumerate (device time, CUDA events on the launching stream), checked
     bit-exactly, then the sample replayed with Floyd and compared with Brent's aggregates."""
     import torch
@@ -611,7 +611,7 @@ def main():
                     "dram_bytes_per_deal": MEMO_DRAM_BYTES_PER_DEAL if mode == 0 and n == 13 else None,
                     "algorithmic_GBps": mbytes / (kernel_ms * 1e-3) / 1e9, "hbm_peak_GBps": hbm_peak,
                     "frac_of_hbm": mbytes / (kernel_ms * 1e-3) / 1e9 / hbm_peak, "hbm_peak_source": hbm_src}
-        # The integer-issue roofline of the turns (north-star's report: turns x ops per turn against the measured
+        # The integer-issue roofline of the turns (turns x ops per turn against the measured
         # LOP3+IMAD ceiling and the nominal issue rate) and, for the memo kernel, the roofline that binds it:
         # random 8-byte table reads against the measured random-gather ceiling of this GPU.
         int_issue = {"achieved": achieved / 1e12, "peak": issue_peak / 1e12, "unit": "Tops/s (INT32 thread-ops)",
